@@ -116,6 +116,17 @@ inline MotionDev make_motion_dev(const fm_motion *m) {
   return d;
 }
 
+// Weight of slot s at call time t.
+__device__ inline float motion_weight(const MotionDev &md, int s, double t) {
+  int k = 0;
+  while (k + 1 < md.n_terms && s >= md.slot0[k + 1]) ++k;
+  const fm_motion_term &T = md.terms[k];
+  const double v = ppoly_eval(T.pp_c, T.pp_x, T.pp_k, T.pp_intervals, T.n_modes, s - md.slot0[k], term_time(t, T),
+                              T.extrapolate);
+  const float w = __double2float_rn(v);
+  return T.kind == FM_TERM_POD_VELOCITY ? __fmul_rn(w, __double2float_rn(t)) : w;
+}
+
 int validate_motion(const fm_motion *m, int64_t n_nodes, const char *who);
 
 // Fills weights[c * slots + s] for n_calls call times (device array).

@@ -40,17 +40,7 @@ __global__ void motion_weights_kernel(MotionDev md, const double *__restrict__ t
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_calls * md.slots) return;
   const int64_t c = idx / md.slots;
-  const int s = (int)(idx - c * md.slots);
-  int k = 0;
-  while (k + 1 < md.n_terms && s >= md.slot0[k + 1]) ++k;
-  const fm_motion_term &T = md.terms[k];
-  const int col = s - md.slot0[k];
-  const double t = times[c];
-  const double te = term_time(t, T);
-  const double v = ppoly_eval(T.pp_c, T.pp_x, T.pp_k, T.pp_intervals, T.n_modes, col, te, T.extrapolate);
-  float w = __double2float_rn(v);
-  if (T.kind == FM_TERM_POD_VELOCITY) w = __fmul_rn(w, __double2float_rn(t));
-  weights[idx] = w;
+  weights[idx] = motion_weight(md, (int)(idx - c * md.slots), times[c]);
 }
 
 int launch_motion_weights(const MotionDev &md, const double *times_dev, int64_t n_calls, float *weights,

@@ -1,6 +1,6 @@
 // Pieces shared by the Signal forms: the mass-weighted magnetisation M * Mxy,
-// the distinct-time runs of the sample times, and the tile list that maps
-// thread blocks to runs.
+// the distinct-time runs of the sample times, how far the samples factor, and
+// the tile list that maps thread blocks to runs.
 #pragma once
 #include "motion.cuh"
 
@@ -10,22 +10,6 @@ namespace fm {
 constexpr int kPlainThreads = 256;
 // SM count of a B200; sizes split-K fan-out so workspace queries need no device.
 constexpr int kSmCount = 148;
-
-// Device view of the sample runs ("time groups"): run g covers samples
-// [start[g], start[g+1]) which share one time t_g.
-struct Runs {
-  int *flag;        // (S,) 1 where a run starts
-  int *gid;         // (S,) inclusive scan of flag
-  int *start;       // (S + 1,) run starts; start[n_runs] = S
-  int *tile_off;    // (S + 1,) first tile of each run
-  int *tile_run;    // (max_tiles,) run of each tile
-  int *tile_s0;     // (max_tiles,) first sample of each tile
-  double *run_t;    // (S,) time of each run, widened to double
-  int *counts;      // (8,) n_runs, n_tiles, then per-form plan values
-  int *error;       // (1,) error bits of the call (kErr*)
-  void *cub_tmp;
-  size_t cub_bytes;
-};
 
 // CSR view of the sparse mass matrix, rows in Eigen's accumulation order.
 struct Csr {
@@ -37,36 +21,79 @@ struct Csr {
   size_t cub_bytes;
 };
 
-int64_t max_tiles_for(int64_t S, int tile);
-
-void carve_runs(Carve &c, int64_t S, int tile, Runs &r);
-void carve_csr(Carve &c, int64_t rows, int64_t nnz, Csr &m);
-
 // Error bits recorded on the device during a Signal call.
 constexpr int kErrTimeout = 1;      // a tensor-core pipeline wait ran out
 constexpr int kErrSparseRow = 2;    // a row index of M outside [0, rows)
 constexpr int kErrTableCalls = 4;   // TABLE motion entries != distinct-time runs
 constexpr int kErrPhaseRange = 8;   // a tensor-core phase k . r may reach 2^27 cycles
 
-// Builds runs and tiles of `tile` samples on the device: counts[0] = runs,
-// counts[1] = tiles.  No host synchronisation.
+// Control words of one problem (zeroed when its descriptor is written).
+constexpr int kCtlFlags = 0;    // kFlag* bits found over the samples and M
+constexpr int kCtlRuns = 1;     // distinct-time runs
+constexpr int kCtlFac = 2;      // factored runs
+constexpr int kCtlTiles = 3;    // tiles of the other runs
+constexpr int kCtlSplits = 4;   // node splits (tensor-core form)
+constexpr int kCtlChunk = 5;    // nodes per split (tensor-core form)
+constexpr int kCtlError = 6;    // kErr* bits
+constexpr int kCtlWords = 16;
+
+// A slab is the Ls = lines x kz samples of one readout index.
+constexpr int kFlagRuns = 1;           // some slab is not exactly one run
+constexpr int kFlagSlabs = 2;          // some slab breaks k = kp + kq (checked additively in FP64)
+constexpr int kFlagOffsets = 4;        // some slab's kz offsets differ from the first slab's
+constexpr int kFlagNotDiagonal = 8;    // M has as many entries as rows but is not diagonal
+
+// Descriptor of one problem's preparation, in device memory.
+struct PrepDev {
+  int64_t S, N, V;
+  int Ls, n_lines, n_kz, n_ro;
+  int n_chunks, chunk;   // the samples in n_chunks stretches of `chunk`
+  int tile;              // samples per tile of an unfactored run
+  int slabs;             // slabs may factor: factored runs are listed apart from the tiles
+  int diag;              // M holds as many entries as rows: diagonal unless shown otherwise
+  int vgroup;            // columns per group of MM (0: one (N, V) matrix)
+  int64_t table_calls;   // entries of a TABLE motion, -1 without one
+  const void *kx, *ky, *kz, *t;
+  const int *indptr, *indices;
+  const void *data, *Mxy;
+  void *MM;
+  int *ctl;
+  unsigned char *slab_bad;   // (n_ro,) slab is not one run or does not factor
+  int *chunk_starts, *chunk_fac, *chunk_tiles;  // (n_chunks,) counts per stretch
+  int *start;            // (S + 1,) run starts; start[n_runs] = S
+  double *run_t;         // (S,) time of each run, widened to double
+  int *frun;             // factored runs, ascending
+  int2 *tiles;           // (run, first sample within it) of every other tile
+  float *weights;        // (n_runs, slots) TERMS motion weights
+  MotionDev md;
+  Csr csr;
+};
+
+// Scratch of one problem: carved the same way when sizing and when running.
+// `slabs`: slabs of more than one kz value may factor (tensor-core form).
+void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool slabs, int vgroup, size_t real_bytes, int *ctl,
+                PrepDev &p);
+// Fills the rest of the descriptor from the arguments.
+void fill_prep(const fm_signal_args *a, PrepDev &p);
+
+// Queues the preparation of n problems (descriptors `host`, copied to the
+// device array `dev`): runs, factoring, M * Mxy, motion weights and tiles.
+// No host synchronisation and no copy from host memory.
 template <typename T>
-int build_runs(const T *t, int64_t S, int tile, Runs &r, cudaStream_t st);
+int launch_prep(const fm_signal_args *probs, const PrepDev *host, int n, PrepDev *dev, cudaStream_t st);
 
-// Sets kErrTableCalls when a TABLE motion does not hold one entry per run.
-int check_table_calls(const fm_motion *m, Runs &r, cudaStream_t st);
+// Reads the error words of n problems (ctl: n rows of kCtlWords), waits for
+// the stream and maps the first error to a status with a message.
+int report_errors(const int *ctl, int n, cudaStream_t st, const char *who);
 
-// Reads and clears the error word (synchronises the stream) and maps it to a
-// status with a message.
-int report_errors(Runs &r, cudaStream_t st, const char *who);
-
-// MM[i, v] = sum_j M[i, j] * Mxy[j, v] accumulated over j ascending (Eigen's
-// column-major sparse x dense product, cpp/feelmri/MRI.cpp:92).
-template <typename T>
-int sparse_times_dense(const fm_signal_args *a, Csr &m, const T *Mxy, T *MM, int *error, cudaStream_t st);
-
-// Motion weights for the runs, with the run count read on the device.
-int launch_run_weights(const MotionDev &md, const double *run_t, const int *n_runs, int64_t max_runs,
-                       float *weights, cudaStream_t st);
+// Element of M Mxy for node n, column v: (N, V) rows, or per group of
+// `vgroup` columns (N, ld) rows with ld = the group's columns rounded up to
+// even (16-byte rows for the bulk copies), groups one after the other.
+__host__ __device__ inline int64_t mm_index(int64_t n, int64_t v, int64_t N, int64_t V, int vgroup) {
+  if (vgroup == 0) return n * V + v;
+  const int64_t g = v / vgroup;
+  const int64_t cols = (V - g * vgroup) < vgroup ? (V - g * vgroup) : vgroup;
+  return g * N * vgroup + n * ((cols + 1) & ~(int64_t)1) + (v - g * vgroup);
+}
 
 }  // namespace fm

@@ -34,7 +34,8 @@ struct PlainDev {
   MotionDev md;
   const float *weights;   // (n_runs, slots) TERMS motion weights
   const T *table;         // TABLE motion (n_runs, N, 3) in T
-  const int *tile_run, *tile_s0, *run_start;
+  const int2 *tiles;      // (run, first sample within it)
+  const int *run_start;
   const int *n_tiles;     // device: number of tiles
   const double *run_t;
   int64_t chunk;          // nodes per split
@@ -67,8 +68,8 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T>
   const int split = blockIdx.y;
   for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
   __syncthreads();  // the previous tile's readers of s_pos / s_w are done
-  const int g = p.tile_run[tile];
-  const int s_begin = p.tile_s0[tile];
+  const int g = p.tiles[tile].x;
+  const int s_begin = p.run_start[g] + p.tiles[tile].y;
   const int s_end = min(p.run_start[g + 1], s_begin + kPlainThreads * SPT);
   const T tg = (T)p.run_t[g];
   const int nv = (int)min((int64_t)VMAX, p.V - v0);
@@ -193,10 +194,8 @@ static int choose_splits(int64_t n_tiles_min, int64_t N) {
 
 template <typename T>
 struct PlainPlan {
-  T *MM;
-  Csr csr;
-  Runs runs;
-  float *weights;
+  PrepDev prep;
+  PrepDev *dev;
   T *partials;
   int splits;
   int tile;
@@ -207,10 +206,9 @@ static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   const int64_t S = a->n_ro * a->n_lines * a->n_kz;
   const int64_t N = a->n_nodes, V = a->n_vencs;
   pl.tile = samples_per_thread<T>(V) * kPlainThreads;
-  pl.MM = c.take<T>((size_t)N * V * 2);
-  carve_csr(c, a->m_rows, a->m_nnz, pl.csr);
-  carve_runs(c, S, pl.tile, pl.runs);
-  pl.weights = c.take<float>((size_t)(S + 1) * motion_slots(a->motion));
+  int *ctl = c.take<int>(kCtlWords);
+  pl.dev = c.take<PrepDev>(1);
+  carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
   pl.splits = choose_splits(ceil_div(S, pl.tile), N);
   pl.partials = (pl.splits > 1) ? c.take<T>((size_t)pl.splits * S * V * 2) : nullptr;
 }
@@ -233,12 +231,10 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
     FM_CUDA(cudaMemsetAsync(out, 0, (size_t)S * V * 2 * sizeof(T), st));
     return FM_OK;
   }
-  FM_TRY(build_runs<T>(static_cast<const T *>(a->t), S, pl.tile, pl.runs, st));
-  FM_TRY(sparse_times_dense<T>(a, pl.csr, static_cast<const T *>(a->Mxy), pl.MM, pl.runs.error, st));
-  FM_TRY(check_table_calls(a->motion, pl.runs, st));
-  const MotionDev md = make_motion_dev(a->motion);
-  FM_TRY(launch_run_weights(md, pl.runs.run_t, pl.runs.counts, S, pl.weights, st));
-  const int64_t max_tiles = max_tiles_for(S, pl.tile);
+  fill_prep(a, pl.prep);
+  FM_TRY(launch_prep<T>(a, &pl.prep, 1, pl.dev, st));
+  const MotionDev &md = pl.prep.md;
+  const int64_t max_tiles = S + S / pl.tile + 1;
 
   PlainDev<T> p{};
   p.N = N; p.S = S; p.V = V;
@@ -248,15 +244,14 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
   p.r0 = static_cast<const T *>(a->r0);
   p.phi = static_cast<const T *>(a->phi);
   p.T2 = static_cast<const T *>(a->T2);
-  p.MM = pl.MM;
+  p.MM = static_cast<const T *>(pl.prep.MM);
   p.md = md;
-  p.weights = (md.kind == FM_MOTION_TERMS) ? pl.weights : nullptr;
+  p.weights = (md.kind == FM_MOTION_TERMS) ? pl.prep.weights : nullptr;
   p.table = (a->motion && a->motion->kind == FM_MOTION_TABLE) ? static_cast<const T *>(a->motion->table) : nullptr;
-  p.n_tiles = pl.runs.counts + 1;
-  p.tile_run = pl.runs.tile_run;
-  p.tile_s0 = pl.runs.tile_s0;
-  p.run_start = pl.runs.start;
-  p.run_t = pl.runs.run_t;
+  p.n_tiles = pl.prep.ctl + kCtlTiles;
+  p.tiles = pl.prep.tiles;
+  p.run_start = pl.prep.start;
+  p.run_t = pl.prep.run_t;
   p.splits = pl.splits;
   p.chunk = ceil_div(N, pl.splits);
   p.out = (pl.splits > 1) ? pl.partials : out;
@@ -290,7 +285,7 @@ int signal_plain_errors(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t w
   PlainPlan<T> pl;
   carve_plain<T>(cv, a, pl);
   FM_TRY(carve_ok(cv, "fm_signal"));
-  return report_errors(pl.runs, ctx->stream, sizeof(T) == 4 ? "fm_signal(F32)" : "fm_signal(F64)");
+  return report_errors(pl.prep.ctl, 1, ctx->stream, sizeof(T) == 4 ? "fm_signal(F32)" : "fm_signal(F64)");
 }
 template int signal_plain_errors<float>(fm_ctx *, const fm_signal_args *, void *, size_t);
 template int signal_plain_errors<double>(fm_ctx *, const fm_signal_args *, void *, size_t);

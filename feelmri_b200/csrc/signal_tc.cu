@@ -36,7 +36,6 @@
 // finish and frees its tensor memory.
 #include <cmath>
 #include <vector>
-#include <cub/cub.cuh>
 
 #include "signal_common.cuh"
 #include "tc_ptx.cuh"
@@ -110,18 +109,20 @@ struct TcDev {
   const float *weights;
   const float *table;
   const double *run_t;
-  const TcRun *runs;
-  const TcItem *items;
+  const int *start;   // run starts (PrepDev)
+  const int *frun;    // factored runs
+  const int2 *tiles;  // tiles of the generic runs
+  int *ctl;           // control words of the problem
   int Qt, NT, kind;  // kind 0: factored runs, 1: generic runs
+  int RU;            // lines per stacked unit
+  int prob, first, n_of, max_splits;  // the problem, its first entry and its entries
   int wrows;         // rows per node buffer: VG weight rows, then (stacked runs) nrun D rows
   int stacked;       // items hold several runs (D in the A rows, B without decay)
   int mm_ld;         // row stride of MM (float2): this group's columns, padded to even
   int tma;           // node blocks are staged by bulk copies (aligned inputs, room in smem)
   int mstage;        // 3 r: a single POD term's mode rows are staged with each node block (0: read from global)
-  const int *plan;  // device: [2] factored items, [3] generic items, [4] splits, [5] nodes per split
   float2 *partials; // (splits, S, V) when splits > 1
   float2 *out;
-  int *error;
 };
 
 // One launch works through a table of entries (one per problem, Mxy column
@@ -133,22 +134,64 @@ struct TcBatchDev {
   int acc_cols;  // tensor-memory columns of the widest entry (accumulator; the running sum follows)
 };
 
-// Work list of one entry, read from the device-side plan.
+// Work list of one entry, from the problem's control words.
 struct TcWork {
-  int splits, item0, n_items;
+  int splits, n_items;
+  bool stack;  // items are consecutive lines of the runs laid end to end
   int64_t chunk;
   float2 *out;
 };
 
+// Runs can be stacked into one unit when the positions do not depend on the
+// run (no motion) and every run is a factored slab of the full (lines x kz)
+// shape with the same kz offsets, exactly (flags of the sample scan).
+__device__ inline bool tc_stacked(const TcDev &p) {
+  return p.stacked && !(p.ctl[kCtlFlags] & (kFlagRuns | kFlagSlabs | kFlagOffsets));
+}
+
+__device__ inline int tc_items_per_run(const TcDev &p) {
+  return (int)(ceil_div(p.n_lines, kTcRows) * ceil_div(p.n_kz, p.Qt));
+}
+
+__device__ inline int tc_n_items(const TcDev &p) {
+  if (p.kind != 0) return p.ctl[kCtlTiles];
+  if (tc_stacked(p)) return (int)ceil_div((int64_t)p.ctl[kCtlRuns] * p.n_lines, (int64_t)p.RU);
+  return p.ctl[kCtlFac] * tc_items_per_run(p);
+}
+
 __device__ inline TcWork tc_work(const TcDev &p) {
-  const int kind = p.kind;
   TcWork W;
-  W.splits = p.plan[4];
-  W.chunk = p.plan[5];
-  W.item0 = kind == 0 ? 0 : p.plan[2];
-  W.n_items = kind == 0 ? p.plan[2] : p.plan[3];
+  W.splits = p.ctl[kCtlSplits];
+  W.chunk = p.ctl[kCtlChunk];
+  W.n_items = tc_n_items(p);
+  W.stack = p.kind == 0 && tc_stacked(p);
   W.out = W.splits > 1 ? p.partials : p.out;
   return W;
+}
+
+__device__ inline TcItem tc_item(const TcDev &p, const TcWork &W, int i) {
+  TcItem t;
+  if (p.kind != 0) {
+    const int2 k = p.tiles[i];
+    t.run = k.x; t.p0 = k.y; t.q0 = 0; t.nrun = 1;
+    t.rows = min(kTcRows, p.start[k.x + 1] - p.start[k.x] - k.y);
+  } else if (W.stack) {
+    const int64_t L0 = (int64_t)i * p.RU, total = (int64_t)p.ctl[kCtlRuns] * p.n_lines;
+    t.run = (int)(L0 / p.n_lines);
+    t.p0 = (int)(L0 - (int64_t)t.run * p.n_lines);
+    t.q0 = 0;
+    t.rows = (int)min((int64_t)p.RU, total - L0);
+    t.nrun = (t.p0 + t.rows - 1) / p.n_lines + 1;
+  } else {
+    const int c = tc_items_per_run(p), nq = (int)ceil_div(p.n_kz, p.Qt);
+    const int w = i % c;
+    t.run = p.frun[i / c];
+    t.p0 = (w / nq) * kTcRows;
+    t.q0 = (w % nq) * p.Qt;
+    t.nrun = 1;
+    t.rows = min(kTcRows, p.n_lines - t.p0);
+  }
+  return t;
 }
 
 // Shared-memory layout.  Strides of the weight and phase tables are padded
@@ -257,8 +300,11 @@ __device__ inline TcUnit tc_unit(const TcDev &p, const TcWork &W, int u) {
   TcUnit U;
   const int item = u % W.n_items;
   U.split = u / W.n_items;
-  U.it = p.items[W.item0 + item];
-  U.run = p.runs[U.it.run];
+  U.it = tc_item(p, W, item);
+  U.run.start = p.start[U.it.run];
+  U.run.factored = p.kind == 0 ? 1 : 0;
+  U.run.P = U.run.factored ? p.n_lines : p.start[U.it.run + 1] - U.run.start;
+  U.run.Q = U.run.factored ? p.n_kz : 1;
   U.P_tile = p.stacked ? U.run.P : min(kTcRows, U.run.P - U.it.p0);
   U.Q_tile = min(p.Qt, U.run.Q - U.it.q0);
   U.rows = U.it.rows;
@@ -593,7 +639,7 @@ __device__ inline void tc_final(const TcDev &p, const TcWork &W, const TcUnit &U
   int r_row = 0, line = 0;
   if (row_ok) tc_row_line(p, U, row, r_row, line);
   const int qvg = U.Q_tile * p.VG;
-  const int start = row_ok ? p.runs[U.it.run + r_row].start : 0;
+  const int start = row_ok ? p.start[U.it.run + r_row] : 0;
   const int s_row = start + (U.run.factored ? line * p.n_kz + U.it.q0 : line);
   const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
   const int n_acc = tc_parts(p.NT), AW = p.NT, sum_col = tc_sum_col(p.NT);
@@ -792,7 +838,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_c
         int r, line;
         tc_row_line(p, U, row, r, line);
         a_drow = VG + r;
-        const int start = r == 0 ? U.run.start : p.runs[U.it.run + r].start;
+        const int start = r == 0 ? U.run.start : p.start[U.it.run + r];
         const int s_p = start + (fac ? line * p.n_kz : line);
         kx0 = p.kx[s_p];
         ky0 = p.ky[s_p];
@@ -1087,7 +1133,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_c
         // every phase of the unit had |k . r| <= kmax rmax: the fixed-point
         // reduction holds below 2^28 cycles (2^27 leaves a margin)
         if (!((double)__int_as_float(*kmax) * (double)__int_as_float(*rmax) < 134217728.0))
-          atomicOr(p.error, kErrPhaseRange);
+          atomicOr(p.ctl + kCtlError, kErrPhaseRange);
         *kmax = 0;
         *rmax = 0;
       }
@@ -1098,7 +1144,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_c
       float2 *dst = W.out + (int64_t)U.split * p.S * p.V;
       int r, line;
       tc_row_line(p, U, tid, r, line);
-      const int start = p.runs[U.it.run + r].start;
+      const int start = p.start[U.it.run + r];
       const int s_row = start + (fac ? line * p.n_kz + U.it.q0 : line);
       for (int q = 0; q < U.Q_tile; ++q)
         for (int v = 0; v < VG; ++v) dst[(int64_t)(s_row + q) * p.V + p.v0 + v] = make_float2(0.f, 0.f);
@@ -1114,151 +1160,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_c
   __syncthreads();
   // a wait that ran out is reported for every problem of the launch
   if (*abort_flag)
-    for (int e = tid; e < B.n_entries; e += kTcThreads) atomicOr(B.entries[e].error, kErrTimeout);
+    for (int e = tid; e < B.n_entries; e += kTcThreads) atomicOr(B.entries[e].ctl + kCtlError, kErrTimeout);
   if (warp == 0) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, kTcTmemCols);
   }
 }
 
-// ---- run classification and work items ---------------------------------
-
-// One block per run: a run is factored when it covers exactly one
-// (lines x kz) slab and every sample satisfies k = kp_j + kq_k in FP64.
-__global__ void tc_classify_kernel(const float *__restrict__ kx, const float *__restrict__ ky,
-                                   const float *__restrict__ kz, const int *__restrict__ start,
-                                   const int *__restrict__ counts, int n_lines, int n_kz, TcRun *__restrict__ runs) {
-  const int n_runs = counts[0];
-  for (int g = blockIdx.x; g < n_runs; g += gridDim.x) {
-  __syncthreads();
-  const int s0 = start[g], len = start[g + 1] - s0;
-  const int Ls = n_lines * n_kz;
-  __shared__ int sep;
-  if (threadIdx.x == 0) sep = (len == Ls && Ls > 1 && n_kz > 1 && s0 % Ls == 0) ? 1 : 0;
-  __syncthreads();
-  if (sep) {
-    const double b0[3] = {kx[s0], ky[s0], kz[s0]};
-    for (int idx = threadIdx.x; idx < Ls; idx += blockDim.x) {
-      const int jl = idx / n_kz, kk = idx % n_kz;
-      const int s = s0 + idx, sj = s0 + jl * n_kz, sk = s0 + kk;
-      const double a[3] = {kx[s], ky[s], kz[s]};
-      const double pj[3] = {kx[sj], ky[sj], kz[sj]};
-      const double qk[3] = {kx[sk], ky[sk], kz[sk]};
-      bool good = true;
-      for (int c = 0; c < 3; ++c) good = good && (a[c] == pj[c] + (qk[c] - b0[c]));
-      if (!good) atomicExch(&sep, 0);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    TcRun r;
-    r.start = s0;
-    r.factored = sep;
-    r.P = sep ? n_lines : len;
-    r.Q = sep ? n_kz : 1;
-    runs[g] = r;
-  }
-  }  // runs
-}
-
-// Runs can be stacked into one unit when the positions do not depend on the
-// run (no motion) and every run is a factored slab of the full (lines x kz)
-// shape with the same kz offsets kq = k(q) - k(first sample), exactly.
-// `flag` starts non-zero; any run that breaks a condition clears it.
-__global__ void tc_stack_check_kernel(const float *__restrict__ kx, const float *__restrict__ ky,
-                                      const float *__restrict__ kz, const TcRun *__restrict__ runs,
-                                      const int *__restrict__ counts, int n_lines, int n_kz, int *__restrict__ flag) {
-  const int n_runs = counts[0];
-  if (n_runs <= 0) return;
-  const int s0 = runs[0].start;
-  const int64_t total = (int64_t)n_runs * n_kz;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int g = (int)(idx / n_kz), q = (int)(idx % n_kz);
-    const TcRun r = runs[g];
-    bool ok = r.factored && r.P == n_lines && r.Q == n_kz;
-    if (ok) {
-      const int a = r.start, b = s0;
-      ok = ((double)kx[a + q] - (double)kx[a]) == ((double)kx[b + q] - (double)kx[b]) &&
-           ((double)ky[a + q] - (double)ky[a]) == ((double)ky[b + q] - (double)ky[b]) &&
-           ((double)kz[a + q] - (double)kz[a]) == ((double)kz[b + q] - (double)kz[b]);
-    }
-    if (!ok) atomicExch(flag, 0);
-  }
-}
-
-// Item counts per run, factored runs in one list and the rest in another.
-// With stacking (stack != nullptr and *stack set) the runs' P lines are laid
-// end to end and cut into items of RU lines: run g opens the items whose
-// first line falls in it.
-__device__ inline int64_t tc_packed_first(int64_t g, int P, int RU) { return ceil_div(g * P, (int64_t)RU); }
-__global__ void tc_count_kernel(const TcRun *__restrict__ runs, const int *__restrict__ counts, int Qt,
-                                int *__restrict__ nf, int *__restrict__ ng, int64_t S, const int *__restrict__ stack,
-                                int P, int RU) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = counts[0];
-  if (g > S) return;
-  if (g >= n) {
-    nf[g] = 0;
-    ng[g] = 0;
-    return;
-  }
-  if (stack && *stack) {
-    nf[g] = (int)(tc_packed_first(g + 1, P, RU) - tc_packed_first(g, P, RU));
-    ng[g] = 0;
-    return;
-  }
-  const TcRun r = runs[g];
-  const int items = (int)(ceil_div(r.P, kTcRows) * ceil_div(r.Q, r.factored ? Qt : 1));
-  nf[g] = r.factored ? items : 0;
-  ng[g] = r.factored ? 0 : items;
-}
-
-// Items of one Mxy column group: factored first, then generic; their counts
-// go to plan[2] and plan[3].
-__global__ void tc_fill_kernel(const TcRun *__restrict__ runs, const int *__restrict__ counts, int Qt,
-                               const int *__restrict__ of, const int *__restrict__ og, TcItem *__restrict__ items,
-                               int *__restrict__ plan, const int *__restrict__ stack, int P, int RU) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = counts[0];
-  if (g > n) return;
-  if (g == n) {
-    plan[2] = of[n];
-    plan[3] = og[n];
-    return;
-  }
-  if (stack && *stack) {
-    const int64_t i0 = tc_packed_first(g, P, RU), i1 = tc_packed_first(g + 1, P, RU);
-    const int64_t total = (int64_t)n * P;
-    for (int64_t i = i0; i < i1; ++i) {
-      const int64_t L0 = i * RU;
-      TcItem t;
-      t.run = g;
-      t.p0 = (int)(L0 - (int64_t)g * P);
-      t.q0 = 0;
-      t.rows = (int)((total - L0) < RU ? (total - L0) : RU);
-      t.nrun = (int)((L0 + t.rows - 1) / P - g + 1);
-      items[of[g] + (i - i0)] = t;
-    }
-    return;
-  }
-  const TcRun r = runs[g];
-  const int qt = r.factored ? Qt : 1;
-  const int nq = (int)ceil_div(r.Q, qt);
-  const int np = (int)ceil_div(r.P, kTcRows);
-  // factored items first, then the generic ones (offset by the factored total)
-  const int base = r.factored ? of[g] : of[n] + og[g];
-  for (int a = 0; a < np; ++a)
-    for (int b = 0; b < nq; ++b) {
-      TcItem t;
-      t.run = g;
-      t.p0 = a * kTcRows;
-      t.q0 = b * qt;
-      t.nrun = 1;
-      t.rows = (r.P - t.p0) < kTcRows ? (r.P - t.p0) : kTcRows;
-      items[base + a * nq + b] = t;
-    }
-}
+// ---- plan --------------------------------------------------------------
 
 // Node-range splits: enough work units that the persistent blocks finish
 // together (units per block close to an integer), each split at least 2048
@@ -1280,35 +1189,52 @@ __host__ __device__ inline int tc_choose_splits(int64_t items, int64_t N, int ma
   return best;
 }
 
-// Splits of one problem, shared by all its column groups (plan rows of 8
-// ints): from the node count per split when tuned, else balanced over the SMs.
-__global__ void tc_plan_kernel(int *__restrict__ plan, int n_groups, int64_t N, int max_splits, int split_nodes) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int64_t items = 0;
-  for (int g = 0; g < n_groups; ++g) items += plan[8 * g + 2] + plan[8 * g + 3];
-  int splits;
-  if (split_nodes > 0) {
-    const int64_t s = ceil_div(N, (int64_t)split_nodes);
-    splits = (int)(s < 1 ? 1 : (s > max_splits ? max_splits : s));
-  } else {
-    splits = tc_choose_splits(items, N, max_splits);
+// Node splits of every problem, shared by all its entries (from the node
+// count per split when tuned, else balanced over the SMs), and the running
+// unit counts of the launch's entries.  One block.
+constexpr int kTcPlanThreads = 1024;
+__global__ void __launch_bounds__(kTcPlanThreads) tc_plan_kernel(const TcDev *__restrict__ entries, int n,
+                                                                 int split_nodes, int *__restrict__ offsets,
+                                                                 int *__restrict__ first) {
+  for (int e = threadIdx.x; e < n; e += kTcPlanThreads) {
+    const TcDev &p = entries[e];
+    if (e != p.first) continue;
+    first[p.prob] = e;
+    int splits;
+    if (split_nodes > 0) {
+      const int64_t s = ceil_div(p.N, (int64_t)split_nodes);
+      splits = (int)(s < 1 ? 1 : (s > p.max_splits ? p.max_splits : s));
+    } else {
+      int64_t items = 0;
+      for (int k = 0; k < p.n_of; ++k) items += tc_n_items(entries[e + k]);
+      splits = tc_choose_splits(items, p.N, p.max_splits);
+    }
+    p.ctl[kCtlSplits] = splits;
+    p.ctl[kCtlChunk] = (int)(ceil_div(ceil_div(p.N, splits), kTcNodes) * kTcNodes);
   }
-  const int chunk = (int)(ceil_div(ceil_div(N, splits), kTcNodes) * kTcNodes);
-  for (int g = 0; g < n_groups; ++g) {
-    plan[8 * g + 4] = splits;
-    plan[8 * g + 5] = chunk;
-  }
-}
-
-// Running unit counts of the launch's entries.
-__global__ void tc_batch_plan_kernel(const TcDev *__restrict__ entries, int n, int *__restrict__ offsets) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int acc = 0;
-  offsets[0] = 0;
-  for (int e = 0; e < n; ++e) {
-    const int *pl = entries[e].plan;
-    acc += (entries[e].kind == 0 ? pl[2] : pl[3]) * pl[4];
-    offsets[e + 1] = acc;
+  __syncthreads();
+  __shared__ int part[kTcPlanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  if (threadIdx.x == 0) offsets[0] = 0;
+  for (int e0 = 0; e0 < n; e0 += kTcPlanThreads) {
+    const int e = e0 + threadIdx.x;
+    int v = e < n ? tc_n_items(entries[e]) * *(volatile int *)(entries[e].ctl + kCtlSplits) : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v += o;
+    }
+    __syncthreads();
+    if (lane == 31) part[warp] = v;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int i = 0; i < kTcPlanThreads / 32; ++i) {
+      if (i < warp) before += part[i];
+      total += part[i];
+    }
+    if (e < n) offsets[e + 1] = base + before + v;
+    base += total;
   }
 }
 
@@ -1327,47 +1253,27 @@ __global__ void tc_write_entries_kernel(const __grid_constant__ TcEntryChunk c, 
   for (int i = threadIdx.x; i < words; i += blockDim.x) d[i] = src[i];
 }
 
-// M Mxy regrouped per column group: group g holds (N, mm_ld_g) rows with
-// mm_ld_g = its column count rounded up to even (16-byte rows for the bulk
-// copies); groups of 8 columns are consecutive.
-__global__ void tc_group_mm_kernel(const float2 *__restrict__ MM, int64_t N, int V, float2 *__restrict__ MMg) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= N * V) return;
-  const int64_t n = e / V;
-  const int v = (int)(e % V);
-  const int g = v / kTcVGroup, vi = v % kTcVGroup;
-  const int vg = (V - g * kTcVGroup) < kTcVGroup ? (V - g * kTcVGroup) : kTcVGroup;
-  const int ld = (vg + 1) & ~1;
-  MMg[(int64_t)g * N * kTcVGroup + n * ld + vi] = MM[e];
-}
-
-__global__ void tc_reduce_kernel(const float2 *__restrict__ part, const int *__restrict__ plan, int64_t count,
-                                 float2 *__restrict__ out) {
-  const int splits = plan[4];
+// Sums of the node splits, in split order, for every problem (grid y).
+__global__ void tc_reduce_kernel(const TcDev *__restrict__ entries, const int *__restrict__ first) {
+  const TcDev &p = entries[first[blockIdx.y]];
+  const int splits = p.ctl[kCtlSplits];
   if (splits <= 1) return;
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
-  float2 acc = part[e];
-  for (int k = 1; k < splits; ++k) {
-    const float2 v = part[(int64_t)k * count + e];
-    acc.x += v.x;
-    acc.y += v.y;
+  const float2 *part = p.partials;
+  const int64_t count = p.S * p.V;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
+    float2 acc = part[e];
+    for (int k = 1; k < splits; ++k) {
+      const float2 v = part[(int64_t)k * count + e];
+      acc.x += v.x;
+      acc.y += v.y;
+    }
+    p.out[e] = acc;
   }
-  out[e] = acc;
 }
 
 // Workspace of one problem.
 struct TcPlan {
-  float *MM;
-  float2 *MMg;    // M Mxy per column group (tc_group_mm_kernel)
-  Csr csr;
-  Runs runs;
-  float *weights;
-  TcRun *tcruns;
-  TcItem *items;  // n_groups lists of 2 S + 2
-  int *nf, *ng, *of, *og;
-  int *plan;      // n_groups rows of 8 ints
-  int *stack;     // runs can be stacked (set on the device)
+  PrepDev prep;
   float2 *partials;
   int n_groups, max_splits;
 };
@@ -1381,25 +1287,12 @@ static int tc_max_splits(int64_t S, int64_t V) {
 
 static int tc_groups(int64_t V) { return (int)ceil_div(V, (int64_t)kTcVGroup); }
 
-static void carve_tc(Carve &c, const fm_signal_args *a, TcPlan &pl) {
+static void carve_tc(Carve &c, const fm_signal_args *a, int *ctl, TcPlan &pl) {
   const int64_t S = a->n_ro * a->n_lines * a->n_kz;
-  const int64_t N = a->n_nodes, V = a->n_vencs;
-  pl.n_groups = tc_groups(V);
-  pl.MM = c.take<float>((size_t)N * V * 2);
-  pl.MMg = c.take<float2>((size_t)pl.n_groups * N * kTcVGroup);
-  carve_csr(c, a->m_rows, a->m_nnz, pl.csr);
-  carve_runs(c, S, kTcRows, pl.runs);
-  pl.weights = c.take<float>((size_t)(S + 1) * motion_slots(a->motion));
-  pl.tcruns = c.take<TcRun>(S + 1);
-  pl.items = c.take<TcItem>((size_t)pl.n_groups * (2 * S + 2));
-  pl.nf = c.take<int>(S + 2);
-  pl.ng = c.take<int>(S + 2);
-  pl.of = c.take<int>(S + 2);
-  pl.og = c.take<int>(S + 2);
-  pl.plan = c.take<int>((size_t)8 * (pl.n_groups > 0 ? pl.n_groups : 1));
-  pl.stack = c.take<int>(4);
-  pl.max_splits = tc_max_splits(S, V);
-  pl.partials = c.take<float2>((size_t)pl.max_splits * S * V);
+  pl.n_groups = tc_groups(a->n_vencs);
+  carve_prep(c, a, kTcRows, true, kTcVGroup, sizeof(float), ctl, pl.prep);
+  pl.max_splits = tc_max_splits(S, a->n_vencs);
+  pl.partials = c.take<float2>((size_t)pl.max_splits * S * a->n_vencs);
 }
 
 // Entries of a launch: per problem, per column group, both run kinds.
@@ -1409,12 +1302,23 @@ static int tc_n_entries(const fm_signal_args *probs, int n) {
   return e;
 }
 
-static void carve_batch(Carve &c, const fm_signal_args *probs, int n, TcPlan *plans, TcDev **entries,
-                        int **offsets) {
-  for (int i = 0; i < n; ++i) carve_tc(c, &probs[i], plans[i]);
+struct TcBatchPlan {
+  std::vector<TcPlan> probs;
+  int *ctl;       // kCtlWords per problem
+  PrepDev *prep;  // descriptors of the problems that have work
+  TcDev *entries;
+  int *offsets, *first;
+};
+
+static void carve_batch(Carve &c, const fm_signal_args *probs, int n, TcBatchPlan &b) {
+  b.probs.resize(n > 0 ? n : 1);
+  b.ctl = c.take<int>((size_t)kCtlWords * (n > 0 ? n : 1));
+  b.prep = c.take<PrepDev>(n > 0 ? n : 1);
+  b.first = c.take<int>(n > 0 ? n : 1);
   const int ne = tc_n_entries(probs, n);
-  *entries = c.take<TcDev>(ne > 0 ? ne : 1);
-  *offsets = c.take<int>(ne + 1);
+  b.entries = c.take<TcDev>(ne > 0 ? ne : 1);
+  b.offsets = c.take<int>(ne + 1);
+  for (int i = 0; i < n; ++i) carve_tc(c, &probs[i], b.ctl ? b.ctl + (size_t)kCtlWords * i : nullptr, b.probs[i]);
 }
 
 // Tile shape of a column group: up to 128 (q, v) pairs per tile and at most
@@ -1474,60 +1378,20 @@ static void tc_shape(int Qt, int VG, int &NT, int &acc_cols) {
 
 static size_t tc_batch_workspace(const fm_signal_args *probs, int n) {
   Carve c(nullptr, 0);
-  std::vector<TcPlan> plans(n > 0 ? n : 1);
-  TcDev *entries;
-  int *offsets;
-  carve_batch(c, probs, n, plans.data(), &entries, &offsets);
+  TcBatchPlan b;
+  carve_batch(c, probs, n, b);
   return c.used;
 }
 
 size_t tc_workspace(const fm_signal_args *a) { return tc_batch_workspace(a, 1); }
 
-// Preparation of one problem (runs, M Mxy, motion weights, run kinds, items
-// and splits); fills its launch entries.  Returns the number of entries.
-static int tc_prepare(const fm_signal_args *a, TcPlan &pl, const fm_tc_tuning *tune, TcDev *host_entries,
-                      cudaStream_t st, const char *who) {
+// Launch entries of one problem; returns their number.
+static int tc_entries(const fm_signal_args *a, const TcPlan &pl, const fm_tc_tuning *tune, int prob, int e0,
+                      TcDev *host_entries) {
   const int64_t S = a->n_ro * a->n_lines * a->n_kz;
   const int64_t N = a->n_nodes, V = a->n_vencs;
-  if (S == 0 || V == 0) return 0;
-  float2 *out = static_cast<float2 *>(a->out);
-  if (N == 0) {
-    FM_CUDA(cudaMemsetAsync(out, 0, (size_t)S * V * sizeof(float2), st));
-    return 0;
-  }
-  FM_REQUIRE(a->n_lines * a->n_kz < (1LL << 30), FM_ERR_SHAPE, "%s: slab too large", who);
-  const float *kx = static_cast<const float *>(a->kx), *ky = static_cast<const float *>(a->ky),
-              *kz = static_cast<const float *>(a->kz);
-  FM_TRY(build_runs<float>(static_cast<const float *>(a->t), S, kTcRows, pl.runs, st));
-  FM_TRY(sparse_times_dense<float>(a, pl.csr, static_cast<const float *>(a->Mxy), pl.MM, pl.runs.error, st));
-  FM_TRY(check_table_calls(a->motion, pl.runs, st));
-  tc_group_mm_kernel<<<(unsigned)ceil_div(N * V, 256), 256, 0, st>>>(reinterpret_cast<const float2 *>(pl.MM), N,
-                                                                     (int)V, pl.MMg);
-  count_launch();
-  FM_TRY(check_launch("tc_group_mm_kernel"));
-  const MotionDev md = make_motion_dev(a->motion);
-  FM_TRY(launch_run_weights(md, pl.runs.run_t, pl.runs.counts, S, pl.weights, st));
-  const int64_t cls_blocks = S < 8 * kSmCount ? S : 8 * kSmCount;
-  tc_classify_kernel<<<(unsigned)cls_blocks, 256, 0, st>>>(kx, ky, kz, pl.runs.start, pl.runs.counts,
-                                                           (int)a->n_lines, (int)a->n_kz, pl.tcruns);
-  count_launch();
-  FM_TRY(check_launch("tc_classify_kernel"));
-  // stacking check (the same for every column group)
-  bool may_stack = false;
-  for (int g = 0; g < pl.n_groups; ++g) {
-    const int64_t v0 = (int64_t)g * kTcVGroup;
-    const int VG = (int)((V - v0) < kTcVGroup ? (V - v0) : kTcVGroup);
-    if (tc_stack_runs(a, VG, tc_qt(a, VG, tune)) > 1) may_stack = true;
-  }
-  if (may_stack) {
-    FM_CUDA(cudaMemsetAsync(pl.stack, 1, sizeof(int), st));
-    const int64_t work = S;  // n_runs x n_kz <= S
-    const unsigned blocks = (unsigned)(work / 256 + 1 < 4 * kSmCount ? work / 256 + 1 : 4 * kSmCount);
-    tc_stack_check_kernel<<<blocks, 256, 0, st>>>(kx, ky, kz, pl.tcruns, pl.runs.counts, (int)a->n_lines,
-                                                   (int)a->n_kz, pl.stack);
-    count_launch();
-    FM_TRY(check_launch("tc_stack_check_kernel"));
-  }
+  const PrepDev &pr = pl.prep;
+  const MotionDev &md = pr.md;
   int ne = 0;
   for (int g = 0; g < pl.n_groups; ++g) {
     const int64_t v0 = (int64_t)g * kTcVGroup;
@@ -1535,45 +1399,34 @@ static int tc_prepare(const fm_signal_args *a, TcPlan &pl, const fm_tc_tuning *t
     const int Qt_f = tc_qt(a, VG, tune);
     const int R = tc_stack_runs(a, VG, Qt_f);
     const int RU = R > 1 ? tc_pack_rows((int)a->n_lines, R) : 0;
-    const int *stack = R > 1 ? pl.stack : nullptr;
-    TcItem *items = pl.items + (size_t)g * (2 * S + 2);
-    int *plan = pl.plan + 8 * g;
-    const unsigned gb = (unsigned)ceil_div(S + 1, 256);
-    tc_count_kernel<<<gb, 256, 0, st>>>(pl.tcruns, pl.runs.counts, Qt_f, pl.nf, pl.ng, S, stack, (int)a->n_lines, RU);
-    count_launch();
-    FM_TRY(check_launch("tc_count_kernel"));
-    size_t cb = pl.runs.cub_bytes;
-    FM_CUDA(cub::DeviceScan::ExclusiveSum(pl.runs.cub_tmp, cb, pl.nf, pl.of, (int)(S + 1), st));
-    cb = pl.runs.cub_bytes;
-    FM_CUDA(cub::DeviceScan::ExclusiveSum(pl.runs.cub_tmp, cb, pl.ng, pl.og, (int)(S + 1), st));
-    count_launch(2);
-    tc_fill_kernel<<<gb, 256, 0, st>>>(pl.tcruns, pl.runs.counts, Qt_f, pl.of, pl.og, items, plan, stack,
-                                       (int)a->n_lines, RU);
-    count_launch();
-    FM_TRY(check_launch("tc_fill_kernel"));
     for (int kind = 0; kind < 2; ++kind) {
       TcDev &p = host_entries[ne++];
       p = TcDev{};
       p.N = N; p.S = S; p.V = V;
       p.v0 = (int)v0; p.VG = VG;
       p.n_lines = (int)a->n_lines; p.n_kz = (int)a->n_kz;
-      p.kx = kx; p.ky = ky; p.kz = kz;
+      p.kx = static_cast<const float *>(a->kx);
+      p.ky = static_cast<const float *>(a->ky);
+      p.kz = static_cast<const float *>(a->kz);
       p.r0 = static_cast<const float *>(a->r0);
       p.phi = static_cast<const float *>(a->phi);
       p.T2 = static_cast<const float *>(a->T2);
-      p.MM = pl.MMg + (size_t)g * N * kTcVGroup;
+      p.MM = static_cast<const float2 *>(pr.MM) + (size_t)g * N * kTcVGroup;
       p.mm_ld = (VG + 1) & ~1;
       p.md = md;
-      p.weights = (md.kind == FM_MOTION_TERMS) ? pl.weights : nullptr;
+      p.weights = (md.kind == FM_MOTION_TERMS) ? pr.weights : nullptr;
       p.table = (a->motion && a->motion->kind == FM_MOTION_TABLE) ? static_cast<const float *>(a->motion->table)
                                                                    : nullptr;
-      p.run_t = pl.runs.run_t;
-      p.runs = pl.tcruns;
-      p.items = items;
-      p.plan = plan;
+      p.run_t = pr.run_t;
+      p.start = pr.start;
+      p.frun = pr.frun;
+      p.tiles = pr.tiles;
+      p.ctl = pr.ctl;
+      p.RU = RU;
+      p.prob = prob; p.first = e0; p.n_of = 2 * pl.n_groups;
+      p.max_splits = pl.max_splits;
       p.partials = pl.partials;
-      p.out = out;
-      p.error = pl.runs.error;
+      p.out = static_cast<float2 *>(a->out);
       p.kind = kind;
       p.Qt = kind == 0 ? Qt_f : 1;
       // a stacked unit's node buffers add one D row per run
@@ -1598,44 +1451,40 @@ static int tc_prepare(const fm_signal_args *a, TcPlan &pl, const fm_tc_tuning *t
         p.mstage = 3 * md.terms[0].n_modes;
     }
   }
-  tc_plan_kernel<<<1, 32, 0, st>>>(pl.plan, pl.n_groups, N, pl.max_splits, tune ? tune->split_nodes : 0);
-  count_launch();
-  FM_TRY(check_launch("tc_plan_kernel"));
   return ne;
 }
 
 // Signal for n problems: per-problem preparation, then one persistent
 // tensor-core launch over all of their work units, then the split sums.
-constexpr int kTcSideStreams = 8;  // helper streams for the per-problem preparations of a batch
-
 static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc_tuning *tune, void *ws,
                     size_t ws_bytes, const char *who) {
   cudaStream_t st = ctx->stream;
   Carve cv(ws, ws_bytes);
-  std::vector<TcPlan> plans(n > 0 ? n : 1);
-  TcDev *entries;
-  int *offsets;
-  carve_batch(cv, probs, n, plans.data(), &entries, &offsets);
+  TcBatchPlan b;
+  carve_batch(cv, probs, n, b);
   FM_TRY(carve_ok(cv, who));
   std::vector<TcDev> host(tc_n_entries(probs, n) + 1);
+  std::vector<fm_signal_args> work;
+  std::vector<PrepDev> prep;
   int ne = 0;
-  // the problems' preparations are independent: with several problems they
-  // run on helper streams forked from the launch stream and joined back
-  // before the persistent launch (in a captured graph: parallel branches)
-  const int K = n >= 4 ? kTcSideStreams : 0;
-  if (K > 0) {
-    FM_TRY(ctx_side_streams(ctx, K));
-    FM_TRY(ctx_fork(ctx, K));
+  int64_t widest = 0;  // outputs of the largest problem
+  for (int i = 0; i < n; ++i) {
+    const fm_signal_args *a = &probs[i];
+    const int64_t S = a->n_ro * a->n_lines * a->n_kz, count = S * a->n_vencs;
+    if (count == 0) continue;
+    if (a->n_nodes == 0) {
+      FM_CUDA(cudaMemsetAsync(a->out, 0, (size_t)count * sizeof(float2), st));
+      continue;
+    }
+    FM_REQUIRE(a->n_lines * a->n_kz < (1LL << 30), FM_ERR_SHAPE, "%s: slab too large", who);
+    fill_prep(a, b.probs[i].prep);
+    ne += tc_entries(a, b.probs[i], tune, (int)prep.size(), ne, host.data() + ne);
+    work.push_back(*a);
+    prep.push_back(b.probs[i].prep);
+    if (count > widest) widest = count;
   }
-  int prep = FM_OK;
-  for (int i = 0; i < n && prep == FM_OK; ++i) {
-    const int k = tc_prepare(&probs[i], plans[i], tune, host.data() + ne, K > 0 ? ctx->side[i % K] : st, who);
-    if (k < 0) prep = k;
-    else ne += k;
-  }
-  if (K > 0) FM_TRY(ctx_join(ctx, K));
-  if (prep != FM_OK) return prep;
   if (ne == 0) return FM_OK;
+  FM_TRY(launch_prep<float>(work.data(), prep.data(), (int)prep.size(), b.prep, st));
   int acc_cols = 32;
   size_t smem = 0;
   bool modes = false;
@@ -1656,16 +1505,16 @@ static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc
     TcEntryChunk c;
     c.n = (ne - e0) < kTcEntriesPerWrite ? (ne - e0) : kTcEntriesPerWrite;
     for (int k = 0; k < c.n; ++k) c.e[k] = host[e0 + k];
-    tc_write_entries_kernel<<<1, 256, 0, st>>>(c, entries + e0);
+    tc_write_entries_kernel<<<1, 256, 0, st>>>(c, b.entries + e0);
     count_launch();
     FM_TRY(check_launch("tc_write_entries_kernel"));
   }
-  tc_batch_plan_kernel<<<1, 32, 0, st>>>(entries, ne, offsets);
+  tc_plan_kernel<<<1, kTcPlanThreads, 0, st>>>(b.entries, ne, tune ? tune->split_nodes : 0, b.offsets, b.first);
   count_launch();
-  FM_TRY(check_launch("tc_batch_plan_kernel"));
+  FM_TRY(check_launch("tc_plan_kernel"));
   TcBatchDev B;
-  B.entries = entries;
-  B.offsets = offsets;
+  B.entries = b.entries;
+  B.offsets = b.offsets;
   B.n_entries = ne;
   B.acc_cols = acc_cols;
   {
@@ -1676,12 +1525,10 @@ static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc
     count_launch();
     FM_TRY(check_launch("signal_tc_kernel"));
   }
-  for (int i = 0; i < n; ++i) {
-    const fm_signal_args *a = &probs[i];
-    const int64_t count = a->n_ro * a->n_lines * a->n_kz * a->n_vencs;
-    if (count == 0 || a->n_nodes == 0) continue;
-    tc_reduce_kernel<<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(plans[i].partials, plans[i].plan, count,
-                                                                      static_cast<float2 *>(a->out));
+  const int64_t rb = ceil_div(widest, 256);
+  for (size_t i0 = 0; i0 < prep.size(); i0 += 65535) {
+    const unsigned y = (unsigned)(prep.size() - i0 < 65535 ? prep.size() - i0 : 65535);
+    tc_reduce_kernel<<<dim3((unsigned)(rb < 4 * kSmCount ? rb : 4 * kSmCount), y), 256, 0, st>>>(b.entries, b.first + i0);
     count_launch();
     FM_TRY(check_launch("tc_reduce_kernel"));
   }
@@ -1695,19 +1542,28 @@ int signal_tc(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes) {
 static int tc_batch_errors(fm_ctx *ctx, const fm_signal_args *probs, int n, void *ws, size_t ws_bytes,
                            const char *who) {
   Carve cv(ws, ws_bytes);
-  std::vector<TcPlan> plans(n > 0 ? n : 1);
-  TcDev *entries;
-  int *offsets;
-  carve_batch(cv, probs, n, plans.data(), &entries, &offsets);
+  TcBatchPlan b;
+  carve_batch(cv, probs, n, b);
   FM_TRY(carve_ok(cv, who));
+  // the problems that had work, in stretches (the others' words were never set)
   int rc = FM_OK;
-  for (int i = 0; i < n; ++i) {
-    const fm_signal_args *a = &probs[i];
-    if (a->n_ro * a->n_lines * a->n_kz == 0 || a->n_vencs == 0 || a->n_nodes == 0) continue;
-    const int r = report_errors(plans[i].runs, ctx->stream, who);
+  bool waited = false;
+  for (int i = 0; i < n;) {
+    auto idle = [&](int k) {
+      return probs[k].n_ro * probs[k].n_lines * probs[k].n_kz == 0 || probs[k].n_vencs == 0 || probs[k].n_nodes == 0;
+    };
+    if (idle(i)) {
+      ++i;
+      continue;
+    }
+    int j = i;
+    while (j < n && !idle(j)) ++j;
+    const int r = report_errors(b.probs[i].prep.ctl, j - i, ctx->stream, who);
+    waited = true;
     if (r != FM_OK && rc == FM_OK) rc = r;
+    i = j;
   }
-  if (n == 0) FM_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (!waited) FM_CUDA(cudaStreamSynchronize(ctx->stream));
   return rc;
 }
 
