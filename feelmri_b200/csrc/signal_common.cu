@@ -51,6 +51,7 @@ void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool slabs, int vgr
   p.n_kz = (int)(p.S > 0 ? a->n_kz : 1);
   p.Ls = p.n_lines * p.n_kz;
   p.slabs = slabs && p.n_kz > 1;
+  p.stat = p.n_ro > 1 && p.Ls > 1 && (a->motion == nullptr || a->motion->kind == FM_MOTION_NONE);
   p.tile = tile;
   p.vgroup = vgroup;
   const int64_t want = ceil_div(p.S, 1024);
@@ -173,6 +174,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
         if (p.slabs) {
           p.slab_bad[i] = 1;
           if (w == 0) p.slab_bad[i - 1] = 1;
+        }
+      }
+      if (p.stat) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const T k = kc[d][s];
+          if (!(k == kc[d][(int64_t)i * p.Ls])) flags |= kFlagInSlab << d;
+          if (!(k == kc[d][w])) flags |= kFlagAcross << d;
         }
       }
       if (p.slabs) {

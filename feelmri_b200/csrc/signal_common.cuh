@@ -42,6 +42,18 @@ constexpr int kFlagRuns = 1;           // some slab is not exactly one run
 constexpr int kFlagSlabs = 2;          // some slab breaks k = kp + kq (checked additively in FP64)
 constexpr int kFlagOffsets = 4;        // some slab's kz offsets differ from the first slab's
 constexpr int kFlagNotDiagonal = 8;    // M has as many entries as rows but is not diagonal
+constexpr int kFlagInSlab = 1 << 8;    // << c: component c of k varies inside some slab
+constexpr int kFlagAcross = 1 << 11;   // << c: component c differs from the first slab's
+
+// Components of k that go with the run, and whether the samples factor as
+// k(i, j, k) = k_run(i) + k_slab(j, k): every slab is one run and each component
+// is either the same throughout every slab (it goes with the run) or the same
+// in every slab (it goes with the place in the slab).
+__device__ inline int prep_run_comps(const int *ctl) { return (ctl[kCtlFlags] / kFlagAcross) & 7; }
+__device__ inline bool prep_static(const int *ctl) {
+  const int f = ctl[kCtlFlags];
+  return !(f & kFlagRuns) && ((f / kFlagInSlab) & (f / kFlagAcross) & 7) == 0;
+}
 
 // Descriptor of one problem's preparation, in device memory.
 struct PrepDev {
@@ -49,6 +61,7 @@ struct PrepDev {
   int Ls, n_lines, n_kz, n_ro;
   int n_chunks, chunk;   // the samples in n_chunks stretches of `chunk`
   int tile;              // samples per tile of an unfactored run
+  int stat;              // runs may factor out (no motion, several runs of several samples)
   int slabs;             // slabs may factor: factored runs are listed apart from the tiles
   int diag;              // M holds as many entries as rows: diagonal unless shown otherwise
   int vgroup;            // columns per group of MM (0: one (N, V) matrix)

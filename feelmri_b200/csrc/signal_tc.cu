@@ -21,19 +21,27 @@
 //   fixed point, to 2^-24 cycles) before the FP32 sin/cos, so far nodes at
 //   high k keep their digits.
 //
-// Block (persistent, one per SM, 16 warps): in factored units warps 0-7
-// write the A tiles and warps 8-15 the B tiles and the phase tables; in
-// generic units every warp writes A (16 nodes per pipeline stage, a ring of
-// 4 stages in shared memory in the 64-byte swizzled K-major layout).
-// Threads 0-127 also derive the node blocks.  After each group's
-// barrier one thread (warp 7, lane 0) issues the group's MMAs; warp 0 owns
-// the tensor memory.  tcgen05.commit frees a ring slot when the MMAs that
-// read it have completed.  The tensor core's FP32 accumulation truncates, so
-// the accumulator only collects 32 stages; all warps then fold it into an FP32
-// (round-to-nearest) running sum kept in the other half of tensor memory.
-// Blocks loop over work units (row/column tile of a run x node range).  All
-// waits are bounded: on timeout the block records an error, lets its MMAs
-// finish and frees its tensor memory.
+// Block (persistent, one per SM, 16 warps, each with a role of its own and
+// mbarriers between them): warps 0-12 write the operand tiles into a ring of
+// stages (16 nodes each) in shared memory, in the 64-byte swizzled K-major
+// layout; warps 13 and 14 form the node blocks (128 nodes: moved positions,
+// weights) ahead of them; one thread of warp 15 issues the MMAs of each written
+// stage and releases its slot by tcgen05.commit.  The tensor core's FP32
+// accumulation truncates, so the accumulator only collects 32 stages; warps 0-7
+// then fold it into an FP32 (round-to-nearest) running sum kept in the other
+// half of tensor memory.  Blocks loop over work units (row/column tile of a run
+// x node range), each role on its own.  All waits are bounded: on timeout the
+// block records an error, lets its MMAs finish and frees its tensor memory.
+//
+// What bounds it: operand writing, i.e. the instruction rate of the half-rate
+// integer pipe and FP64 beside running MMAs; a stage takes about 1,600 cycles
+// on wide tiles (128 pairs of 4 columns; its MMAs need 768), 900 on generic
+// ones.  Measured on a B200, with one barrier for the whole block every two or
+// four stages and one warp writing operands and issuing MMAs before:
+// 200,740 nodes x 96 x 96 x 32 x 4 columns 9,274 -> 8,070 us, radial 50,021 x
+// 65,536 x 8 columns with 10 modes 8,687 -> 5,350, 16 uneven phantoms 3,821 ->
+// 2,410 (with runs as columns, kTcRuns).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -44,47 +52,36 @@ namespace fm {
 
 constexpr int kTcRows = 128;        // UMMA M
 constexpr int kTcNodes = 16;        // nodes per stage -> K = 32 (two UMMA K steps)
-constexpr int kTcStages = 4;
-// Generic units use a ring of their own (kTcRingGen slots of their small
-// stages, which always fit), with their own barriers and stage counter, so
-// that a group's producers need not wait for the previous group's MMAs.  At
-// a unit's end every MMA has completed, so the two rings may share the
-// shared memory.
-constexpr int kTcRingGen = 8;
+constexpr int kTcMinRing = 3, kTcMaxRing = 8;  // pipeline stages in shared memory
 constexpr int kTcBlockNodes = 128;  // nodes whose per-run data is formed together
 constexpr int kTcStagesPerBlock = kTcBlockNodes / kTcNodes;
-constexpr int kTcProducerWarps = 16;
-constexpr int kTcProducers = 32 * kTcProducerWarps;  // every thread of the block
-constexpr int kTcThreads = kTcProducers;
+constexpr int kTcThreads = 512;
 constexpr int kTcVGroup = 8;        // Mxy columns per launch
+// Warp roles.  Warps 0-12 write the operand tiles, 13 and 14 form the node
+// blocks, 15 issues the MMAs.  A stage's A is written by one warp per 32 rows,
+// its B tile by one or two warps; such groups take the stages in turn, so that
+// each warp waits, fences and signals once for all it does in a stage.  No
+// more groups take turns than the ring has slots: a warp's next slot has then
+// been released at most one round ago, and its barrier's parity is
+// unambiguous.  Warps 0-7 also fold the accumulator and write the results.
+constexpr int kTcDrainWarps = 8;
+constexpr int kTcOperandWarps = 13;
+constexpr int kTcStageArrivals = 6;  // at most 4 A and 2 B warps; the first A warp arrives for the missing ones
+constexpr int kTcNodeWarp = 13;
+constexpr int kTcMmaWarp = 15;
 // Stages accumulated in the tensor-memory accumulator before it is folded
 // into an FP32 round-to-nearest running sum (also in tensor memory).  The
 // tensor core's FP32 accumulation truncates, so its error grows with the
 // number of MMAs added into one accumulator; 32 stages (512 nodes, 192 MMAs)
 // keep it near 1e-5.
 constexpr int kTcDrain = 32;
-// Stages a generic (unfactored, N = 16) unit writes between two barriers.  At
-// most kTcStages: a group's stages must use distinct ring slots, whose
-// previous MMAs went out at an earlier barrier (so no wait can depend on the
-// group's own MMAs).
-constexpr int kTcGenGroup = 4;
-// Stages a factored unit writes between two barriers.  The B warps compute
-// the phase table of stage st + kTcFacGroup during stage st, so the table
-// ring holds 2 kTcFacGroup buffers (kTcEBufs).
-constexpr int kTcFacGroup = 2;
-constexpr int kTcEBufs = 2 * kTcFacGroup;
+// Node buffers: one is written while others are still read.  The operand
+// warps are up to a ring apart, so with two buffers of eight stages the next
+// block was often late.
+constexpr int kTcMinNodeBufs = 2, kTcMaxNodeBufs = 4;
 constexpr uint64_t kTcWaitNs = 2000000000ull;
-static_assert(kTcGenGroup <= kTcStages && (kTcRingGen & (kTcRingGen - 1)) == 0 &&
-                  kTcStagesPerBlock % kTcGenGroup == 0 && kTcDrain % kTcGenGroup == 0,
-              "generic stage groups must fit the ring, the node blocks and the accumulation groups");
-static_assert(kTcFacGroup <= kTcStages && kTcStagesPerBlock % kTcFacGroup == 0 && kTcDrain % kTcFacGroup == 0 &&
-                  (kTcEBufs & (kTcEBufs - 1)) == 0 && kTcFacGroup <= 2,
-              "factored stage groups: the node block is requested at stage 2 and derived at stage 4 of 8");
 constexpr uint32_t kAStageBytes = kTcRows * 2 * kTcNodes * 2;  // 128 rows x 32 K x bf16 = 8 KB
 
-struct TcRun {
-  int start, P, Q, factored;
-};
 // A work item: `rows` lines from line p0 and columns q0.. of run `run`, or
 // (stacked problems) `rows` consecutive lines of the problem's runs laid end
 // to end, from line p0 of run `run` on: unit row i is line (p0 + i) % P of
@@ -97,6 +94,18 @@ struct TcRun {
 struct TcItem {
   int run, p0, q0, nrun, rows;
 };
+
+// Kinds of launch entries (one problem's Mxy column group each).
+constexpr int kTcSlab = 0;     // factored runs: rows lines, columns (kz, v)
+constexpr int kTcGeneric = 1;  // other runs: rows samples, columns v
+// Runs as columns, for a problem without motion whose k factors between the
+// run and the place in the slab (kFlagStatic*): rows are the samples of a
+// slab, columns (run, v); A = exp(-2 pi i k_slab . r), B = exp(-2 pi i k_run . r)
+// exp(-t / T2) exp(i phi t) M Mxy.  Slabs of few kz values then give wide
+// tiles: a 32 x 32 x 8 grid of one coil has 64 units of 8 pairs as lines x kz
+// (16 pairs of columns for 128 lines of 4 runs) and 2 units of 32 pairs here.
+constexpr int kTcRuns = 2;
+constexpr int kTcKinds = 3;
 
 struct TcDev {
   int64_t N, S, V;
@@ -113,16 +122,26 @@ struct TcDev {
   const int *frun;    // factored runs
   const int2 *tiles;  // tiles of the generic runs
   int *ctl;           // control words of the problem
-  int Qt, NT, kind;  // kind 0: factored runs, 1: generic runs
+  int Qt, NT, kind;
   int RU;            // lines per stacked unit
+  int use_runs;      // runs become columns where k factors that way (kTcRuns)
   int prob, first, n_of, max_splits;  // the problem, its first entry and its entries
   int wrows;         // rows per node buffer: VG weight rows, then (stacked runs) nrun D rows
-  int stacked;       // items hold several runs (D in the A rows, B without decay)
+  int stacked;       // items may hold several runs (D in the A rows, B without decay)
   int mm_ld;         // row stride of MM (float2): this group's columns, padded to even
   int tma;           // node blocks are staged by bulk copies (aligned inputs, room in smem)
   int mstage;        // 3 r: a single POD term's mode rows are staged with each node block (0: read from global)
   float2 *partials; // (splits, S, V) when splits > 1
   float2 *out;
+};
+
+// Shared-memory layout of a launch, the same for all its entries (the warps
+// cross from one unit to the next on their own, so a ring slot or node buffer
+// must not move): barriers, `ring` stages, two node buffers (positions,
+// weight rows), two staging areas of raw node blocks.
+struct TcGeom {
+  uint32_t stage_bytes, ring;
+  uint32_t node_bufs, pos, w, wrows, raw, raw_bytes, total;
 };
 
 // One launch works through a table of entries (one per problem, Mxy column
@@ -131,7 +150,7 @@ struct TcBatchDev {
   const TcDev *entries;
   const int *offsets;  // device: n_entries + 1 running unit counts
   int n_entries;
-  int acc_cols;  // tensor-memory columns of the widest entry (accumulator; the running sum follows)
+  TcGeom geom;
 };
 
 // Work list of one entry, from the problem's control words.
@@ -154,7 +173,12 @@ __device__ inline int tc_items_per_run(const TcDev &p) {
 }
 
 __device__ inline int tc_n_items(const TcDev &p) {
-  if (p.kind != 0) return p.ctl[kCtlTiles];
+  if (p.use_runs && prep_static(p.ctl)) {
+    if (p.kind != kTcRuns) return 0;
+    return (int)(ceil_div((int64_t)p.n_lines * p.n_kz, kTcRows) * ceil_div(p.ctl[kCtlRuns], p.Qt));
+  }
+  if (p.kind == kTcRuns) return 0;
+  if (p.kind == kTcGeneric) return p.ctl[kCtlTiles];
   if (tc_stacked(p)) return (int)ceil_div((int64_t)p.ctl[kCtlRuns] * p.n_lines, (int64_t)p.RU);
   return p.ctl[kCtlFac] * tc_items_per_run(p);
 }
@@ -164,17 +188,23 @@ __device__ inline TcWork tc_work(const TcDev &p) {
   W.splits = p.ctl[kCtlSplits];
   W.chunk = p.ctl[kCtlChunk];
   W.n_items = tc_n_items(p);
-  W.stack = p.kind == 0 && tc_stacked(p);
+  W.stack = p.kind == kTcSlab && tc_stacked(p);
   W.out = W.splits > 1 ? p.partials : p.out;
   return W;
 }
 
 __device__ inline TcItem tc_item(const TcDev &p, const TcWork &W, int i) {
   TcItem t;
-  if (p.kind != 0) {
+  if (p.kind == kTcGeneric) {
     const int2 k = p.tiles[i];
     t.run = k.x; t.p0 = k.y; t.q0 = 0; t.nrun = 1;
     t.rows = min(kTcRows, p.start[k.x + 1] - p.start[k.x] - k.y);
+  } else if (p.kind == kTcRuns) {
+    const int nq = (int)ceil_div(p.ctl[kCtlRuns], p.Qt);
+    t.run = 0; t.nrun = 1;
+    t.p0 = (i / nq) * kTcRows;
+    t.q0 = (i % nq) * p.Qt;
+    t.rows = min(kTcRows, p.n_lines * p.n_kz - t.p0);
   } else if (W.stack) {
     const int64_t L0 = (int64_t)i * p.RU, total = (int64_t)p.ctl[kCtlRuns] * p.n_lines;
     t.run = (int)(L0 / p.n_lines);
@@ -194,44 +224,35 @@ __device__ inline TcItem tc_item(const TcDev &p, const TcWork &W, int i) {
   return t;
 }
 
-// Shared-memory layout.  Strides of the weight and phase tables are padded
-// (130 and 18 complex values) so that the B producers' 16-byte reads of
-// different columns fall in different banks.
-constexpr int kWStride = kTcBlockNodes + 2;
+// A weight row of a node buffer is a row of real parts and one of imaginary
+// parts, kWStride floats each (padded, so that 16-byte reads of different
+// rows fall in different banks).
+constexpr int kWStride = kTcBlockNodes + 4;
+constexpr uint32_t kTcPosBytes = 3 * kTcBlockNodes * 8;  // x, y, z rows of a node buffer (FP64)
+constexpr int kTcComps = 4;  // x, y, z and (runs as columns) the run's time
 constexpr uint32_t kTcSmemMax = 232448;  // dynamic shared memory a block may opt in to
-constexpr int kEStride = kTcNodes + 2;
 
-// Barriers and the tensor-memory address live in the first kTcFront bytes
-// (fixed, since the tile layout after them changes from unit to unit).
+// Barriers, the tensor-memory address and small shared values.
 constexpr uint32_t kTcFront = 1024;
-constexpr uint32_t kTcBars = 0, kTcMisc = 128;
-
-struct TcSmem {
-  uint32_t stage_bytes, a_hi, a_lo, b_hi, b_lo;  // offsets inside a stage
-  uint32_t stages, pos, w, etab, raw, total;
+constexpr uint32_t kTcMisc = 256;
+struct TcBars {
+  uint64_t full[kTcMaxRing], empty[kTcMaxRing];
+  uint64_t accfull, accfree;
+  uint64_t nodefull[kTcMaxNodeBufs], nodeempty[kTcMaxNodeBufs], rawfull[2];
+  uint64_t done;
+};
+static_assert(kTcMinRing >= 3, "three groups of A warps take turns");
+static_assert(sizeof(TcBars) <= kTcMisc, "barriers fit before the other shared values");
+struct TcMisc {
+  uint32_t tmem;
+  int abort_flag;
+  int rmax[kTcMaxNodeBufs];  // largest |x| + |y| + |z| of each node buffer (float bits)
 };
 
-// Node data is double-buffered: block b is read while block b + 1 is written.
-__host__ __device__ inline TcSmem tc_smem_layout(int NT, int VG, int Qt, int ring = kTcStages) {
-  // VG here is the weight rows per node buffer (TcDev::wrows)
-  TcSmem L;
-  L.a_hi = 0;
-  L.a_lo = kAStageBytes;
-  L.b_hi = 2 * kAStageBytes;
-  L.b_lo = 2 * kAStageBytes + NT * 2 * kTcNodes * 2;
-  L.stage_bytes = 2 * kAStageBytes + 2 * NT * 2 * kTcNodes * 2;
-  L.stages = kTcFront;
-  uint32_t off = kTcFront + (uint32_t)ring * L.stage_bytes;
-  L.pos = off;  // [2][3][128] double: x, y, z of the moved nodes
-  off += 2 * 3 * kTcBlockNodes * 8;
-  L.w = off;  // [2][VG][kWStride] float2
-  off += 2 * VG * kWStride * 8;
-  L.etab = off;  // [kTcEBufs][Qt][kEStride] float2, by stage
-  off += kTcEBufs * Qt * kEStride * 8;
-  L.raw = off;  // staging of one raw node block (bulk copies), when used
-  L.total = off;
-  return L;
-}
+// Narrow and wide tiles (tensor-memory layout and MMAs below).
+__host__ __device__ inline bool tc_narrow(int NT) { return NT <= 128; }
+
+__host__ __device__ inline uint32_t tc_stage_bytes(int NT) { return 2 * kAStageBytes + 2 * NT * 2 * kTcNodes * 2; }
 
 // Bytes of one raw node block: positions, T2, phi and the group's M Mxy rows.
 __host__ __device__ inline uint32_t tc_raw_bytes(int mm_ld) {
@@ -255,31 +276,80 @@ __host__ __device__ inline uint32_t sw64_offset(uint32_t row, uint32_t k) {
   return row * 64 + ((((k >> 3) ^ (row >> 1)) & 3) << 4) + (k & 7) * 2;
 }
 
+// Two FP32 values in one 64-bit register pair: the packed add, multiply and
+// multiply-add issue once for both.
+struct F2 {
+  unsigned long long v;
+};
+__device__ inline F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ inline void f2_get(F2 x, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ inline F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ inline F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+__device__ inline uint32_t bf16_pair(float a, float b) {
+  uint32_t r;  // a in the low half (cvt.rn.bf16x2 puts its first source in the upper half)
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+
+// a - h and b - h' for the BF16 pair (h, h'), exactly: the mixed-precision
+// multiply-add takes the BF16 operand as it is.  Shifting it into place first
+// (two instructions of the half-rate integer pipe a pair) made a split twice
+// as long: 8 cycles against 4.2.
+__device__ inline void minus_bf16(float a, float b, uint32_t pair, float &da, float &db) {
+  const uint16_t minus_one = 0xbf80;
+  asm("{\n\t.reg .b16 l, h;\n\t"
+      "mov.b32 {l, h}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, l, %3, %4;\n\t"
+      "fma.rn.f32.bf16 %1, h, %3, %5;\n\t}"
+      : "=&f"(da), "=f"(db)
+      : "r"(pair), "h"(minus_one), "f"(a), "f"(b));
+}
+
 // hi = bf16(x), lo = bf16(x - hi) for the pair (a, b); bits of (hi_a, hi_b)
-// and (lo_a, lo_b) with a in the low half (cvt.rn.bf16x2 puts its first
-// source in the upper half).
+// and (lo_a, lo_b) with a in the low half.
 __device__ inline void split_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
-  uint32_t h, l;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
-  const float ha = __uint_as_float(h << 16), hb = __uint_as_float(h & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(b - hb), "f"(a - ha));
-  hi = h;
-  lo = l;
+  float la, lb;
+  hi = bf16_pair(a, b);
+  minus_bf16(a, b, hi, la, lb);
+  lo = bf16_pair(la, lb);
+}
+// The same for (a, b) and for (b, -a).
+__device__ inline void split_pair_im(float a, float b, uint32_t &hi, uint32_t &lo, uint32_t &hi_im, uint32_t &lo_im) {
+  hi = bf16_pair(a, b);
+  hi_im = bf16_pair(b, -a);
+  float la, lb;
+  minus_bf16(a, b, hi, la, lb);
+  lo = bf16_pair(la, lb);
+  lo_im = bf16_pair(lb, -la);
 }
 
 // cos and sin of 2 pi c for c in cycles given in FP64.  c is reduced modulo
 // one in fixed point: adding 1.5 * 2^29 leaves a double whose last place is
 // 2^-23, so its low 32 bits hold round(c * 2^23) modulo 2^32 and their low
-// 23 bits, sign-extended, are c - rint(c) in units of 2^-23 (error at most
-// 2^-24 cycles, for |c| < 2^28).  This keeps the reduction off the
-// transcendental unit (no rint, no double-to-float conversion): one FP64
-// add, a signed bit-field extract and an integer-to-float conversion, then
-// the FP32 sin/cos.
+// 23 bits, moved to the top of the word, are c - rint(c) in units of 2^-32
+// (error at most 2^-24 cycles, for |c| < 2^28).  This keeps the reduction off
+// the transcendental unit (no rint, no double-to-float conversion): one FP64
+// add, a shift and an integer-to-float conversion, then the FP32 sin/cos.
+// FP64 shares its unit with the tensor core (a DFMA takes 3.2 times as long
+// while N = 256 MMAs run); forming the phases by 32 x 32-bit integer multiplies
+// instead was slower all the same (flow case 9.6 against 8.3 ms), since the
+// half-rate integer pipe is the busier one here.
 __device__ inline void cycles_cos_sin(double c, float &co, float &s) {
-  const int lo = __double2loint(__dadd_rn(c, 805306368.0));
-  int frac;  // the low 23 bits, sign-extended
-  asm("bfe.s32 %0, %1, 0, 23;" : "=r"(frac) : "r"(lo));
-  __sincosf(__int2float_rn(frac) * 7.490140565847157e-07f, &s, &co);  // 2 pi / 2^23
+  const int frac = (int)((unsigned)__double2loint(__dadd_rn(c, 805306368.0)) << 9);
+  __sincosf(__int2float_rn(frac) * 1.4629180792671596e-09f, &s, &co);  // 2 pi / 2^32
 }
 
 __device__ inline void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -288,11 +358,16 @@ __device__ inline void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint3
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d));
 }
 
+__device__ inline void st_shared(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+
 struct TcUnit {
   TcItem it;
-  TcRun run;  // the first run
-  int split, P_tile, Q_tile, n_stages, n_groups;
-  int rows, pairs;  // active A rows and column pairs (Q_tile VG); P_tile: lines per run when stacked
+  int start;      // first sample of the first run
+  int P;          // lines per run (factored) or samples of the run
+  int split, Q_tile, n_stages, n_groups;
+  int rows;       // active A rows
   int64_t n_begin, n_end;
 };
 
@@ -301,14 +376,11 @@ __device__ inline TcUnit tc_unit(const TcDev &p, const TcWork &W, int u) {
   const int item = u % W.n_items;
   U.split = u / W.n_items;
   U.it = tc_item(p, W, item);
-  U.run.start = p.start[U.it.run];
-  U.run.factored = p.kind == 0 ? 1 : 0;
-  U.run.P = U.run.factored ? p.n_lines : p.start[U.it.run + 1] - U.run.start;
-  U.run.Q = U.run.factored ? p.n_kz : 1;
-  U.P_tile = p.stacked ? U.run.P : min(kTcRows, U.run.P - U.it.p0);
-  U.Q_tile = min(p.Qt, U.run.Q - U.it.q0);
+  U.start = p.start[U.it.run];
+  U.P = p.kind == kTcSlab ? p.n_lines : p.start[U.it.run + 1] - U.start;
+  U.Q_tile = p.kind == kTcSlab ? min(p.Qt, p.n_kz - U.it.q0)
+                               : (p.kind == kTcRuns ? min(p.Qt, p.ctl[kCtlRuns] - U.it.q0) : 1);
   U.rows = U.it.rows;
-  U.pairs = U.Q_tile * p.VG;
   U.n_begin = (int64_t)U.split * W.chunk;
   U.n_end = min(p.N, U.n_begin + W.chunk);
   U.n_stages = U.n_end > U.n_begin ? (int)ceil_div(U.n_end - U.n_begin, kTcNodes) : 0;
@@ -316,255 +388,399 @@ __device__ inline TcUnit tc_unit(const TcDev &p, const TcWork &W, int u) {
   return U;
 }
 
+// Entry of unit u: offsets[e] <= u < offsets[e + 1].
+__device__ inline int tc_entry_of(const TcBatchDev &B, int u) {
+  int lo = 0, hi = B.n_entries;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (B.offsets[mid] <= u) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 // Run (relative to the unit's first) and line of unit row `row` (TcItem).
 __device__ inline void tc_row_line(const TcDev &p, const TcUnit &U, int row, int &r, int &line) {
   if (p.stacked) {
     const int lr = U.it.p0 + row;
-    r = lr / U.P_tile;
-    line = lr % U.P_tile;
+    r = lr / U.P;
+    line = lr % U.P;
   } else {
     r = 0;
     line = U.it.p0 + row;
   }
 }
 
+// Output sample of unit row `row` and its first column, and the step from one
+// column q to the next (every run of a stacked unit shares the columns).
+__device__ inline void tc_out_sample(const TcDev &p, const TcUnit &U, int row, int64_t &s_row, int64_t &s_q) {
+  int r, line;
+  tc_row_line(p, U, row, r, line);
+  if (p.kind == kTcRuns) {
+    s_q = (int64_t)p.n_lines * p.n_kz;
+    s_row = U.it.q0 * s_q + line;
+    return;
+  }
+  s_q = 1;
+  s_row = p.start[U.it.run + r] + (p.kind == kTcSlab ? (int64_t)line * p.n_kz + U.it.q0 : line);
+}
+
 // Bounded wait that gives up at once after any earlier timeout of the block
 // (the flag lives in shared memory), so a broken pipeline ends quickly.
 __device__ inline bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-  if (ptx::mbar_try_wait(bar, parity)) return true;
+  if (ptx::mbar_try_wait_long(bar, parity)) return true;
   if (*abort_flag) return false;
   if (ptx::mbar_wait(bar, parity, kTcWaitNs)) return true;
   *abort_flag = 1;
   return false;
 }
 
-// Before a group of stages ending with global stage gl is written: the MMAs
-// that last read its ring slots are done.  They complete in issue order, so
-// waiting for the slot of the group's last stage (stage gl - kTcStages)
-// covers the earlier ones.
-__device__ inline void tc_wait_group(uint64_t *empty, uint32_t gl, volatile int *abort_flag) {
-  tc_wait(&empty[gl & (kTcStages - 1)], ((gl / kTcStages) & 1) ^ 1, abort_flag);
-}
-
-// Shared-memory maximum of non-negative ints over the active lanes of a
-// warp: one atomic per warp instead of one per thread on the same address.
-__device__ inline void tc_note_max(int *dst, int v) {
-  const unsigned mask = __activemask();
-  const int m = __reduce_max_sync(mask, v);
-  if ((threadIdx.x & 31) == __ffs(mask) - 1) atomicMax(dst, m);
-}
-
-// Records |kx| + |ky| + |kz| of a phase row (float bits; a NaN counts as too large).
-__device__ inline void tc_note_k(int *kmax, double kx, double ky, double kz) {
-  const float s = (float)(fabs(kx) + fabs(ky) + fabs(kz));
-  tc_note_max(kmax, __float_as_int(s) & 0x7fffffff);
-}
-
-__device__ inline void prefetch_l1(const void *ptr) { asm volatile("prefetch.global.L1 [%0];" ::"l"(ptr)); }
-
-// Raw node data loaded two stages before it is derived (global loads in
-// flight meanwhile).  With a single rank-1 POD term (the flow and respiratory
-// POD fits of the examples) the node's mode row is loaded into registers with
-// it; otherwise the mode rows are prefetched into L1 for the displacement.
-constexpr int kTcRegModes = 1;
-struct TcRaw {
-  float x, y, z, t2, phi;
-  float2 m[kTcVGroup];
-  float pmx[kTcRegModes], pmy[kTcRegModes], pmz[kTcRegModes];
+// Ring position of a warp: slot and the parity its `full` barrier completes
+// with (its `empty` barrier is waited for with the opposite one).
+struct TcRing {
+  uint32_t slot, phase;
+  __device__ inline void seek(uint32_t stage, uint32_t ring) {
+    slot = stage % ring;
+    phase = (stage / ring) & 1;
+  }
+  __device__ inline void advance(uint32_t stages, uint32_t ring) {
+    slot += stages;
+    while (slot >= ring) {
+      slot -= ring;
+      phase ^= 1;
+    }
+  }
 };
-// Mode count of the register-resident displacement, or -1 when the motion
-// is not a single POD term of at most kTcRegModes modes.
-__device__ inline int tc_reg_modes(const TcDev &p) {
-  return (p.md.kind == FM_MOTION_TERMS && p.md.n_terms == 1 && p.md.terms[0].kind != FM_TERM_RESPIRATORY &&
-          p.md.terms[0].n_modes <= kTcRegModes) ? p.md.terms[0].n_modes : -1;
+
+// float bits of |x| + |y| + |z| (a NaN compares above every number)
+__device__ inline int tc_abs_sum(double x, double y, double z) {
+  return __float_as_int((float)(fabs(x) + fabs(y) + fabs(z))) & 0x7fffffff;
 }
 
-__device__ inline void tc_prefetch_modes(const TcDev &p, int64_t n, TcRaw &rr) {
-  if (p.md.kind != FM_MOTION_TERMS) return;
-  const int rm = tc_reg_modes(p);
-  if (rm >= 0) {
-    const float *Phi = p.md.terms[0].modes + (size_t)n * 3 * rm;
-#pragma unroll
-    for (int m = 0; m < kTcRegModes; ++m) {
-      rr.pmx[m] = m < rm ? __ldg(Phi + m) : 0.f;
-      rr.pmy[m] = m < rm ? __ldg(Phi + rm + m) : 0.f;
-      rr.pmz[m] = m < rm ? __ldg(Phi + 2 * rm + m) : 0.f;
-    }
-    return;
-  }
-  for (int k = 0; k < p.md.n_terms; ++k) {
-    const fm_motion_term &T = p.md.terms[k];
-    if (T.kind == FM_TERM_RESPIRATORY) continue;
-    const float *Phi = T.modes + (size_t)n * 3 * T.n_modes;
-    prefetch_l1(Phi);
-    prefetch_l1(Phi + 3 * T.n_modes - 1);
-  }
+// ---- node blocks ---------------------------------------------------------
+
+// Raw data of one node block in a staging area.
+struct TcRawView {
+  const float *r0, *T2, *phi;
+  const float2 *MM;
+  const float *modes;
+};
+__device__ inline TcRawView tc_raw_view(const unsigned char *staging, int mm_ld) {
+  TcRawView v;
+  v.r0 = reinterpret_cast<const float *>(staging);
+  v.T2 = v.r0 + 3 * kTcBlockNodes;
+  v.phi = v.T2 + kTcBlockNodes;
+  v.MM = reinterpret_cast<const float2 *>(v.phi + kTcBlockNodes);
+  v.modes = reinterpret_cast<const float *>(staging + tc_raw_bytes(mm_ld));
+  return v;
 }
 
-__device__ inline void tc_load_raw(const TcDev &p, int64_t n, TcRaw &r) {
-  r.x = p.r0[3 * n + 0];
-  r.y = p.r0[3 * n + 1];
-  r.z = p.r0[3 * n + 2];
-  r.t2 = p.T2[n];
-  r.phi = p.phi[n];
-#pragma unroll
-  for (int v = 0; v < kTcVGroup; ++v)
-    if (v < p.VG) r.m[v] = p.MM[n * p.mm_ld + v];
-  tc_prefetch_modes(p, n, r);
+// What the node warps need of an entry and a unit, held in registers: reading
+// the entry again for every node cost more than the nodes' arithmetic (a block
+// took 5,100 cycles at 8 columns and 10 modes, 2,900 at 4 columns and one
+// mode, and set the pace of the whole block).
+struct TcNodeArgs {
+  const float *r0, *T2, *phi, *modes, *wrun, *table;
+  const float2 *MM;
+  int VG, mm_ld, mstage, wrows, nrun;
+  bool stacked, runs;
+  float t;  // the run's time; stacked: lane k holds run k's
+  float w;  // lane k: motion weight k of a staged term
+};
+
+__device__ inline TcNodeArgs tc_node_args(const TcDev &p, const TcUnit &U, int lane) {
+  TcNodeArgs a;
+  a.r0 = p.r0; a.T2 = p.T2; a.phi = p.phi;
+  a.MM = p.MM;
+  a.VG = p.VG; a.mm_ld = p.mm_ld; a.mstage = p.mstage; a.wrows = p.wrows; a.nrun = U.it.nrun;
+  a.modes = p.mstage ? p.md.terms[0].modes : nullptr;
+  a.wrun = p.weights ? p.weights + (int64_t)U.it.run * p.md.slots : nullptr;
+  a.table = p.table ? p.table + (int64_t)U.it.run * p.N * 3 : nullptr;
+  a.stacked = p.stacked != 0;
+  a.runs = p.kind == kTcRuns;
+  a.t = (float)p.run_t[U.it.run + (a.stacked && lane < a.nrun ? lane : 0)];
+  a.w = p.mstage && 3 * lane < p.mstage ? a.wrun[p.md.slot0[0] + lane] : 0.f;
+  return a;
 }
 
-// Per-run node quantities of one node into slot `slot` of a node buffer:
-// moved position (in FP64 for the phase products) and the decayed,
-// off-resonance rotated weights W' = (M Mxy)[n, v] exp(-t / T2) exp(i phi t).
-// Nodes past the range get position 0 and zero weights, so they add nothing.
-__device__ inline void tc_derive(const TcDev &p, const TcUnit &U, int64_t n, const TcRaw &r, const float *wrun,
-                                 double *pos, float2 *wblk, int slot, int *rmax, const float *smodes = nullptr) {
-  if (n < U.n_end) {
-    float x = r.x, y = r.y, z = r.z;
-    const int rm = tc_reg_modes(p);
-    if (rm >= 0) {
-      // motion_disp for one POD term, modes from registers (same arithmetic)
-      const float *wk = wrun + p.md.slot0[0];
-      float tx = 0.f, ty = 0.f, tz = 0.f;
+// Requests the raw data of the full node block at n0 (one thread).
+__device__ inline void tc_request_block(const TcNodeArgs &a, int64_t n0, unsigned char *staging, uint64_t *rawfull) {
+  const TcRawView v = tc_raw_view(staging, a.mm_ld);
+  // the staging area's previous readers are past a barrier; order their
+  // reads before the copies
+  ptx::fence_proxy_async_smem();
+  ptx::mbar_arrive_expect_tx(rawfull, tc_raw_bytes(a.mm_ld) + tc_mode_bytes(a.mstage));
+  ptx::bulk_copy_g2s((void *)v.r0, a.r0 + 3 * n0, 12 * kTcBlockNodes, rawfull);
+  ptx::bulk_copy_g2s((void *)v.T2, a.T2 + n0, 4 * kTcBlockNodes, rawfull);
+  ptx::bulk_copy_g2s((void *)v.phi, a.phi + n0, 4 * kTcBlockNodes, rawfull);
+  ptx::bulk_copy_g2s((void *)v.MM, a.MM + n0 * a.mm_ld, 8 * kTcBlockNodes * a.mm_ld, rawfull);
+  // mode rows of node n0 onwards: 12 r bytes per node, n0 a multiple of 16
+  // and the rows 16-byte aligned (checked on the host)
+  if (a.mstage) ptx::bulk_copy_g2s((void *)v.modes, a.modes + n0 * a.mstage, tc_mode_bytes(a.mstage), rawfull);
+}
+
+// Node quantities of the block at n0 into a node buffer (one warp, nodes lane,
+// lane + 32 ..): moved position (in FP64 for the phase
+// products) and the decayed, off-resonance rotated weights
+// W' = (M Mxy)[n, v] exp(-t / T2) exp(i phi t) of the run.  Nodes past the
+// range get position 0 and zero weights, so they add nothing.  Returns the
+// largest |x| + |y| + |z| for the phase range check (float bits).
+__device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, int64_t n0, int64_t n_end, bool staged,
+                                         const TcRawView &raw, unsigned char *buf, float *wblk, int slot0) {
+  constexpr int kPer = kTcBlockNodes / 32, kStep = 32;
+  double *pos = reinterpret_cast<double *>(buf);
+  float x[kPer], y[kPer], z[kPer], t2[kPer], phi[kPer];
+  bool in[kPer];
 #pragma unroll
-      for (int m = 0; m < kTcRegModes; ++m) {
-        const float wm = m < rm ? wk[m] : 0.f;
-        tx = fmaf(r.pmx[m], wm, tx);
-        ty = fmaf(r.pmy[m], wm, ty);
-        tz = fmaf(r.pmz[m], wm, tz);
-      }
-      x = x + tx; y = y + ty; z = z + tz;
-    } else if (p.md.kind == FM_MOTION_TERMS) {
-      float dx, dy, dz;
-      if (smodes) {
-        // the single POD term's sum (motion_disp's products in its order),
-        // the mode row read from the staged block
-        const int rk = p.md.terms[0].n_modes;
-        const float *Phi = smodes + slot * 3 * rk, *wk = wrun + p.md.slot0[0];
-        dx = 0.f; dy = 0.f; dz = 0.f;
-#pragma unroll 1
-        for (int m = 0; m < rk; ++m) {
-          const float wm = wk[m];
-          dx = fmaf(Phi[m], wm, dx);
-          dy = fmaf(Phi[rk + m], wm, dy);
-          dz = fmaf(Phi[2 * rk + m], wm, dz);
-        }
-      } else {
-        motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
-      }
-      x = x + dx; y = y + dy; z = z + dz;
-    } else if (p.table) {
-      const float *d = p.table + ((int64_t)U.it.run * p.N + n) * 3;
-      x = x + d[0]; y = y + d[1]; z = z + d[2];
-    }
-    pos[slot] = (double)x;
-    pos[kTcBlockNodes + slot] = (double)y;
-    pos[2 * kTcBlockNodes + slot] = (double)z;
-    // |x| + |y| + |z| for the phase range check (a NaN counts as too large)
-    tc_note_max(rmax, __float_as_int(fabsf(x) + fabsf(y) + fabsf(z)) & 0x7fffffff);
-    // decay exp(-t / T2) and off-resonance rotation exp(i phi t) of a run:
-    // the fast exponential of -t (1 / T2), and the phase phi t reduced in
-    // cycles in FP64 before the fast sin/cos (cycles_cos_sin), as the A and B
-    // tiles do (both within a few 1e-7 of the accurate functions)
-    const float inv_t2 = __frcp_rn(r.t2);
-    if (p.stacked) {
-      // the weights without decay (B), then one D_r = decay e^{i phi t_r} row per run (A)
-#pragma unroll
-      for (int v = 0; v < kTcVGroup; ++v)
-        if (v < p.VG) wblk[v * kWStride + slot] = r.m[v];
-      for (int k = 0; k < U.it.nrun; ++k) {
-        const float tg = (float)p.run_t[U.it.run + k];
-        const float decay = __expf(-tg * inv_t2);
-        float so, co;
-        cycles_cos_sin((double)(r.phi * tg) * 0.15915494309189535, co, so);
-        wblk[(p.VG + k) * kWStride + slot] = make_float2(decay * co, decay * so);
-      }
+  for (int i = 0; i < kPer; ++i) {
+    const int slot = slot0 + i * kStep;
+    const int64_t n = n0 + slot;
+    in[i] = n < n_end;
+    if (staged) {
+      x[i] = raw.r0[3 * slot]; y[i] = raw.r0[3 * slot + 1]; z[i] = raw.r0[3 * slot + 2];
+      t2[i] = raw.T2[slot];
+      phi[i] = raw.phi[slot];
+    } else if (in[i]) {
+      x[i] = a.r0[3 * n]; y[i] = a.r0[3 * n + 1]; z[i] = a.r0[3 * n + 2];
+      t2[i] = a.T2[n];
+      phi[i] = a.phi[n];
     } else {
-      const float tg = (float)p.run_t[U.it.run];
-      const float decay = __expf(-tg * inv_t2);
-      float so, co;
-      cycles_cos_sin((double)(r.phi * tg) * 0.15915494309189535, co, so);
-      const float er = decay * co, ei = decay * so;
-#pragma unroll
-      for (int v = 0; v < kTcVGroup; ++v)
-        if (v < p.VG)
-          wblk[v * kWStride + slot] = make_float2(r.m[v].x * er - r.m[v].y * ei, r.m[v].x * ei + r.m[v].y * er);
+      x[i] = y[i] = z[i] = phi[i] = 0.f;
+      t2[i] = 1.f;
     }
-  } else {
-    pos[slot] = 0.0;
-    pos[kTcBlockNodes + slot] = 0.0;
-    pos[2 * kTcBlockNodes + slot] = 0.0;
-    for (int v = 0; v < p.wrows; ++v) wblk[v * kWStride + slot] = make_float2(0.f, 0.f);
   }
-}
-
-// Node block blk + 1 of a unit (threads 0-127, one node each), in two calls
-// some stages apart.  request: a full block with p.tma is requested by bulk
-// copies into the staging area (thread 0; completion on rawfull), any other
-// block by register loads.  Otherwise the block is derived into the other
-// node buffer.  raw_seq counts the staged blocks (the rawfull phase).
-template <bool kModes>
-__device__ inline void tc_stage_block(const TcDev &p, const TcUnit &U, int tid, uint32_t blk, bool request,
-                                      TcRaw &raw, uint32_t &raw_seq, unsigned char *staging, uint64_t *rawfull,
-                                      const float *wrun, double *pos_next, float2 *w_next,
-                                      volatile int *abort_flag, int *rmax) {
-  const int64_t n0 = U.n_begin + (int64_t)(blk + 1) * kTcBlockNodes;
-  const int64_t n1 = n0 + tid;
-  const bool staged = p.tma && n0 + kTcBlockNodes <= U.n_end;
-  float *sr0 = reinterpret_cast<float *>(staging);
-  float *sT2 = sr0 + 3 * kTcBlockNodes;
-  float *sphi = sT2 + kTcBlockNodes;
-  float2 *sMM = reinterpret_cast<float2 *>(sphi + kTcBlockNodes);
-  // the block's POD mode rows, after the raw block (TcDev::mstage)
-  float *smodes = reinterpret_cast<float *>(staging + tc_raw_bytes(p.mm_ld));
-  if (request) {
-    if (staged) {
-      if (tid == 0) {
-        // the staging area's previous readers (the last block's derive) are
-        // past this stage's barriers; order their reads before the copies
-        ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive_expect_tx(rawfull, tc_raw_bytes(p.mm_ld) + (kModes ? tc_mode_bytes(p.mstage) : 0u));
-        ptx::bulk_copy_g2s(sr0, p.r0 + 3 * n0, 12 * kTcBlockNodes, rawfull);
-        ptx::bulk_copy_g2s(sT2, p.T2 + n0, 4 * kTcBlockNodes, rawfull);
-        ptx::bulk_copy_g2s(sphi, p.phi + n0, 4 * kTcBlockNodes, rawfull);
-        ptx::bulk_copy_g2s(sMM, p.MM + n0 * p.mm_ld, 8 * kTcBlockNodes * p.mm_ld, rawfull);
-        // mode rows of node n0 onwards: 12 r bytes per node, n0 a multiple of
-        // 16 and the rows 16-byte aligned (checked on the host)
-        if (kModes && p.mstage)
-          ptx::bulk_copy_g2s(smodes, p.md.terms[0].modes + n0 * p.mstage, tc_mode_bytes(p.mstage), rawfull);
+  if (staged && a.mstage) {
+    // the single POD term's sum (motion_disp's products in its order), the
+    // mode rows read from the staged block
+    const int rk = a.mstage / 3;
+    float dx[kPer], dy[kPer], dz[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) dx[i] = dy[i] = dz[i] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < rk; ++k) {
+      const float wm = __shfl_sync(0xffffffffu, a.w, k);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const float *Phi = raw.modes + (slot0 + i * kStep) * a.mstage + k;
+        dx[i] = fmaf(Phi[0], wm, dx[i]);
+        dy[i] = fmaf(Phi[rk], wm, dy[i]);
+        dz[i] = fmaf(Phi[2 * rk], wm, dz[i]);
       }
-      if (!(kModes && p.mstage)) tc_prefetch_modes(p, n1, raw);
-    } else if (n1 < U.n_end) {
-      tc_load_raw(p, n1, raw);
     }
-  } else {
-    if (staged) {
-      tc_wait(rawfull, raw_seq & 1, abort_flag);
-      ++raw_seq;
-      raw.x = sr0[3 * tid];
-      raw.y = sr0[3 * tid + 1];
-      raw.z = sr0[3 * tid + 2];
-      raw.t2 = sT2[tid];
-      raw.phi = sphi[tid];
 #pragma unroll
-      for (int v = 0; v < kTcVGroup; ++v)
-        if (v < p.VG) raw.m[v] = sMM[tid * p.mm_ld + v];
+    for (int i = 0; i < kPer; ++i) {
+      x[i] = x[i] + dx[i]; y[i] = y[i] + dy[i]; z[i] = z[i] + dz[i];
     }
-    tc_derive(p, U, n1, raw, wrun, pos_next, w_next, tid, rmax, kModes && staged && p.mstage ? smodes : nullptr);
+  } else if (a.wrun || a.table) {
+#pragma unroll 1
+    for (int i = 0; i < kPer; ++i) {
+      const int64_t n = n0 + slot0 + i * kStep;
+      if (n >= n_end) continue;
+      float dx, dy, dz;
+      if (a.wrun) {
+        motion_disp(p.md, a.wrun, n, p.N, dx, dy, dz);
+      } else {
+        dx = a.table[3 * n]; dy = a.table[3 * n + 1]; dz = a.table[3 * n + 2];
+      }
+      // (compile-time indices keep the arrays in registers)
+#pragma unroll
+      for (int q = 0; q < kPer; ++q)
+        if (q == i) {
+          x[q] = x[q] + dx; y[q] = y[q] + dy; z[q] = z[q] + dz;
+        }
+    }
+  }
+  int rmax = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int slot = slot0 + i * kStep;
+    pos[slot] = (double)x[i];
+    pos[kTcBlockNodes + slot] = (double)y[i];
+    pos[2 * kTcBlockNodes + slot] = (double)z[i];
+    rmax = max(rmax, __float_as_int(fabsf(x[i]) + fabsf(y[i]) + fabsf(z[i])) & 0x7fffffff);
+  }
+  // decay exp(-t / T2) and off-resonance rotation exp(i phi t) of a run: the
+  // fast exponential of -t (1 / T2), and the phase phi t reduced in cycles in
+  // FP64 before the fast sin/cos (cycles_cos_sin), as the A and B tiles do
+  // (both within a few 1e-7 of the accurate functions).  Stacked: the weights
+  // without decay (B), then one D_r = decay e^{i phi t_r} row per run (A).
+  // Runs as columns: the weights without decay, then 1 / T2 and (FP64) phi in
+  // cycles, from which B forms each run's factor.
+  const int nd = a.runs ? 0 : (a.stacked ? a.nrun : 1);
+  float inv_t2[kPer], er[kPer], ei[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) inv_t2[i] = __frcp_rn(t2[i]);
+  if (a.runs) {
+    double *ph = reinterpret_cast<double *>(wblk + 2 * (a.VG + 1) * kWStride);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      wblk[2 * a.VG * kWStride + slot0 + i * kStep] = in[i] ? inv_t2[i] : 0.f;
+      ph[slot0 + i * kStep] = (double)phi[i] * 0.15915494309189535;
+    }
+  }
+#pragma unroll 1
+  for (int k = 0; k < nd; ++k) {
+    const float tg = a.stacked ? __shfl_sync(0xffffffffu, a.t, k) : a.t;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const float decay = in[i] ? __expf(-tg * inv_t2[i]) : 0.f;
+      float so, co;
+      cycles_cos_sin((double)(phi[i] * tg) * 0.15915494309189535, co, so);
+      er[i] = in[i] ? decay * co : 0.f;
+      ei[i] = in[i] ? decay * so : 0.f;
+      if (a.stacked) {
+        wblk[2 * (a.VG + k) * kWStride + slot0 + i * kStep] = er[i];
+        wblk[(2 * (a.VG + k) + 1) * kWStride + slot0 + i * kStep] = ei[i];
+      }
+    }
+  }
+  const bool plain = a.stacked || a.runs;
+  auto put = [&](int v, int slot, float2 m, float dr, float di) {
+    wblk[2 * v * kWStride + slot] = plain ? m.x : m.x * dr - m.y * di;
+    wblk[(2 * v + 1) * kWStride + slot] = plain ? m.y : m.x * di + m.y * dr;
+  };
+#pragma unroll 1
+  for (int v = 0; v < a.VG; v += 2) {  // rows of M Mxy hold column pairs
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int slot = slot0 + i * kStep;
+      float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (staged) m = *reinterpret_cast<const float4 *>(raw.MM + slot * a.mm_ld + v);
+      else if (in[i]) m = *reinterpret_cast<const float4 *>(a.MM + (n0 + slot) * a.mm_ld + v);
+      put(v, slot, make_float2(m.x, m.y), er[i], ei[i]);
+      if (v + 1 < a.VG) put(v + 1, slot, make_float2(m.z, m.w), er[i], ei[i]);
+    }
+  }
+  return rmax;
+}
+
+// ---- operand tiles -------------------------------------------------------
+
+// Phases k . r of two nodes, in cycles; kRuns: less phi t (ph in cycles, time k[3]).
+template <bool kRuns>
+__device__ __forceinline__ void tc_phase2(const double *pos, const double (&k)[kTcComps], const double *ph, float &c0,
+                                          float &s0, float &c1, float &s1) {
+  const double2 x = *reinterpret_cast<const double2 *>(pos);
+  const double2 y = *reinterpret_cast<const double2 *>(pos + kTcBlockNodes);
+  const double2 z = *reinterpret_cast<const double2 *>(pos + 2 * kTcBlockNodes);
+  double a = k[0] * x.x, b = k[0] * x.y;
+  if (kRuns) {
+    const double2 f = *reinterpret_cast<const double2 *>(ph);
+    a = fma(-k[3], f.x, a);
+    b = fma(-k[3], f.y, b);
+  }
+  cycles_cos_sin(fma(k[2], z.x, fma(k[1], y.x, a)), c0, s0);
+  cycles_cos_sin(fma(k[2], z.y, fma(k[1], y.y, b)), c1, s1);
+}
+
+// A'[row][2n..2n+1] = (Re A, -Im A) = (cos, sin) of 2 pi kp . r_n of 8 nodes;
+// in a stacked unit A is multiplied by the row's run factor D_r(n):
+// (Re, -Im) of (cos - i sin)(dr + i di) = (cos dr + sin di, sin dr - cos di).
+// addr: the row's first 16-byte chunk (hi tile); the second is d_k2 = +/-16
+// bytes from it (swizzled chunk positions 2 half and 2 half + 1 differ in
+// their lowest bit), the lo tile kAStageBytes on.
+template <bool kStacked>
+__device__ __forceinline__ void tc_write_a(const double *pos, const double (&kd)[kTcComps], const float *dp,
+                                           uint32_t addr, int d_k2) {
+  uint32_t h[8], l[8];
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    float c0, s0, c1, s1;
+    tc_phase2<false>(pos + i, kd, nullptr, c0, s0, c1, s1);
+    if (kStacked) {
+      const float2 dr = *reinterpret_cast<const float2 *>(dp + i);
+      const float2 di = *reinterpret_cast<const float2 *>(dp + kWStride + i);
+      const float r0 = fmaf(c0, dr.x, s0 * di.x), r1 = fmaf(c1, dr.y, s1 * di.y);
+      s0 = fmaf(s0, dr.x, -(c0 * di.x));
+      s1 = fmaf(s1, dr.y, -(c1 * di.y));
+      c0 = r0;
+      c1 = r1;
+    }
+    split_pair(c0, s0, h[i], l[i]);
+    split_pair(c1, s1, h[i + 1], l[i + 1]);
+  }
+  st_shared_v4(addr, h[0], h[1], h[2], h[3]);
+  st_shared_v4(addr + d_k2, h[4], h[5], h[6], h[7]);
+  st_shared_v4(addr + kAStageBytes, l[0], l[1], l[2], l[3]);
+  st_shared_v4(addr + kAStageBytes + d_k2, l[4], l[5], l[6], l[7]);
+}
+
+// B'^T rows of one kz value q and 8 nodes, all VG columns: re row `row` =
+// (Re B, Im B), im row NT/2 + row = (Im B, -Re B), B = e_q(n) W'(n, v),
+// e_q = exp(-2 pi i kq . r_n), row = v Qt + q (the lanes of a warp hold
+// consecutive q, so their 16-byte stores fall in different banks; rows
+// q VG + v took 570 cycles a task at VG = 4 against 220).  wblk: the
+// block's weight rows; node0: the first of the 8 nodes.
+// kRuns: q is a run of time t and B also carries its decay and off-resonance
+// rotation, e_q = exp(-2 pi i kq . r_n + i phi_n t) exp(-t / T2_n).
+template <bool kRuns>
+__device__ __forceinline__ void tc_write_b(const double *pos, const double (&kd)[kTcComps], const float *wblk,
+                                           int node0, int VG, int row, int Qt, int half, uint32_t b_tile,
+                                           uint32_t d_lo, uint32_t d_im) {
+  F2 er[4], ei[4], ni[4];  // node pairs; ni = -ei
+  const float *rate = wblk + 2 * VG * kWStride + node0;  // kRuns: 1 / T2, then phi in cycles
+  const double *ph = reinterpret_cast<const double *>(wblk + 2 * (VG + 1) * kWStride) + node0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float c0, s0, c1, s1;
+    tc_phase2<kRuns>(pos + 2 * i, kd, ph + 2 * i, c0, s0, c1, s1);
+    if (kRuns) {
+      const float2 inv = *reinterpret_cast<const float2 *>(rate + 2 * i);
+      const float t = (float)kd[3], d0 = __expf(-t * inv.x), d1 = __expf(-t * inv.y);
+      c0 *= d0; s0 *= d0;
+      c1 *= d1; s1 *= d1;
+    }
+    er[i] = f2(c0, c1);
+    ni[i] = f2(s0, s1);
+    ei[i] = f2(-s0, -s1);
+  }
+  const float *wp = wblk + node0;
+#pragma unroll 1
+  for (int v = 0; v < VG; ++v, row += Qt, wp += 2 * kWStride) {
+    const float4 *wr4 = reinterpret_cast<const float4 *>(wp), *wi4 = reinterpret_cast<const float4 *>(wp + kWStride);
+    const uint32_t b = b_tile + sw64_offset(row, 16 * half);
+    const int d_k2 = ((row >> 1) & 1) != 0 ? -16 : 16;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // four nodes: one 16-byte chunk of each tile
+      const float4 wr = wr4[i], wi = wi4[i];
+      uint32_t h[4], l[4], hm[4], lm[4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const F2 r2 = j ? f2(wr.z, wr.w) : f2(wr.x, wr.y), i2 = j ? f2(wi.z, wi.w) : f2(wi.x, wi.y);
+        const int k = 2 * i + j;
+        float b0r, b1r, b0i, b1i;
+        f2_get(f2_fma(er[k], r2, f2_mul(ni[k], i2)), b0r, b1r);
+        f2_get(f2_fma(er[k], i2, f2_mul(ei[k], r2)), b0i, b1i);
+        split_pair_im(b0r, b0i, h[2 * j], l[2 * j], hm[2 * j], lm[2 * j]);
+        split_pair_im(b1r, b1i, h[2 * j + 1], l[2 * j + 1], hm[2 * j + 1], lm[2 * j + 1]);
+      }
+      const uint32_t at = b + (i ? d_k2 : 0);
+      st_shared_v4(at, h[0], h[1], h[2], h[3]);
+      st_shared_v4(at + d_lo, l[0], l[1], l[2], l[3]);
+      st_shared_v4(at + d_im, hm[0], hm[1], hm[2], hm[3]);
+      st_shared_v4(at + d_im + d_lo, lm[0], lm[1], lm[2], lm[3]);
+    }
   }
 }
 
-// Phase table of one stage of a factored unit: e_q(n) = exp(-2 pi i kq_q . r_n)
-// for q = q0 (and q0 + 32) and the two nodes n0, n0 + 1 of this thread.
-__device__ inline void tc_phase_pair(const double *pb, float2 *et, int q, int n0, double kx, double ky, double kz) {
-  const double2 x = *reinterpret_cast<const double2 *>(pb + n0);
-  const double2 y = *reinterpret_cast<const double2 *>(pb + kTcBlockNodes + n0);
-  const double2 z = *reinterpret_cast<const double2 *>(pb + 2 * kTcBlockNodes + n0);
-  float c0, s0, c1, s1;
-  cycles_cos_sin(fma(kz, z.x, fma(ky, y.x, kx * x.x)), c0, s0);
-  cycles_cos_sin(fma(kz, z.y, fma(ky, y.y, kx * x.y)), c1, s1);
-  *reinterpret_cast<float4 *>(et + q * kEStride + n0) = make_float4(c0, -s0, c1, -s1);
+// B'^T rows of a generic unit: B is only the weights of the VG columns.  The
+// four A warps of a stage write it, one element a lane: column lane % 8, node
+// 4 (warp % 4) + lane / 8 (a warp of its own took 700 cycles a stage for it,
+// the whole of A takes 600).
+__device__ __forceinline__ void tc_write_b_generic(const float *w, int VG, int quad, uint32_t b_tile, uint32_t d_lo,
+                                                   uint32_t d_im) {
+  const int lane = threadIdx.x & 31, v = lane & 7, node = 4 * quad + (lane >> 3);
+  if (v >= VG) return;
+  uint32_t h, l, hm, lm;
+  split_pair_im(w[2 * v * kWStride + node], w[(2 * v + 1) * kWStride + node], h, l, hm, lm);
+  // the im row is a multiple of 8 rows on, so its swizzle is the same
+  const uint32_t b = b_tile + sw64_offset(v, 2 * node);
+  st_shared(b, h);
+  st_shared(b + d_lo, l);
+  st_shared(b + d_im, hm);
+  st_shared(b + d_im + d_lo, lm);
 }
+
+// ---- accumulator ---------------------------------------------------------
 
 // Tensor memory (all 512 columns of the SM).  Wide tiles (NT > 128): the
 // accumulator in columns [0, NT) collects all three products.  Narrow tiles
@@ -577,73 +793,67 @@ __device__ inline void tc_phase_pair(const double *pb, float2 *et, int q, int n0
 // sum follows at column sum_col.  In each part, column j < NT/2 is the real
 // part of pair j and column NT/2 + j its imaginary part.
 constexpr uint32_t kTcTmemCols = 512;
-__host__ __device__ inline bool tc_narrow(int NT) { return NT <= 128; }
 __host__ __device__ inline int tc_parts(int NT) { return tc_narrow(NT) ? 2 : 1; }
 __host__ __device__ inline int tc_sum_col(int NT) { return ((tc_parts(NT) * NT) + 31) & ~31; }
 
-// Folds the accumulator (group gg, complete once accfull's phase gg & 1
-// has flipped) into the running sum: sum = part_0 (+ part_1) for the first
-// group, else sum + (part_0 (+ part_1)), in FP32 round-to-nearest.  Warp w
-// handles TMEM lanes of quarter w % 4 and column quarter w / 4.  The next MMA
-// into the accumulator is issued after a block barrier.
-__device__ inline void tc_fold(const TcDev &p, uint64_t *accfull, uint32_t tmem, int gg, bool first,
-                               volatile int *abort_flag) {
+// Folds the accumulator (complete) into the running sum: sum = part_0
+// (+ part_1) for the first group, else sum + (part_0 (+ part_1)), in FP32
+// round-to-nearest.  Warps 0-7: warp w handles TMEM lanes of quarter w % 4
+// and every other 8 columns.
+// Waits for the group (accfull, `parity`) and hands the accumulator back.  Not
+// inlined: it runs once in 32 stages, and its registers would be the stage
+// loops'.
+__device__ __noinline__ void tc_fold(TcBars *bars, uint32_t parity, int NT, uint32_t tmem, bool first,
+                                     volatile int *abort_flag) {
   const int warp = threadIdx.x >> 5;
-  tc_wait(accfull, gg & 1, abort_flag);
+  tc_wait(&bars->accfull, parity, abort_flag);
+  __syncwarp();
   ptx::tc_fence_after();
-  const int NT = p.NT, n_acc = tc_parts(NT), sum_col = tc_sum_col(NT);
-  const int quarter = warp & 3, cq = warp >> 2;
-  const int cpq = ((NT / 4 + 15) / 16) * 16;
-  const int c_begin = cq * cpq, c_end = min(NT, c_begin + cpq);
-  const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-  for (int c0 = c_begin; c0 < c_end; c0 += 16) {
-    uint32_t a[16];
-    ptx::tmem_ld16(tmem + lanes + (uint32_t)c0, a);
+  const int sum_col = tc_sum_col(NT);
+  const bool narrow = tc_narrow(NT);
+  const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll 2
+  for (int c0 = (warp >> 2) * 8; c0 < NT; c0 += 16) {
+    uint32_t a[8], b[8], r[8];
+    ptx::tmem_ld8(base + (uint32_t)c0, a);
+    if (narrow) ptx::tmem_ld8(base + (uint32_t)(NT + c0), b);
+    if (!first) ptx::tmem_ld8(base + (uint32_t)(sum_col + c0), r);
     ptx::tmem_wait_ld();
-    // the other accumulators, then the running sum, in halves of 8 columns
-    for (int k = 1; k <= n_acc; ++k) {
-      if (k == n_acc && first) break;
-      const int col = (k == n_acc ? sum_col : k * NT) + c0;
+    if (narrow) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t r[8];
-        ptx::tmem_ld8(tmem + lanes + (uint32_t)(col + 8 * h), r);
-        ptx::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          a[8 * h + i] = k == n_acc ? __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(a[8 * h + i]))
-                                    : __float_as_uint(__uint_as_float(a[8 * h + i]) + __uint_as_float(r[i]));
-      }
+      for (int i = 0; i < 8; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) + __uint_as_float(b[i]));
     }
-    ptx::tmem_st16(tmem + lanes + (uint32_t)(sum_col + c0), a);
+    if (!first) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(a[i]));
+    }
+    ptx::tmem_st8(base + (uint32_t)(sum_col + c0), a);
   }
   ptx::tmem_wait_st();
   ptx::tc_fence_before();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(&bars->accfree);
 }
 
 // Writes the unit's result: running sum (when earlier groups were folded) +
-// the accumulator of the last group gg (its parts added in order), to the
-// output samples.  Warp w reads TMEM lanes of quarter w % 4 and every fourth
-// chunk of 8 pairs starting at w / 4.
-__device__ inline void tc_final(const TcDev &p, const TcWork &W, const TcUnit &U, uint64_t *accfull,
-                                uint32_t tmem, int gg, bool has_sum, volatile int *abort_flag) {
+// the accumulator of the last group (its parts added in order), to the output
+// samples.  Warps 0-7: warp w reads TMEM lanes of quarter w % 4 and every
+// other chunk of 8 pairs.
+__device__ __forceinline__ void tc_final(const TcDev &p, const TcWork &W, const TcUnit &U, uint32_t tmem,
+                                         bool has_sum) {
   const int tid = threadIdx.x, warp = tid >> 5;
-  tc_wait(accfull, gg & 1, abort_flag);
   ptx::tc_fence_after();
   const int quarter = warp & 3;
   const int row = quarter * 32 + (tid & 31);
-  const int NH = p.NT >> 1;
+  const int NH = p.NT >> 1, VG = p.VG;
   const bool row_ok = row < U.rows;
   float2 *dst = W.out + (int64_t)U.split * p.S * p.V;
-  // every run of a stacked unit shares the column pairs
-  int r_row = 0, line = 0;
-  if (row_ok) tc_row_line(p, U, row, r_row, line);
-  const int qvg = U.Q_tile * p.VG;
-  const int start = row_ok ? p.start[U.it.run + r_row] : 0;
-  const int s_row = start + (U.run.factored ? line * p.n_kz + U.it.q0 : line);
+  const int Qt = p.Qt, n_pairs = Qt * VG;  // pair j: column v = j / Qt, q = j % Qt
+  int64_t s_row = 0, s_q = 0;
+  if (row_ok) tc_out_sample(p, U, row, s_row, s_q);
   const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
   const int n_acc = tc_parts(p.NT), AW = p.NT, sum_col = tc_sum_col(p.NT);
-  for (int c0 = (warp >> 2) * 8; c0 < NH; c0 += 32) {
+  for (int c0 = (warp >> 2) * 8; c0 < n_pairs; c0 += 16) {
     uint32_t r[8], m[8];
     ptx::tmem_ld8(taddr + (uint32_t)c0, r);
     ptx::tmem_ld8(taddr + (uint32_t)(NH + c0), m);
@@ -675,487 +885,369 @@ __device__ inline void tc_final(const TcDev &p, const TcWork &W, const TcUnit &U
       }
     }
     if (!row_ok) continue;
+    int vv = c0 / Qt, q = c0 - vv * Qt;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float re = re8[i], im = im8[i];
-      const int jj = c0 + i;  // pair (q, v)
-      if (jj >= qvg) continue;
-      const int q = jj / p.VG, vv = jj % p.VG;
-      if (q < U.Q_tile) dst[(int64_t)(s_row + q) * p.V + p.v0 + vv] = make_float2(re, im);
+      if (q < U.Q_tile && vv < VG) dst[(s_row + q * s_q) * p.V + p.v0 + vv] = make_float2(re8[i], im8[i]);
+      if (++q == Qt) {
+        q = 0;
+        ++vv;
+      }
     }
   }
   ptx::tc_fence_before();
 }
 
-// MMAs of one stage (global stage index g, stage-local st of a unit with
-// n_stages stages): A_hi B_hi + A_hi B_lo + A_lo B_hi over the two K steps
-// into the accumulator (overwritten at a group's first stage); the stage's
-// shared memory is released by a commit to empty[s], and the group's
-// accumulator by a commit to accfull after the group's last stage.  kFence:
-// the call orders its MMAs after the group barrier itself (otherwise the
-// caller has done so once for the group).  Called by
-// the whole issuing warp (warp 7): the descriptors are warp-uniform, and
-// lane 0 issues the MMAs and commits (it is the thread whose operations the
-// commits track).
-template <bool kFence>
-__device__ inline void tc_issue(const TcSmem &L, uint32_t sbase, uint32_t tmem, uint32_t idesc, int NT,
-                                uint64_t *empty, uint64_t *accfull, uint32_t s, uint32_t st, uint32_t n_stages,
-                                uint32_t lane) {
-  if (kFence) ptx::tc_fence_after();
+// MMAs of one stage (first: the first stage of an accumulation group, which
+// overwrites the accumulator): A_hi B_hi + A_hi B_lo + A_lo B_hi over the two
+// K steps.  Called by the one thread that issues every MMA and commit.
+template <bool kNarrow>
+__device__ __forceinline__ void tc_issue(uint32_t stage_addr, uint32_t tmem, uint32_t idesc, uint32_t idesc2,
+                                         uint32_t d_blo, bool first) {
   // Descriptors (ptx::smem_desc_sw64): the tiles of a stage differ only in
   // the start-address field, address / 16 (below 2^14 in shared memory, and
   // every tile and stage offset a multiple of 16), so the stage's field is
   // formed once and each tile's is one add; the high word is constant.
-  const uint32_t f0 = ((sbase + L.stages + s * L.stage_bytes) >> 4) | (1u << 16);  // + LBO
+  const uint32_t f0 = (stage_addr >> 4) | (1u << 16);                             // + LBO
   constexpr uint32_t kDescHi = (512u >> 4) | (1u << 14) | (4u << 29);            // SBO, version, 64B swizzle
-  // the drain group's first stage overwrites the accumulator; everything is
-  // computed before the first MMA goes out
-  const uint32_t acc0 = (st % kTcDrain) == 0 ? 0u : 1u;
-  uint64_t ad[2][2], bd[2][2];
+  const uint32_t acc0 = first ? 0u : 1u;
+  constexpr uint32_t a_lo = kAStageBytes >> 4, b_hi = 2 * kAStageBytes >> 4;
+  auto desc = [&](uint32_t off) { return ((uint64_t)kDescHi << 32) | (f0 + off); };
 #pragma unroll
   for (int ks = 0; ks < 2; ++ks) {
     // K step ks: elements 16 ks .. 16 ks + 15, bytes 32 ks .. of every row
-    ad[ks][0] = ((uint64_t)kDescHi << 32) | (f0 + ((L.a_hi + ks * 32) >> 4));
-    ad[ks][1] = ((uint64_t)kDescHi << 32) | (f0 + ((L.a_lo + ks * 32) >> 4));
-    bd[ks][0] = ((uint64_t)kDescHi << 32) | (f0 + ((L.b_hi + ks * 32) >> 4));
-    bd[ks][1] = ((uint64_t)kDescHi << 32) | (f0 + ((L.b_lo + ks * 32) >> 4));
-  }
-  if (tc_narrow(NT)) {
-    // A_hi [B_hi; B_lo] (N = 2 NT, both tiles from b_hi on), then A_lo B_hi
-    const uint32_t idesc2 = ptx::idesc_bf16_f32(kTcRows, 2 * NT);
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      ptx::mma_bf16_lane0(tmem, ad[ks][0], bd[ks][0], idesc2, ks == 0 ? acc0 : 1u, lane);
-      ptx::mma_bf16_lane0(tmem, ad[ks][1], bd[ks][0], idesc, 1u, lane);
-    }
-  } else {
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      ptx::mma_bf16_lane0(tmem, ad[ks][0], bd[ks][0], idesc, ks == 0 ? acc0 : 1u, lane);
-      ptx::mma_bf16_lane0(tmem, ad[ks][0], bd[ks][1], idesc, 1u, lane);
-      ptx::mma_bf16_lane0(tmem, ad[ks][1], bd[ks][0], idesc, 1u, lane);
+    const uint32_t acc = ks == 0 ? acc0 : 1u;
+    if (kNarrow) {
+      // A_hi [B_hi; B_lo] (N = 2 NT, both tiles from b_hi on), then A_lo B_hi
+      ptx::mma_bf16(tmem, desc(2 * ks), desc(b_hi + 2 * ks), idesc2, acc);
+      ptx::mma_bf16(tmem, desc(a_lo + 2 * ks), desc(b_hi + 2 * ks), idesc, 1u);
+    } else {
+      ptx::mma_bf16(tmem, desc(2 * ks), desc(b_hi + 2 * ks), idesc, acc);
+      ptx::mma_bf16(tmem, desc(2 * ks), desc(b_hi + d_blo + 2 * ks), idesc, 1u);
+      ptx::mma_bf16(tmem, desc(a_lo + 2 * ks), desc(b_hi + 2 * ks), idesc, 1u);
     }
   }
-  ptx::mma_commit_lane0(&empty[s], lane);
-  if ((st % kTcDrain) == kTcDrain - 1 || st == n_stages - 1) ptx::mma_commit_lane0(accfull, lane);
 }
 
-// kModes: some entry stages POD mode rows with its node blocks (TcDev::mstage);
-// the instance without that code is the one every other launch uses.
-template <bool kModes>
+// ---- warp roles ----------------------------------------------------------
+
+// Warp 15, one elected thread: a stage's MMAs once its operands are written;
+// each stage's slot is released by a commit to its `empty` barrier, the
+// accumulator handed over by a commit to accfull after a group's last stage
+// and taken back at accfree.  The election (not a test of the lane number)
+// tells the compiler that one thread runs, so the descriptors go straight to
+// uniform registers: an MMA issues in 40 cycles, against 100 under a lane
+// predicate (whatever its shape), and a commit adds none, against 80-230.
+template <bool kNarrow>
+__device__ __forceinline__ void tc_mma_unit(const TcGeom &G, TcBars *bars, uint32_t stages, uint32_t tmem, int NT,
+                                            int nst, TcRing &r, uint32_t &group, volatile int *abort_flag) {
+  const uint32_t idesc = ptx::idesc_bf16_f32(kTcRows, NT), idesc2 = ptx::idesc_bf16_f32(kTcRows, 2 * NT);
+  for (int st = 0; st < nst; ++st) {
+    const bool first = (st % kTcDrain) == 0;
+    if (first) tc_wait(&bars->accfree, (group & 1) ^ 1, abort_flag);
+    tc_wait(&bars->full[r.slot], r.phase, abort_flag);
+    ptx::tc_fence_after();
+    tc_issue<kNarrow>(stages + r.slot * G.stage_bytes, tmem, idesc, idesc2, (uint32_t)NT * 64 >> 4, first);
+    ptx::mma_commit(&bars->empty[r.slot]);
+    if ((st % kTcDrain) == kTcDrain - 1 || st == nst - 1) {
+      ptx::mma_commit(&bars->accfull);
+      ++group;
+    }
+    r.advance(1, G.ring);
+  }
+}
+
+__device__ __forceinline__ void tc_role_mma(const TcBatchDev &B, TcBars *bars, uint32_t stages, uint32_t tmem,
+                                            int n_units, volatile int *abort_flag) {
+  if (ptx::elect_one()) {
+    TcRing r;
+    r.seek(0, B.geom.ring);
+    uint32_t group = 0;
+    for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+      const int e = tc_entry_of(B, u);
+      const TcDev &p = B.entries[e];
+      const int NT = p.NT, nst = tc_unit(p, tc_work(p), u - B.offsets[e]).n_stages;
+      if (tc_narrow(NT)) tc_mma_unit<true>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
+      else tc_mma_unit<false>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
+    }
+    // all issued MMAs complete before the tensor memory is released
+    ptx::mma_commit(&bars->done);
+    if (!ptx::mbar_wait(&bars->done, 0, kTcWaitNs)) *abort_flag = 1;
+  }
+  __syncwarp();
+}
+
+// Warps 13 and 14: the node blocks in turn, ahead of their readers; a full
+// block's raw data is fetched by bulk copies into the warp's staging area while
+// the other warp's block is formed.
+__device__ __forceinline__ void tc_role_nodes(const TcBatchDev &B, TcBars *bars, TcMisc *misc, unsigned char *smem,
+                                              int n_units, volatile int *abort_flag) {
+  const int d = (threadIdx.x >> 5) - kTcNodeWarp, lane = threadIdx.x & 31;
+  const TcGeom &G = B.geom;
+  float *w_all = reinterpret_cast<float *>(smem + G.w);
+  unsigned char *staging = smem + G.raw + d * G.raw_bytes;
+  const TcRawView none{};
+  uint32_t block0 = 0;  // blocks of earlier units
+  uint32_t rs = 0;      // blocks staged so far by this warp
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    const int e = tc_entry_of(B, u);
+    const TcDev &p = B.entries[e];
+    const TcUnit U = tc_unit(p, tc_work(p), u - B.offsets[e]);
+    const int n_blocks = (U.n_stages + kTcStagesPerBlock - 1) / kTcStagesPerBlock;
+    const TcNodeArgs a = tc_node_args(p, U, lane);
+    const bool tma = p.tma != 0;
+    auto n_at = [&](int blk) { return U.n_begin + (int64_t)blk * kTcBlockNodes; };
+    auto staged = [&](int blk) { return tma && n_at(blk + 1) <= U.n_end; };
+    auto request = [&](int blk) {
+      if (blk < n_blocks && staged(blk) && lane == 0) tc_request_block(a, n_at(blk), staging, &bars->rawfull[d]);
+    };
+    const int first = (d + block0) & 1;
+    request(first);
+    TcRing nr;  // the block's node buffer
+    nr.seek(block0 + first, G.node_bufs);
+    for (int blk = first; blk < n_blocks; blk += 2) {
+      const uint32_t b = nr.slot;
+      const bool now = staged(blk);
+      tc_wait(&bars->nodeempty[b], nr.phase ^ 1, abort_flag);
+      if (now) {
+        tc_wait(&bars->rawfull[d], rs & 1, abort_flag);
+        ++rs;
+      }
+      __syncwarp();  // the derive exchanges values between lanes
+      int rmax = tc_derive(p, a, n_at(blk), U.n_end, now, now ? tc_raw_view(staging, a.mm_ld) : none,
+                           smem + G.pos + b * kTcPosBytes, w_all + b * G.wrows * 2 * kWStride, lane);
+      rmax = __reduce_max_sync(0xffffffffu, rmax);
+      if (lane == 0) misc->rmax[b] = rmax;
+      __syncwarp();  // the block is written and the staging area read
+      if (lane == 0) ptx::mbar_arrive(&bars->nodefull[b]);
+      request(blk + 2);
+      nr.advance(2, G.node_bufs);
+    }
+    block0 += n_blocks;
+  }
+}
+
+// Warps 0-12: operand tiles; warps 0-7 also fold the accumulator and write
+// the results.
+__device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *bars, TcMisc *misc, unsigned char *smem,
+                                                 uint32_t stages, uint32_t tmem, int n_units,
+                                                 volatile int *abort_flag) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const TcGeom &G = B.geom;
+  const float *w_all = reinterpret_cast<const float *>(smem + G.w);
+  const uint32_t ring = G.ring, stage_bytes = G.stage_bytes;
+  uint32_t stage0 = 0, group0 = 0;  // stages and accumulation groups of earlier units
+  TcRing nr;                        // next node buffer
+  nr.seek(0, G.node_bufs);
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    const int e = tc_entry_of(B, u);
+    const TcDev &p = B.entries[e];
+    const TcUnit U = tc_unit(p, tc_work(p), u - B.offsets[e]);
+    const int NT = p.NT, VG = p.VG, Qt = p.Qt, Q_tile = U.Q_tile, nst = U.n_stages;
+    const int n_blocks = (nst + kTcStagesPerBlock - 1) / kTcStagesPerBlock;
+    const bool stacked = p.stacked != 0, generic = p.kind == kTcGeneric, runs = p.kind == kTcRuns;
+    const int cmask = runs ? prep_run_comps(p.ctl) : 0;  // components of k that go with the run
+    const bool drains = warp < kTcDrainWarps;
+    // turns: three groups of A warps for a generic unit (they write its B too),
+    // else two, and the other warps on B: two per stage (a node half each)
+    // when the tile has more than 16 columns and there are warps for it
+    const int nrg = (U.rows + 31) >> 5, a_groups = generic ? 3 : 2, nA = a_groups * nrg;
+    const bool is_a = warp < nA, both = Q_tile <= 16;
+    const int b_per = both || kTcOperandWarps - nA < 4 ? 1 : 2;
+    const int b_groups = generic ? 0 : min((kTcOperandWarps - nA) / b_per, (int)ring);
+    const uint32_t d_lo = (uint32_t)NT * 64, d_im = (uint32_t)(NT >> 1) * 64;
+    // the unit's node blocks, each acquired and released in order by every
+    // warp (a barrier's phases could otherwise be counted twice)
+    int blk = -1, rmax = 0;
+    uint32_t nbuf = 0;
+    auto release = [&]() {
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&bars->nodeempty[nbuf]);
+    };
+    auto acquire = [&](int to) {
+      while (blk < to) {
+        tc_wait(&bars->nodefull[nr.slot], nr.phase, abort_flag);
+        rmax = max(rmax, misc->rmax[nr.slot]);
+        nbuf = nr.slot;
+        nr.advance(1, G.node_bufs);
+        if (++blk < to) release();
+      }
+    };
+    // accumulation groups folded into the running sum: group g (not the last)
+    // when the ring is full of the next group's stages, so that the tensor
+    // core has work as soon as the accumulator is free again
+    int folded = 0;
+    auto fold_before = [&](int st) {
+      while (folded < U.n_groups - 1 && st >= (folded + 1) * kTcDrain + (int)ring - 1) {
+        tc_fold(bars, (group0 + folded) & 1, NT, tmem, folded == 0, abort_flag);
+        ++folded;
+      }
+    };
+    TcRing r;
+    int kmax = -1;  // |k| of this thread's phases (float bits)
+    if (is_a) {
+      // rows 32 rg .. of every a_groups-th stage
+      const int grp = warp / nrg, rg = warp - grp * nrg, row = rg * 32 + lane;
+      double kd[kTcComps] = {0, 0, 0, 0};
+      int a_drow = 0;
+      if (row < U.rows) {
+        int rr, line;
+        tc_row_line(p, U, row, rr, line);
+        a_drow = 2 * (VG + rr) * kWStride;
+        const int s_p = (rr == 0 ? U.start : p.start[U.it.run + rr]) + (p.kind == kTcSlab ? line * p.n_kz : line);
+        kd[0] = cmask & 1 ? 0.0 : (double)p.kx[s_p];
+        kd[1] = cmask & 2 ? 0.0 : (double)p.ky[s_p];
+        kd[2] = cmask & 4 ? 0.0 : (double)p.kz[s_p];
+        kmax = tc_abs_sum(kd[0], kd[1], kd[2]);
+      }
+      const uint32_t row_off = sw64_offset(row, 0), row_off1 = sw64_offset(row, 16);
+      const int d_k2 = ((row >> 1) & 1) != 0 ? -16 : 16;
+      const uint32_t arrive = rg != 0 ? 1 : kTcStageArrivals - (nrg - 1) - (generic ? 0 : b_per);
+      r.seek(stage0 + grp, ring);
+      for (int st = grp; st < nst; st += a_groups) {
+        if (drains) fold_before(st);
+        acquire(st / kTcStagesPerBlock);
+        tc_wait(&bars->empty[r.slot], r.phase ^ 1, abort_flag);
+        const uint32_t j = st & (kTcStagesPerBlock - 1);
+        const uint32_t stg = stages + r.slot * stage_bytes;
+        const float *wp = w_all + nbuf * G.wrows * 2 * kWStride + j * kTcNodes;
+        if (generic)
+          for (int quad = rg; quad < 4; quad += nrg)
+            tc_write_b_generic(wp, VG, quad, stg + 2 * kAStageBytes, d_lo, d_im);
+        const double *pos = reinterpret_cast<const double *>(smem + G.pos + nbuf * kTcPosBytes) + j * kTcNodes;
+#pragma unroll 1
+        for (int n = 0; n < 16; n += 8) {
+          const uint32_t addr = stg + (n ? row_off1 : row_off);
+          if (stacked) tc_write_a<true>(pos + n, kd, wp + a_drow + n, addr, d_k2);
+          else tc_write_a<false>(pos + n, kd, nullptr, addr, d_k2);
+        }
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_n(&bars->full[r.slot], arrive);
+        if (st + a_groups >= nst || (st + a_groups) / kTcStagesPerBlock > blk) release();
+        r.advance(a_groups, ring);
+      }
+    } else {
+      // the B tile of every b_groups-th stage, or a node half of it: lanes hold
+      // the columns q, 32 at a time, or up to 16 of them and both node halves
+      const int grp = (warp - nA) / b_per, half0 = both ? lane >> 4 : (warp - nA) - grp * b_per;
+      const int lq = both ? lane & 15 : lane, half_step = both ? 2 : b_per;
+      r.seek(stage0 + grp, ring);
+      for (int st = grp; st < nst && grp < b_groups; st += b_groups) {
+        if (drains) fold_before(st);
+        acquire(st / kTcStagesPerBlock);
+        tc_wait(&bars->empty[r.slot], r.phase ^ 1, abort_flag);
+        const uint32_t j = st & (kTcStagesPerBlock - 1);
+        const uint32_t b_tile = stages + r.slot * stage_bytes + 2 * kAStageBytes;
+        const double *pos = reinterpret_cast<const double *>(smem + G.pos + nbuf * kTcPosBytes) + j * kTcNodes;
+        const float *wblk = w_all + nbuf * G.wrows * 2 * kWStride;
+#pragma unroll 1
+        for (int q0 = 0; q0 < Q_tile; q0 += 32) {
+          // lanes past the tile repeat its last column and write nothing
+          const int q = min(q0 + lq, Q_tile - 1);
+          const bool mine = q0 + lq < Q_tile;
+          double kd[kTcComps] = {0, 0, 0, 0};
+          if (runs) {
+            const int s_q = p.start[U.it.q0 + q];
+            kd[0] = cmask & 1 ? (double)p.kx[s_q] : 0.0;
+            kd[1] = cmask & 2 ? (double)p.ky[s_q] : 0.0;
+            kd[2] = cmask & 4 ? (double)p.kz[s_q] : 0.0;
+            kd[3] = p.run_t[U.it.q0 + q];
+          } else {
+            const int s_q = U.start + U.it.q0 + q;
+            kd[0] = (double)p.kx[s_q] - (double)p.kx[U.start];
+            kd[1] = (double)p.ky[s_q] - (double)p.ky[U.start];
+            kd[2] = (double)p.kz[s_q] - (double)p.kz[U.start];
+          }
+          kmax = max(kmax, tc_abs_sum(kd[0], kd[1], kd[2]));
+#pragma unroll 1
+          for (int half = half0; half < 2; half += half_step) {
+            if (!mine) continue;
+            const int n0 = j * kTcNodes + 8 * half;
+            if (runs) tc_write_b<true>(pos + 8 * half, kd, wblk, n0, VG, q, Qt, half, b_tile, d_lo, d_im);
+            else tc_write_b<false>(pos + 8 * half, kd, wblk, n0, VG, q, Qt, half, b_tile, d_lo, d_im);
+          }
+        }
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->full[r.slot]);
+        if (st + b_groups >= nst || (st + b_groups) / kTcStagesPerBlock > blk) release();
+        r.advance(b_groups, ring);
+      }
+    }
+    while (blk < n_blocks - 1) {  // blocks past this warp's last stage
+      if (drains) fold_before((blk + 1) * kTcStagesPerBlock);
+      acquire(blk + 1);
+      release();
+    }
+    // the groups that no later stage of this warp led to fold: the MMAs, and
+    // with them the other warps, may wait for them
+    if (drains) fold_before(nst + kTcDrain + (int)ring);
+    // every warp has written its stages of this unit, so that none starts the
+    // next unit's turns more than a round of the ring ahead of the MMAs
+    ptx::named_barrier(2, 32 * kTcOperandWarps);
+    // every phase of the unit had |k . r| <= kmax rmax: the fixed-point
+    // reduction holds below 2^28 cycles (2^27 leaves a margin)
+    if (kmax >= 0 && !((double)__int_as_float(kmax) * (double)__int_as_float(rmax) < 134217728.0))
+      atomicOr(p.ctl + kCtlError, kErrPhaseRange);
+    if (drains) {
+      if (nst > 0) {
+        tc_wait(&bars->accfull, (group0 + folded) & 1, abort_flag);
+        __syncwarp();
+        // the unit read again, rather than kept in registers over the loops
+        const TcWork Wf = tc_work(p);
+        tc_final(p, Wf, tc_unit(p, Wf, u - B.offsets[e]), tmem, folded > 0);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->accfree);
+      } else if (warp < 4 && warp * 32 + lane < U.rows) {
+        // no nodes in this split: its share of the tile is zero
+        const TcWork W = tc_work(p);
+        float2 *dst = W.out + (int64_t)U.split * p.S * p.V;
+        int64_t s_row, s_q;
+        tc_out_sample(p, U, warp * 32 + lane, s_row, s_q);
+        for (int q = 0; q < Q_tile; ++q)
+          for (int v = 0; v < VG; ++v) dst[(s_row + q * s_q) * p.V + p.v0 + v] = make_float2(0.f, 0.f);
+      }
+    }
+    stage0 += nst;
+    group0 += U.n_groups;
+  }
+}
+
 __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_constant__ TcBatchDev B) {
   extern __shared__ __align__(1024) unsigned char smem[];
   // work sizes come from the device-side plan, so the launch needs no host
   // synchronisation (and can be captured in a CUDA graph)
   const int n_units = B.offsets[B.n_entries];
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  uint64_t *empty = reinterpret_cast<uint64_t *>(smem + kTcBars);
-  uint64_t *gempty = empty + kTcStages;  // the generic ring's slots
-  uint64_t *accfull = gempty + kTcRingGen;
-  uint64_t *done = accfull + 1;
-  uint64_t *rawfull = done + 1;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kTcMisc);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kTcMisc + 4);
-  // largest |kx|+|ky|+|kz| of the unit's phases and |x|+|y|+|z| of its moved
-  // nodes (float bits), for the check that the fixed-point phase reduction
-  // applies (cycles_cos_sin)
-  int *kmax = reinterpret_cast<int *>(smem + kTcMisc + 8);
-  int *rmax = reinterpret_cast<int *>(smem + kTcMisc + 12);
-  const uint32_t sbase = ptx::smem_addr(smem);
-
+  const int tid = threadIdx.x, warp = tid >> 5;
+  TcBars *bars = reinterpret_cast<TcBars *>(smem);
+  TcMisc *misc = reinterpret_cast<TcMisc *>(smem + kTcMisc);
+  volatile int *abort_flag = &misc->abort_flag;
   if (tid == 0) {
-    for (int s = 0; s < kTcStages + kTcRingGen; ++s) ptx::mbar_init(&empty[s], 1);
-    ptx::mbar_init(accfull, 1);
-    ptx::mbar_init(done, 1);
-    ptx::mbar_init(rawfull, 1);
-    *abort_flag = 0;
-    *kmax = 0;
-    *rmax = 0;
+    for (int s = 0; s < kTcMaxRing; ++s) {
+      ptx::mbar_init(&bars->full[s], kTcStageArrivals);
+      ptx::mbar_init(&bars->empty[s], 1);
+    }
+    ptx::mbar_init(&bars->accfull, 1);
+    ptx::mbar_init(&bars->accfree, kTcDrainWarps);
+    for (int b = 0; b < kTcMaxNodeBufs; ++b) {
+      ptx::mbar_init(&bars->nodefull[b], 1);
+      ptx::mbar_init(&bars->nodeempty[b], kTcOperandWarps);
+    }
+    for (int b = 0; b < 2; ++b) ptx::mbar_init(&bars->rawfull[b], 1);
+    ptx::mbar_init(&bars->done, 1);
+    misc->abort_flag = 0;
     ptx::fence_mbar_init();
   }
-  if (warp == 0) ptx::tmem_alloc(tmem_slot, kTcTmemCols);
+  if (warp == 0) ptx::tmem_alloc(&misc->tmem, kTcTmemCols);
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = tmem_slot[0];
-
-  // Roles (warp-uniform).  Warps 0-7 write A: rows 32 (w >> 1) + lane, nodes
-  // 8 (w & 1) .. + 7 of every stage.  Warps 8-15 write B: pairs
-  // 32 ((w - 8) >> 1) + lane, same node halves, and the next stage's phase
-  // table.  Threads 0-127 also derive the node blocks.  One thread of warp 7
-  // issues a stage's MMAs after the block barrier that follows the stage
-  // (every writer has fenced its stores to the async proxy by then).  Both
-  // roles pass the same barriers and drains in the same order.
-  const bool a_role = warp < 8;
-  const int rw = a_role ? warp : warp - 8;
-  const int row = (rw >> 1) * 32 + lane;  // A row or B pair
-  const int half = rw & 1;                // nodes 8 half .. 8 half + 7 of a stage
-  const bool loader = tid < kTcBlockNodes;
-  const bool issuer = tid == 7 * 32;  // lane 0 of warp 7: the thread that issues every MMA
-  // phase-table thread: q = (tid - 256) / 8 (+ 32), nodes 2 ((tid - 256) % 8) + {0, 1}
-  const int tq = (tid - 256) >> 3, tn = ((tid - 256) & 7) * 2;
-  uint32_t gst = 0, raw_seq = 0;
-  uint32_t gsg = 0;  // stages of generic units so far (their ring's counter)
-  int gbase = 0;
-  TcRaw raw;
-  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-    // the unit's entry: offsets[e] <= u < offsets[e + 1]
-    int e_lo = 0, e_hi = B.n_entries;
-    while (e_hi - e_lo > 1) {
-      const int mid = (e_lo + e_hi) >> 1;
-      if (B.offsets[mid] <= u) e_lo = mid; else e_hi = mid;
-    }
-    const TcDev &p = B.entries[e_lo];
-    const TcWork W = tc_work(p);
-    const int NT = p.NT, NH = NT >> 1, VG = p.VG, Qt = p.Qt, WR = p.wrows;
-    const TcSmem L = tc_smem_layout(NT, WR, Qt, p.kind == 0 ? kTcStages : kTcRingGen);
-    double *pos_all = reinterpret_cast<double *>(smem + L.pos);
-    float2 *w_all = reinterpret_cast<float2 *>(smem + L.w);
-    float2 *etab = reinterpret_cast<float2 *>(smem + L.etab);
-    const uint32_t sstages = sbase + L.stages;
-    const uint32_t idesc = ptx::idesc_bf16_f32(kTcRows, NT);
-    // operand addresses inside a stage: the thread's first 8-K chunk; the
-    // second chunk is d_k2 = +/-16 bytes from it (swizzled chunk positions
-    // 2 half and 2 half + 1 differ in their lowest bit), the lo tile d_lo
-    // bytes on and (B) the imaginary row block d_im bytes on
-    const uint32_t o_hi = (a_role ? L.a_hi : L.b_hi) + sw64_offset(row, 16 * half);
-    const int d_k2 = ((((2 * half) ^ (row >> 1)) & 1) != 0) ? -16 : 16;
-    const uint32_t d_lo = a_role ? L.a_lo - L.a_hi : L.b_lo - L.b_hi;
-    const uint32_t d_im = (uint32_t)NH * 64;
-    const bool b_rows = row < NH;
-    const TcUnit U = tc_unit(p, W, u - B.offsets[e_lo]);
-    const bool fac = U.run.factored != 0;
-    const uint32_t nst = (uint32_t)U.n_stages;
-    ptx::named_barrier(1, kTcProducers);  // the previous unit's readers are done
-    // per-unit row data in registers
-    double kx0 = 0, ky0 = 0, kz0 = 0, kx1 = 0, ky1 = 0, kz1 = 0;  // A: kp of the row; B: kq of q and q + 32
-    int bq = 0, bw = 0;  // B: phase-table row and weight row of the pair
-    int a_drow = 0;      // A of a stacked unit: the row's D row in the node buffer
-    if (a_role) {
-      if (row < U.rows) {
-        // the row's run (r = 0 unless stacked) and line
-        int r, line;
-        tc_row_line(p, U, row, r, line);
-        a_drow = VG + r;
-        const int start = r == 0 ? U.run.start : p.start[U.it.run + r];
-        const int s_p = start + (fac ? line * p.n_kz : line);
-        kx0 = p.kx[s_p];
-        ky0 = p.ky[s_p];
-        kz0 = p.kz[s_p];
-        if (nst > 0) tc_note_k(kmax, kx0, ky0, kz0);
-      }
-    } else {
-      if (row < U.pairs) {
-        bq = row / VG;
-        bw = row % VG;
-      }
-      if (fac) {
-        const int s_0 = U.run.start;
-        if (tq < U.Q_tile) {
-          const int s_q = U.run.start + U.it.q0 + tq;
-          kx0 = (double)p.kx[s_q] - (double)p.kx[s_0];
-          ky0 = (double)p.ky[s_q] - (double)p.ky[s_0];
-          kz0 = (double)p.kz[s_q] - (double)p.kz[s_0];
-          if (nst > 0) tc_note_k(kmax, kx0, ky0, kz0);
-        }
-        if (tq + 32 < U.Q_tile) {
-          const int s_q = U.run.start + U.it.q0 + tq + 32;
-          kx1 = (double)p.kx[s_q] - (double)p.kx[s_0];
-          ky1 = (double)p.ky[s_q] - (double)p.ky[s_0];
-          kz1 = (double)p.kz[s_q] - (double)p.kz[s_0];
-          if (nst > 0) tc_note_k(kmax, kx1, ky1, kz1);
-        }
-      }
-    }
-    const bool t_on0 = !a_role && fac && tq < U.Q_tile, t_on1 = !a_role && fac && tq + 32 < U.Q_tile;
-    const float *wrun = p.weights ? p.weights + (int64_t)U.it.run * p.md.slots : nullptr;
-    const uint32_t n_blocks = (nst + kTcStagesPerBlock - 1) / kTcStagesPerBlock;
-    // prologue: node block 0 into buffer 0
-    if (loader && nst > 0) {
-      const int64_t n = U.n_begin + tid;
-      if (n < U.n_end) tc_load_raw(p, n, raw);
-      tc_derive(p, U, n, raw, wrun, pos_all, w_all, tid, rmax);
-    }
-    ptx::named_barrier(1, kTcProducers);  // block 0 is visible
-    // phase tables of the first group's stages (block 0, buffers 0 ..)
-    for (uint32_t st = 0; st < kTcFacGroup && st < nst; ++st) {
-      float2 *et = etab + st * Qt * kEStride;
-      if (t_on0) tc_phase_pair(pos_all + st * kTcNodes, et, tq, tn, kx0, ky0, kz0);
-      if (t_on1) tc_phase_pair(pos_all + st * kTcNodes, et, tq + 32, tn, kx1, ky1, kz1);
-    }
-    // the first group's tables are read by other warps than their writers
-    if (fac) ptx::named_barrier(1, kTcProducers);
-    const uint32_t g0 = gst, gg0 = gsg;
-    int next_drain = 0;
-    if (!fac) {
-      // ------------------------------------------- generic unit, all warps --
-      // B is only the weights of the unit's VG columns (NT = 16), so every
-      // warp writes A: rows 32 (w % 4) + lane, nodes 4 (w / 4) .. + 3 of a
-      // stage; threads 0-127 also write one B element (pair tid % 8, node
-      // tid / 8).  Pairs past VG hold values no output reads.
-      const int grow = (warp & 3) * 32 + lane, gc = warp >> 2;
-      double gx = 0, gy = 0, gz = 0;
-      if (grow < U.P_tile) {
-        const int s_p = U.run.start + U.it.p0 + grow;
-        gx = p.kx[s_p];
-        gy = p.ky[s_p];
-        gz = p.kz[s_p];
-        if (nst > 0) tc_note_k(kmax, gx, gy, gz);
-      }
-      const bool g_active = (warp & 3) * 32 < U.P_tile;
-      const uint32_t ga0 = L.a_hi + sw64_offset(grow, 8 * gc);
-      const uint32_t gl0 = L.a_lo + sw64_offset(grow, 8 * gc);
-      const int gpair = tid & 7, gnode = tid >> 3;
-      const bool g_b = tid < kTcRows && gpair < NH;
-      const int gv = gpair < VG ? gpair : 0;
-      const uint32_t gbr = sw64_offset(gpair, 2 * gnode), gbi = sw64_offset(NH + gpair, 2 * gnode);
-      // The MMAs of a generic stage are small (N = 16), so the producers
-      // write kTcGenGroup stages between barriers and the issuer sends them
-      // together: one barrier per group instead of one per stage.  Groups
-      // divide the 8-stage node blocks, so a block derived at stage 6 is
-      // visible after its group's barrier, before any stage of it is read.
-      for (uint32_t sg = 0; sg < nst; sg += kTcGenGroup) {
-        const uint32_t s_end = min(nst, sg + (uint32_t)kTcGenGroup);
-        for (uint32_t st = sg; st < s_end; ++st) {
-          const uint32_t g = gg0 + st, s = g & (kTcRingGen - 1);
-          const uint32_t j = st & (kTcStagesPerBlock - 1), blk = st / kTcStagesPerBlock, buf = blk & 1;
-          if (loader && blk + 1 < n_blocks && (j == 0 || j == 4))
-            tc_stage_block<kModes>(p, U, tid, blk, j == 0, raw, raw_seq, smem + L.raw, rawfull, wrun,
-                           pos_all + (buf ^ 1) * 3 * kTcBlockNodes, w_all + (buf ^ 1) * WR * kWStride, abort_flag,
-                           rmax);
-          // the MMAs that last read stage s were sent at an earlier barrier
-          tc_wait(&gempty[s], ((g / kTcRingGen) & 1) ^ 1, abort_flag);
-          const uint32_t stg = sstages + s * L.stage_bytes;
-          if (g_active) {
-            const double *px = pos_all + buf * 3 * kTcBlockNodes + j * kTcNodes + 4 * gc;
-            uint32_t h[4], l[4];
-#pragma unroll
-            for (int u4 = 0; u4 < 4; u4 += 2) {
-              const double2 x = *reinterpret_cast<const double2 *>(px + u4);
-              const double2 y = *reinterpret_cast<const double2 *>(px + kTcBlockNodes + u4);
-              const double2 z = *reinterpret_cast<const double2 *>(px + 2 * kTcBlockNodes + u4);
-              float c0, s0, c1, s1;
-              cycles_cos_sin(fma(gz, z.x, fma(gy, y.x, gx * x.x)), c0, s0);
-              cycles_cos_sin(fma(gz, z.y, fma(gy, y.y, gx * x.y)), c1, s1);
-              split_pair(c0, s0, h[u4], l[u4]);
-              split_pair(c1, s1, h[u4 + 1], l[u4 + 1]);
-            }
-            st_shared_v4(stg + ga0, h[0], h[1], h[2], h[3]);
-            st_shared_v4(stg + gl0, l[0], l[1], l[2], l[3]);
-          }
-          if (g_b) {
-            const float2 wv = w_all[(buf * WR + gv) * kWStride + j * kTcNodes + gnode];
-            uint32_t hb, lb;
-            split_pair(wv.x, wv.y, hb, lb);
-            const uint32_t hm = __byte_perm(hb, 0u, 0x1032) ^ 0x80000000u, lm = __byte_perm(lb, 0u, 0x1032) ^ 0x80000000u;
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + L.b_hi + gbr), "r"(hb));
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + L.b_lo + gbr), "r"(lb));
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + L.b_hi + gbi), "r"(hm));
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + L.b_lo + gbi), "r"(lm));
-          }
-        }
-        ptx::fence_proxy_async_smem();
-        // every writer of the group is done: its MMAs go out now
-        ptx::named_barrier(1, kTcProducers);
-        if (warp == 7) {
-          ptx::tc_fence_after();
-          for (uint32_t st = sg; st < s_end; ++st)
-            tc_issue<false>(L, sbase, tmem, idesc, NT, gempty, accfull, (gg0 + st) & (kTcRingGen - 1), st, nst, lane);
-        }
-        // an accumulation group ended with this group: fold it before the
-        // next group's MMAs (which go out at the next barrier)
-        if (s_end < nst && (s_end & (kTcDrain - 1)) == 0) {
-          tc_fold(p, accfull, tmem, gbase + next_drain, next_drain == 0, abort_flag);
-          ++next_drain;
-        }
-      }
-    } else if (a_role) {
-      // ------------------------------------------------------- A rows --
-      // kTcFacGroup stages between barriers; the group's MMAs go out at its
-      // barrier.  Node block blk + 1 is requested at j == 2 and derived at
-      // j == 4 into the other buffer: that buffer's readers (block blk - 1)
-      // are done, and the phase tables of block blk + 1's first stages are
-      // computed after the barrier that ends the derive's group.
-      const bool active = (rw >> 1) * 32 < U.rows;
-      for (uint32_t sg = 0; sg < nst; sg += kTcFacGroup) {
-        const uint32_t s_end = min(nst, sg + (uint32_t)kTcFacGroup);
-        // a group's stages lie in one node block (groups divide the blocks)
-        const uint32_t jg = sg & (kTcStagesPerBlock - 1), blk = sg / kTcStagesPerBlock, buf = blk & 1;
-        if (loader && blk + 1 < n_blocks && (jg == 2 || jg == 4))
-          tc_stage_block<kModes>(p, U, tid, blk, jg == 2, raw, raw_seq, smem + L.raw, rawfull, wrun,
-                         pos_all + (buf ^ 1) * 3 * kTcBlockNodes, w_all + (buf ^ 1) * WR * kWStride, abort_flag,
-                         rmax);
-        tc_wait_group(empty, g0 + s_end - 1, abort_flag);
-#pragma unroll
-        for (uint32_t i = 0; i < (uint32_t)kTcFacGroup; ++i) {
-          const uint32_t st = sg + i;
-          if (st >= s_end) break;
-          const uint32_t s = (g0 + st) & (kTcStages - 1), j = jg + i;
-          if (active) {
-            // A'[row][2n..2n+1] = (Re A, -Im A) = (cos, sin) of 2 pi kp . r_n;
-            // in a stacked unit A is multiplied by the row's run factor D_r(n):
-            // (Re, -Im) of (cos - i sin)(dr + i di) = (cos dr + sin di, sin dr - cos di)
-            const uint32_t stg = sstages + s * L.stage_bytes;
-            const double *px = pos_all + buf * 3 * kTcBlockNodes + j * kTcNodes + 8 * half;
-            uint32_t h[8], l[8];
-            if (p.stacked) {
-              const float4 *dp = reinterpret_cast<const float4 *>(w_all + (buf * WR + a_drow) * kWStride +
-                                                                  j * kTcNodes + 8 * half);
-#pragma unroll
-              for (int u4 = 0; u4 < 8; u4 += 2) {
-                const double2 x = *reinterpret_cast<const double2 *>(px + u4);
-                const double2 y = *reinterpret_cast<const double2 *>(px + kTcBlockNodes + u4);
-                const double2 z = *reinterpret_cast<const double2 *>(px + 2 * kTcBlockNodes + u4);
-                float c0, s0, c1, s1;
-                cycles_cos_sin(fma(kz0, z.x, fma(ky0, y.x, kx0 * x.x)), c0, s0);
-                cycles_cos_sin(fma(kz0, z.y, fma(ky0, y.y, kx0 * x.y)), c1, s1);
-                const float4 d = dp[u4 >> 1];
-                split_pair(fmaf(c0, d.x, s0 * d.y), fmaf(s0, d.x, -(c0 * d.y)), h[u4], l[u4]);
-                split_pair(fmaf(c1, d.z, s1 * d.w), fmaf(s1, d.z, -(c1 * d.w)), h[u4 + 1], l[u4 + 1]);
-              }
-            } else {
-#pragma unroll
-              for (int u4 = 0; u4 < 8; u4 += 2) {
-                const double2 x = *reinterpret_cast<const double2 *>(px + u4);
-                const double2 y = *reinterpret_cast<const double2 *>(px + kTcBlockNodes + u4);
-                const double2 z = *reinterpret_cast<const double2 *>(px + 2 * kTcBlockNodes + u4);
-                float c0, s0, c1, s1;
-                cycles_cos_sin(fma(kz0, z.x, fma(ky0, y.x, kx0 * x.x)), c0, s0);
-                cycles_cos_sin(fma(kz0, z.y, fma(ky0, y.y, kx0 * x.y)), c1, s1);
-                split_pair(c0, s0, h[u4], l[u4]);
-                split_pair(c1, s1, h[u4 + 1], l[u4 + 1]);
-              }
-            }
-            const uint32_t a_st = stg + o_hi;
-            st_shared_v4(a_st, h[0], h[1], h[2], h[3]);
-            st_shared_v4(a_st + d_k2, h[4], h[5], h[6], h[7]);
-            st_shared_v4(a_st + d_lo, l[0], l[1], l[2], l[3]);
-            st_shared_v4(a_st + d_lo + d_k2, l[4], l[5], l[6], l[7]);
-          }
-        }
-        ptx::fence_proxy_async_smem();
-        // every writer of the group is done (and its phase tables of the next
-        // group are visible after this barrier): its MMAs go out now
-        ptx::named_barrier(1, kTcProducers);
-        if (warp == 7)
-          for (uint32_t st = sg; st < s_end; ++st)
-            tc_issue<true>(L, sbase, tmem, idesc, NT, empty, accfull, (g0 + st) % kTcStages, st, nst, lane);
-        // an accumulation group ended with this group: fold it before the
-        // next group's MMAs go out
-        if (s_end < nst && (s_end & (kTcDrain - 1)) == 0) {
-          tc_fold(p, accfull, tmem, gbase + next_drain, next_drain == 0, abort_flag);
-          ++next_drain;
-        }
-      }
-    } else {
-      // ------------------------------------------------------- B rows --
-      for (uint32_t sg = 0; sg < nst; sg += kTcFacGroup) {
-        const uint32_t s_end = min(nst, sg + (uint32_t)kTcFacGroup);
-        const uint32_t jg = sg & (kTcStagesPerBlock - 1), buf = (sg / kTcStagesPerBlock) & 1;
-        tc_wait_group(empty, g0 + s_end - 1, abort_flag);
-#pragma unroll
-        for (uint32_t i = 0; i < (uint32_t)kTcFacGroup; ++i) {
-          const uint32_t st = sg + i;
-          if (st >= s_end) break;
-          const uint32_t s = (g0 + st) & (kTcStages - 1), j = jg + i;
-          // B'^T rows: re row `row` = (Re B, Im B), im row NT/2 + row =
-          // (Im B, -Re B), B = e_q(n) W'(n, v).  Pairs past Q_tile VG hold
-          // values no output reads.  Threads past the tile's NT/2 pairs have
-          // no B element (their warps only take part in the phase table).
-          if (b_rows) {
-          const float4 *wp =
-              reinterpret_cast<const float4 *>(w_all + (buf * WR + bw) * kWStride + j * kTcNodes + 8 * half);
-          float br[8], bi[8];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 w2 = wp[i];
-            br[2 * i] = w2.x; bi[2 * i] = w2.y; br[2 * i + 1] = w2.z; bi[2 * i + 1] = w2.w;
-          }
-          {
-            const float4 *ep = reinterpret_cast<const float4 *>(etab + ((st & (kTcEBufs - 1)) * Qt + bq) * kEStride +
-                                                                8 * half);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 e2 = ep[i];
-              const float wr0 = br[2 * i], wi0 = bi[2 * i], wr1 = br[2 * i + 1], wi1 = bi[2 * i + 1];
-              br[2 * i] = e2.x * wr0 - e2.y * wi0;
-              bi[2 * i] = e2.x * wi0 + e2.y * wr0;
-              br[2 * i + 1] = e2.z * wr1 - e2.w * wi1;
-              bi[2 * i + 1] = e2.z * wi1 + e2.w * wr1;
-            }
-          }
-          uint32_t hr[8], lr[8], hm[8], lm[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            split_pair(br[i], bi[i], hr[i], lr[i]);
-            hm[i] = __byte_perm(hr[i], 0u, 0x1032) ^ 0x80000000u;
-            lm[i] = __byte_perm(lr[i], 0u, 0x1032) ^ 0x80000000u;
-          }
-          {
-            const uint32_t stg = sstages + s * L.stage_bytes;
-            const uint32_t b_st = stg + o_hi;
-            st_shared_v4(b_st, hr[0], hr[1], hr[2], hr[3]);
-            st_shared_v4(b_st + d_k2, hr[4], hr[5], hr[6], hr[7]);
-            st_shared_v4(b_st + d_lo, lr[0], lr[1], lr[2], lr[3]);
-            st_shared_v4(b_st + d_lo + d_k2, lr[4], lr[5], lr[6], lr[7]);
-            st_shared_v4(b_st + d_im, hm[0], hm[1], hm[2], hm[3]);
-            st_shared_v4(b_st + d_im + d_k2, hm[4], hm[5], hm[6], hm[7]);
-            st_shared_v4(b_st + d_im + d_lo, lm[0], lm[1], lm[2], lm[3]);
-            st_shared_v4(b_st + d_im + d_lo + d_k2, lm[4], lm[5], lm[6], lm[7]);
-          }
-          }  // b_rows
-          // the phase table of stage st + kTcFacGroup (next group) into its
-          // buffer, whose last readers (stage st - kTcFacGroup) are past the
-          // previous group's barrier
-          if (t_on0 && st + kTcFacGroup < nst) {
-            const uint32_t st1 = st + kTcFacGroup;
-            const double *pb = pos_all + ((st1 / kTcStagesPerBlock) & 1) * 3 * kTcBlockNodes +
-                               (st1 & (kTcStagesPerBlock - 1)) * kTcNodes;
-            float2 *et = etab + (st1 & (kTcEBufs - 1)) * Qt * kEStride;
-            tc_phase_pair(pb, et, tq, tn, kx0, ky0, kz0);
-            if (t_on1) tc_phase_pair(pb, et, tq + 32, tn, kx1, ky1, kz1);
-          }
-        }
-        ptx::fence_proxy_async_smem();
-        ptx::named_barrier(1, kTcProducers);
-        if (s_end < nst && (s_end & (kTcDrain - 1)) == 0) {
-          tc_fold(p, accfull, tmem, gbase + next_drain, next_drain == 0, abort_flag);
-          ++next_drain;
-        }
-      }
-    }
-    if (fac) gst = g0 + nst;
-    else gsg = gg0 + nst;
-    if (nst > 0) {
-      ptx::named_barrier(1, kTcProducers);  // the unit's last stage is written
-      if (tid == 0) {
-        // every phase of the unit had |k . r| <= kmax rmax: the fixed-point
-        // reduction holds below 2^28 cycles (2^27 leaves a margin)
-        if (!((double)__int_as_float(*kmax) * (double)__int_as_float(*rmax) < 134217728.0))
-          atomicOr(p.ctl + kCtlError, kErrPhaseRange);
-        *kmax = 0;
-        *rmax = 0;
-      }
-    }
-    if (U.n_groups > 0) tc_final(p, W, U, accfull, tmem, gbase + U.n_groups - 1, U.n_groups > 1, abort_flag);
-    if (U.n_groups == 0 && tid < U.rows) {
-      // no nodes in this split: its share of the tile is zero
-      float2 *dst = W.out + (int64_t)U.split * p.S * p.V;
-      int r, line;
-      tc_row_line(p, U, tid, r, line);
-      const int start = p.start[U.it.run + r];
-      const int s_row = start + (fac ? line * p.n_kz + U.it.q0 : line);
-      for (int q = 0; q < U.Q_tile; ++q)
-        for (int v = 0; v < VG; ++v) dst[(int64_t)(s_row + q) * p.V + p.v0 + v] = make_float2(0.f, 0.f);
-    }
-    gbase += U.n_groups;
-  }
-  if (issuer) {
-    // all issued MMAs complete before the tensor memory is released
-    ptx::mma_commit(done);
-    if (!ptx::mbar_wait(done, 0, kTcWaitNs)) *abort_flag = 1;
-  }
+  const uint32_t tmem = *(volatile uint32_t *)&misc->tmem;
+  const uint32_t stages = ptx::smem_addr(smem) + kTcFront;
+  if (warp == kTcMmaWarp) tc_role_mma(B, bars, stages, tmem, n_units, abort_flag);
+  else if (warp >= kTcNodeWarp) tc_role_nodes(B, bars, misc, smem, n_units, abort_flag);
+  else tc_role_operands(B, bars, misc, smem, stages, tmem, n_units, abort_flag);
   ptx::tc_fence_before();
   __syncthreads();
   // a wait that ran out is reported for every problem of the launch
@@ -1169,20 +1261,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) signal_tc_kernel(const __grid_c
 
 // ---- plan --------------------------------------------------------------
 
-// Node-range splits: enough work units that the persistent blocks finish
-// together (units per block close to an integer), each split at least 2048
-// nodes; fewer splits win ties.
-__host__ __device__ inline int tc_choose_splits(int64_t items, int64_t N, int max_splits) {
+// Node-range splits: the least estimated time of the persistent blocks, in
+// stages: rounds of units times a unit's stages plus its set-up and write
+// (about 12 stages), and the partial sums written and read back (a stage, about
+// 0.4 us, moves some 2.6 MB).  Splits of at least 128 nodes (one node block).
+__host__ __device__ inline int tc_choose_splits(int64_t items, int64_t N, int64_t outputs, int max_splits) {
   if (items <= 0) return 1;
   int best = 1;
-  double best_eff = -1.0;
+  double best_cost = 0.0;
   for (int s = 1; s <= max_splits; ++s) {
-    if (s > 1 && ceil_div(N, s) < 2048) break;
-    const double units = (double)items * s;
-    const double per_block = units / kSmCount;
-    const double eff = per_block / ceil(per_block) * (units < kSmCount ? units / kSmCount : 1.0);
-    if (eff > best_eff + 0.02) {
-      best_eff = eff;
+    if (s > 1 && ceil_div(N, s) < kTcBlockNodes) break;
+    const double rounds = (double)ceil_div(items * s, (int64_t)kSmCount);
+    const double cost = rounds * ((double)ceil_div(ceil_div(N, s), kTcNodes) + 12.0) +
+                        (s > 1 ? s * (double)outputs * 16.0 / 2.6e6 : 0.0);
+    if (s == 1 || cost < best_cost) {
+      best_cost = cost;
       best = s;
     }
   }
@@ -1207,7 +1300,7 @@ __global__ void __launch_bounds__(kTcPlanThreads) tc_plan_kernel(const TcDev *__
     } else {
       int64_t items = 0;
       for (int k = 0; k < p.n_of; ++k) items += tc_n_items(entries[e + k]);
-      splits = tc_choose_splits(items, p.N, p.max_splits);
+      splits = tc_choose_splits(items, p.N, p.S * p.V, p.max_splits);
     }
     p.ctl[kCtlSplits] = splits;
     p.ctl[kCtlChunk] = (int)(ceil_div(ceil_div(p.N, splits), kTcNodes) * kTcNodes);
@@ -1278,11 +1371,13 @@ struct TcPlan {
   int n_groups, max_splits;
 };
 
+// Most node splits of a problem: 16 while their partial sums stay within a
+// gigabyte, more for small outputs (up to 64 in 32 MB), which have few units.
 static int tc_max_splits(int64_t S, int64_t V) {
   const int64_t bytes_per = S * V * 8;
-  int64_t s = bytes_per > 0 ? (1LL << 30) / bytes_per : 16;
-  if (s > 16) s = 16;
-  return (int)(s < 1 ? 1 : s);
+  if (bytes_per <= 0) return 1;
+  const int64_t s = std::min<int64_t>(16, (1LL << 30) / bytes_per), small = std::min<int64_t>(64, (32LL << 20) / bytes_per);
+  return (int)std::max<int64_t>(1, std::max(s, small));
 }
 
 static int tc_groups(int64_t V) { return (int)ceil_div(V, (int64_t)kTcVGroup); }
@@ -1298,7 +1393,7 @@ static void carve_tc(Carve &c, const fm_signal_args *a, int *ctl, TcPlan &pl) {
 // Entries of a launch: per problem, per column group, both run kinds.
 static int tc_n_entries(const fm_signal_args *probs, int n) {
   int e = 0;
-  for (int i = 0; i < n; ++i) e += 2 * tc_groups(probs[i].n_vencs);
+  for (int i = 0; i < n; ++i) e += kTcKinds * tc_groups(probs[i].n_vencs);
   return e;
 }
 
@@ -1323,20 +1418,35 @@ static void carve_batch(Carve &c, const fm_signal_args *probs, int n, TcBatchPla
 
 // Tile shape of a column group: up to 128 (q, v) pairs per tile and at most
 // 64 kz values (fewer when tuned).
-static void tc_shape(int Qt, int VG, int &NT, int &acc_cols);
-
 static int tc_qt(const fm_signal_args *a, int VG, const fm_tc_tuning *tune) {
   int cap = (128 / VG < 64) ? 128 / VG : 64;
   if (tune && tune->kz_cap > 0 && tune->kz_cap < cap) cap = tune->kz_cap;
-  int Qt = (int)((a->n_kz < cap) ? a->n_kz : cap);
-  // narrower tiles until the tiles, node buffers and phase-table ring fit in
-  // shared memory (stacked runs are limited to what then fits)
-  for (;;) {
-    int NT, acc;
-    tc_shape(Qt, VG, NT, acc);
-    if (Qt <= 8 || tc_smem_layout(NT, VG, Qt).total <= kTcSmemMax) return Qt;
-    Qt -= 8;
-  }
+  return (int)((a->n_kz < cap) ? a->n_kz : cap);
+}
+
+// Columns of a tile of Qt VG pairs: real and imaginary parts.
+static int tc_nt(int Qt, int VG) { return (int)ceil_div(2 * Qt * VG, 16) * 16; }
+
+// Layout of a launch for stages of `stage_bytes`, `wrows` weight rows per node
+// buffer and staging areas of raw_bytes each (ring 0 when min_ring stages and
+// two node buffers do not fit).
+static TcGeom tc_geom(uint32_t stage_bytes, uint32_t wrows, uint32_t raw_bytes, uint32_t min_ring = kTcMinRing) {
+  TcGeom g{};
+  g.stage_bytes = stage_bytes;
+  g.wrows = wrows;
+  g.raw_bytes = (raw_bytes + 127) & ~127u;
+  const uint32_t buf = kTcPosBytes + wrows * 2 * kWStride * 4;
+  const uint32_t fixed = kTcFront + 2 * g.raw_bytes;
+  // as many node buffers as leave room for min_ring stages, then the stages
+  for (g.node_bufs = kTcMaxNodeBufs; g.node_bufs >= kTcMinNodeBufs; --g.node_bufs)
+    if (fixed + g.node_bufs * buf + min_ring * stage_bytes <= kTcSmemMax) break;
+  if (g.node_bufs < kTcMinNodeBufs) return g;
+  g.ring = std::min<uint32_t>(kTcMaxRing, (kTcSmemMax - fixed - g.node_bufs * buf) / stage_bytes);
+  g.pos = kTcFront + g.ring * stage_bytes;
+  g.w = g.pos + g.node_bufs * kTcPosBytes;
+  g.raw = g.w + g.node_bufs * wrows * 2 * kWStride * 4;
+  g.total = g.raw + 2 * g.raw_bytes;
+  return g;
 }
 
 // Runs a stacked unit may touch, for a column group: stacking needs whole
@@ -1353,9 +1463,7 @@ static int tc_stack_runs(const fm_signal_args *a, int VG, int Qt) {
   int R = P >= kTcRows ? 2 : (kTcRows % P == 0 ? kTcRows / P : (kTcRows - 1 + P - 1) / P + 1);
   if (R > kTcMaxStack) R = kTcMaxStack;
   // the tiles and node buffers must fit in shared memory
-  int NT, acc;
-  tc_shape(Qt, VG, NT, acc);
-  while (R > 1 && tc_smem_layout(NT, VG + R, Qt).total > kTcSmemMax) --R;
+  while (R > 1 && tc_geom(tc_stage_bytes(tc_nt(Qt, VG)), VG + R, 0).ring == 0) --R;
   return R < 2 ? 1 : R;
 }
 
@@ -1370,12 +1478,6 @@ static int tc_pack_rows(int P, int R) {
   return (R - 1) * P;
 }
 
-static void tc_shape(int Qt, int VG, int &NT, int &acc_cols) {
-  NT = (int)ceil_div(2 * Qt * VG, 16) * 16;
-  acc_cols = 32;
-  while (acc_cols < NT) acc_cols <<= 1;
-}
-
 static size_t tc_batch_workspace(const fm_signal_args *probs, int n) {
   Carve c(nullptr, 0);
   TcBatchPlan b;
@@ -1384,6 +1486,28 @@ static size_t tc_batch_workspace(const fm_signal_args *probs, int n) {
 }
 
 size_t tc_workspace(const fm_signal_args *a) { return tc_batch_workspace(a, 1); }
+
+// A node's mode rows are staged up to this many modes (15 KB per block).
+constexpr int kTcMaxStagedModes = 10;
+
+// Runs per tile when runs are columns: up to 128 pairs, the tiles about equal.
+static int tc_runs_qt(const fm_signal_args *a, int VG) {
+  const int64_t cap = 128 / VG, tiles = ceil_div(a->n_ro, cap);
+  return (int)ceil_div(a->n_ro, tiles > 0 ? tiles : 1);
+}
+
+// Whether runs as columns (where k allows it) take less time than lines x kz
+// tiles: units times the time of a unit's stage, which is about 600 + 6 NT
+// cycles (measured 700 at NT = 16, 2,200 at NT = 256: the A tile is always
+// written in full, so wide tiles pay).
+static bool tc_prefers_runs(const fm_signal_args *a, int VG, int Qt, int RU, int Qt_r) {
+  auto cost = [&](int64_t units, int qt) { return units * (600 + 6 * (int64_t)tc_nt(qt, VG)); };
+  const int64_t slab_units = RU > 0 ? ceil_div(a->n_ro * a->n_lines, (int64_t)RU)
+                                    : a->n_ro * ceil_div(a->n_lines, (int64_t)kTcRows) * ceil_div(a->n_kz, (int64_t)Qt);
+  const int64_t runs_units = ceil_div(a->n_lines * a->n_kz, (int64_t)kTcRows) * ceil_div(a->n_ro, (int64_t)Qt_r);
+  if (a->n_kz < 2) return true;  // otherwise generic: one column group per 128 samples
+  return cost(runs_units, Qt_r) < cost(slab_units, Qt);
+}
 
 // Launch entries of one problem; returns their number.
 static int tc_entries(const fm_signal_args *a, const TcPlan &pl, const fm_tc_tuning *tune, int prob, int e0,
@@ -1399,7 +1523,9 @@ static int tc_entries(const fm_signal_args *a, const TcPlan &pl, const fm_tc_tun
     const int Qt_f = tc_qt(a, VG, tune);
     const int R = tc_stack_runs(a, VG, Qt_f);
     const int RU = R > 1 ? tc_pack_rows((int)a->n_lines, R) : 0;
-    for (int kind = 0; kind < 2; ++kind) {
+    const int Qt_r = tc_runs_qt(a, VG);
+    const int use_runs = pr.stat && tc_prefers_runs(a, VG, Qt_f, RU, Qt_r);
+    for (int kind = 0; kind < kTcKinds; ++kind) {
       TcDev &p = host_entries[ne++];
       p = TcDev{};
       p.N = N; p.S = S; p.V = V;
@@ -1423,31 +1549,25 @@ static int tc_entries(const fm_signal_args *a, const TcPlan &pl, const fm_tc_tun
       p.tiles = pr.tiles;
       p.ctl = pr.ctl;
       p.RU = RU;
-      p.prob = prob; p.first = e0; p.n_of = 2 * pl.n_groups;
+      p.prob = prob; p.first = e0; p.n_of = kTcKinds * pl.n_groups;
       p.max_splits = pl.max_splits;
       p.partials = pl.partials;
       p.out = static_cast<float2 *>(a->out);
       p.kind = kind;
-      p.Qt = kind == 0 ? Qt_f : 1;
+      p.Qt = kind == kTcSlab ? Qt_f : (kind == kTcRuns && use_runs ? Qt_r : 1);
       // a stacked unit's node buffers add one D row per run
-      const int Rk = kind == 0 ? R : 1;
+      const int Rk = kind == kTcSlab ? R : 1;
       p.stacked = Rk > 1 ? 1 : 0;
-      p.wrows = VG + (Rk > 1 ? Rk : 0);
-      int acc_cols;
-      tc_shape(p.Qt, VG, p.NT, acc_cols);
-      // node blocks by bulk copies when the inputs are 16-byte aligned and the
-      // staging area fits next to the tiles
-      const bool aligned = ((uintptr_t)p.r0 % 16 == 0) && ((uintptr_t)p.T2 % 16 == 0) &&
-                           ((uintptr_t)p.phi % 16 == 0) && ((uintptr_t)p.MM % 16 == 0);
-      const int ring = kind == 0 ? kTcStages : kTcRingGen;
-      p.tma = aligned && tc_smem_layout(p.NT, p.wrows, p.Qt, ring).total + tc_raw_bytes(p.mm_ld) <= kTcSmemMax;
-      // the mode rows of a single POD term of several modes are staged with
-      // the node blocks (a rank-1 term is held in registers instead) when
-      // they are 16-byte aligned and there is room after the raw block
+      p.wrows = VG + (kind == kTcRuns && use_runs ? 2 : (Rk > 1 ? Rk : 0));
+      p.NT = tc_nt(p.Qt, VG);
+      p.use_runs = use_runs;
+      // node blocks by bulk copies when the inputs are 16-byte aligned; the
+      // mode rows of a single POD term with them (tc_batch drops either when
+      // the staging areas do not fit)
+      p.tma = ((uintptr_t)p.r0 % 16 == 0) && ((uintptr_t)p.T2 % 16 == 0) && ((uintptr_t)p.phi % 16 == 0) &&
+              ((uintptr_t)p.MM % 16 == 0);
       if (p.tma && md.kind == FM_MOTION_TERMS && md.n_terms == 1 && md.terms[0].kind != FM_TERM_RESPIRATORY &&
-          md.terms[0].n_modes > kTcRegModes && (uintptr_t)md.terms[0].modes % 16 == 0 &&
-          tc_smem_layout(p.NT, p.wrows, p.Qt, ring).total + tc_raw_bytes(p.mm_ld) +
-                  tc_mode_bytes(3 * md.terms[0].n_modes) <= kTcSmemMax)
+          (uintptr_t)md.terms[0].modes % 16 == 0 && md.terms[0].n_modes <= kTcMaxStagedModes)
         p.mstage = 3 * md.terms[0].n_modes;
     }
   }
@@ -1485,22 +1605,30 @@ static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc
   }
   if (ne == 0) return FM_OK;
   FM_TRY(launch_prep<float>(work.data(), prep.data(), (int)prep.size(), b.prep, st));
-  int acc_cols = 32;
-  size_t smem = 0;
-  bool modes = false;
-  auto staging = [&](const TcDev &d) -> size_t {
-    return d.tma ? tc_raw_bytes(d.mm_ld) + tc_mode_bytes(d.mstage) : 0;
-  };
+  // one layout for all entries; staging areas (first without the mode rows,
+  // then altogether) give way to the operand ring
+  uint32_t stage = 0, wrows = 0, raw = 0, raw_modes = 0;
   for (int e = 0; e < ne; ++e) {
-    modes = modes || host[e].mstage != 0;
-    int NT = host[e].NT, ac = 32;
-    while (ac < NT) ac <<= 1;
-    if (ac > acc_cols) acc_cols = ac;
-    const int ring = host[e].kind == 0 ? kTcStages : kTcRingGen;
-    const size_t sm = tc_smem_layout(NT, host[e].wrows, host[e].Qt, ring).total + staging(host[e]);
-    if (sm > smem) smem = sm;
+    stage = std::max(stage, tc_stage_bytes(host[e].NT));
+    wrows = std::max(wrows, (uint32_t)host[e].wrows);
+    if (!host[e].tma) continue;
+    raw = std::max(raw, tc_raw_bytes(host[e].mm_ld));
+    raw_modes = std::max(raw_modes, tc_raw_bytes(host[e].mm_ld) + tc_mode_bytes(host[e].mstage));
   }
-  FM_REQUIRE(smem <= kTcSmemMax, FM_ERR_UNSUPPORTED, "%s: tile needs %zu bytes of shared memory", who, smem);
+  // in order of what costs least to give up: the mode rows' staging, the third
+  // stage of slack in the ring, all staging
+  TcGeom geom = tc_geom(stage, wrows, raw_modes, 4);
+  if (geom.ring == 0) {
+    geom = tc_geom(stage, wrows, raw, 4);
+    if (geom.ring == 0) geom = tc_geom(stage, wrows, raw_modes);
+    if (geom.ring == 0) geom = tc_geom(stage, wrows, raw);
+    if (geom.ring == 0) geom = tc_geom(stage, wrows, 0);
+  }
+  for (int e = 0; e < ne; ++e) {
+    if (tc_raw_bytes(host[e].mm_ld) + tc_mode_bytes(host[e].mstage) > geom.raw_bytes) host[e].mstage = 0;
+    if (tc_raw_bytes(host[e].mm_ld) > geom.raw_bytes) host[e].tma = 0;
+  }
+  FM_REQUIRE(geom.ring != 0, FM_ERR_UNSUPPORTED, "%s: stages of %u bytes do not fit in shared memory", who, stage);
   for (int e0 = 0; e0 < ne; e0 += kTcEntriesPerWrite) {
     TcEntryChunk c;
     c.n = (ne - e0) < kTcEntriesPerWrite ? (ne - e0) : kTcEntriesPerWrite;
@@ -1516,12 +1644,11 @@ static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc
   B.entries = b.entries;
   B.offsets = b.offsets;
   B.n_entries = ne;
-  B.acc_cols = acc_cols;
+  B.geom = geom;
   {
     ScopedTimer timer(ctx, "signal_tc");
-    auto kernel = modes ? signal_tc_kernel<true> : signal_tc_kernel<false>;
-    FM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<kSmCount, kTcThreads, smem, st>>>(B);
+    FM_CUDA(cudaFuncSetAttribute(signal_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)geom.total));
+    signal_tc_kernel<<<kSmCount, kTcThreads, geom.total, st>>>(B);
     count_launch();
     FM_TRY(check_launch("signal_tc_kernel"));
   }

@@ -28,6 +28,10 @@ __device__ inline void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
+__device__ inline void mbar_arrive_n(uint64_t *bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
+}
+
 __device__ inline bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -53,12 +57,27 @@ __device__ inline bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// One wait of up to a millisecond for the phase of `parity`: the warp is
+// suspended meanwhile and issues nothing (a loop of short waits takes issue
+// slots from the warps it waits for).
+__device__ inline bool mbar_try_wait_long(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity), "r"(1000000u)
+      : "memory");
+  return ok != 0;
+}
+
 // Waits for the phase of `parity` to complete; false after `limit_ns`.
 __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity, uint64_t limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait_long(bar, parity)) return true;
   const uint64_t t0 = globaltimer();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait_long(bar, parity)) return true;
     if (globaltimer() - t0 > limit_ns) return false;
   }
 }
@@ -140,40 +159,23 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
          | ((M >> 4) << 24);  // M / 16
 }
 
+// One thread of the converged warp.
+__device__ inline bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// No memory clobber: the MMA reads shared memory through the async proxy
+// (ordered by the writers' proxy fence and the barrier before it), and as a
+// volatile asm it stays in order with the other volatile asm (waits, fences,
+// commits).
 __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same MMA executed by a whole warp with only lane 0 issuing it (the
-// predicate is evaluated inside the instruction sequence, so the warp stays
-// converged and the warp-uniform descriptors need no per-thread moves).
-__device__ inline void mma_bf16_lane0(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                      uint32_t accumulate, uint32_t lane) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.eq.u32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lane));
-  // no memory clobber: the MMA reads shared memory through the async proxy
-  // (ordered by the writers' proxy fence and the block barrier before it),
-  // and as a volatile asm it stays in order with the other volatile asm
-  // (waits, barriers, commits), so a clobber would only force the caller's
-  // values out of registers between consecutive MMAs
-}
-
-// mma_commit issued by lane 0 of a converged warp.
-__device__ inline void mma_commit_lane0(uint64_t *bar, uint32_t lane) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.eq.u32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar)),
-      "r"(lane));
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
 // Arrives on `bar` once all previously issued tcgen05.mma of this thread
@@ -184,17 +186,6 @@ __device__ inline void mma_commit(uint64_t *bar) {
                : "memory");
 }
 
-// 32 lanes x 32 bits, 16 consecutive columns per thread.
-__device__ inline void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 // 32 lanes x 32 bits, 8 consecutive columns per thread.
 __device__ inline void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -203,14 +194,11 @@ __device__ inline void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "memory");
 }
 
-// 32 lanes x 32 bits, 16 consecutive columns per thread (store).
-__device__ inline void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
+// 32 lanes x 32 bits, 8 consecutive columns per thread (store).
+__device__ inline void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 
 __device__ inline void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }

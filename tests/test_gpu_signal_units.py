@@ -1,0 +1,90 @@
+"""Signal work units at the sizes where they can go wrong, against the FP64
+oracle: partial row and column tiles of every unit kind, few rows, node ranges
+that end inside a stage or block, the run and sparse-matrix preparation.
+
+Tolerances: the split-BF16 form keeps hi hi + hi lo + lo hi, so a product is
+off by at most about 3 x 2^-17 of its size; over incoherent sums that is below
+the form's bar of 1e-4 relative L2."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from oracle import fp64
+from feelmri_b200 import workloads as W
+from feelmri_b200.MRI import Signal, signal_call_times
+
+pytestmark = pytest.mark.gpu
+
+TC_TOL = 1e-4
+
+
+def _case(n, V, seed=0):
+    rng = np.random.default_rng(seed)
+    r0 = rng.uniform(-0.04, 0.04, (n, 3)).astype(np.float32)
+    Mxy = ((rng.normal(size=(n, V)) + 1j * rng.normal(size=(n, V))) * 0.1).astype(np.complex64)
+    phi = W.off_resonance(n)
+    T2 = rng.uniform(50.0, 100.0, n).astype(np.float32)
+    M = sp.diags(rng.uniform(1e-7, 3e-7, n)).tocsc()
+    return r0, M, Mxy, phi, T2
+
+
+def _ref(M, traj, t, r0, phi, T2, Mxy, pod=None):
+    disp = None if pod is None else np.stack([pod(x) for x in signal_call_times(t)[1:]])
+    return fp64.signal(sp.csc_matrix(M), *traj.points, t, r0, phi, T2, Mxy, disp=disp, pi_mode="float")
+
+
+def _traj(kind, res):
+    if kind == "cartesian":
+        return W.cartesian(res=res)
+    if kind == "spiral":
+        return W.spiral_stack(n_ro=res[0], n_interleaves=res[1], n_kz=res[2])
+    return W.radial3d(n_ro=res[0], n_spokes=res[1], kmax=300.0)
+
+
+@pytest.mark.parametrize("kind,res,V,n,motion", [
+    ("cartesian", (5, 16, 8), 1, 700, False),     # runs as columns: 5 runs, one row tile
+    ("cartesian", (17, 11, 3), 1, 129, False),    # 17 columns: both node halves apart
+    ("cartesian", (33, 7, 5), 2, 513, False),     # 35 rows, 33 runs of 2 columns
+    ("cartesian", (70, 13, 4), 1, 300, False),    # 70 runs in one tile, 52 rows
+    ("cartesian", (150, 9, 1), 1, 257, False),    # two column tiles, kz = 1
+    ("cartesian", (20, 40, 9), 8, 400, False),    # 20 runs of 8 columns: two column tiles
+    ("cartesian", (3, 96, 32), 4, 1111, True),    # wide slab, three row groups
+    ("cartesian", (3, 33, 40), 3, 600, True),     # 33 rows, 40 kz values
+    ("cartesian", (2, 130, 70), 1, 200, True),    # a second row tile of two rows
+    ("spiral", (40, 3, 16), 2, 515, False),       # stacked runs
+    ("spiral", (9, 20, 17), 1, 100, False),       # stacked, more than 16 kz values
+    ("radial", (6, 31, 1), 8, 1030, True),        # generic, one row group
+    ("radial", (4, 64, 1), 3, 2050, False),       # generic, two row groups
+    ("radial", (3, 300, 1), 9, 130, True),        # generic, two column groups, partial row tile
+])
+def test_tensor_core_units(cuda, kind, res, V, n, motion):
+    r0, M, Mxy, phi, T2 = _case(n, V)
+    traj = _traj(kind, res)
+    pod = W.sinusoidal_pod(n, n_modes=3, amp=1e-3, period=50.0, n_frames=8) if motion else None
+    K = Signal(0, M, traj.points, traj.t, r0, phi, T2, Mxy, pod, precision="bf16x3")
+    assert fp64.rel_l2(K, _ref(M, traj, traj.t, r0, phi, T2, Mxy, pod)) < TC_TOL
+
+
+@pytest.mark.parametrize("precision,tol", [("bf16x3", TC_TOL), (None, 1e-5)])
+@pytest.mark.parametrize("what", ["line_times", "sample_times", "merged_runs", "permutation", "shared_rows"])
+def test_runs_and_sparse_products(cuda, what, precision, tol):
+    """Sample times that do not follow the slabs, and mass matrices of as many
+    entries as rows that are not diagonal."""
+    n, V = 900, 2
+    r0, M, Mxy, phi, T2 = _case(n, V, seed=3)
+    traj = W.cartesian(res=(6, 10, 4))
+    t = traj.t.copy()
+    rng = np.random.default_rng(5)
+    if what == "line_times":
+        t += (np.arange(10, dtype=np.float32) * 0.001)[None, :, None]
+    elif what == "sample_times":
+        t = (2.0 + 0.001 * np.arange(t.size, dtype=np.float32)).reshape(t.shape)
+    elif what == "merged_runs":
+        t[2] = t[1]  # two slabs are one run
+        t[4, 5:] += np.float32(0.01)  # one slab is two
+    elif what == "permutation":
+        M = sp.csc_matrix((M.diagonal(), (rng.permutation(n), np.arange(n))), shape=(n, n))
+    else:  # n entries, several in one row, some columns empty
+        M = sp.csc_matrix((M.diagonal(), (rng.integers(0, n, n), np.sort(rng.integers(0, n, n)))), shape=(n, n))
+    K = Signal(0, M, traj.points, t, r0, phi, T2, Mxy, None, precision=precision)
+    assert fp64.rel_l2(K, _ref(M, traj, t, r0, phi, T2, Mxy)) < tol
