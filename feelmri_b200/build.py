@@ -21,6 +21,7 @@ SOURCES = [
     "bloch.cu",
     "signal_common.cu",
     "signal_plain.cu",
+    "signal_gemm.cu",
     "signal_tc.cu",
     "signal.cu",
     "mass.cu",

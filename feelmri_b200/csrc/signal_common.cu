@@ -40,7 +40,7 @@ static void carve_csr(Carve &c, int64_t rows, int64_t nnz, Csr &m) {
   m.cub_tmp = c.take<char>(m.cub_bytes);
 }
 
-void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool slabs, int vgroup, size_t real_bytes, int *ctl,
+void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool tensor_core, int vgroup, size_t real_bytes, int *ctl,
                 PrepDev &p) {
   p = PrepDev{};
   p.S = a->n_ro * a->n_lines * a->n_kz;
@@ -50,8 +50,11 @@ void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool slabs, int vgr
   p.n_lines = (int)(p.S > 0 ? a->n_lines : 1);
   p.n_kz = (int)(p.S > 0 ? a->n_kz : 1);
   p.Ls = p.n_lines * p.n_kz;
-  p.slabs = slabs && p.n_kz > 1;
+  p.slabs = tensor_core && p.n_kz > 1;
   p.stat = p.n_ro > 1 && p.Ls > 1 && (a->motion == nullptr || a->motion->kind == FM_MOTION_NONE);
+  const int64_t most_cols = 1 << 30;  // columns of a factored product are counted in int
+  p.slab_cover = !tensor_core && p.n_kz > 1 && p.n_lines > 1 && p.n_kz * p.V < most_cols;
+  p.run_cover = !tensor_core && p.stat && p.n_ro * p.V < most_cols;
   p.tile = tile;
   p.vgroup = vgroup;
   const int64_t want = ceil_div(p.S, 1024);
@@ -184,6 +187,15 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
           if (!(k == kc[d][w])) flags |= kFlagAcross << d;
         }
       }
+      if (p.slab_cover) {
+        const int j = w / p.n_kz;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const T k = kc[d][s];
+          if (!(k == kc[d][(int64_t)i * p.Ls + (int64_t)j * p.n_kz])) flags |= kFlagAlongKz << d;
+          if (!(k == kc[d][(int64_t)i * p.Ls + (w - j * p.n_kz)])) flags |= kFlagOverLines << d;
+        }
+      }
       if (p.slabs) {
         // k(j, k) == kp_j + kq_k exactly, kq the slab's kz offsets
         const int j = w / p.n_kz, k = w - j * p.n_kz;
@@ -267,6 +279,11 @@ struct Cplx<double> {
   using type = double2;
 };
 
+// The whole problem goes through a factored CUDA-core form.
+__device__ inline bool prep_covered(const PrepDev &p) {
+  return prep_form(p.run_cover, p.slab_cover, p.ctl) != kFormPlain;
+}
+
 // Factored runs (fac) and tiles of the others (tiles) that run g opens.
 __device__ inline void prep_run_items(const PrepDev &p, int g, bool &fac, int &tiles) {
   const int s0 = p.start[g], len = p.start[g + 1] - s0;
@@ -305,7 +322,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
   const int c = blockIdx.x;
   if (c >= p.n_chunks) return;
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = min(n_runs, (c + 1) * per);
+  const int g1 = prep_covered(p) ? 0 : min(n_runs, (c + 1) * per);
   int nf = 0, nt = 0;
   for (int g = c * per + threadIdx.x; g < g1; g += kPrepThreads) {
     bool fac;
@@ -404,7 +421,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_fill_kernel(const PrepDev *
   int t0 = block_prefix(p.chunk_tiles, c);
   const int n_runs = p.ctl[kCtlRuns];
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = min(n_runs, (c + 1) * per);
+  const int g1 = prep_covered(p) ? 0 : min(n_runs, (c + 1) * per);
   for (int gb = c * per; gb < g1; gb += kPrepThreads) {
     const int g = gb + threadIdx.x;
     bool fac = false;

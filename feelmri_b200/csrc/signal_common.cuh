@@ -44,6 +44,8 @@ constexpr int kFlagOffsets = 4;        // some slab's kz offsets differ from the
 constexpr int kFlagNotDiagonal = 8;    // M has as many entries as rows but is not diagonal
 constexpr int kFlagInSlab = 1 << 8;    // << c: component c of k varies inside some slab
 constexpr int kFlagAcross = 1 << 11;   // << c: component c differs from the first slab's
+constexpr int kFlagAlongKz = 1 << 14;  // << c: component c varies along some line's kz values
+constexpr int kFlagOverLines = 1 << 17;  // << c: component c varies over some slab's lines at one kz
 
 // Components of k that go with the run, and whether the samples factor as
 // k(i, j, k) = k_run(i) + k_slab(j, k): every slab is one run and each component
@@ -61,6 +63,8 @@ struct PrepDev {
   int Ls, n_lines, n_kz, n_ro;
   int n_chunks, chunk;   // the samples in n_chunks stretches of `chunk`
   int tile;              // samples per tile of an unfactored run
+  int slab_cover;        // slabs that factor by components are not listed as tiles (CUDA-core forms)
+  int run_cover;         // nor is anything where the runs factor out
   int stat;              // runs may factor out (no motion, several runs of several samples)
   int slabs;             // slabs may factor: factored runs are listed apart from the tiles
   int diag;              // M holds as many entries as rows: diagonal unless shown otherwise
@@ -82,9 +86,24 @@ struct PrepDev {
   Csr csr;
 };
 
+// Components of k that go with kz within a slab, and whether every run is a
+// slab whose k factors as k_line(j) + k_kz(k), each component in one factor.
+__device__ inline int prep_kz_comps(const int *ctl) { return (ctl[kCtlFlags] / kFlagAlongKz) & 7; }
+__device__ inline bool prep_slab(const int *ctl) {
+  const int f = ctl[kCtlFlags];
+  return !(f & kFlagRuns) && ((f / kFlagAlongKz) & (f / kFlagOverLines) & 7) == 0;
+}
+
+// The CUDA-core form that sums a problem.
+enum { kFormRuns, kFormSlabs, kFormPlain };
+__device__ inline int prep_form(bool run_cover, bool slab_cover, const int *ctl) {
+  return run_cover && prep_static(ctl) ? kFormRuns : (slab_cover && prep_slab(ctl) ? kFormSlabs : kFormPlain);
+}
+
 // Scratch of one problem: carved the same way when sizing and when running.
-// `slabs`: slabs of more than one kz value may factor (tensor-core form).
-void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool slabs, int vgroup, size_t real_bytes, int *ctl,
+// `tensor_core`: factored slabs are listed for the tensor-core form (else for
+// the factored CUDA-core form).
+void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool tensor_core, int vgroup, size_t real_bytes, int *ctl,
                 PrepDev &p);
 // Fills the rest of the descriptor from the arguments.
 void fill_prep(const fm_signal_args *a, PrepDev &p);

@@ -1,4 +1,5 @@
-// Plain CUDA-core forms of Signal (FP32 drop-in and FP64).
+// Plain CUDA-core forms of Signal (FP32 drop-in and FP64), for samples whose
+// wave vectors do not factor (signal_gemm.cu takes the others).
 //
 // Restates Signal<T> (cpp/feelmri/MRI.cpp:38-159 with motion, :196-298
 // without): for every sample s of run g (time t_g)
@@ -10,7 +11,10 @@
 // shared memory; the per-run node quantities (moved position, phase offset,
 // decayed weight) are formed once per block and node.  Node ranges may be
 // split over blocks; partial sums are then added in a fixed order.
+#include <algorithm>
+
 #include "signal_common.cuh"
+#include "signal_gemm.cuh"
 
 namespace fm {
 
@@ -156,14 +160,37 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T>
   }  // tiles
 }
 
-// out[e] = sum over splits in order of partial[split][e].
+// out[e] = sum over the node splits of partial[split][e]: eight threads of a
+// block each sum every eighth split in order, then their sums in order.  The
+// splits are those of the form that worked.
+struct SplitCounts {
+  int run_cover, slab_cover;
+  int splits[3];  // by form
+};
+constexpr int kReduceLanes = 8, kReduceElems = 32;
 template <typename T>
-__global__ void split_reduce_kernel(const T *__restrict__ part, int splits, int64_t count, T *__restrict__ out) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
-  T acc = part[e];
-  for (int k = 1; k < splits; ++k) acc += part[(int64_t)k * count + e];
-  out[e] = acc;
+__global__ void __launch_bounds__(kReduceLanes *kReduceElems) split_reduce_kernel(const T *__restrict__ part, SplitCounts c,
+                                                                                  const int *__restrict__ ctl,
+                                                                                  int64_t count, T *__restrict__ out) {
+  __shared__ T sums[kReduceLanes][kReduceElems];
+  const int splits = c.splits[prep_form(c.run_cover, c.slab_cover, ctl)];
+  if (splits <= 1) return;
+  const int lane = threadIdx.x & (kReduceElems - 1), k0 = threadIdx.x / kReduceElems;
+  for (int64_t e0 = (int64_t)blockIdx.x * kReduceElems; e0 < count; e0 += (int64_t)gridDim.x * kReduceElems) {
+    const int64_t e = e0 + lane;
+    T acc = T(0);
+    if (e < count)
+      for (int k = k0; k < splits; k += kReduceLanes) acc += part[(int64_t)k * count + e];
+    __syncthreads();
+    sums[k0][lane] = acc;
+    __syncthreads();
+    if (k0 == 0 && e < count) {
+      T s = sums[0][lane];
+#pragma unroll
+      for (int i = 1; i < kReduceLanes; ++i) s += sums[i][lane];
+      out[e] = s;
+    }
+  }
 }
 
 template <typename T, int VMAX>
@@ -197,6 +224,7 @@ struct PlainPlan {
   PrepDev prep;
   PrepDev *dev;
   T *partials;
+  GemmPlan gemm[2];
   int splits;
   int tile;
 };
@@ -210,7 +238,9 @@ static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   pl.dev = c.take<PrepDev>(1);
   carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
   pl.splits = choose_splits(ceil_div(S, pl.tile), N);
-  pl.partials = (pl.splits > 1) ? c.take<T>((size_t)pl.splits * S * V * 2) : nullptr;
+  plan_gemm<T>(a, pl.prep, pl.splits, pl.gemm);
+  const int most = std::max(pl.splits, std::max(pl.gemm[0].splits, pl.gemm[1].splits));
+  pl.partials = most > 1 ? c.take<T>((size_t)most * S * V * 2) : nullptr;
 }
 
 int validate_signal(const fm_signal_args *a, const char *who);
@@ -270,9 +300,12 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
     count_launch();
     FM_TRY(check_launch("signal_plain_kernel"));
   }
-  if (pl.splits > 1) {
-    const int64_t count = S * V * 2;
-    split_reduce_kernel<T><<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(pl.partials, pl.splits, count, out);
+  FM_TRY(launch_gemm<T>(a, pl.prep, pl.gemm, out, pl.partials, st));
+  if (pl.partials) {
+    const int64_t count = S * V * 2, blocks = ceil_div(count, kReduceElems);
+    const SplitCounts c{pl.prep.run_cover, pl.prep.slab_cover, {pl.gemm[0].splits, pl.gemm[1].splits, pl.splits}};
+    split_reduce_kernel<T><<<(unsigned)(blocks < 32 * kSmCount ? blocks : 32 * kSmCount), kReduceLanes * kReduceElems, 0,
+                             st>>>(pl.partials, c, pl.prep.ctl, count, out);
     count_launch();
     FM_TRY(check_launch("split_reduce_kernel"));
   }

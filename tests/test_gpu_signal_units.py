@@ -88,3 +88,55 @@ def test_runs_and_sparse_products(cuda, what, precision, tol):
         M = sp.csc_matrix((M.diagonal(), (rng.integers(0, n, n), np.sort(rng.integers(0, n, n)))), shape=(n, n))
     K = Signal(0, M, traj.points, t, r0, phi, T2, Mxy, None, precision=precision)
     assert fp64.rel_l2(K, _ref(M, traj, t, r0, phi, T2, Mxy)) < tol
+
+
+# CUDA-core forms whose samples factor: rounding of the FP64 form is some 1e-15 a
+# term and does not add up coherently over these few nodes; FP32 has the bar of
+# its drop-in form.
+@pytest.mark.parametrize("precision,tol", [("f64", 1e-13), (None, 1e-5)])
+@pytest.mark.parametrize("res,V,n,motion", [
+    ((2, 3, 1), 1, 17, False),      # one thread's rows and columns
+    ((64, 64, 1), 1, 700, False),   # one full tile (FP64)
+    ((65, 9, 1), 1, 129, False),    # a second column tile of one column
+    ((7, 43, 3), 3, 515, False),    # 129 rows: a second row tile of one
+    ((5, 11, 2), 70, 65, False),    # more columns per run than a tile holds
+    ((4, 6, 5), 13, 33, True),      # 65 columns of 13 weights
+    ((3, 131, 2), 2, 301, True),    # three row tiles
+    ((2, 2, 80), 1, 1, True),       # one node
+    ((3, 5, 16), 4, 2049, True),    # stage ends
+    ((1, 40, 6), 2, 500, False),    # one run: slabs
+])
+def test_factored_forms(cuda, res, V, n, motion, precision, tol):
+    r0, M, Mxy, phi, T2 = _case(n, V)
+    traj = _traj("cartesian", res)
+    pod = W.sinusoidal_pod(n, n_modes=3, amp=1e-3, period=50.0, n_frames=8) if motion else None
+    pts, t = traj.points, traj.t
+    if precision == "f64":
+        r0, phi, T2, t = (a.astype(np.float64) for a in (r0, phi, T2, t))
+        pts = tuple(np.asarray(p, np.float64) for p in pts)
+        Mxy = Mxy.astype(np.complex128)
+    K = Signal(0, M, pts, t, r0, phi, T2, Mxy, pod)
+    assert K.dtype == Mxy.dtype
+    ref = fp64.signal(sp.csc_matrix(M), *pts, t, r0, phi, T2, Mxy, pi_mode="float",
+                      disp=None if pod is None else np.stack([pod(x) for x in signal_call_times(t)[1:]]))
+    # displacements are FP32 numbers in both
+    assert fp64.rel_l2(K, ref) < (tol if pod is None or precision is None else 1e-6)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_factored_forms_far_and_not_finite(cuda, dtype):
+    """Phases of millions of cycles, and nodes at no finite place."""
+    n = 80
+    r0, M, Mxy, phi, T2 = _case(n, 1)
+    traj = W.cartesian(res=(4, 6, 3))
+    c = lambda a: np.asarray(a, dtype)
+    pts = [c(p) for p in traj.points]
+    pts[1] = c(np.float32(pts[1] * 1e6))
+    args = (c(traj.t), c(r0), c(phi), c(T2), Mxy.astype(np.complex64 if dtype == np.float32 else np.complex128))
+    K = Signal(0, M, tuple(pts), *args, None)
+    ref = fp64.signal(sp.csc_matrix(M), *pts, *args, disp=None, pi_mode="float")
+    assert fp64.rel_l2(K, ref) < 1e-5
+    for bad in (np.nan, np.inf):
+        r1 = args[1].copy()
+        r1[3, 2] = bad
+        assert np.isnan(Signal(0, M, tuple(pts), args[0], r1, *args[2:], None)).all()
