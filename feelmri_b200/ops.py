@@ -583,12 +583,24 @@ def mass_assemble(elems, nodes, qweights, tab):
     N = nodes.shape[0]
     indptr = torch.empty((N + 1,), dtype=torch.int32, device=dev)
     ctx = ctx_for(dev)
-    L.check(L.lib().fm_mass_assemble(ctx, C.byref(a), is_double, C.byref(nnz), indptr.data_ptr(), None, None, 0,
-                                     ws.data_ptr(), ws.numel()))
+
+    def assemble(indices, data):
+        L.check(L.lib().fm_mass_assemble(ctx, C.byref(a), is_double, C.byref(nnz), indptr.data_ptr(), _ptr(indices),
+                                         _ptr(data), 0 if data is None else data.numel(), ws.data_ptr(), ws.numel()))
+
+    # one pass into arrays that hold every triplet, then the entries alone; a mesh
+    # of more than 1 GiB of triplets is counted first instead
+    triplets = elems.numel() * elems.shape[1]
+    if 0 < triplets * (4 + nodes.element_size()) <= 1 << 30:
+        indices = torch.empty((triplets,), dtype=torch.int32, device=dev)
+        data = torch.empty((triplets,), dtype=nodes.dtype, device=dev)
+        assemble(indices, data)
+        return indptr, indices[:nnz.value].clone(), data[:nnz.value].clone()
+    assemble(None, None)
     indices = torch.empty((nnz.value,), dtype=torch.int32, device=dev)
     data = torch.empty((nnz.value,), dtype=nodes.dtype, device=dev)
-    L.check(L.lib().fm_mass_assemble(ctx, C.byref(a), is_double, C.byref(nnz), indptr.data_ptr(),
-                                     indices.data_ptr(), data.data_ptr(), nnz.value, ws.data_ptr(), ws.numel()))
+    if nnz.value:
+        assemble(indices, data)
     return indptr, indices, data
 
 
