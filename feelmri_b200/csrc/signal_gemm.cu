@@ -224,7 +224,7 @@ __device__ inline void gemm_rows(unsigned char *A, const double *krow, int mask,
   int m = threadIdx.x / per, r = threadIdx.x - m * per;
   while (m < cnt) {
     if constexpr (sizeof(T) == 4) {
-      f32x2 re, im, neg;
+      float re0, im0, re1, im1;
       double c0, c1;
       c0 = c1 = 0.0;
 #pragma unroll
@@ -235,10 +235,11 @@ __device__ inline void gemm_rows(unsigned char *A, const double *krow, int mask,
           c0 = fma(k.x, at, c0);
           c1 = fma(k.y, at, c1);
         }
-      cis_cycles2(c0, c1, re, im, neg);
-      f32x2 *a = reinterpret_cast<f32x2 *>(A) + (m * (per >> 2) + (r >> 2)) * 8 + (r & 3);
-      a[0] = re;
-      a[4] = im;
+      cis_cycles(c0, re0, im0);
+      cis_cycles(c1, re1, im1);
+      float2 *a = reinterpret_cast<float2 *>(A) + (m * (per >> 2) + (r >> 2)) * 8 + (r & 3);
+      a[0] = make_float2(re0, re1);
+      a[4] = make_float2(im0, im1);
     } else {
       Cycles c0, c1;
       phase_pair(krow, rows, 2 * r, 2 * r + 1, d, m, m, mask, c0, c1);
@@ -278,10 +279,8 @@ __device__ inline void gemm_cols(unsigned char *B, const double *kcol, int mask,
         c0 = fma(u, d[4 * kGemmNodes + m], c0);
         c1 = fma(u, d[4 * kGemmNodes + m + 1], c1);
       }
-      f32x2 re, im, neg;
-      cis_cycles2(c0, c1, re, im, neg);
-      unpack2(re, er[0], er[1]);
-      unpack2(im, ei[0], ei[1]);
+      cis_cycles(c0, er[0], ei[0]);
+      cis_cycles(c1, er[1], ei[1]);
     } else {
       Cycles c0, c1;
       phase_pair(kcol, cols, q, q, d, m, m + 1, mask, c0, c1);

@@ -9,25 +9,15 @@
 // taken of the phase in radians.  One thread block covers up to
 // kPlainThreads * SPT samples of one run and sweeps a node range staged in
 // shared memory; the per-run node quantities (moved position, phase offset,
-// decayed weight) are formed once per block and node.  Node ranges may be
+// decayed weight) are formed once per tile and node.  Node ranges may be
 // split over blocks; partial sums are then added in a fixed order.
 #include <algorithm>
 
+#include "cycles.cuh"
 #include "signal_common.cuh"
 #include "signal_gemm.cuh"
 
 namespace fm {
-
-template <typename T>
-struct V4;
-template <>
-struct V4<float> {
-  using type = float4;
-};
-template <>
-struct V4<double> {
-  using type = double4;
-};
 
 template <typename T>
 struct PlainDev {
@@ -48,29 +38,19 @@ struct PlainDev {
   T two_pi;
 };
 
-template <typename T>
-__device__ inline void sincos_t(T x, T *s, T *c);
-template <>
-__device__ inline void sincos_t<float>(float x, float *s, float *c) { sincosf(x, s, c); }
-template <>
-__device__ inline void sincos_t<double>(double x, double *s, double *c) { sincos(x, s, c); }
+constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an SM holds in FP32
 
-template <typename T>
-__device__ inline T exp_t(T x);
-template <>
-__device__ inline float exp_t<float>(float x) { return expf(x); }
-template <>
-__device__ inline double exp_t<double>(double x) { return exp(x); }
-
-template <typename T, int VMAX, int SPT, int NT>
-__global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T> p, int v0) {
-  using T4 = typename V4<T>::type;
-  __shared__ T4 s_pos[NT];             // moved x, y, z and phi * t
+template <int VMAX, int NT>
+__global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<double> p, int v0) {
+  using T = double;
+  constexpr int SPT = 1;
+  __shared__ double4 s_pos[NT];             // moved x, y, z and phi * t
   __shared__ T s_w[NT][2 * VMAX];      // decayed M * Mxy columns v0 .. v0 + VMAX
 
   const int n_tiles = *p.n_tiles;
-  const int split = blockIdx.y;
-  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+  const int64_t items = (int64_t)n_tiles * p.splits;
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+  const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
   __syncthreads();  // the previous tile's readers of s_pos / s_w are done
   const int g = p.tiles[tile].x;
   const int s_begin = p.run_start[g] + p.tiles[tile].y;
@@ -112,12 +92,12 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T>
         const T *d = p.table + ((int64_t)g * p.N + n) * 3;
         x = x + (T)d[0]; y = y + (T)d[1]; z = z + (T)d[2];
       }
-      T4 pp;
+      double4 pp;
       pp.x = x; pp.y = y; pp.z = z;
       pp.w = p.phi[n] * tg;                       // phi_off (MRI.cpp:124)
       s_pos[j] = pp;
       const T invT2 = T(1) / p.T2[n];
-      const T decay = exp_t<T>(-tg * invT2);      // T2_decay (MRI.cpp:127)
+      const T decay = exp(-tg * invT2);      // T2_decay (MRI.cpp:127)
       const T *mm = p.MM + (n * p.V + v0) * 2;
 #pragma unroll
       for (int v = 0; v < VMAX; ++v) {
@@ -127,13 +107,13 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T>
     }
     __syncthreads();
     for (int j = 0; j < cnt; ++j) {
-      const T4 pp = s_pos[j];
+      const double4 pp = s_pos[j];
 #pragma unroll
       for (int q = 0; q < SPT; ++q) {
         // phase = -kx_ x - ky_ y - kz_ z + phi_off   (MRI.cpp:143-146)
         const T ph = fma(-kzs[q], pp.z, fma(-kys[q], pp.y, -kxs[q] * pp.x)) + pp.w;
         T sn, cs;
-        sincos_t<T>(ph, &sn, &cs);
+        sincos(ph, &sn, &cs);
 #pragma unroll
         for (int v = 0; v < VMAX; ++v) {
           const T wr = s_w[j][2 * v + 0], wi = s_w[j][2 * v + 1];
@@ -157,6 +137,96 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<T>
       }
     }
   }
+  }  // tiles
+}
+
+// FP32: two samples per thread, their phases in FP64 cycles.  A phase is three multiply-adds on the FP64 pipe,
+// which the rest leaves idle, and its reduction exact (cycles.cuh), where the
+// reference rounds the phase in radians to FP32; what comes after is FP32 as
+// there.  Bound by issue: per sample-node some 40 instructions for the phase and
+// its sin/cos and 4 a column, 77% of the issue rate.  20,011 nodes x 128 runs x
+// 255 samples x 8 columns on a B200: 2944 us with sincosf of a rounded phase, one
+// sample per thread and tiles dealt out split by split, 1730 us now.
+constexpr int kPlain32Threads = 128;
+constexpr int kPlainNodes = 128;  // nodes staged at a time
+template <int VMAX>
+__global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(PlainDev<float> p, int v0) {
+  __shared__ double4 s_pos[kPlainNodes];         // moved x, y, z and phi t in cycles
+  __shared__ float2 s_w[kPlainNodes][VMAX];  // decayed M * Mxy
+
+  const int n_tiles = *p.n_tiles;
+  const int64_t items = (int64_t)n_tiles * p.splits;
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
+    __syncthreads();  // the previous tile's readers of s_pos / s_w are done
+    const int g = p.tiles[tile].x;
+    const int s0 = p.run_start[g] + p.tiles[tile].y + threadIdx.x, s1 = s0 + kPlain32Threads;
+    const int s_end = p.run_start[g + 1];
+    const float tg = (float)p.run_t[g];
+    const int nv = (int)min((int64_t)VMAX, p.V - v0);
+    // -k in units of 2 pi with a float-rounded pi
+    auto scaled = [&](const float *k, int s) { return s < s_end ? -(double)k[s] * kPiRatio : 0.0; };
+    const double kx0 = scaled(p.kx, s0), ky0 = scaled(p.ky, s0), kz0 = scaled(p.kz, s0);
+    const double kx1 = scaled(p.kx, s1), ky1 = scaled(p.ky, s1), kz1 = scaled(p.kz, s1);
+    float2 acc0[VMAX], acc1[VMAX];
+#pragma unroll
+    for (int v = 0; v < VMAX; ++v) acc0[v] = acc1[v] = make_float2(0.f, 0.f);
+
+    const int64_t n_begin = (int64_t)split * p.chunk;
+    const int64_t n_end = min(p.N, n_begin + p.chunk);
+    const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
+    for (int64_t nb = n_begin; nb < n_end; nb += kPlainNodes) {
+      const int cnt = (int)min((int64_t)kPlainNodes, n_end - nb);
+      __syncthreads();
+      for (int j = threadIdx.x; j < cnt; j += kPlain32Threads) {
+        const int64_t n = nb + j;
+        float x = p.r0[3 * n + 0], y = p.r0[3 * n + 1], z = p.r0[3 * n + 2];
+        if (p.md.kind == FM_MOTION_TERMS) {
+          float dx, dy, dz;
+          motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
+          x = x + dx; y = y + dy; z = z + dz;
+        } else if (p.table) {
+          const float *d = p.table + ((int64_t)g * p.N + n) * 3;
+          x = x + d[0]; y = y + d[1]; z = z + d[2];
+        }
+        double4 pp;
+        pp.x = x; pp.y = y; pp.z = z;
+        pp.w = (double)p.phi[n] * tg * kInv2Pi;     // phi_off (MRI.cpp:124)
+        s_pos[j] = pp;
+        const float invT2 = 1.f / p.T2[n];
+        const float decay = expf(-tg * invT2);      // T2_decay (MRI.cpp:127)
+        const float *mm = p.MM + (n * p.V + v0) * 2;
+#pragma unroll
+        for (int v = 0; v < VMAX; ++v) {
+          const float wr = v < nv ? mm[2 * v + 0] * decay : 0.f, wi = v < nv ? mm[2 * v + 1] * decay : 0.f;
+          s_w[j][v] = make_float2(wr, wi);
+        }
+      }
+      __syncthreads();
+#pragma unroll 2
+      for (int j = 0; j < cnt; ++j) {
+        const double4 pp = s_pos[j];
+        // phase = -kx_ x - ky_ y - kz_ z + phi_off   (MRI.cpp:143-146)
+        float c0, s0n, c1, s1n;
+        cis_cycles(fma(kx0, pp.x, fma(ky0, pp.y, fma(kz0, pp.z, pp.w))), c0, s0n);
+        cis_cycles(fma(kx1, pp.x, fma(ky1, pp.y, fma(kz1, pp.z, pp.w))), c1, s1n);
+#pragma unroll
+        for (int v = 0; v < VMAX; ++v) {
+          const float2 w = s_w[j][v];
+          acc0[v].x = fmaf(c0, w.x, fmaf(-s0n, w.y, acc0[v].x));
+          acc0[v].y = fmaf(c0, w.y, fmaf(s0n, w.x, acc0[v].y));
+          acc1[v].x = fmaf(c1, w.x, fmaf(-s1n, w.y, acc1[v].x));
+          acc1[v].y = fmaf(c1, w.y, fmaf(s1n, w.x, acc1[v].y));
+        }
+      }
+    }
+
+    float2 *dst = reinterpret_cast<float2 *>(p.out) + (int64_t)split * p.S * p.V + v0;
+#pragma unroll
+    for (int v = 0; v < VMAX; ++v) {
+      if (v < nv && s0 < s_end) dst[(int64_t)s0 * p.V + v] = acc0[v];
+      if (v < nv && s1 < s_end) dst[(int64_t)s1 * p.V + v] = acc1[v];
+    }
   }  // tiles
 }
 
@@ -194,29 +264,28 @@ __global__ void __launch_bounds__(kReduceLanes *kReduceElems) split_reduce_kerne
 }
 
 template <typename T, int VMAX>
-static void launch_plain(const PlainDev<T> &p, int64_t max_tiles, int v0, int spt, cudaStream_t st) {
-  constexpr int NT = 128;
-  const int64_t per_split = (4LL * kSmCount + p.splits - 1) / p.splits;
-  dim3 grid((unsigned)(max_tiles < per_split ? max_tiles : per_split), (unsigned)p.splits);
-  if (spt == 2) signal_plain_kernel<T, VMAX, 2, NT><<<grid, kPlainThreads, 0, st>>>(p, v0);
-  else signal_plain_kernel<T, VMAX, 1, NT><<<grid, kPlainThreads, 0, st>>>(p, v0);
+static void launch_plain(const PlainDev<T> &p, int64_t max_tiles, int v0, cudaStream_t st) {
+  const int64_t most = max_tiles * p.splits;
+  const unsigned grid = (unsigned)(most < kPlainBlocks ? most : kPlainBlocks);
+  if constexpr (sizeof(T) == 4) signal_plain32_kernel<VMAX><<<grid, kPlain32Threads, 0, st>>>(p, v0);
+  else signal_plain_kernel<VMAX, kPlainNodes><<<grid, kPlainThreads, 0, st>>>(p, v0);
 }
 
-// Samples per thread: two for FP32 with few columns, else one.
-template <typename T>
-static int samples_per_thread(int64_t V) {
-  return (sizeof(T) == 4 && V <= 4) ? 2 : 1;
-}
-
-// Split count: enough blocks to fill the GPU, bounded by the node count.
-static int choose_splits(int64_t n_tiles_min, int64_t N) {
-  const int64_t want = 4LL * kSmCount;
-  int64_t s = (n_tiles_min >= want) ? 1 : ceil_div(want, n_tiles_min > 0 ? n_tiles_min : 1);
-  s = s < 1 ? 1 : s;
-  const int64_t by_nodes = ceil_div(N, 1024);
-  if (s > by_nodes) s = by_nodes;
-  if (s > 64) s = 64;
-  return (int)(s < 1 ? 1 : s);
+// Split count for slabs cut to `tiles` tiles: the most tiles that a block takes,
+// over the splits, and 1% a split for its partial sums; at least 1024 nodes a
+// split.  128 tiles go to 592 blocks in 9 splits, 2 for each block and 0.22 of a
+// tile's time; in the fewest splits that give every block one (5), it is 0.4.
+static int choose_splits(int64_t tiles, int64_t N) {
+  int best = 1;
+  double best_cost = 0.0;
+  for (int s = 1; s <= 64 && (s == 1 || N / s >= 1024); ++s) {
+    const double cost = (double)ceil_div(tiles * s, (int64_t)kPlainBlocks) / s * (1.0 + 0.01 * s);
+    if (s == 1 || cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 template <typename T>
@@ -233,11 +302,11 @@ template <typename T>
 static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   const int64_t S = a->n_ro * a->n_lines * a->n_kz;
   const int64_t N = a->n_nodes, V = a->n_vencs;
-  pl.tile = samples_per_thread<T>(V) * kPlainThreads;
+  pl.tile = sizeof(T) == 4 ? 2 * kPlain32Threads : kPlainThreads;
   int *ctl = c.take<int>(kCtlWords);
   pl.dev = c.take<PrepDev>(1);
   carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
-  pl.splits = choose_splits(ceil_div(S, pl.tile), N);
+  pl.splits = choose_splits(S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1, N);
   plan_gemm<T>(a, pl.prep, pl.splits, pl.gemm);
   const int most = std::max(pl.splits, std::max(pl.gemm[0].splits, pl.gemm[1].splits));
   pl.partials = most > 1 ? c.take<T>((size_t)most * S * V * 2) : nullptr;
@@ -289,14 +358,13 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
   const float pi_f = 3.14159265358979323846f;
   p.two_pi = (T)2.0 * (T)pi_f;
 
-  const int spt = samples_per_thread<T>(V);
   ScopedTimer timer(ctx, sizeof(T) == 4 ? "signal_f32" : "signal_f64");
   for (int v0 = 0; v0 < V; v0 += 8) {
     const int64_t nv = V - v0;
-    if (nv <= 1) launch_plain<T, 1>(p, max_tiles, v0, spt, st);
-    else if (nv <= 2) launch_plain<T, 2>(p, max_tiles, v0, spt, st);
-    else if (nv <= 4) launch_plain<T, 4>(p, max_tiles, v0, spt, st);
-    else launch_plain<T, 8>(p, max_tiles, v0, spt, st);
+    if (nv <= 1) launch_plain<T, 1>(p, max_tiles, v0, st);
+    else if (nv <= 2) launch_plain<T, 2>(p, max_tiles, v0, st);
+    else if (nv <= 4) launch_plain<T, 4>(p, max_tiles, v0, st);
+    else launch_plain<T, 8>(p, max_tiles, v0, st);
     count_launch();
     FM_TRY(check_launch("signal_plain_kernel"));
   }

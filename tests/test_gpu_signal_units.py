@@ -140,3 +140,32 @@ def test_factored_forms_far_and_not_finite(cuda, dtype):
         r1 = args[1].copy()
         r1[3, 2] = bad
         assert np.isnan(Signal(0, M, tuple(pts), args[0], r1, *args[2:], None)).all()
+
+
+# The unfactored FP32 form at the edges of its tiles of 256 samples, node stages
+# of 128 and column groups of 8; phases of millions of cycles; nodes at no finite
+# place.  Its drop-in form's bar.
+@pytest.mark.parametrize("res,V,n,motion", [
+    ((1, 1, 1), 1, 1, False),
+    ((3, 128, 1), 2, 127, False),
+    ((3, 129, 1), 3, 129, True),
+    ((2, 256, 1), 8, 256, False),
+    ((2, 257, 1), 9, 2049, True),
+    ((1, 700, 1), 5, 1500, False),
+])
+def test_unfactored_form(cuda, res, V, n, motion):
+    r0, M, Mxy, phi, T2 = _case(n, V)
+    traj = _traj("radial", res)
+    pod = W.sinusoidal_pod(n, n_modes=3, amp=1e-3, period=50.0, n_frames=8) if motion else None
+    pts = [np.asarray(p, np.float32) for p in traj.points]
+    for scale in (1.0, 1e6):
+        k = (pts[0], np.float32(pts[1] * scale), pts[2])
+        K = Signal(0, M, k, traj.t, r0, phi, T2, Mxy, pod)
+        ref = fp64.signal(sp.csc_matrix(M), *k, traj.t, r0, phi, T2, Mxy, pi_mode="float",
+                          disp=None if pod is None else np.stack([pod(x) for x in signal_call_times(traj.t)[1:]]))
+        if scale == 1.0 or pod is None:  # the displaced place is rounded to FP32
+            assert fp64.rel_l2(K, ref) < 1e-5
+    for bad in (np.nan, np.inf):
+        r1 = r0.copy()
+        r1[0, 1] = bad
+        assert np.isnan(Signal(0, M, traj.points, traj.t, r1, phi, T2, Mxy, pod)).all()
