@@ -19,7 +19,7 @@
 // Block: a tile of rows x (q, v) pairs, 8 x 4 (FP64: 4 x 4) per thread, operands
 // of 16 nodes at a time in shared memory.  Forming a pair of elements costs some
 // 100 instructions, a product of a thread's block with a node 128 multiply-adds:
-// issue bounds the FP32 form (1.5 10^9 warp instructions at 63% of the issue
+// issue bounds the FP32 form (1.46 10^9 warp instructions at 66% of the issue
 // rate in the flow case below, two thirds of them multiply-adds), the latency of
 // forming operands and the set-up of short node ranges the FP64 one.  Plain
 // multiply-adds, not packed ones: those need one operand twice in registers,
@@ -28,7 +28,7 @@
 //
 // Kernel time on a B200, one sin/cos per node-sample (signal_plain_kernel)
 // against this: FP32 50,021 nodes x 48 runs x 48 lines x 16 kz x 4 columns with
-// flow 6152 us -> 1976 us (the multiply-adds alone take 820 us), FP64 20,011
+// flow 6152 us -> 1970 us (the multiply-adds alone take 820 us), FP64 20,011
 // nodes x 64 runs x 64 lines 1403 us -> 67 us (multiply-adds 18 us).
 #include <algorithm>
 
@@ -192,49 +192,37 @@ struct GemmAcc<double> {
   __device__ double2 get(int i, int j) const { return make_double2(re[i][j], im[i][j]); }
 };
 
-// Phases of two factor elements, k[i0] at node m0 and k[i1] at node m1, over the
-// components of `mask`: a sum in FP64, or (FP64 form) with what rounding leaves
-// out.
-__device__ inline void phase_pair(const double *k, int stride, int i0, int i1, const double *d, int m0, int m1, int mask,
+// Phases of two factor elements, k[i0] at node m0 and k[i1] at node m1: sums in
+// FP64 (FP32 form), or with what rounding leaves out (FP64 form).
+__device__ inline void phase_pair(const double *k, int stride, int i0, int i1, const double *d, int m0, int m1,
                                   double &c0, double &c1) {
-  c0 = c1 = 0.0;
-#pragma unroll
-  for (int x = 0; x < 3; ++x)
-    if ((mask >> x) & 1) {
-      c0 = fma(k[x * stride + i0], d[x * kGemmNodes + m0], c0);
-      c1 = fma(k[x * stride + i1], d[x * kGemmNodes + m1], c1);
-    }
+  c0 = fma(k[2 * stride + i0], d[2 * kGemmNodes + m0], fma(k[stride + i0], d[kGemmNodes + m0], k[i0] * d[m0]));
+  c1 = fma(k[2 * stride + i1], d[2 * kGemmNodes + m1], fma(k[stride + i1], d[kGemmNodes + m1], k[i1] * d[m1]));
 }
-__device__ inline void phase_pair(const double *k, int stride, int i0, int i1, const double *d, int m0, int m1, int mask,
+__device__ inline void phase_pair(const double *k, int stride, int i0, int i1, const double *d, int m0, int m1,
                                   Cycles &c0, Cycles &c1) {
 #pragma unroll
-  for (int x = 0; x < 3; ++x)
-    if ((mask >> x) & 1) {
-      c0.add(k[x * stride + i0], k[(x + 3) * stride + i0], d[x * kGemmNodes + m0]);
-      c1.add(k[x * stride + i1], k[(x + 3) * stride + i1], d[x * kGemmNodes + m1]);
-    }
+  for (int x = 0; x < 3; ++x) {
+    c0.add(k[x * stride + i0], k[(x + 3) * stride + i0], d[x * kGemmNodes + m0]);
+    c1.add(k[x * stride + i1], k[(x + 3) * stride + i1], d[x * kGemmNodes + m1]);
+  }
 }
 
 // Row factor of a stage: a thread's elements are pairs of rows at a node, every
 // nt-th of the stage.
 template <typename T>
-__device__ inline void gemm_rows(unsigned char *A, const double *krow, int mask, int rows, const double *d, int cnt, int nt) {
+__device__ inline void gemm_rows(unsigned char *A, const double *krow, int rows, const double *d, int cnt, int nt) {
   const int per = rows / 2;
   const int dm = nt / per, dr = nt - dm * per;
   int m = threadIdx.x / per, r = threadIdx.x - m * per;
   while (m < cnt) {
     if constexpr (sizeof(T) == 4) {
       float re0, im0, re1, im1;
-      double c0, c1;
-      c0 = c1 = 0.0;
-#pragma unroll
-      for (int x = 0; x < 3; ++x)
-        if ((mask >> x) & 1) {
-          const double2 k = reinterpret_cast<const double2 *>(krow + x * rows)[r];
-          const double at = d[x * kGemmNodes + m];
-          c0 = fma(k.x, at, c0);
-          c1 = fma(k.y, at, c1);
-        }
+      const double2 *k = reinterpret_cast<const double2 *>(krow) + r;
+      const double2 kx = k[0], ky = k[per], kz = k[2 * per];
+      const double x = d[m], y = d[kGemmNodes + m], z = d[2 * kGemmNodes + m];
+      const double c0 = fma(kz.x, z, fma(ky.x, y, kx.x * x));
+      const double c1 = fma(kz.y, z, fma(ky.y, y, kx.y * x));
       cis_cycles(c0, re0, im0);
       cis_cycles(c1, re1, im1);
       float2 *a = reinterpret_cast<float2 *>(A) + (m * (per >> 2) + (r >> 2)) * 8 + (r & 3);
@@ -242,7 +230,7 @@ __device__ inline void gemm_rows(unsigned char *A, const double *krow, int mask,
       a[4] = make_float2(im0, im1);
     } else {
       Cycles c0, c1;
-      phase_pair(krow, rows, 2 * r, 2 * r + 1, d, m, m, mask, c0, c1);
+      phase_pair(krow, rows, 2 * r, 2 * r + 1, d, m, m, c0, c1);
       double re0, im0, re1, im1;
       c0.cis(re0, im0);
       c1.cis(re1, im1);
@@ -262,7 +250,7 @@ __device__ inline void gemm_rows(unsigned char *A, const double *krow, int mask,
 // Column factor of a stage: the elements of q at two nodes, then its V columns.
 // `off` columns of q0 lie before the tile.
 template <typename T>
-__device__ inline void gemm_cols(unsigned char *B, const double *kcol, int mask, const unsigned char *slots, int cols, int n_cols,
+__device__ inline void gemm_cols(unsigned char *B, const double *kcol, const unsigned char *slots, int cols, int n_cols,
                                  int nq, int V, int nv, int off, bool runs, const double *d,
                                  const typename GemmType<T>::V2 *w, int cnt, int nt) {
   constexpr int kPer = 2;
@@ -273,7 +261,7 @@ __device__ inline void gemm_cols(unsigned char *B, const double *kcol, int mask,
     T er[kPer], ei[kPer];
     if constexpr (sizeof(T) == 4) {
       double c0, c1;
-      phase_pair(kcol, cols, q, q, d, m, m + 1, mask, c0, c1);
+      phase_pair(kcol, cols, q, q, d, m, m + 1, c0, c1);
       if (runs) {
         const double u = kcol[6 * cols + q] * kInv2Pi;
         c0 = fma(u, d[4 * kGemmNodes + m], c0);
@@ -283,7 +271,7 @@ __device__ inline void gemm_cols(unsigned char *B, const double *kcol, int mask,
       cis_cycles(c1, er[1], ei[1]);
     } else {
       Cycles c0, c1;
-      phase_pair(kcol, cols, q, q, d, m, m + 1, mask, c0, c1);
+      phase_pair(kcol, cols, q, q, d, m, m + 1, c0, c1);
       if (runs) {
         c0.add_turn(d[4 * kGemmNodes + m], kcol[6 * cols + q]);
         c1.add_turn(d[4 * kGemmNodes + m + 1], kcol[6 * cols + q]);
@@ -355,9 +343,7 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
   const T *kc[3] = {p.kx, p.ky, p.kz};
   const int64_t s0 = (int64_t)g * Ls;  // first sample of the slab (runs are slabs here)
   // -k float(pi) / pi, split in two
-  int mask = 0;  // components that are not 0 throughout: rows, columns << 3
-  auto scaled = [&](double *dst, int stride, double k, bool here, int bit) {
-    if (here && k != 0.0) mask |= 1 << bit;
+  auto scaled = [&](double *dst, int stride, double k, bool here) {
     const double hi = here ? -k * kPiRatio : 0.0;
     dst[0] = hi;
     dst[3 * stride] = here ? fma(-k, kPiRatio, -hi) - k * kPiRatioLo : 0.0;
@@ -365,19 +351,13 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
   for (int i = tid; i < rows; i += nt) {
     const int r = row0 + min(i, n_rows - 1);
     const int64_t s = p.runs ? r : s0 + (int64_t)r * p.n_kz;
-    for (int d = 0; d < 3; ++d) scaled(krow + d * rows + i, rows, (double)kc[d][s], !((cm >> d) & 1), d);
+    for (int d = 0; d < 3; ++d) scaled(krow + d * rows + i, rows, (double)kc[d][s], !((cm >> d) & 1));
   }
   for (int i = tid; i < nq; i += nt) {
     const int64_t s = p.runs ? (int64_t)(q0 + i) * Ls : s0 + q0 + i;
-    for (int d = 0; d < 3; ++d) scaled(kcol + d * cols + i, cols, (double)kc[d][s], (cm >> d) & 1, d + 3);
+    for (int d = 0; d < 3; ++d) scaled(kcol + d * cols + i, cols, (double)kc[d][s], (cm >> d) & 1);
     kcol[6 * cols + i] = p.runs ? p.run_t[q0 + i] : 0.0;
   }
-  // a component that is 0 for the whole tile is left out (a node that is not at a
-  // finite place is made not a number in its weights)
-  int masks = 0;
-#pragma unroll
-  for (int b = 0; b < 6; ++b) masks |= __syncthreads_or((mask >> b) & 1) ? 1 << b : 0;
-  const int row_mask = masks & 7, col_mask = masks >> 3;
   const double tg = p.runs ? 0.0 : p.run_t[g];
   const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
   const int64_t n_begin = (int64_t)split * p.chunk, n_end = min(p.N, n_begin + p.chunk);
@@ -403,7 +383,6 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
         tx = tx + t[0]; ty = ty + t[1]; tz = tz + t[2];
       }
       x = (double)tx; y = (double)ty; z = (double)tz;
-      const bool finite = isfinite(x) && isfinite(y) && isfinite(z);
       if (p.runs) {
         f = (double)inv;
         h = (double)phi;
@@ -426,7 +405,6 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
           m.x = o.x * wr - o.y * wi;
           m.y = o.x * wi + o.y * wr;
         }
-        if (!finite) m.x = m.y = T(NAN);
         w[i] = m;
         if (++v == V) v = 0;
       }
@@ -454,8 +432,8 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
     const double *d = node + blk * 5 * kGemmNodes + m0;
     const V2 *w = reinterpret_cast<const V2 *>(smem + L.w) + (blk * kGemmNodes + m0) * nv;
     unsigned char *at = smem + (st & 1) * L.stage;
-    gemm_rows<T>(at + L.a, krow, row_mask, rows, d, cnt, nt);
-    gemm_cols<T>(at + L.b, kcol, col_mask, slots, cols, n_cols, nq, V, nv, off, p.runs, d, w, cnt, nt);
+    gemm_rows<T>(at + L.a, krow, rows, d, cnt, nt);
+    gemm_cols<T>(at + L.b, kcol, slots, cols, n_cols, nq, V, nv, off, p.runs, d, w, cnt, nt);
   };
   // two operand stages: one is formed while the other is multiplied, so a stage
   // costs one barrier and the warps of a block need not be in step.  Node data
@@ -521,9 +499,9 @@ static void gemm_shape(int64_t P, int64_t C, int64_t V, GemmPlan &g) {
 // Node splits: the least estimated time, in operand stages of a block that has
 // its SM to itself.  The blocks of an SM share its arithmetic, so their stages
 // add up, at a rate that grows with the warps there (latency: 8 / warps on top);
-// a block costs about 4 stages to set up and write, and a round of blocks 6 more
+// a block costs about 3 stages to set up and write, and a round of blocks 6 more
 // in latency; partial sums are
-// written and read back at some 5 MB a stage.  Splits of at least 64 nodes and
+// written and read back at some 20 MB a stage.  Splits of at least 64 nodes and
 // 256 MB of partial sums, and at least as many as the unfactored form takes, so
 // that no sum in the form's type is longer than there.
 static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int least) {
@@ -537,7 +515,7 @@ static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int leas
     const int64_t on_sm = ceil_div(units * s, (int64_t)kSmCount);
     const double warps = (double)std::min(on_sm, per_sm) * (g.threads / 32);
     const double cost = (double)on_sm * ((double)N / s / kGemmStage) * (1.0 + 8.0 / warps) +
-                        4.0 * (double)on_sm + 6.0 * (double)ceil_div(on_sm, per_sm) + (s > 1 ? 2.0 * s * (double)out_bytes / 5e6 : 0.0);
+                        3.0 * (double)on_sm + 6.0 * (double)ceil_div(on_sm, per_sm) + (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
     if (s == least || cost < best_cost) {
       best = s;
       best_cost = cost;
