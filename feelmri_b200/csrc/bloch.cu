@@ -6,6 +6,7 @@
 // all time steps; per-step scalars (rf, G, dt, motion weights) are read as
 // warp-uniform loads.  Step i -> i+1 uses rf[i+1], G[i+1], dt[i+1]; dt[0] is
 // ignored; e1/e2 are recomputed only when dt changes (BlochSimulator.cpp:69-99).
+#include <climits>
 #include <mutex>
 
 #include <math_constants.h>
@@ -16,11 +17,19 @@ namespace fm {
 
 // Step segments: runs of consecutive steps with the same dt and the same
 // RF-off state, so that the sweep tests neither per step.  seg[0] holds the
-// count G; seg[1 + g] the first step of segment g with the flags below;
-// seg[1 + G] the number of steps.
+// count G (and kSegWide); seg[1 + g] the first step of segment g with the flags
+// below; seg[1 + G] the number of steps.
 constexpr int kSegNoRf = 1 << 30;  // rf = 0 on every step of the segment
 constexpr int kSegDt = 1 << 29;    // dt changes at the first step (e1, e2 recomputed)
+constexpr int kSegFlat = INT_MIN;  // RF off and the field of a node the same on every step
 constexpr int kSegStep = kSegDt - 1;
+constexpr int kSegWide = kWideFlag;  // seg[0]: some motion weight is not within kWide
+constexpr int kSegCount = kSegWide - 1;
+
+// Where the field of a node stays the same: nowhere; on steps without gradient,
+// where Bz = dB at any finite place; on steps with the gradient of the one
+// before, for nodes that do not move.
+enum { kFlatNone, kFlatNoGradient, kFlatSameGradient };
 
 // Pass of one block of threads over the n_time samples of one solve (or one
 // block of a sequence): step parameters, the dt-changed flags (:72), the step
@@ -28,7 +37,7 @@ constexpr int kSegStep = kSegDt - 1;
 // (BlochSimulator.cpp:82-83) is all that is sequential.  One thread for all of
 // it took 22 us for 709 samples on a B200, this takes 3 us.
 constexpr int kPrepSteps = 256;
-__device__ inline void bloch_prep_range(int64_t n_time, float gamma, const float2 *__restrict__ rf,
+__device__ inline void bloch_prep_range(int64_t n_time, float gamma, int flat_rule, const float2 *__restrict__ rf,
                                         const float *__restrict__ G, const float *__restrict__ dt,
                                         float4 *__restrict__ sa, float4 *__restrict__ sb, int *__restrict__ seg,
                                         double *__restrict__ call_t) {
@@ -53,9 +62,28 @@ __device__ inline void bloch_prep_range(int64_t n_time, float gamma, const float
         const float2 q = rf[i];
         was = q.x == 0.f && q.y == 0.f;
       }
+      const float *g = G + 3 * (i + 1);
+      auto still = [&](const float *h) {  // step with gradient h whose field is that of the segment
+        if (flat_rule == kFlatNoGradient) return h[0] == 0.f && h[1] == 0.f && h[2] == 0.f;
+        return h[0] == h[-3] && h[1] == h[-2] && h[2] == h[-1];
+      };
+      bool flat = false, was_flat = false;
+      if (flat_rule == kFlatNoGradient) {
+        flat = norf && still(g);
+        was_flat = was && still(g - 3);
+      } else if (flat_rule == kFlatSameGradient && i > 0) {
+        bool was2 = false;
+        if (i > 1) {
+          const float2 q = rf[i - 1];
+          was2 = q.x == 0.f && q.y == 0.f;
+        }
+        flat = norf && was && still(g);
+        was_flat = was && was2 && still(g - 3);
+      }
       sa[i] = make_float4(r.x, r.y, __fmaf_rn(r.x, r.x, __fmul_rn(r.y, r.y)), __fmul_rn(mhg, d));
-      sb[i] = make_float4(G[3 * (i + 1) + 0], G[3 * (i + 1) + 1], G[3 * (i + 1) + 2], d);
-      if (i == 0 || changed || norf != was) head = (int)i | (norf ? kSegNoRf : 0) | (changed ? kSegDt : 0);
+      sb[i] = make_float4(g[0], g[1], g[2], d);
+      if (i == 0 || changed || norf != was || flat != was_flat)
+        head = (int)i | (norf ? kSegNoRf : 0) | (changed ? kSegDt : 0) | (flat ? kSegFlat : 0);
       s_t[tid] = d;
     }
     const unsigned heads = __ballot_sync(0xffffffffu, head != -1);
@@ -87,11 +115,12 @@ __device__ inline void bloch_prep_range(int64_t n_time, float gamma, const float
   }
 }
 
-__global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, float gamma, const float2 *__restrict__ rf,
+__global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, float gamma, int flat_rule,
+                                                                const float2 *__restrict__ rf,
                                                                 const float *__restrict__ G, const float *__restrict__ dt,
                                                                 float4 *__restrict__ sa, float4 *__restrict__ sb,
                                                                 int *__restrict__ seg, double *__restrict__ call_t) {
-  bloch_prep_range(n_time, gamma, rf, G, dt, sa, sb, seg, call_t);
+  bloch_prep_range(n_time, gamma, flat_rule, rf, G, dt, sa, sb, seg, call_t);
 }
 
 // Sequence form: a block of threads per block.  Block b's samples start at
@@ -99,12 +128,12 @@ __global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, 
 // more than steps); its segment list at offset_b + b (n_time_b + 1 ints).
 // Its motion calls are the samples offset_b .. offset_b + n_time_b - 1.
 __global__ void __launch_bounds__(kPrepSteps) bloch_seq_prep_kernel(
-    const fm_bloch_block *__restrict__ blocks, float gamma, const float2 *__restrict__ rf, const float *__restrict__ G,
+    const fm_bloch_block *__restrict__ blocks, float gamma, int flat_rule, const float2 *__restrict__ rf, const float *__restrict__ G,
     const float *__restrict__ dt, float4 *__restrict__ sa, float4 *__restrict__ sb, int *__restrict__ seg,
     double *__restrict__ call_t, int *__restrict__ call_block) {
   const int b = blockIdx.x;
   const int64_t o = blocks[b].offset, nt = blocks[b].n_time, step0 = o - b;
-  bloch_prep_range(nt, gamma, rf + o, G + 3 * o, dt + o, sa + step0, sb + step0, seg + o + b,
+  bloch_prep_range(nt, gamma, flat_rule, rf + o, G + 3 * o, dt + o, sa + step0, sb + step0, seg + o + b,
                    call_t ? call_t + o : nullptr);
   if (call_block)
     for (int64_t i = threadIdx.x; i < nt; i += kPrepSteps) call_block[o + i] = b;
@@ -140,6 +169,7 @@ struct BlochNode {
   float2 mxy;
   float mz;
   float e1, e2, rec;  // rec = (1 - e1) M0, recomputed with e1
+  bool within;        // place and modes within kWide
 };
 
 // MODE: 0 static, 1 TERMS with the POD modes of one term in registers,
@@ -157,6 +187,7 @@ __device__ __forceinline__ void bloch_node_load(const BlochDev &p, int64_t n, Bl
   s.mz = p.Mz0[n];
   s.e1 = 0.f; s.e2 = 0.f; s.rec = 0.f;
   s.r_pod = 0;
+  s.within = fabsf(s.x) <= kWide && fabsf(s.y) <= kWide && fabsf(s.z) <= kWide;
   if (MODE == 1 || MODE == 4) {
     const fm_motion_term &T = p.md.terms[p.pod_term];
     s.r_pod = T.n_modes;
@@ -166,6 +197,7 @@ __device__ __forceinline__ void bloch_node_load(const BlochDev &p, int64_t n, Bl
       s.phx[m] = (m < s.r_pod) ? __ldg(Phi + m) : 0.f;
       s.phy[m] = (m < s.r_pod) ? __ldg(Phi + s.r_pod + m) : 0.f;
       s.phz[m] = (m < s.r_pod) ? __ldg(Phi + 2 * s.r_pod + m) : 0.f;
+      s.within = s.within && fabsf(s.phx[m]) <= kWide && fabsf(s.phy[m]) <= kWide && fabsf(s.phz[m]) <= kWide;
     }
   }
 }
@@ -230,10 +262,11 @@ __device__ __forceinline__ void bloch_position(const BlochDev &p, const BlochNod
 }
 
 // One segment of `count` steps (one dt, one RF state; flags from the prep
-// pass), step parameters from sa / sb, first motion call call0.  HIST:
+// pass; flat: a flat segment's field is to be taken from its first step), step
+// parameters from sa / sb, first motion call call0.  HIST:
 // history columns written through hist_m / hist_z (the first step's column).
 template <int MODE, int RMAX, bool HIST>
-__device__ __forceinline__ void bloch_segment(const BlochDev &p, BlochNode<RMAX> &s, int flags, const float4 *sa,
+__device__ __forceinline__ void bloch_segment(const BlochDev &p, BlochNode<RMAX> &s, int flags, bool flat, const float4 *sa,
                                               const float4 *sb, int count, int64_t call0, float2 *hist_m,
                                               float *hist_z) {
   const float *wrow = (MODE == 4) ? p.weights + call0 * p.md.slots + p.md.slot0[p.pod_term] : nullptr;
@@ -252,7 +285,43 @@ __device__ __forceinline__ void bloch_segment(const BlochDev &p, BlochNode<RMAX>
   float2 mxy = s.mxy;
   float mz = s.mz;
   const float e1 = s.e1, e2 = s.e2, rec = s.rec;
-  if (flags & kSegNoRf) {
+  if ((flags & kSegFlat) && (MODE == 0 || MODE == 4) && flat) {
+    // The step below with its field, and so its rotation, formed once.  43% of
+    // the steps of an imaging sequence with spacing blocks: 100,003 nodes with
+    // four modes, 4656 steps, 3180 us -> 1917 us on a B200; 5003 nodes at
+    // rest, 59 steps, 16 us -> 7 us.
+    float c, ca_i, a2, ca2r, ca2i;
+    {
+      const float4 b = *sb;
+      float px, py, pz;
+      bloch_position<MODE, RMAX>(p, s, call0, wrow, px, py, pz);
+      const float Bz = __fadd_rn(fmaf(pz, b.z, fmaf(py, b.y, __fmul_rn(px, b.x))), s.db);
+      const float sq = __fmul_rn(Bz, Bz);
+      float Bn = (sq == CUDART_INF_F) ? sq : fabsf(Bz);
+      Bn = (Bn < 1e-12f) ? 1e-12f : Bn;
+      const float nz = __fmul_rn(Bz, __frcp_rn(Bn));
+      float sn;
+      sincosf(__fmul_rn(Bn, sa->w), &sn, &c);
+      ca_i = nz * sn;
+      a2 = fmaf(c, c, ca_i * ca_i);
+      ca2r = c * c - ca_i * ca_i;
+      ca2i = 2.f * c * ca_i;
+    }
+#pragma unroll 4
+    for (int i = 0; i < count; ++i) {
+      const float nmr = ca2r * mxy.x - ca2i * mxy.y;
+      const float nmi = ca2r * mxy.y + ca2i * mxy.x;
+      mxy.x = nmr * e2;
+      mxy.y = nmi * e2;
+      mz = fmaf(a2 * mz, e1, rec);
+      if (HIST) {
+        *hist_m = mxy;
+        *hist_z = mz;
+        hist_m += p.n;
+        hist_z += p.n;
+      }
+    }
+  } else if (flags & kSegNoRf) {
     // No RF on these steps: beta = 0, so the update reduces to
     // Mxy' = conj(alpha)^2 Mxy, Mz' = |alpha|^2 Mz; the dropped terms of
     // the general form below are exact zeros.  |rf|^2 is 0, and
@@ -365,12 +434,13 @@ __global__ void __launch_bounds__(128) bloch_kernel(BlochDev p) {
     p.Mxy_hist[n] = s.mxy;
     p.Mz_hist[n] = s.mz;
   }
-  const int n_seg = p.seg[0];
+  const int n_seg = p.seg[0] & kSegCount;
+  const bool flat = MODE == 0 || (s.within && !(p.seg[0] & kSegWide));
   const int *segp = p.seg + 1;
   for (int g = 0; g < n_seg; ++g) {
     const int e0 = segp[g];
     const int i0 = e0 & kSegStep, i1 = segp[g + 1] & kSegStep;
-    bloch_segment<MODE, RMAX, HIST>(p, s, e0, p.sa + i0, p.sb + i0, i1 - i0, (int64_t)i0 + 1,
+    bloch_segment<MODE, RMAX, HIST>(p, s, e0, flat, p.sa + i0, p.sb + i0, i1 - i0, (int64_t)i0 + 1,
                                     HIST ? p.Mxy_hist + (int64_t)(i0 + 1) * p.n + n : nullptr,
                                     HIST ? p.Mz_hist + (int64_t)(i0 + 1) * p.n + n : nullptr);
   }
@@ -403,12 +473,13 @@ __global__ void __launch_bounds__(128) bloch_seq_kernel(BlochDev p, BlochSeqDev 
     const fm_bloch_block &B = q.blocks[b];
     const int64_t o = B.offset, step0 = o - b;
     const int *segp = q.seg + o + b;
-    const int n_seg = segp[0];
+    const int n_seg = segp[0] & kSegCount;
+    const bool flat = MODE == 0 || (s.within && !(segp[0] & kSegWide));
     s.e1 = 0.f; s.e2 = 0.f; s.rec = 0.f;
     for (int g = 0; g < n_seg; ++g) {
       const int e0 = segp[1 + g];
       const int i0 = e0 & kSegStep, i1 = segp[2 + g] & kSegStep;
-      bloch_segment<MODE, RMAX, false>(p, s, e0, p.sa + step0 + i0, p.sb + step0 + i0, i1 - i0, o + i0 + 1,
+      bloch_segment<MODE, RMAX, false>(p, s, e0, flat, p.sa + step0 + i0, p.sb + step0 + i0, i1 - i0, o + i0 + 1,
                                        nullptr, nullptr);
     }
     if (B.store >= 0) {
@@ -425,7 +496,8 @@ __global__ void __launch_bounds__(128) bloch_seq_kernel(BlochDev p, BlochSeqDev 
 // timeshifts replace the terms' (update_timeshift(t0) before each block).
 __global__ void motion_weights_seq_kernel(MotionDev md, const double *__restrict__ times, int64_t n_calls,
                                           const int *__restrict__ call_block,
-                                          const fm_bloch_block *__restrict__ blocks, float *__restrict__ weights) {
+                                          const fm_bloch_block *__restrict__ blocks, float *__restrict__ weights,
+                                          int *__restrict__ seg) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_calls * md.slots) return;
   const int64_t c = idx / md.slots;
@@ -443,6 +515,7 @@ __global__ void motion_weights_seq_kernel(MotionDev md, const double *__restrict
   float w = __double2float_rn(v);
   if (T.kind == FM_TERM_POD_VELOCITY) w = __fmul_rn(w, __double2float_rn(t));
   weights[idx] = w;
+  if (!(fabsf(w) <= kWide)) atomicOr(seg + B.offset + call_block[c], kSegWide);
 }
 
 template <int MODE, int RMAX>
@@ -526,6 +599,15 @@ static void dispatch_bloch_mode(const MotionDev &md, int &pod_term, L &l) {
       l.template run<1, 32>();
     }
   }
+}
+
+// Which steps have a node's field in common, by what dispatch_bloch_mode takes.
+static int flat_rule(const MotionDev &md) {
+  if (md.kind == FM_MOTION_NONE) return kFlatSameGradient;
+  if (md.kind == FM_MOTION_TERMS && md.n_terms == 1 && md.terms[0].kind != FM_TERM_RESPIRATORY &&
+      md.terms[0].n_modes <= 32)
+    return kFlatNoGradient;
+  return kFlatNone;
 }
 
 struct SolveLaunch {
@@ -635,11 +717,11 @@ int fm_bloch_solve_f32(fm_ctx *ctx, const fm_bloch_args *a, void *workspace, siz
   if (a->n_pos == 0) return FM_OK;
 
   const MotionDev md = make_motion_dev(a->motion);
-  bloch_prep_kernel<<<1, kPrepSteps, 0, st>>>(a->n_time, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa,
+  bloch_prep_kernel<<<1, kPrepSteps, 0, st>>>(a->n_time, a->gamma, flat_rule(md), reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa,
                                      sb, seg, md.kind == FM_MOTION_TERMS ? call_t : nullptr);
   count_launch();
   FM_TRY(check_launch("bloch_prep_kernel"));
-  FM_TRY(launch_motion_weights(md, call_t, a->n_time, weights, st));
+  FM_TRY(launch_motion_weights(md, call_t, a->n_time, weights, st, seg));
 
   BlochDev p{};
   p.n = a->n_pos;
@@ -694,14 +776,14 @@ int fm_bloch_sequence_f32(fm_ctx *ctx, const fm_bloch_sequence_args *a, void *wo
                           st));
   const bool terms = md.kind == FM_MOTION_TERMS;
   bloch_seq_prep_kernel<<<(unsigned)a->n_blocks, kPrepSteps, 0, st>>>(
-      w.blocks, a->gamma, reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, w.sa, w.sb, w.seg,
+      w.blocks, a->gamma, flat_rule(md), reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, w.sa, w.sb, w.seg,
       terms ? w.call_t : nullptr, terms ? w.call_block : nullptr);
   count_launch();
   FM_TRY(check_launch("bloch_seq_prep_kernel"));
   if (terms) {
     const int64_t total = a->n_samples * md.slots;
     motion_weights_seq_kernel<<<(unsigned)ceil_div(total, 128), 128, 0, st>>>(md, w.call_t, a->n_samples,
-                                                                               w.call_block, w.blocks, w.weights);
+                                                                               w.call_block, w.blocks, w.weights, w.seg);
     count_launch();
     FM_TRY(check_launch("motion_weights_seq_kernel"));
   }

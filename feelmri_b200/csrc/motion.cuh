@@ -129,9 +129,14 @@ __device__ inline float motion_weight(const MotionDev &md, int s, double t) {
 
 int validate_motion(const fm_motion *m, int64_t n_nodes, const char *who);
 
-// Fills weights[c * slots + s] for n_calls call times (device array).
+// Sums of up to 32 products of numbers within kWide are finite.
+constexpr float kWide = 1e15f;
+constexpr int kWideFlag = 1 << 30;
+
+// Fills weights[c * slots + s] for n_calls call times (device array); sets
+// kWideFlag in *wide (unless null) where a weight is not within kWide.
 int launch_motion_weights(const MotionDev &md, const double *times_dev, int64_t n_calls, float *weights,
-                          cudaStream_t st);
+                          cudaStream_t st, int *wide = nullptr);
 
 // Displacement of node n at one call from the weights of that call.
 __device__ inline void motion_disp(const MotionDev &md, const float *__restrict__ w, int64_t n, int64_t n_nodes,

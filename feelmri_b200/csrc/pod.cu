@@ -36,19 +36,22 @@ int validate_motion(const fm_motion *m, int64_t n_nodes, const char *who) {
 
 // One thread per (call, slot).
 __global__ void motion_weights_kernel(MotionDev md, const double *__restrict__ times, int64_t n_calls,
-                                      float *__restrict__ weights) {
+                                      float *__restrict__ weights, int *__restrict__ wide) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_calls * md.slots) return;
   const int64_t c = idx / md.slots;
-  weights[idx] = motion_weight(md, (int)(idx - c * md.slots), times[c]);
+  const float w = motion_weight(md, (int)(idx - c * md.slots), times[c]);
+  weights[idx] = w;
+  if (wide && !(fabsf(w) <= kWide)) atomicOr(wide, kWideFlag);
 }
 
 int launch_motion_weights(const MotionDev &md, const double *times_dev, int64_t n_calls, float *weights,
-                          cudaStream_t st) {
+                          cudaStream_t st, int *wide) {
   if (md.kind != FM_MOTION_TERMS || n_calls == 0) return FM_OK;
   const int64_t total = n_calls * md.slots;
   const int threads = 128;
-  motion_weights_kernel<<<(unsigned)ceil_div(total, threads), threads, 0, st>>>(md, times_dev, n_calls, weights);
+  motion_weights_kernel<<<(unsigned)ceil_div(total, threads), threads, 0, st>>>(md, times_dev, n_calls, weights,
+                                                                                   wide);
   count_launch();
   return check_launch("motion_weights_kernel");
 }
