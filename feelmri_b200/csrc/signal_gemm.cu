@@ -28,8 +28,8 @@
 //
 // Kernel time on a B200, one sin/cos per node-sample (signal_plain_kernel)
 // against this: FP32 50,021 nodes x 48 runs x 48 lines x 16 kz x 4 columns with
-// flow 6152 us -> 1970 us (the multiply-adds alone take 820 us), FP64 20,011
-// nodes x 64 runs x 64 lines 1403 us -> 67 us (multiply-adds 18 us).
+// flow 6152 us -> 2050 us (the multiply-adds alone take 820 us), FP64 20,011
+// nodes x 64 runs x 64 lines 1403 us -> 68 us (multiply-adds 18 us).
 #include <algorithm>
 
 #include "cycles.cuh"
@@ -40,6 +40,10 @@ namespace fm {
 
 constexpr int kGemmNodes = 32;  // nodes whose data are formed at a time
 constexpr int kGemmStage = 16;  // nodes per operand stage
+// Stages summed in registers before their sum is added to the output.  Rounding
+// of one long sum is the largest error of the FP32 form: on 200,740 nodes
+// 1.4e-5, and 2.5e-6 with the sums cut, for 4% of the time.
+constexpr int kGemmFold = 2048 / kGemmStage;
 constexpr int kGemmCols = 4;    // columns per thread
 constexpr int kGemmSlots = 16 * kGemmCols;
 constexpr int kGemmMaxThreads = 256;
@@ -414,7 +418,6 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
     d[0] = x; d[kGemmNodes] = y; d[2 * kGemmNodes] = z; d[3 * kGemmNodes] = f; d[4 * kGemmNodes] = h;
   };
   GemmAcc<T> acc;
-  acc.clear();
   const int tr = tid / TC, tc = tid - tr * TC;
   const bool works = tr < TR;
   unsigned char *slots = smem + L.slot;
@@ -443,7 +446,9 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
   if (n_stages > 0) form_stage(0);
   __syncthreads();
   int turn = 0;
-  for (int st = 0; st < n_stages; ++st) {
+  for (int fold = 0; fold == 0 || fold < n_stages; fold += kGemmFold) {
+  acc.clear();
+  for (int st = fold; st < min(n_stages, fold + kGemmFold); ++st) {
     if (st % kPerBlock == 0 && st + kPerBlock < n_stages) {
       turn = turn + 1 == warps ? 0 : turn + 1;
       form_nodes(st / kPerBlock + 1, turn);
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
     }
     __syncthreads();
   }
-  if (!works) return;
+  if (!works) continue;
   V2 *dst = reinterpret_cast<V2 *>(p.out) + (int64_t)split * p.S * p.V;
 #pragma unroll
   for (int i = 0; i < RT; ++i) {
@@ -474,8 +479,15 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
       if (c >= n_cols) continue;
       const int q = (col0 + c) / V, v = col0 + c - q * V;
       const int64_t s = p.runs ? (int64_t)q * Ls + row0 + r : s0 + (int64_t)(row0 + r) * p.n_kz + q;
-      dst[s * p.V + v] = acc.get(i, j);
+      V2 sum = acc.get(i, j);
+      if (fold > 0) {
+        const V2 before = dst[s * p.V + v];
+        sum.x += before.x;
+        sum.y += before.y;
+      }
+      dst[s * p.V + v] = sum;
     }
+  }
   }
 }
 
@@ -499,9 +511,9 @@ static void gemm_shape(int64_t P, int64_t C, int64_t V, GemmPlan &g) {
 // Node splits: the least estimated time, in operand stages of a block that has
 // its SM to itself.  The blocks of an SM share its arithmetic, so their stages
 // add up, at a rate that grows with the warps there (latency: 8 / warps on top);
-// a block costs about 3 stages to set up and write, and a round of blocks 6 more
-// in latency; partial sums are
-// written and read back at some 20 MB a stage.  Splits of at least 64 nodes and
+// a block costs about 3 stages to set up and write, and a round of blocks 30 more
+// in latency and uneven ends; partial sums are written and read back at some 20 MB
+// a stage.  Splits of at least 64 nodes and
 // 256 MB of partial sums, and at least as many as the unfactored form takes, so
 // that no sum in the form's type is longer than there.
 static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int least) {
@@ -515,7 +527,7 @@ static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int leas
     const int64_t on_sm = ceil_div(units * s, (int64_t)kSmCount);
     const double warps = (double)std::min(on_sm, per_sm) * (g.threads / 32);
     const double cost = (double)on_sm * ((double)N / s / kGemmStage) * (1.0 + 8.0 / warps) +
-                        3.0 * (double)on_sm + 6.0 * (double)ceil_div(on_sm, per_sm) + (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
+                        3.0 * (double)on_sm + 30.0 * (double)ceil_div(on_sm, per_sm) + (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
     if (s == least || cost < best_cost) {
       best = s;
       best_cost = cost;

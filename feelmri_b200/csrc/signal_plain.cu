@@ -146,9 +146,10 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<do
 // there.  Bound by issue: per sample-node some 40 instructions for the phase and
 // its sin/cos and 4 a column, 77% of the issue rate.  20,011 nodes x 128 runs x
 // 255 samples x 8 columns on a B200: 2944 us with sincosf of a rounded phase, one
-// sample per thread and tiles dealt out split by split, 1730 us now.
+// sample per thread and tiles dealt out split by split, 1830 us now.
 constexpr int kPlain32Threads = 128;
 constexpr int kPlainNodes = 128;  // nodes staged at a time
+constexpr int kPlainFold = 2048;  // nodes in one sum: a longer one is the largest error of the form
 template <int VMAX>
 __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(PlainDev<float> p, int v0) {
   __shared__ double4 s_pos[kPlainNodes];         // moved x, y, z and phi t in cycles
@@ -169,14 +170,17 @@ __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(Plai
     const double kx0 = scaled(p.kx, s0), ky0 = scaled(p.ky, s0), kz0 = scaled(p.kz, s0);
     const double kx1 = scaled(p.kx, s1), ky1 = scaled(p.ky, s1), kz1 = scaled(p.kz, s1);
     float2 acc0[VMAX], acc1[VMAX];
+    // nodes are rows of a sparse matrix of 32-bit indices
+    const int n_begin = (int)((int64_t)split * p.chunk);
+    const int n_end = (int)min(p.N, n_begin + p.chunk);
+    const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
+    // a sum of kPlainFold nodes in registers at a time, then added to the output
+    for (int fold = n_begin;;) {
+      const int fold_end = fold + min(kPlainFold, n_end - fold);
 #pragma unroll
     for (int v = 0; v < VMAX; ++v) acc0[v] = acc1[v] = make_float2(0.f, 0.f);
-
-    const int64_t n_begin = (int64_t)split * p.chunk;
-    const int64_t n_end = min(p.N, n_begin + p.chunk);
-    const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
-    for (int64_t nb = n_begin; nb < n_end; nb += kPlainNodes) {
-      const int cnt = (int)min((int64_t)kPlainNodes, n_end - nb);
+    for (int nb = fold; nb < fold_end; nb += kPlainNodes) {
+      const int cnt = min(kPlainNodes, fold_end - nb);
       __syncthreads();
       for (int j = threadIdx.x; j < cnt; j += kPlain32Threads) {
         const int64_t n = nb + j;
@@ -222,10 +226,20 @@ __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(Plai
     }
 
     float2 *dst = reinterpret_cast<float2 *>(p.out) + (int64_t)split * p.S * p.V + v0;
+    auto put = [&](float2 &to, float2 sum) {
+      if (fold > n_begin) {
+        sum.x += to.x;
+        sum.y += to.y;
+      }
+      to = sum;
+    };
 #pragma unroll
     for (int v = 0; v < VMAX; ++v) {
-      if (v < nv && s0 < s_end) dst[(int64_t)s0 * p.V + v] = acc0[v];
-      if (v < nv && s1 < s_end) dst[(int64_t)s1 * p.V + v] = acc1[v];
+      if (v < nv && s0 < s_end) put(dst[(int64_t)s0 * p.V + v], acc0[v]);
+      if (v < nv && s1 < s_end) put(dst[(int64_t)s1 * p.V + v], acc1[v]);
+    }
+    fold = fold_end;
+    if (fold >= n_end) break;
     }
   }  // tiles
 }

@@ -169,3 +169,23 @@ def test_unfactored_form(cuda, res, V, n, motion):
         r1 = r0.copy()
         r1[0, 1] = bad
         assert np.isnan(Signal(0, M, traj.points, traj.t, r1, phi, T2, Mxy, pod)).all()
+
+
+@pytest.mark.parametrize("kind,res,dtype,tol", [
+    ("cartesian", (600, 8, 2), np.float32, 1e-5),  # factored
+    ("cartesian", (600, 8, 2), np.float64, 1e-6),  # displacements are FP32 numbers
+    ("radial", (600, 40, 1), np.float32, 1e-5),    # unfactored
+])
+def test_sums_cut_within_a_node_range(cuda, kind, res, dtype, tol):
+    """So many runs that a node range is longer than one sum in registers."""
+    n, V = 12000, 2
+    r0, M, Mxy, phi, T2 = _case(n, V)
+    traj = _traj(kind, res)
+    pod = W.sinusoidal_pod(n, n_modes=2, amp=1e-3, period=50.0, n_frames=8)
+    c = lambda a: np.asarray(a, dtype)
+    pts, args = tuple(c(p) for p in traj.points), (c(traj.t), c(r0), c(phi), c(T2))
+    K = Signal(0, M, pts, *args, Mxy.astype(np.complex64 if dtype == np.float32 else np.complex128), pod)
+    pick = np.random.default_rng(2).permutation(traj.t.size)[:300]
+    disp = np.stack([pod(x) for x in signal_call_times(args[0])[1:]])
+    ref = fp64.signal(sp.csc_matrix(M), *pts, *args, Mxy, pi_mode="float", disp=disp, sample_idx=pick)
+    assert fp64.rel_l2(K.reshape(-1, V)[pick], ref) < tol
