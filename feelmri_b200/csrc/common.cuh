@@ -27,6 +27,10 @@ struct fm_ctx {
 
 namespace fm {
 
+// SM count of a B200; sizes grids and split-K fan-out so workspace queries need no
+// device.
+constexpr int kSmCount = 148;
+
 // Thread-local last error (read through fm_last_error).
 void set_error(int code, const char *fmt, ...);
 int last_code();

@@ -8,8 +8,6 @@ namespace fm {
 
 // Samples per tile of the plain (CUDA-core) forms.
 constexpr int kPlainThreads = 256;
-// SM count of a B200; sizes split-K fan-out so workspace queries need no device.
-constexpr int kSmCount = 148;
 
 // CSR view of the sparse mass matrix, rows in Eigen's accumulation order.
 struct Csr {

@@ -78,3 +78,21 @@ def test_moving_steps(cuda, modes):
     pod.update_timeshift(np.float32(np.nan))
     m, z = _solve(rf, 0 * G, dt, r0, Mxy, Mz, dB, T1, T2, pod)
     assert np.isnan(m[:, 1:]).all()
+
+
+@pytest.mark.parametrize("n", [1, 129, 148 * 128, 148 * 128 + 1])
+def test_one_launch_and_two(cuda, n):
+    """257 steps are prepared by their own launch, the first 256 of them (up to
+    148 blocks of nodes) within the sweep: the same bits."""
+    rng = np.random.default_rng(11)
+    rf, G, dt = (np.concatenate([a, a[1:], a[1:]]) for a in _steps(4))
+    rf, G, dt = rf[:258], G[:258], dt[:258]
+    assert rf.size == 258
+    r0 = rng.uniform(-0.05, 0.05, (n, 3)).astype(np.float32)
+    T1, T2 = np.full(n, 1000, np.float32), np.full(n, 80, np.float32)
+    dB = rng.normal(0, 1e-4, n).astype(np.float32)
+    Mxy, Mz = np.full(n, 0.3 - 0.2j, np.complex64), np.full(n, 0.7, np.float32)
+    m, z = _solve(rf, G, dt, r0, Mxy, Mz, dB, T1, T2, None)
+    a, b = _solve(rf[:257], G[:257], dt[:257], r0, Mxy, Mz, dB, T1, T2, None)
+    np.testing.assert_array_equal(a, m[:, :257])
+    np.testing.assert_array_equal(b, z[:, :257])
