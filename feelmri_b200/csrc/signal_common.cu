@@ -279,9 +279,17 @@ struct Cplx<double> {
   using type = double2;
 };
 
-// The whole problem goes through a factored CUDA-core form.
-__device__ inline bool prep_covered(const PrepDev &p) {
-  return prep_form(p.run_cover, p.slab_cover, p.ctl) != kFormPlain;
+// A TABLE motion must hold one entry per run: a shorter one would be read past
+// its end, so a problem without them is given no work at all (its error word is
+// set, and the call reports it).
+__device__ inline bool prep_table_mismatch(const PrepDev &p) {
+  return p.table_calls >= 0 && p.table_calls != p.ctl[kCtlRuns];
+}
+
+// Nothing of the problem is listed: it goes through a factored CUDA-core form as
+// a whole, or has no work.
+__device__ inline bool prep_unlisted(const PrepDev &p) {
+  return prep_table_mismatch(p) || prep_form(p.run_cover, p.slab_cover, p.ctl) != kFormPlain;
 }
 
 // Factored runs (fac) and tiles of the others (tiles) that run g opens.
@@ -318,11 +326,11 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
       p.weights[idx] = motion_weight(p.md, (int)(idx - g * p.md.slots), p.run_t[g]);
     }
   }
-  if (tid == 0 && p.table_calls >= 0 && p.table_calls != n_runs) atomicOr(p.ctl + kCtlError, kErrTableCalls);
+  if (tid == 0 && prep_table_mismatch(p)) atomicOr(p.ctl + kCtlError, kErrTableCalls);
   const int c = blockIdx.x;
   if (c >= p.n_chunks) return;
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = prep_covered(p) ? 0 : min(n_runs, (c + 1) * per);
+  const int g1 = prep_unlisted(p) ? 0 : min(n_runs, (c + 1) * per);
   int nf = 0, nt = 0;
   for (int g = c * per + threadIdx.x; g < g1; g += kPrepThreads) {
     bool fac;
@@ -421,7 +429,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_fill_kernel(const PrepDev *
   int t0 = block_prefix(p.chunk_tiles, c);
   const int n_runs = p.ctl[kCtlRuns];
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = prep_covered(p) ? 0 : min(n_runs, (c + 1) * per);
+  const int g1 = prep_unlisted(p) ? 0 : min(n_runs, (c + 1) * per);
   for (int gb = c * per; gb < g1; gb += kPrepThreads) {
     const int g = gb + threadIdx.x;
     bool fac = false;

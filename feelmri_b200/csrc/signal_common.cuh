@@ -92,9 +92,11 @@ __device__ inline bool prep_slab(const int *ctl) {
   return !(f & kFlagRuns) && ((f / kFlagAlongKz) & (f / kFlagOverLines) & 7) == 0;
 }
 
-// The CUDA-core form that sums a problem.
+// The CUDA-core form that sums a problem.  A problem whose motion table does not
+// match its runs goes to the unfactored form, for which it has no tiles.
 enum { kFormRuns, kFormSlabs, kFormPlain };
 __device__ inline int prep_form(bool run_cover, bool slab_cover, const int *ctl) {
+  if (ctl[kCtlError] & kErrTableCalls) return kFormPlain;
   return run_cover && prep_static(ctl) ? kFormRuns : (slab_cover && prep_slab(ctl) ? kFormSlabs : kFormPlain);
 }
 
