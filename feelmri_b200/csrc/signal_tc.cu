@@ -424,10 +424,15 @@ __device__ inline void tc_out_sample(const TcDev &p, const TcUnit &U, int row, i
   s_row = p.start[U.it.run + r] + (p.kind == kTcSlab ? (int64_t)line * p.n_kz + U.it.q0 : line);
 }
 
-// Bounded wait that gives up at once after any earlier timeout of the block
-// (the flag lives in shared memory), so a broken pipeline ends quickly.
+// Bounded wait; false when it ran out, and at once after any earlier one of the
+// block did (the flag lives in shared memory).  The MMA and node roles end with a
+// failed wait; the operand warps, which share a barrier, walk on without waiting
+// to the end of their unit and leave there together.  So a block ends soon after
+// the first wait that ran out, whatever work is left.  Every arrival but the copies'
+// is a single one: arrivals that no wait made room for then complete phases that
+// nobody trusts any more, where a count above what a phase has left would fault.
 __device__ inline bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-  if (ptx::mbar_try_wait_long(bar, parity)) return true;
+  if (ptx::mbar_test_wait(bar, parity)) return true;
   if (*abort_flag) return false;
   if (ptx::mbar_wait(bar, parity, kTcWaitNs)) return true;
   *abort_flag = 1;
@@ -939,13 +944,13 @@ __device__ __forceinline__ void tc_issue(uint32_t stage_addr, uint32_t tmem, uin
 // uniform registers: an MMA issues in 40 cycles, against 100 under a lane
 // predicate (whatever its shape), and a commit adds none, against 80-230.
 template <bool kNarrow>
-__device__ __forceinline__ void tc_mma_unit(const TcGeom &G, TcBars *bars, uint32_t stages, uint32_t tmem, int NT,
+__device__ __forceinline__ bool tc_mma_unit(const TcGeom &G, TcBars *bars, uint32_t stages, uint32_t tmem, int NT,
                                             int nst, TcRing &r, uint32_t &group, volatile int *abort_flag) {
   const uint32_t idesc = ptx::idesc_bf16_f32(kTcRows, NT), idesc2 = ptx::idesc_bf16_f32(kTcRows, 2 * NT);
   for (int st = 0; st < nst; ++st) {
     const bool first = (st % kTcDrain) == 0;
-    if (first) tc_wait(&bars->accfree, (group & 1) ^ 1, abort_flag);
-    tc_wait(&bars->full[r.slot], r.phase, abort_flag);
+    if (first && !tc_wait(&bars->accfree, (group & 1) ^ 1, abort_flag)) return false;
+    if (!tc_wait(&bars->full[r.slot], r.phase, abort_flag)) return false;
     ptx::tc_fence_after();
     tc_issue<kNarrow>(stages + r.slot * G.stage_bytes, tmem, idesc, idesc2, (uint32_t)NT * 64 >> 4, first);
     ptx::mma_commit(&bars->empty[r.slot]);
@@ -955,6 +960,7 @@ __device__ __forceinline__ void tc_mma_unit(const TcGeom &G, TcBars *bars, uint3
     }
     r.advance(1, G.ring);
   }
+  return true;
 }
 
 __device__ __forceinline__ void tc_role_mma(const TcBatchDev &B, TcBars *bars, uint32_t stages, uint32_t tmem,
@@ -967,8 +973,9 @@ __device__ __forceinline__ void tc_role_mma(const TcBatchDev &B, TcBars *bars, u
       const int e = tc_entry_of(B, u);
       const TcDev &p = B.entries[e];
       const int NT = p.NT, nst = tc_unit(p, tc_work(p), u - B.offsets[e]).n_stages;
-      if (tc_narrow(NT)) tc_mma_unit<true>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
-      else tc_mma_unit<false>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
+      const bool ok = tc_narrow(NT) ? tc_mma_unit<true>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag)
+                                    : tc_mma_unit<false>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
+      if (!ok) break;
     }
     // all issued MMAs complete before the tensor memory is released
     ptx::mma_commit(&bars->done);
@@ -1008,12 +1015,14 @@ __device__ __forceinline__ void tc_role_nodes(const TcBatchDev &B, TcBars *bars,
     for (int blk = first; blk < n_blocks; blk += 2) {
       const uint32_t b = nr.slot;
       const bool now = staged(blk);
-      tc_wait(&bars->nodeempty[b], nr.phase ^ 1, abort_flag);
+      bool ok = tc_wait(&bars->nodeempty[b], nr.phase ^ 1, abort_flag);
       if (now) {
-        tc_wait(&bars->rawfull[d], rs & 1, abort_flag);
+        // a copy in flight is waited for even where the block gives up: it must not
+        // land in the shared memory of another
+        if (!ptx::mbar_wait(&bars->rawfull[d], rs & 1, kTcWaitNs)) *abort_flag = 1, ok = false;
         ++rs;
       }
-      __syncwarp();  // the derive exchanges values between lanes
+      if (!__all_sync(0xffffffffu, ok)) return;  // (also converges the warp: the derive exchanges values between lanes)
       int rmax = tc_derive(p, a, n_at(blk), U.n_end, now, now ? tc_raw_view(staging, a.mm_ld) : none,
                            smem + G.pos + b * kTcPosBytes, w_all + b * G.wrows * 2 * kWStride, lane);
       rmax = __reduce_max_sync(0xffffffffu, rmax);
@@ -1102,7 +1111,7 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
       }
       const uint32_t row_off = sw64_offset(row, 0), row_off1 = sw64_offset(row, 16);
       const int d_k2 = ((row >> 1) & 1) != 0 ? -16 : 16;
-      const uint32_t arrive = rg != 0 ? 1 : kTcStageArrivals - (nrg - 1) - (generic ? 0 : b_per);
+      const int arrive = rg != 0 ? 1 : kTcStageArrivals - (nrg - 1) - (generic ? 0 : b_per);
       r.seek(stage0 + grp, ring);
       for (int st = grp; st < nst; st += a_groups) {
         if (drains) fold_before(st);
@@ -1123,7 +1132,7 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
         }
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_n(&bars->full[r.slot], arrive);
+        if (lane < arrive) ptx::mbar_arrive(&bars->full[r.slot]);
         if (st + a_groups >= nst || (st + a_groups) / kTcStagesPerBlock > blk) release();
         r.advance(a_groups, ring);
       }
@@ -1184,8 +1193,9 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
     // with them the other warps, may wait for them
     if (drains) fold_before(nst + kTcDrain + (int)ring);
     // every warp has written its stages of this unit, so that none starts the
-    // next unit's turns more than a round of the ring ahead of the MMAs
-    ptx::named_barrier(2, 32 * kTcOperandWarps);
+    // next unit's turns more than a round of the ring ahead of the MMAs; after a
+    // wait that ran out, all leave here together
+    if (ptx::named_barrier_or(2, 32 * kTcOperandWarps, *abort_flag)) break;
     // every phase of the unit had |k . r| <= kmax rmax: the fixed-point
     // reduction holds below 2^28 cycles (2^27 leaves a margin)
     if (kmax >= 0 && !((double)__int_as_float(kmax) * (double)__int_as_float(rmax) < 134217728.0))

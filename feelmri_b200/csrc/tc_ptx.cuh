@@ -28,22 +28,6 @@ __device__ inline void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-__device__ inline void mbar_arrive_n(uint64_t *bar, uint32_t n) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
-}
-
-__device__ inline bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // Non-blocking test of the phase of `parity`.
 __device__ inline bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
@@ -102,8 +86,18 @@ __device__ inline void bulk_copy_g2s(void *dst_smem, const void *src_gmem, uint3
 // (the tensor core reading its operands).
 __device__ inline void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-__device__ inline void named_barrier(uint32_t id, uint32_t threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+// Barrier of `threads` threads that tells each whether `v` held in any of them.
+__device__ inline bool named_barrier_or(uint32_t id, uint32_t threads, bool v) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %3, 0;\n\t"
+      "bar.red.or.pred p, %1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any)
+      : "r"(id), "r"(threads), "r"((uint32_t)v)
+      : "memory");
+  return any != 0;
 }
 
 // ---- tensor memory ------------------------------------------------------
