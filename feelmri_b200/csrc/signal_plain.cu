@@ -287,12 +287,14 @@ static void launch_plain(const PlainDev<T> &p, int64_t max_tiles, int v0, cudaSt
 
 // Split count for slabs cut to `tiles` tiles: the most tiles that a block takes,
 // over the splits, and 1% a split for its partial sums; at least 1024 nodes a
-// split.  128 tiles go to 592 blocks in 9 splits, 2 for each block and 0.22 of a
-// tile's time; in the fewest splits that give every block one (5), it is 0.4.
-static int choose_splits(int64_t tiles, int64_t N) {
+// split and 256 MB of partial sums (`out_bytes` a split).  128 tiles go to 592
+// blocks in 9 splits, 2 for each block and 0.22 of a tile's time; in the fewest
+// splits that give every block one (5), it is 0.4.
+constexpr int64_t kPartialBytes = 256LL << 20;
+static int choose_splits(int64_t tiles, int64_t N, int64_t out_bytes) {
   int best = 1;
   double best_cost = 0.0;
-  for (int s = 1; s <= 64 && (s == 1 || N / s >= 1024); ++s) {
+  for (int s = 1; s <= 64 && (s == 1 || (N / s >= 1024 && s * out_bytes <= kPartialBytes)); ++s) {
     const double cost = (double)ceil_div(tiles * s, (int64_t)kPlainBlocks) / s * (1.0 + 0.01 * s);
     if (s == 1 || cost < best_cost) {
       best = s;
@@ -320,7 +322,8 @@ static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   int *ctl = c.take<int>(kCtlWords);
   pl.dev = c.take<PrepDev>(1);
   carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
-  pl.splits = choose_splits(S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1, N);
+  pl.splits = choose_splits(S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1, N,
+                            S * V * 2 * (int64_t)sizeof(T));
   plan_gemm<T>(a, pl.prep, pl.splits, pl.gemm);
   const int most = std::max(pl.splits, std::max(pl.gemm[0].splits, pl.gemm[1].splits));
   pl.partials = most > 1 ? c.take<T>((size_t)most * S * V * 2) : nullptr;

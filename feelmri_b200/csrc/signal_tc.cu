@@ -1382,11 +1382,13 @@ struct TcPlan {
 };
 
 // Most node splits of a problem: 16 while their partial sums stay within a
-// gigabyte, more for small outputs (up to 64 in 32 MB), which have few units.
-static int tc_max_splits(int64_t S, int64_t V) {
+// gigabyte, more for small outputs (up to 64 in 32 MB, of a node block at least),
+// which have few units.
+static int tc_max_splits(int64_t S, int64_t V, int64_t N) {
   const int64_t bytes_per = S * V * 8;
   if (bytes_per <= 0) return 1;
-  const int64_t s = std::min<int64_t>(16, (1LL << 30) / bytes_per), small = std::min<int64_t>(64, (32LL << 20) / bytes_per);
+  const int64_t s = std::min<int64_t>(16, (1LL << 30) / bytes_per);
+  const int64_t small = std::min(std::min<int64_t>(64, (32LL << 20) / bytes_per), ceil_div(N, (int64_t)kTcBlockNodes));
   return (int)std::max<int64_t>(1, std::max(s, small));
 }
 
@@ -1396,7 +1398,7 @@ static void carve_tc(Carve &c, const fm_signal_args *a, int *ctl, TcPlan &pl) {
   const int64_t S = a->n_ro * a->n_lines * a->n_kz;
   pl.n_groups = tc_groups(a->n_vencs);
   carve_prep(c, a, kTcRows, true, kTcVGroup, sizeof(float), ctl, pl.prep);
-  pl.max_splits = tc_max_splits(S, a->n_vencs);
+  pl.max_splits = tc_max_splits(S, a->n_vencs, a->n_nodes);
   pl.partials = c.take<float2>((size_t)pl.max_splits * S * a->n_vencs);
 }
 
