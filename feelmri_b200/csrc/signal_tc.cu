@@ -73,8 +73,12 @@ constexpr int kTcMmaWarp = 15;
 // into an FP32 round-to-nearest running sum (also in tensor memory).  The
 // tensor core's FP32 accumulation truncates, so its error grows with the
 // number of MMAs added into one accumulator; 32 stages (512 nodes, 192 MMAs)
-// keep it near 1e-5.
-constexpr int kTcDrain = 32;
+// keep it near 1e-5.  On wide tiles all three products go to one accumulator, on
+// narrow ones two (tensor memory below): where runs are columns, which makes wide
+// tiles of problems that had narrow ones, 21 stages (126 MMAs) keep the error at
+// that of a narrow tile's 32 (128 MMAs).  512 like nodes are off by
+// 4.0e-6 of their sum on a narrow tile, by 5.2e-6 on a wide one with 32, 2.6e-6 with 21.
+constexpr int kTcDrain = 32, kTcDrainRuns = 21;
 // Node buffers: one is written while others are still read.  The operand
 // warps are up to a ring apart, so with two buffers of eight stages the next
 // block was often late.
@@ -123,6 +127,7 @@ struct TcDev {
   const int2 *tiles;  // tiles of the generic runs
   int *ctl;           // control words of the problem
   int Qt, NT, kind;
+  int drain;         // stages of an accumulation group
   int RU;            // lines per stacked unit
   int use_runs;      // runs become columns where k factors that way (kTcRuns)
   int prob, first, n_of, max_splits;  // the problem, its first entry and its entries
@@ -367,6 +372,7 @@ struct TcUnit {
   int start;      // first sample of the first run
   int P;          // lines per run (factored) or samples of the run
   int split, Q_tile, n_stages, n_groups;
+  int drain;      // TcDev::drain
   int rows;       // active A rows
   int64_t n_begin, n_end;
 };
@@ -384,7 +390,8 @@ __device__ inline TcUnit tc_unit(const TcDev &p, const TcWork &W, int u) {
   U.n_begin = (int64_t)U.split * W.chunk;
   U.n_end = min(p.N, U.n_begin + W.chunk);
   U.n_stages = U.n_end > U.n_begin ? (int)ceil_div(U.n_end - U.n_begin, kTcNodes) : 0;
-  U.n_groups = (int)ceil_div(U.n_stages, kTcDrain);
+  U.drain = p.drain;
+  U.n_groups = (U.n_stages + U.drain - 1) / U.drain;
   return U;
 }
 
@@ -945,18 +952,21 @@ __device__ __forceinline__ void tc_issue(uint32_t stage_addr, uint32_t tmem, uin
 // predicate (whatever its shape), and a commit adds none, against 80-230.
 template <bool kNarrow>
 __device__ __forceinline__ bool tc_mma_unit(const TcGeom &G, TcBars *bars, uint32_t stages, uint32_t tmem, int NT,
-                                            int nst, TcRing &r, uint32_t &group, volatile int *abort_flag) {
+                                            int nst, int drain, TcRing &r, uint32_t &group,
+                                            volatile int *abort_flag) {
   const uint32_t idesc = ptx::idesc_bf16_f32(kTcRows, NT), idesc2 = ptx::idesc_bf16_f32(kTcRows, 2 * NT);
+  int in_group = 0;  // stages of the group issued
   for (int st = 0; st < nst; ++st) {
-    const bool first = (st % kTcDrain) == 0;
+    const bool first = in_group == 0;
     if (first && !tc_wait(&bars->accfree, (group & 1) ^ 1, abort_flag)) return false;
     if (!tc_wait(&bars->full[r.slot], r.phase, abort_flag)) return false;
     ptx::tc_fence_after();
     tc_issue<kNarrow>(stages + r.slot * G.stage_bytes, tmem, idesc, idesc2, (uint32_t)NT * 64 >> 4, first);
     ptx::mma_commit(&bars->empty[r.slot]);
-    if ((st % kTcDrain) == kTcDrain - 1 || st == nst - 1) {
+    if (++in_group == drain || st == nst - 1) {
       ptx::mma_commit(&bars->accfull);
       ++group;
+      in_group = 0;
     }
     r.advance(1, G.ring);
   }
@@ -972,9 +982,11 @@ __device__ __forceinline__ void tc_role_mma(const TcBatchDev &B, TcBars *bars, u
     for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
       const int e = tc_entry_of(B, u);
       const TcDev &p = B.entries[e];
-      const int NT = p.NT, nst = tc_unit(p, tc_work(p), u - B.offsets[e]).n_stages;
-      const bool ok = tc_narrow(NT) ? tc_mma_unit<true>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag)
-                                    : tc_mma_unit<false>(B.geom, bars, stages, tmem, NT, nst, r, group, abort_flag);
+      const int NT = p.NT;
+      const TcUnit U = tc_unit(p, tc_work(p), u - B.offsets[e]);
+      const bool ok =
+          tc_narrow(NT) ? tc_mma_unit<true>(B.geom, bars, stages, tmem, NT, U.n_stages, U.drain, r, group, abort_flag)
+                        : tc_mma_unit<false>(B.geom, bars, stages, tmem, NT, U.n_stages, U.drain, r, group, abort_flag);
       if (!ok) break;
     }
     // all issued MMAs complete before the tensor memory is released
@@ -1087,7 +1099,7 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
     // core has work as soon as the accumulator is free again
     int folded = 0;
     auto fold_before = [&](int st) {
-      while (folded < U.n_groups - 1 && st >= (folded + 1) * kTcDrain + (int)ring - 1) {
+      while (folded < U.n_groups - 1 && st >= (folded + 1) * U.drain + (int)ring - 1) {
         tc_fold(bars, (group0 + folded) & 1, NT, tmem, folded == 0, abort_flag);
         ++folded;
       }
@@ -1191,7 +1203,7 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
     }
     // the groups that no later stage of this warp led to fold: the MMAs, and
     // with them the other warps, may wait for them
-    if (drains) fold_before(nst + kTcDrain + (int)ring);
+    if (drains) fold_before(nst + U.drain + (int)ring);
     // every warp has written its stages of this unit, so that none starts the
     // next unit's turns more than a round of the ring ahead of the MMAs; after a
     // wait that ran out, all leave here together
@@ -1573,6 +1585,7 @@ static int tc_entries(const fm_signal_args *a, const TcPlan &pl, const fm_tc_tun
       p.wrows = VG + (kind == kTcRuns && use_runs ? 2 : (Rk > 1 ? Rk : 0));
       p.NT = tc_nt(p.Qt, VG);
       p.use_runs = use_runs;
+      p.drain = kind == kTcRuns && !tc_narrow(p.NT) ? kTcDrainRuns : kTcDrain;
       // node blocks by bulk copies when the inputs are 16-byte aligned; the
       // mode rows of a single POD term with them (tc_batch drops either when
       // the staging areas do not fit)

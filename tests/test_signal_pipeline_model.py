@@ -7,7 +7,12 @@ import random
 
 import pytest
 
-DRAIN, BLOCK, OPERANDS, DRAINS, ARRIVALS = 32, 8, 13, 8, 6
+BLOCK, OPERANDS, DRAINS, ARRIVALS = 8, 13, 8, 6
+
+
+def drain_of(generic, narrow):
+    """Stages of an accumulation group."""
+    return 32 if generic or narrow else 21
 
 
 class Bar:
@@ -50,15 +55,16 @@ class Block:
 
     def mma(self):
         stage = group = 0
-        for n, *_ in self.units:
+        for n, _, generic, narrow in self.units:
+            drain = drain_of(generic, narrow)
             for st in range(n):
-                if st % DRAIN == 0 and not (yield from self.wait(self.accfree, (group & 1) ^ 1, group)):
+                if st % drain == 0 and not (yield from self.wait(self.accfree, (group & 1) ^ 1, group)):
                     return
                 slot, turn = stage % self.ring, stage // self.ring
                 if not (yield from self.wait(self.full[slot], turn & 1, turn + 1)):
                     return
                 self.empty[slot].arrive()
-                if st % DRAIN == DRAIN - 1 or st == n - 1:
+                if st % drain == drain - 1 or st == n - 1:
                     self.accfull.arrive()
                     group += 1
                 stage += 1
@@ -79,7 +85,8 @@ class Block:
         stage0 = group0 = next_buf = 0
         drains = warp < DRAINS
         for unit, (n, groups, generic, narrow) in enumerate(self.units):
-            blocks, n_acc = -(-n // BLOCK), -(-n // DRAIN)
+            drain = drain_of(generic, narrow)
+            blocks, n_acc = -(-n // BLOCK), -(-n // drain)
             a_groups = 3 if generic else 2
             n_a = a_groups * groups
             is_a = warp < n_a
@@ -101,7 +108,7 @@ class Block:
 
             def fold_before(st):
                 nonlocal folded
-                while drains and folded < n_acc - 1 and st >= (folded + 1) * DRAIN + self.ring - 1:
+                while drains and folded < n_acc - 1 and st >= (folded + 1) * drain + self.ring - 1:
                     g = group0 + folded
                     yield from self.wait(self.accfull, g & 1, g + 1)
                     self.accfree.arrive()
@@ -120,7 +127,7 @@ class Block:
                 yield from fold_before((blk + 1) * BLOCK)
                 yield from acquire(blk + 1)
                 self.nodeempty[buf].arrive()
-            yield from fold_before(n + DRAIN + self.ring)
+            yield from fold_before(n + drain + self.ring)
             # the barrier that also tells whether any warp knows of a failed wait
             if len(self.unit_any) == unit:
                 self.unit_any.append(False)
