@@ -51,6 +51,7 @@ void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool tensor_core, i
   p.n_kz = (int)(p.S > 0 ? a->n_kz : 1);
   p.Ls = p.n_lines * p.n_kz;
   p.slabs = tensor_core && p.n_kz > 1;
+  p.turns = tensor_core;
   p.stat = p.n_ro > 1 && p.Ls > 1 && (a->motion == nullptr || a->motion->kind == FM_MOTION_NONE);
   const int64_t most_cols = 1 << 30;  // columns of a factored product are counted in int
   p.slab_cover = !tensor_core && p.n_kz > 1 && p.n_lines > 1 && p.n_kz * p.V < most_cols;
@@ -78,7 +79,7 @@ void carve_prep(Carve &c, const fm_signal_args *a, int tile, bool tensor_core, i
 void fill_prep(const fm_signal_args *a, PrepDev &p) {
   p.diag = a->m_nnz == a->m_rows ? 1 : 0;
   p.table_calls = (a->motion && a->motion->kind == FM_MOTION_TABLE) ? a->motion->table_calls : -1;
-  p.kx = a->kx; p.ky = a->ky; p.kz = a->kz; p.t = a->t;
+  p.kx = a->kx; p.ky = a->ky; p.kz = a->kz; p.t = a->t; p.phi = a->phi;
   p.indptr = a->m_indptr; p.indices = a->m_indices; p.data = a->m_data;
   p.Mxy = a->Mxy;
   p.md = make_motion_dev(a->motion);
@@ -115,6 +116,19 @@ __device__ inline int block_sum(int v) {
   int s = 0;
 #pragma unroll
   for (int i = 0; i < kPrepThreads / 32; ++i) s += part[i];
+  return s;
+}
+
+// Largest of v over the block's threads, in every thread.
+__device__ inline int block_max(int v) {
+  __shared__ int part[kPrepThreads / 32];
+  v = __reduce_max_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int s = part[0];
+#pragma unroll
+  for (int i = 1; i < kPrepThreads / 32; ++i) s = max(s, part[i]);
   return s;
 }
 
@@ -162,6 +176,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   const T *t = static_cast<const T *>(p.t);
   const T *kc[3] = {static_cast<const T *>(p.kx), static_cast<const T *>(p.ky), static_cast<const T *>(p.kz)};
   int flags = 0;
+  int phi_max = 0, t_max = 0;  // float bits
+  if (p.turns) {
+    const T *phi = static_cast<const T *>(p.phi);
+    for (int64_t n = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; n < p.N; n += (int64_t)gridDim.x * kPrepThreads)
+      phi_max = max(phi_max, __float_as_int((float)phi[n]) & 0x7fffffff);
+  }
   const int c = blockIdx.x;
   if (c < p.n_chunks) {
     const int64_t s0 = (int64_t)c * p.chunk, s1 = min(p.S, s0 + p.chunk);
@@ -169,6 +189,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
     for (int64_t s = s0 + threadIdx.x; s < s1; s += kPrepThreads) {
       const bool first = starts_run(t, s);
       starts += first ? 1 : 0;
+      if (p.turns && t[s] == t[s]) t_max = max(t_max, __float_as_int((float)t[s]) & 0x7fffffff);
       const int i = (int)((unsigned)s / (unsigned)p.Ls), w = (int)s - i * p.Ls;
       if (first != (w == 0)) {
         // slab i is not exactly one run (nor the slab before it, when a run
@@ -226,6 +247,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   }
   flags = __reduce_or_sync(0xffffffffu, flags);
   if ((threadIdx.x & 31) == 0 && flags) atomicOr(p.ctl + kCtlFlags, flags);
+  if (p.turns) {
+    phi_max = block_max(phi_max);
+    t_max = block_max(t_max);
+    if (threadIdx.x == 0 && phi_max) atomicMax(p.ctl + kCtlPhi, phi_max);
+    if (threadIdx.x == 0 && t_max) atomicMax(p.ctl + kCtlTime, t_max);
+  }
 }
 
 // ---- runs ----------------------------------------------------------------
@@ -460,8 +487,8 @@ int report_errors(const int *ctl, int n, cudaStream_t st, const char *who) {
     FM_REQUIRE(!(h & kErrTimeout), FM_ERR_TIMEOUT, "%s: a tensor-core pipeline wait timed out", who);
     FM_REQUIRE(!(h & kErrPhaseRange), FM_ERR_ARG,
                "%s: the split-BF16 form reduces phases k . r in fixed point and needs (|kx|+|ky|+|kz|) * "
-               "(|x|+|y|+|z|) below 2^27 cycles for every sample and moved node (or finite positions); use "
-               "precision f32 or f64",
+               "(|x|+|y|+|z|) below 2^27 cycles for every sample and moved node (or finite positions), and "
+               "off-resonance phases phi t below 2^27 cycles; use precision f32 or f64",
                who);
   }
   return FM_OK;

@@ -23,7 +23,7 @@ struct Csr {
 constexpr int kErrTimeout = 1;      // a tensor-core pipeline wait ran out
 constexpr int kErrSparseRow = 2;    // a row index of M outside [0, rows)
 constexpr int kErrTableCalls = 4;   // TABLE motion entries != distinct-time runs
-constexpr int kErrPhaseRange = 8;   // a tensor-core phase k . r may reach 2^27 cycles
+constexpr int kErrPhaseRange = 8;   // a tensor-core phase k . r or phi t may be out of its reduction's range
 
 // Control words of one problem (zeroed when its descriptor is written).
 constexpr int kCtlFlags = 0;    // kFlag* bits found over the samples and M
@@ -33,6 +33,8 @@ constexpr int kCtlTiles = 3;    // tiles of the other runs
 constexpr int kCtlSplits = 4;   // node splits (tensor-core form)
 constexpr int kCtlChunk = 5;    // nodes per split (tensor-core form)
 constexpr int kCtlError = 6;    // kErr* bits
+constexpr int kCtlPhi = 7;      // largest |phi| (float bits; a NaN counts as largest; tensor-core form)
+constexpr int kCtlTime = 8;     // largest |t|, NaN apart (float bits; tensor-core form)
 constexpr int kCtlWords = 16;
 
 // A slab is the Ls = lines x kz samples of one readout index.
@@ -65,10 +67,11 @@ struct PrepDev {
   int run_cover;         // nor is anything where the runs factor out
   int stat;              // runs may factor out (no motion, several runs of several samples)
   int slabs;             // slabs may factor: factored runs are listed apart from the tiles
+  int turns;             // the largest |phi| and |t| are wanted
   int diag;              // M holds as many entries as rows: diagonal unless shown otherwise
   int vgroup;            // columns per group of MM (0: one (N, V) matrix)
   int64_t table_calls;   // entries of a TABLE motion, -1 without one
-  const void *kx, *ky, *kz, *t;
+  const void *kx, *ky, *kz, *t, *phi;
   const int *indptr, *indices;
   const void *data, *Mxy;
   void *MM;

@@ -1304,6 +1304,16 @@ __host__ __device__ inline int tc_choose_splits(int64_t items, int64_t N, int64_
   return best;
 }
 
+// Off-resonance phases phi t that their reduction holds for (cycles_cos_sin), in
+// radians: up to 2^28 cycles, and where they are added to k . r of up to 2^27 (runs
+// as columns) up to 2^27.  Every node goes with every run, so the largest |phi| and
+// |t| tell.
+constexpr float kTcTurn = 1.6866e9f, kTcTurnRuns = 8.433e8f;
+__device__ inline bool tc_turns_in_range(const TcDev &p) {
+  const float turn = __int_as_float(p.ctl[kCtlPhi]) * __int_as_float(p.ctl[kCtlTime]);
+  return turn < (p.use_runs && prep_static(p.ctl) ? kTcTurnRuns : kTcTurn);
+}
+
 // Node splits of every problem, shared by all its entries (from the node
 // count per split when tuned, else balanced over the SMs), and the running
 // unit counts of the launch's entries.  One block.
@@ -1313,6 +1323,7 @@ __global__ void __launch_bounds__(kTcPlanThreads) tc_plan_kernel(const TcDev *__
                                                                  int *__restrict__ first) {
   for (int e = threadIdx.x; e < n; e += kTcPlanThreads) {
     const TcDev &p = entries[e];
+    if (!tc_turns_in_range(p)) atomicOr(p.ctl + kCtlError, kErrPhaseRange);
     if (e != p.first) continue;
     first[p.prob] = e;
     int splits;

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from feelmri_b200 import ops, workloads as W
+from feelmri_b200._lib import FeelMRIError
 from feelmri_b200._motion import lower, table_motion
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,33 @@ def test_table_of_another_number_of_runs_in_a_batch(cuda):
         ops.signal_batch([(inp, table_motion(whole[:6]), outs[0]), (inp, table_motion(whole[:5]), outs[1])])
     alone = ops.signal_batch([(inp, table_motion(whole[:6]), None)])[0]
     assert torch.equal(outs[0], alone) and (outs[1] == 7.0).all()
+
+
+@pytest.mark.parametrize("kind", ["runs", "slabs", "samples"])
+@pytest.mark.parametrize("phi,refused", [(float("nan"), True), (float("inf"), True), (-2.0 ** 26, True),
+                                         (2.0 ** 22, False), (0.0, False)])
+def test_off_resonance_out_of_range(cuda, kind, phi, refused):
+    """The split-BF16 form reduces phi t as it does k . r: beyond its range (here t up
+    to 32 ms or more, so 2^31 rad) the call fails instead of returning a finite wrong
+    signal; 2^22 rad / ms is within it."""
+    n = 200
+    traj = W.radial3d(n_ro=40, n_spokes=30, kmax=300.0) if kind == "samples" else W.cartesian(res=(40, 6, 5))
+    inp = _inputs(n, 1, traj, "bf16x3", cuda)
+    inp.t = inp.t + 30.0
+    inp.phi[7] = phi
+    pod = W.sinusoidal_pod(n, n_modes=2) if kind == "slabs" else None
+    motion = lower(pod, n, cuda)
+    if refused:
+        with pytest.raises(FeelMRIError, match="off-resonance"):
+            ops.signal(inp, motion, "bf16x3")
+        with pytest.raises(FeelMRIError, match="off-resonance"):
+            ops.signal_batch([(inp, motion, None)])
+    else:
+        assert torch.isfinite(torch.view_as_real(ops.signal(inp, motion, "bf16x3"))).all()
+    if kind == "slabs":
+        return  # (nodes that move have no finite place at no time, which is refused)
+    # a sample without a time is its own run of no finite signal, not a refusal
+    inp.phi[7] = 0.1
+    inp.t[3, 2] = float("nan")
+    K = torch.view_as_real(ops.signal(inp, motion, "bf16x3"))
+    assert K[3, 2].isnan().all() and K[4].isfinite().all()
