@@ -7,13 +7,17 @@
 //   write   descriptors to device memory, control words and slab flags cleared
 //   scan    one pass over the samples and over M's pattern: run starts per
 //           stretch, which slabs are one run and factor, whether M is diagonal
-//   runs    run starts and times, compacted in order
-//   items   M Mxy (diagonal M), motion weights, factored runs and tiles counted
+//   runs    run starts and times, compacted in order; rows of an M of as many
+//           entries as rows that is not diagonal
+//   items   M Mxy (of such an M or a diagonal one), motion weights, factored runs
+//           and tiles counted
 //   fill    factored runs and tiles, compacted in order
 // These phases are a few microseconds of work each, so launches bound them:
 // one chain per problem (33 launches and copies, the scans two each) took
 // 238 us of device time for a 3,083-node Signal of 2,048 samples, 58 us of it
 // outside the main kernel, and 1.6 ms of a 16-problem batch.
+#include <climits>
+
 #include <cub/cub.cuh>
 
 #include "signal_common.cuh"
@@ -240,8 +244,10 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   }
   if (p.diag) {
     bool diag = true;
-    for (int64_t k = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; k < p.N; k += (int64_t)gridDim.x * kPrepThreads)
+    for (int64_t k = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; k < p.N; k += (int64_t)gridDim.x * kPrepThreads) {
       diag = diag && p.indices[k] == (int)k && p.indptr[k] == (int)k;
+      p.csr.fill[k] = -1;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) diag = diag && p.indptr[p.N] == (int)p.N;
     if (!diag) flags |= kFlagNotDiagonal;
   }
@@ -257,11 +263,44 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
 
 // ---- runs ----------------------------------------------------------------
 
+// M Mxy of an M of as many entries as rows that turned out not to be diagonal
+// (a permuted or partly empty one), with no launch of its own: the entries of a row
+// are linked here, in any order, and summed in that of their positions below.
+//   fill: a row's first entry (-1: none)    pos: the entry after an entry
+//   col: an entry's column                  rowptr: room for the order of long rows
+__device__ inline bool prep_listed(const PrepDev &p) { return p.diag && (p.ctl[kCtlFlags] & kFlagNotDiagonal); }
+__device__ inline void prep_link_rows(const PrepDev &p) {
+  const Csr &m = p.csr;
+  for (int64_t e = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; e < p.N; e += (int64_t)gridDim.x * kPrepThreads) {
+    const int k = (int)e, i = p.indices[k];
+    if (i < 0 || i >= p.N) {
+      atomicOr(p.ctl + kCtlError, kErrSparseRow);
+      continue;
+    }
+    // the entry's column: the last that starts at or before it (each entry is
+    // linked once, whatever indptr holds, so that the lists end)
+    int j = k;
+    if (p.indptr[j] > k || p.indptr[j + 1] <= k) {
+      int lo = 0, hi = (int)p.N;
+      while (hi - lo > 1) {
+        const int mid = lo + (hi - lo) / 2;
+        if (p.indptr[mid] <= k) lo = mid;
+        else hi = mid;
+      }
+      j = lo;
+      if (p.indptr[j] > k || p.indptr[j + 1] <= k) continue;
+    }
+    m.col[k] = j;
+    m.pos[k] = atomicExch(m.fill + i, k);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kPrepThreads) prep_runs_kernel(const PrepDev *__restrict__ probs) {
   const PrepDev &p = probs[blockIdx.y];
   const T *t = static_cast<const T *>(p.t);
   const int c = blockIdx.x;
+  if (prep_listed(p)) prep_link_rows(p);
   if (c >= p.n_chunks) return;
   if (!(p.ctl[kCtlFlags] & kFlagRuns)) {  // run g is slab g
     for (int g = c * kPrepThreads + threadIdx.x; g < p.n_ro; g += p.n_chunks * kPrepThreads) {
@@ -306,6 +345,59 @@ struct Cplx<double> {
   using type = double2;
 };
 
+// Element of M Mxy for row i, column v from the row's linked entries.  Up to
+// kLinkedRow of them are taken in order by looking for the next one each time; a
+// longer row's order is written out and sorted by the thread of its first column,
+// which forms the others too.  Split-BF16 call of 200,000 rows and 2 columns on a
+// B200: 313 us with a diagonal M, 322 us permuted (2979 us with one block of threads
+// for the matrix).
+constexpr int kLinkedRow = 8;
+template <typename T>
+__device__ __noinline__ void prep_linked_row(const PrepDev &p, int64_t i, int64_t v) {
+  using C = typename Cplx<T>::type;
+  const Csr &m = p.csr;
+  const T *w = static_cast<const T *>(p.data);
+  const C *x = static_cast<const C *>(p.Mxy);
+  C *MM = static_cast<C *>(p.MM);
+  auto add = [&](C &acc, int k, int64_t col) {
+    const C xe = x[(int64_t)m.col[k] * p.V + col];
+    acc.x = fma(w[k], xe.x, acc.x);
+    acc.y = fma(w[k], xe.y, acc.y);
+  };
+  const int head = m.fill[i];
+  int n = 0;
+  for (int k = head; k >= 0 && (n <= kLinkedRow || v == 0); k = m.pos[k]) ++n;
+  if (n <= kLinkedRow) {
+    C acc{};
+    for (int done = 0, last = -1; done < n; ++done) {
+      int next = INT_MAX;
+      for (int k = head; k >= 0; k = m.pos[k])
+        if (k > last && k < next) next = k;
+      add(acc, next, v);
+      last = next;
+    }
+    MM[mm_index(i, v, p.N, p.V, p.vgroup)] = acc;
+  } else if (v == 0) {
+    int *order = m.rowptr + atomicAdd(p.ctl + kCtlOrder, n);
+    int at = n;  // the list is about descending
+    for (int k = head; k >= 0; k = m.pos[k]) order[--at] = k;
+    int gap = 1;  // Shell's sort
+    while (gap < n / 3) gap = 3 * gap + 1;
+    for (; gap > 0; gap /= 3)
+      for (int k = gap; k < n; ++k) {
+        const int e = order[k];
+        int q = k - gap;
+        for (; q >= 0 && order[q] > e; q -= gap) order[q + gap] = order[q];
+        order[q + gap] = e;
+      }
+    for (int64_t u = 0; u < p.V; ++u) {
+      C acc{};
+      for (int k = 0; k < n; ++k) add(acc, order[k], u);
+      MM[mm_index(i, u, p.N, p.V, p.vgroup)] = acc;
+    }
+  }
+}
+
 // A TABLE motion must hold one entry per run: a shorter one would be read past
 // its end, so a problem without them is given no work at all (its error word is
 // set, and the call reports it).
@@ -346,6 +438,8 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
       MM[mm_index(n, e - n * p.V, p.N, p.V, p.vgroup)] = r;
     }
   }
+  if (prep_listed(p))
+    for (int64_t e = tid; e < p.N * p.V; e += stride) prep_linked_row<T>(p, e / p.V, e - e / p.V * p.V);
   if (p.md.kind == FM_MOTION_TERMS) {
     const int64_t total = (int64_t)n_runs * p.md.slots;
     for (int64_t idx = tid; idx < total; idx += stride) {
@@ -376,80 +470,9 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
 
 // ---- fill ----------------------------------------------------------------
 
-// M Mxy by one block, for an M of as many entries as rows that turned out not
-// to be diagonal: the phases of the general product below with block barriers
-// between them.  Rare (a lumped mass matrix is diagonal, a consistent one has
-// more entries), so it costs the usual calls no launches.
-template <typename T>
-__device__ void prep_block_product(const PrepDev &p) {
-  using C = typename Cplx<T>::type;
-  const int64_t N = p.N;
-  const int *indptr = p.indptr, *indices = p.indices;
-  const Csr &m = p.csr;
-  const int tid = threadIdx.x;
-  for (int64_t i = tid; i <= N; i += kPrepThreads) m.fill[i] = 0;
-  __syncthreads();
-  for (int64_t k = tid; k < N; k += kPrepThreads) {  // nnz == N
-    const int i = indices[k];
-    if (i < 0 || i >= N) atomicOr(p.ctl + kCtlError, kErrSparseRow);
-    else atomicAdd(m.fill + i, 1);
-  }
-  __syncthreads();
-  int base = 0;
-  for (int64_t b = 0; b <= N; b += kPrepThreads) {
-    const int64_t i = b + tid;
-    const int v = i < N ? m.fill[i] : 0;
-    int total;
-    const int off = block_exclusive(v, total);
-    if (i <= N) m.rowptr[i] = base + off;
-    base += total;
-  }
-  __syncthreads();
-  for (int64_t i = tid; i <= N; i += kPrepThreads) m.fill[i] = 0;
-  __syncthreads();
-  for (int64_t j = tid; j < N; j += kPrepThreads)
-    for (int k = indptr[j]; k < indptr[j + 1]; ++k) {
-      const int i = indices[k];
-      if (i < 0 || i >= N) continue;
-      const int slot = m.rowptr[i] + atomicAdd(m.fill + i, 1);
-      m.col[slot] = (int)j;
-      m.pos[slot] = k;
-    }
-  __syncthreads();
-  for (int64_t i = tid; i < N; i += kPrepThreads) {
-    const int r0 = m.rowptr[i], r1 = m.rowptr[i + 1];
-    for (int k = r0 + 1; k < r1; ++k) {
-      const int pk = m.pos[k], ck = m.col[k];
-      int q = k - 1;
-      while (q >= r0 && m.pos[q] > pk) {
-        m.pos[q + 1] = m.pos[q];
-        m.col[q + 1] = m.col[q];
-        --q;
-      }
-      m.pos[q + 1] = pk;
-      m.col[q + 1] = ck;
-    }
-    for (int64_t v = 0; v < p.V; ++v) {
-      C acc;
-      acc.x = T(0); acc.y = T(0);
-      for (int k = r0; k < r1; ++k) {
-        const T w = static_cast<const T *>(p.data)[m.pos[k]];
-        const C x = static_cast<const C *>(p.Mxy)[(int64_t)m.col[k] * p.V + v];
-        acc.x = fma(w, x.x, acc.x);
-        acc.y = fma(w, x.y, acc.y);
-      }
-      static_cast<C *>(p.MM)[mm_index(i, v, N, p.V, p.vgroup)] = acc;
-    }
-  }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kPrepThreads) prep_fill_kernel(const PrepDev *__restrict__ probs) {
   const PrepDev &p = probs[blockIdx.y];
-  if (blockIdx.x == gridDim.x - 1) {
-    if (p.diag && (p.ctl[kCtlFlags] & kFlagNotDiagonal)) prep_block_product<T>(p);
-    return;
-  }
   const int c = blockIdx.x;
   if (c >= p.n_chunks) return;
   int f0 = block_prefix(p.chunk_fac, c);
@@ -623,13 +646,13 @@ int launch_prep(const fm_signal_args *probs, const PrepDev *host, int n, PrepDev
     prep_scan_kernel<T><<<dim3(wide, y), kPrepThreads, 0, st>>>(d);
     count_launch();
     FM_TRY(check_launch("prep_scan_kernel"));
-    prep_runs_kernel<T><<<dim3(chunks, y), kPrepThreads, 0, st>>>(d);
+    prep_runs_kernel<T><<<dim3(wide, y), kPrepThreads, 0, st>>>(d);
     count_launch();
     FM_TRY(check_launch("prep_runs_kernel"));
     prep_items_kernel<T><<<dim3(wide, y), kPrepThreads, 0, st>>>(d);
     count_launch();
     FM_TRY(check_launch("prep_items_kernel"));
-    prep_fill_kernel<T><<<dim3(chunks + 1, y), kPrepThreads, 0, st>>>(d);
+    prep_fill_kernel<T><<<dim3(chunks, y), kPrepThreads, 0, st>>>(d);
     count_launch();
     FM_TRY(check_launch("prep_fill_kernel"));
   }

@@ -35,6 +35,7 @@ constexpr int kCtlChunk = 5;    // nodes per split (tensor-core form)
 constexpr int kCtlError = 6;    // kErr* bits
 constexpr int kCtlPhi = 7;      // largest |phi| (float bits; a NaN counts as largest; tensor-core form)
 constexpr int kCtlTime = 8;     // largest |t|, NaN apart (float bits; tensor-core form)
+constexpr int kCtlOrder = 9;    // entries of the matrix's long rows put in order
 constexpr int kCtlWords = 16;
 
 // A slab is the Ls = lines x kz samples of one readout index.
