@@ -12,8 +12,8 @@
 // Each component of k belongs wholly to one factor (prep_scan_kernel), so the
 // factors' phases are exact products of the inputs: no rounding is added.  The
 // FP32 form forms phases in FP64, the FP64 form keeps what their rounding leaves
-// out, and both reduce them exactly, where the unfactored form sums them in its
-// type as the reference does; sums over the nodes are in the form's type and no
+// out, and both reduce them exactly, where the unfactored FP64 form sums them in
+// radians as the reference does; sums over the nodes are in the form's type and no
 // longer than there.  2 pi is built from a float-rounded pi (MRI.h:13).
 //
 // Block: a tile of rows x (q, v) pairs, 8 x 4 (FP64: 4 x 4) per thread, operands
@@ -111,10 +111,7 @@ struct GemmSmem {
   }
 };
 
-// Register block of a thread: RT consecutive rows, and the columns that lie in
-// slots tc + 16 j of the staged factor.  All offsets but the node's are
-// constants.
-// Column in slot tc + 16 j.  The low bits are mixed so that the threads that
+// Column in slot tc + 16 j of the staged factor.  The low bits are mixed so that the threads that
 // form the V columns of neighbouring q store to different banks.
 __device__ inline int gemm_col(int j, int tc, int TC) {
   const int c = j * TC + tc;
@@ -131,6 +128,8 @@ __device__ inline void lds2(uint32_t addr, double &a, double &b) {
   asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "r"(addr));
 }
 
+// Register block of a thread: consecutive rows, and the columns that lie in slots
+// tc + 16 j of the staged factor.  All offsets but the node's are constants.
 template <typename T>
 struct GemmAcc;
 template <>
@@ -429,6 +428,7 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
   const uint32_t b_at = (uint32_t)__cvta_generic_to_shared(smem + L.b) + tc * 2 * sizeof(T);
   const int n_stages = (int)ceil_div(max(n_end - n_begin, (int64_t)0), (int64_t)kGemmStage);
   constexpr int kPerBlock = kGemmNodes / kGemmStage;
+  static_assert(kPerBlock > 1, "a node block is formed a barrier before its first stage");
   auto nodes_of = [&](int st) { return (int)min((int64_t)kGemmStage, n_end - n_begin - (int64_t)st * kGemmStage); };
   auto form_stage = [&](int st) {
     const int blk = (st / kPerBlock) & 1, m0 = (st % kPerBlock) * kGemmStage, cnt = nodes_of(st);
@@ -447,47 +447,46 @@ __global__ void __launch_bounds__(kGemmMaxThreads, 2) signal_gemm_kernel(GemmDev
   __syncthreads();
   int turn = 0;
   for (int fold = 0; fold == 0 || fold < n_stages; fold += kGemmFold) {
-  acc.clear();
-  for (int st = fold; st < min(n_stages, fold + kGemmFold); ++st) {
-    if (st % kPerBlock == 0 && st + kPerBlock < n_stages) {
-      turn = turn + 1 == warps ? 0 : turn + 1;
-      form_nodes(st / kPerBlock + 1, turn);
-    }
-    if (kPerBlock == 1) __syncthreads();
-    if (st + 1 < n_stages) form_stage(st + 1);
-    if (works) {
-      const int cnt = nodes_of(st);
-      uint32_t A = a_at + (st & 1) * L.stage, B = b_at + (st & 1) * L.stage;
+    acc.clear();
+    for (int st = fold; st < min(n_stages, fold + kGemmFold); ++st) {
+      if (st % kPerBlock == 0 && st + kPerBlock < n_stages) {
+        turn = turn + 1 == warps ? 0 : turn + 1;
+        form_nodes(st / kPerBlock + 1, turn);
+      }
+      if (st + 1 < n_stages) form_stage(st + 1);
+      if (works) {
+        const int cnt = nodes_of(st);
+        uint32_t A = a_at + (st & 1) * L.stage, B = b_at + (st & 1) * L.stage;
 #pragma unroll 2
-      for (int m = 0; m < cnt; ++m) {
-        acc.node(A, B);
-        A += TR * GemmType<T>::kRowBytes;
-        B += kGemmSlots * 2 * sizeof(T);
+        for (int m = 0; m < cnt; ++m) {
+          acc.node(A, B);
+          A += TR * GemmType<T>::kRowBytes;
+          B += kGemmSlots * 2 * sizeof(T);
+        }
+      }
+      __syncthreads();
+    }
+    if (!works) continue;
+    V2 *dst = reinterpret_cast<V2 *>(p.out) + (int64_t)split * p.S * p.V;
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      const int r = RT * tr + i;
+      if (r >= n_rows) continue;
+#pragma unroll
+      for (int j = 0; j < kGemmCols; ++j) {
+        const int c = gemm_col(j, tc, TC);
+        if (c >= n_cols) continue;
+        const int q = (col0 + c) / V, v = col0 + c - q * V;
+        const int64_t s = p.runs ? (int64_t)q * Ls + row0 + r : s0 + (int64_t)(row0 + r) * p.n_kz + q;
+        V2 sum = acc.get(i, j);
+        if (fold > 0) {
+          const V2 before = dst[s * p.V + v];
+          sum.x += before.x;
+          sum.y += before.y;
+        }
+        dst[s * p.V + v] = sum;
       }
     }
-    __syncthreads();
-  }
-  if (!works) continue;
-  V2 *dst = reinterpret_cast<V2 *>(p.out) + (int64_t)split * p.S * p.V;
-#pragma unroll
-  for (int i = 0; i < RT; ++i) {
-    const int r = RT * tr + i;
-    if (r >= n_rows) continue;
-#pragma unroll
-    for (int j = 0; j < kGemmCols; ++j) {
-      const int c = gemm_col(j, tc, TC);
-      if (c >= n_cols) continue;
-      const int q = (col0 + c) / V, v = col0 + c - q * V;
-      const int64_t s = p.runs ? (int64_t)q * Ls + row0 + r : s0 + (int64_t)(row0 + r) * p.n_kz + q;
-      V2 sum = acc.get(i, j);
-      if (fold > 0) {
-        const V2 before = dst[s * p.V + v];
-        sum.x += before.x;
-        sum.y += before.y;
-      }
-      dst[s * p.V + v] = sum;
-    }
-  }
   }
 }
 
@@ -513,8 +512,7 @@ static void gemm_shape(int64_t P, int64_t C, int64_t V, GemmPlan &g) {
 // add up, at a rate that grows with the warps there (latency: 8 / warps on top);
 // a block costs about 3 stages to set up and write, and a round of blocks 30 more
 // in latency and uneven ends; partial sums are written and read back at some 20 MB
-// a stage.  Splits of at least 64 nodes and
-// 256 MB of partial sums, and at least as many as the unfactored form takes, so
+// a stage.  Splits of at least 64 nodes and 256 MB of partial sums, and at least as many as the unfactored form takes, so
 // that no sum in the form's type is longer than there.
 static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int least) {
   const int64_t units = (int64_t)g.products * g.nr * g.nc;
@@ -527,7 +525,8 @@ static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int leas
     const int64_t on_sm = ceil_div(units * s, (int64_t)kSmCount);
     const double warps = (double)std::min(on_sm, per_sm) * (g.threads / 32);
     const double cost = (double)on_sm * ((double)N / s / kGemmStage) * (1.0 + 8.0 / warps) +
-                        3.0 * (double)on_sm + 30.0 * (double)ceil_div(on_sm, per_sm) + (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
+                        3.0 * (double)on_sm + 30.0 * (double)ceil_div(on_sm, per_sm) +
+                        (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
     if (s == least || cost < best_cost) {
       best = s;
       best_cost = cost;

@@ -4,13 +4,14 @@
 // Restates Signal<T> (cpp/feelmri/MRI.cpp:38-159 with motion, :196-298
 // without): for every sample s of run g (time t_g)
 //   K[s, v] = sum_n exp(i * (-2pi k_s . r_n(t_g) + phi_n t_g)) * MM[n, v] * exp(-t_g / T2_n)
-// with MM = M * Mxy, 2pi built from a float-rounded pi (MRI.h:13, MRI.cpp:73),
-// the phase summed in T as the reference does (MRI.cpp:138-146) and sin/cos
-// taken of the phase in radians.  One thread block covers up to
-// kPlainThreads * SPT samples of one run and sweeps a node range staged in
-// shared memory; the per-run node quantities (moved position, phase offset,
-// decayed weight) are formed once per tile and node.  Node ranges may be
-// split over blocks; partial sums are then added in a fixed order.
+// with MM = M * Mxy and 2pi built from a float-rounded pi (MRI.h:13, MRI.cpp:73).
+// The FP64 form sums the phase in radians and takes sin/cos of that, as the
+// reference does (MRI.cpp:138-146); the FP32 form sums it in FP64 cycles and
+// reduces it exactly (cycles.cuh).  One thread block covers up to 256 samples of
+// one run and sweeps a node range staged in shared memory; the per-run node
+// quantities (moved position, phase offset, decayed weight) are formed once per
+// tile and node.  Node ranges may be split over blocks; partial sums are then added
+// in a fixed order.
 #include <algorithm>
 
 #include "cycles.cuh"
@@ -38,109 +39,92 @@ struct PlainDev {
   T two_pi;
 };
 
+constexpr int kPlainNodes = 128;            // nodes staged at a time
 constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an SM holds in FP32
 
-template <int VMAX, int NT>
+template <int VMAX>
 __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<double> p, int v0) {
-  using T = double;
-  constexpr int SPT = 1;
-  __shared__ double4 s_pos[NT];             // moved x, y, z and phi * t
-  __shared__ T s_w[NT][2 * VMAX];      // decayed M * Mxy columns v0 .. v0 + VMAX
+  __shared__ double4 s_pos[kPlainNodes];         // moved x, y, z and phi * t
+  __shared__ double s_w[kPlainNodes][2 * VMAX];  // decayed M * Mxy columns v0 .. v0 + VMAX
 
   const int n_tiles = *p.n_tiles;
   const int64_t items = (int64_t)n_tiles * p.splits;
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
-  const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
-  __syncthreads();  // the previous tile's readers of s_pos / s_w are done
-  const int g = p.tiles[tile].x;
-  const int s_begin = p.run_start[g] + p.tiles[tile].y;
-  const int s_end = min(p.run_start[g + 1], s_begin + kPlainThreads * SPT);
-  const T tg = (T)p.run_t[g];
-  const int nv = (int)min((int64_t)VMAX, p.V - v0);
-
-  T kxs[SPT], kys[SPT], kzs[SPT];
-  T acc_r[SPT][VMAX], acc_i[SPT][VMAX];
-#pragma unroll
-  for (int q = 0; q < SPT; ++q) {
-    const int s = s_begin + q * kPlainThreads + threadIdx.x;
-    const bool ok = s < s_end;
+    const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
+    __syncthreads();  // the previous tile's readers of s_pos / s_w are done
+    const int g = p.tiles[tile].x;
+    const int s = p.run_start[g] + p.tiles[tile].y + threadIdx.x;
+    const bool in = s < p.run_start[g + 1];
+    const double tg = p.run_t[g];
+    const int nv = (int)min((int64_t)VMAX, p.V - v0);
     // kx_ = two_pi * kloc[0](i,j,k)   (MRI.cpp:138-140)
-    kxs[q] = ok ? p.two_pi * p.kx[s] : T(0);
-    kys[q] = ok ? p.two_pi * p.ky[s] : T(0);
-    kzs[q] = ok ? p.two_pi * p.kz[s] : T(0);
+    const double kx = in ? p.two_pi * p.kx[s] : 0.0;
+    const double ky = in ? p.two_pi * p.ky[s] : 0.0;
+    const double kz = in ? p.two_pi * p.kz[s] : 0.0;
+    double acc_r[VMAX], acc_i[VMAX];
 #pragma unroll
-    for (int v = 0; v < VMAX; ++v) {
-      acc_r[q][v] = T(0);
-      acc_i[q][v] = T(0);
-    }
-  }
+    for (int v = 0; v < VMAX; ++v) acc_r[v] = acc_i[v] = 0.0;
 
-  const int64_t n_begin = (int64_t)split * p.chunk;
-  const int64_t n_end = min(p.N, n_begin + p.chunk);
-  const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
-  for (int64_t nb = n_begin; nb < n_end; nb += NT) {
-    const int cnt = (int)min((int64_t)NT, n_end - nb);
-    __syncthreads();
-    for (int j = threadIdx.x; j < cnt; j += kPlainThreads) {
-      const int64_t n = nb + j;
-      T x = p.r0[3 * n + 0], y = p.r0[3 * n + 1], z = p.r0[3 * n + 2];
-      if (p.md.kind == FM_MOTION_TERMS) {
-        float dx, dy, dz;
-        motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
-        x = x + (T)dx; y = y + (T)dy; z = z + (T)dz;
-      } else if (p.table) {
-        const T *d = p.table + ((int64_t)g * p.N + n) * 3;
-        x = x + (T)d[0]; y = y + (T)d[1]; z = z + (T)d[2];
-      }
-      double4 pp;
-      pp.x = x; pp.y = y; pp.z = z;
-      pp.w = p.phi[n] * tg;                       // phi_off (MRI.cpp:124)
-      s_pos[j] = pp;
-      const T invT2 = T(1) / p.T2[n];
-      const T decay = exp(-tg * invT2);      // T2_decay (MRI.cpp:127)
-      const T *mm = p.MM + (n * p.V + v0) * 2;
+    const int64_t n_begin = (int64_t)split * p.chunk;
+    const int64_t n_end = min(p.N, n_begin + p.chunk);
+    const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
+    for (int64_t nb = n_begin; nb < n_end; nb += kPlainNodes) {
+      const int cnt = (int)min((int64_t)kPlainNodes, n_end - nb);
+      __syncthreads();
+      for (int j = threadIdx.x; j < cnt; j += kPlainThreads) {
+        const int64_t n = nb + j;
+        double x = p.r0[3 * n + 0], y = p.r0[3 * n + 1], z = p.r0[3 * n + 2];
+        if (p.md.kind == FM_MOTION_TERMS) {
+          float dx, dy, dz;
+          motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
+          x = x + (double)dx; y = y + (double)dy; z = z + (double)dz;
+        } else if (p.table) {
+          const double *d = p.table + ((int64_t)g * p.N + n) * 3;
+          x = x + d[0]; y = y + d[1]; z = z + d[2];
+        }
+        double4 pp;
+        pp.x = x; pp.y = y; pp.z = z;
+        pp.w = p.phi[n] * tg;                    // phi_off (MRI.cpp:124)
+        s_pos[j] = pp;
+        const double invT2 = 1.0 / p.T2[n];
+        const double decay = exp(-tg * invT2);   // T2_decay (MRI.cpp:127)
+        const double *mm = p.MM + (n * p.V + v0) * 2;
 #pragma unroll
-      for (int v = 0; v < VMAX; ++v) {
-        s_w[j][2 * v + 0] = (v < nv) ? mm[2 * v + 0] * decay : T(0);
-        s_w[j][2 * v + 1] = (v < nv) ? mm[2 * v + 1] * decay : T(0);
+        for (int v = 0; v < VMAX; ++v) {
+          s_w[j][2 * v + 0] = (v < nv) ? mm[2 * v + 0] * decay : 0.0;
+          s_w[j][2 * v + 1] = (v < nv) ? mm[2 * v + 1] * decay : 0.0;
+        }
       }
-    }
-    __syncthreads();
-    for (int j = 0; j < cnt; ++j) {
-      const double4 pp = s_pos[j];
-#pragma unroll
-      for (int q = 0; q < SPT; ++q) {
+      __syncthreads();
+      for (int j = 0; j < cnt; ++j) {
+        const double4 pp = s_pos[j];
         // phase = -kx_ x - ky_ y - kz_ z + phi_off   (MRI.cpp:143-146)
-        const T ph = fma(-kzs[q], pp.z, fma(-kys[q], pp.y, -kxs[q] * pp.x)) + pp.w;
-        T sn, cs;
+        const double ph = fma(-kz, pp.z, fma(-ky, pp.y, -kx * pp.x)) + pp.w;
+        double sn, cs;
         sincos(ph, &sn, &cs);
 #pragma unroll
         for (int v = 0; v < VMAX; ++v) {
-          const T wr = s_w[j][2 * v + 0], wi = s_w[j][2 * v + 1];
-          acc_r[q][v] = fma(cs, wr, fma(-sn, wi, acc_r[q][v]));
-          acc_i[q][v] = fma(cs, wi, fma(sn, wr, acc_i[q][v]));
+          const double wr = s_w[j][2 * v + 0], wi = s_w[j][2 * v + 1];
+          acc_r[v] = fma(cs, wr, fma(-sn, wi, acc_r[v]));
+          acc_i[v] = fma(cs, wi, fma(sn, wr, acc_i[v]));
         }
       }
     }
-  }
 
-  T *dst = p.out + (int64_t)split * p.S * p.V * 2;
-#pragma unroll
-  for (int q = 0; q < SPT; ++q) {
-    const int s = s_begin + q * kPlainThreads + threadIdx.x;
-    if (s >= s_end) continue;
+    if (!in) continue;
+    double *dst = p.out + ((int64_t)split * p.S * p.V + (int64_t)s * p.V + v0) * 2;
 #pragma unroll
     for (int v = 0; v < VMAX; ++v) {
       if (v < nv) {
-        dst[((int64_t)s * p.V + v0 + v) * 2 + 0] = acc_r[q][v];
-        dst[((int64_t)s * p.V + v0 + v) * 2 + 1] = acc_i[q][v];
+        dst[2 * v + 0] = acc_r[v];
+        dst[2 * v + 1] = acc_i[v];
       }
     }
-  }
   }  // tiles
 }
 
-// FP32: two samples per thread, their phases in FP64 cycles.  A phase is three multiply-adds on the FP64 pipe,
+// FP32: two samples per thread, their phases in FP64 cycles.  A phase is three
+// multiply-adds on the FP64 pipe,
 // which the rest leaves idle, and its reduction exact (cycles.cuh), where the
 // reference rounds the phase in radians to FP32; what comes after is FP32 as
 // there.  Bound by issue: per sample-node some 40 instructions for the phase and
@@ -148,7 +132,6 @@ __global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<do
 // 255 samples x 8 columns on a B200: 2944 us with sincosf of a rounded phase, one
 // sample per thread and tiles dealt out split by split, 1830 us now.
 constexpr int kPlain32Threads = 128;
-constexpr int kPlainNodes = 128;  // nodes staged at a time
 constexpr int kPlainFold = 2048;  // nodes in one sum: a longer one is the largest error of the form
 template <int VMAX>
 __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(PlainDev<float> p, int v0) {
@@ -178,68 +161,68 @@ __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(Plai
     for (int fold = n_begin;;) {
       const int fold_end = fold + min(kPlainFold, n_end - fold);
 #pragma unroll
-    for (int v = 0; v < VMAX; ++v) acc0[v] = acc1[v] = make_float2(0.f, 0.f);
-    for (int nb = fold; nb < fold_end; nb += kPlainNodes) {
-      const int cnt = min(kPlainNodes, fold_end - nb);
-      __syncthreads();
-      for (int j = threadIdx.x; j < cnt; j += kPlain32Threads) {
-        const int64_t n = nb + j;
-        float x = p.r0[3 * n + 0], y = p.r0[3 * n + 1], z = p.r0[3 * n + 2];
-        if (p.md.kind == FM_MOTION_TERMS) {
-          float dx, dy, dz;
-          motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
-          x = x + dx; y = y + dy; z = z + dz;
-        } else if (p.table) {
-          const float *d = p.table + ((int64_t)g * p.N + n) * 3;
-          x = x + d[0]; y = y + d[1]; z = z + d[2];
-        }
-        double4 pp;
-        pp.x = x; pp.y = y; pp.z = z;
-        pp.w = (double)p.phi[n] * tg * kInv2Pi;     // phi_off (MRI.cpp:124)
-        s_pos[j] = pp;
-        const float invT2 = 1.f / p.T2[n];
-        const float decay = expf(-tg * invT2);      // T2_decay (MRI.cpp:127)
-        const float *mm = p.MM + (n * p.V + v0) * 2;
+      for (int v = 0; v < VMAX; ++v) acc0[v] = acc1[v] = make_float2(0.f, 0.f);
+      for (int nb = fold; nb < fold_end; nb += kPlainNodes) {
+        const int cnt = min(kPlainNodes, fold_end - nb);
+        __syncthreads();
+        for (int j = threadIdx.x; j < cnt; j += kPlain32Threads) {
+          const int64_t n = nb + j;
+          float x = p.r0[3 * n + 0], y = p.r0[3 * n + 1], z = p.r0[3 * n + 2];
+          if (p.md.kind == FM_MOTION_TERMS) {
+            float dx, dy, dz;
+            motion_disp(p.md, wrun, n, p.N, dx, dy, dz);
+            x = x + dx; y = y + dy; z = z + dz;
+          } else if (p.table) {
+            const float *d = p.table + ((int64_t)g * p.N + n) * 3;
+            x = x + d[0]; y = y + d[1]; z = z + d[2];
+          }
+          double4 pp;
+          pp.x = x; pp.y = y; pp.z = z;
+          pp.w = (double)p.phi[n] * tg * kInv2Pi;     // phi_off (MRI.cpp:124)
+          s_pos[j] = pp;
+          const float invT2 = 1.f / p.T2[n];
+          const float decay = expf(-tg * invT2);      // T2_decay (MRI.cpp:127)
+          const float *mm = p.MM + (n * p.V + v0) * 2;
 #pragma unroll
-        for (int v = 0; v < VMAX; ++v) {
-          const float wr = v < nv ? mm[2 * v + 0] * decay : 0.f, wi = v < nv ? mm[2 * v + 1] * decay : 0.f;
-          s_w[j][v] = make_float2(wr, wi);
+          for (int v = 0; v < VMAX; ++v) {
+            const float wr = v < nv ? mm[2 * v + 0] * decay : 0.f, wi = v < nv ? mm[2 * v + 1] * decay : 0.f;
+            s_w[j][v] = make_float2(wr, wi);
+          }
         }
-      }
-      __syncthreads();
+        __syncthreads();
 #pragma unroll 2
-      for (int j = 0; j < cnt; ++j) {
-        const double4 pp = s_pos[j];
-        // phase = -kx_ x - ky_ y - kz_ z + phi_off   (MRI.cpp:143-146)
-        float c0, s0n, c1, s1n;
-        cis_cycles(fma(kx0, pp.x, fma(ky0, pp.y, fma(kz0, pp.z, pp.w))), c0, s0n);
-        cis_cycles(fma(kx1, pp.x, fma(ky1, pp.y, fma(kz1, pp.z, pp.w))), c1, s1n);
+        for (int j = 0; j < cnt; ++j) {
+          const double4 pp = s_pos[j];
+          // phase = -kx_ x - ky_ y - kz_ z + phi_off   (MRI.cpp:143-146)
+          float c0, s0n, c1, s1n;
+          cis_cycles(fma(kx0, pp.x, fma(ky0, pp.y, fma(kz0, pp.z, pp.w))), c0, s0n);
+          cis_cycles(fma(kx1, pp.x, fma(ky1, pp.y, fma(kz1, pp.z, pp.w))), c1, s1n);
 #pragma unroll
-        for (int v = 0; v < VMAX; ++v) {
-          const float2 w = s_w[j][v];
-          acc0[v].x = fmaf(c0, w.x, fmaf(-s0n, w.y, acc0[v].x));
-          acc0[v].y = fmaf(c0, w.y, fmaf(s0n, w.x, acc0[v].y));
-          acc1[v].x = fmaf(c1, w.x, fmaf(-s1n, w.y, acc1[v].x));
-          acc1[v].y = fmaf(c1, w.y, fmaf(s1n, w.x, acc1[v].y));
+          for (int v = 0; v < VMAX; ++v) {
+            const float2 w = s_w[j][v];
+            acc0[v].x = fmaf(c0, w.x, fmaf(-s0n, w.y, acc0[v].x));
+            acc0[v].y = fmaf(c0, w.y, fmaf(s0n, w.x, acc0[v].y));
+            acc1[v].x = fmaf(c1, w.x, fmaf(-s1n, w.y, acc1[v].x));
+            acc1[v].y = fmaf(c1, w.y, fmaf(s1n, w.x, acc1[v].y));
+          }
         }
       }
-    }
 
-    float2 *dst = reinterpret_cast<float2 *>(p.out) + (int64_t)split * p.S * p.V + v0;
-    auto put = [&](float2 &to, float2 sum) {
-      if (fold > n_begin) {
-        sum.x += to.x;
-        sum.y += to.y;
-      }
-      to = sum;
-    };
+      float2 *dst = reinterpret_cast<float2 *>(p.out) + (int64_t)split * p.S * p.V + v0;
+      auto put = [&](float2 &to, float2 sum) {
+        if (fold > n_begin) {
+          sum.x += to.x;
+          sum.y += to.y;
+        }
+        to = sum;
+      };
 #pragma unroll
-    for (int v = 0; v < VMAX; ++v) {
-      if (v < nv && s0 < s_end) put(dst[(int64_t)s0 * p.V + v], acc0[v]);
-      if (v < nv && s1 < s_end) put(dst[(int64_t)s1 * p.V + v], acc1[v]);
-    }
-    fold = fold_end;
-    if (fold >= n_end) break;
+      for (int v = 0; v < VMAX; ++v) {
+        if (v < nv && s0 < s_end) put(dst[(int64_t)s0 * p.V + v], acc0[v]);
+        if (v < nv && s1 < s_end) put(dst[(int64_t)s1 * p.V + v], acc1[v]);
+      }
+      fold = fold_end;
+      if (fold >= n_end) break;
     }
   }  // tiles
 }
@@ -282,7 +265,7 @@ static void launch_plain(const PlainDev<T> &p, int64_t max_tiles, int v0, cudaSt
   const int64_t most = max_tiles * p.splits;
   const unsigned grid = (unsigned)(most < kPlainBlocks ? most : kPlainBlocks);
   if constexpr (sizeof(T) == 4) signal_plain32_kernel<VMAX><<<grid, kPlain32Threads, 0, st>>>(p, v0);
-  else signal_plain_kernel<VMAX, kPlainNodes><<<grid, kPlainThreads, 0, st>>>(p, v0);
+  else signal_plain_kernel<VMAX><<<grid, kPlainThreads, 0, st>>>(p, v0);
 }
 
 // Split count for slabs cut to `tiles` tiles: the most tiles that a block takes,
