@@ -42,8 +42,15 @@ struct PlainDev {
 constexpr int kPlainNodes = 128;            // nodes staged at a time
 constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an SM holds in FP32
 
-template <int VMAX>
-__global__ void __launch_bounds__(kPlainThreads) signal_plain_kernel(PlainDev<double> p, int v0) {
+// FP64.  Bound by the FP64 pipe's latency in sincos, so by the warps there:
+// BLOCKS = 2 of them an SM.  Left to itself the compiler takes more than 128
+// registers at two columns and up, and half the blocks: 5,003 nodes x 64 runs x 300
+// samples x 2 columns on a B200 1053 us, 787 us with two.  BLOCKS = 1 where all
+// blocks have an SM to themselves: they are dealt to the chip's unequal parts in
+// equal shares, so that 128 of them would put two on some SMs (8 columns, 100,003
+// nodes: 592 us, 877 us with two).  One column fits two blocks either way.
+template <int VMAX, int BLOCKS>
+__global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(PlainDev<double> p, int v0) {
   __shared__ double4 s_pos[kPlainNodes];         // moved x, y, z and phi * t
   __shared__ double s_w[kPlainNodes][2 * VMAX];  // decayed M * Mxy columns v0 .. v0 + VMAX
 
@@ -261,11 +268,19 @@ __global__ void __launch_bounds__(kReduceLanes *kReduceElems) split_reduce_kerne
 }
 
 template <typename T, int VMAX>
-static void launch_plain(const PlainDev<T> &p, int64_t max_tiles, int v0, cudaStream_t st) {
+static void launch_plain(const PlainDev<T> &p, int64_t tiles, int64_t max_tiles, int v0, cudaStream_t st) {
   const int64_t most = max_tiles * p.splits;
   const unsigned grid = (unsigned)(most < kPlainBlocks ? most : kPlainBlocks);
-  if constexpr (sizeof(T) == 4) signal_plain32_kernel<VMAX><<<grid, kPlain32Threads, 0, st>>>(p, v0);
-  else signal_plain_kernel<VMAX><<<grid, kPlainThreads, 0, st>>>(p, v0);
+  if constexpr (sizeof(T) == 4) {
+    signal_plain32_kernel<VMAX><<<grid, kPlain32Threads, 0, st>>>(p, v0);
+    return;
+  } else if constexpr (VMAX > 1) {
+    if (tiles * p.splits <= kSmCount) {
+      signal_plain_kernel<VMAX, 1><<<grid, kPlainThreads, 0, st>>>(p, v0);
+      return;
+    }
+  }
+  if constexpr (sizeof(T) == 8) signal_plain_kernel<VMAX, 2><<<grid, kPlainThreads, 0, st>>>(p, v0);
 }
 
 // Split count for slabs cut to `tiles` tiles: the most tiles that a block takes,
@@ -295,6 +310,7 @@ struct PlainPlan {
   GemmPlan gemm[2];
   int splits;
   int tile;
+  int64_t tiles;  // of slabs that are runs
 };
 
 template <typename T>
@@ -305,8 +321,8 @@ static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   int *ctl = c.take<int>(kCtlWords);
   pl.dev = c.take<PrepDev>(1);
   carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
-  pl.splits = choose_splits(S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1, N,
-                            S * V * 2 * (int64_t)sizeof(T));
+  pl.tiles = S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1;
+  pl.splits = choose_splits(pl.tiles, N, S * V * 2 * (int64_t)sizeof(T));
   plan_gemm<T>(a, pl.prep, pl.splits, pl.gemm);
   const int most = std::max(pl.splits, std::max(pl.gemm[0].splits, pl.gemm[1].splits));
   pl.partials = most > 1 ? c.take<T>((size_t)most * S * V * 2) : nullptr;
@@ -361,10 +377,10 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
   ScopedTimer timer(ctx, sizeof(T) == 4 ? "signal_f32" : "signal_f64");
   for (int v0 = 0; v0 < V; v0 += 8) {
     const int64_t nv = V - v0;
-    if (nv <= 1) launch_plain<T, 1>(p, max_tiles, v0, st);
-    else if (nv <= 2) launch_plain<T, 2>(p, max_tiles, v0, st);
-    else if (nv <= 4) launch_plain<T, 4>(p, max_tiles, v0, st);
-    else launch_plain<T, 8>(p, max_tiles, v0, st);
+    if (nv <= 1) launch_plain<T, 1>(p, pl.tiles, max_tiles, v0, st);
+    else if (nv <= 2) launch_plain<T, 2>(p, pl.tiles, max_tiles, v0, st);
+    else if (nv <= 4) launch_plain<T, 4>(p, pl.tiles, max_tiles, v0, st);
+    else launch_plain<T, 8>(p, pl.tiles, max_tiles, v0, st);
     count_launch();
     FM_TRY(check_launch("signal_plain_kernel"));
   }
