@@ -13,8 +13,8 @@
 // factors' phases are exact products of the inputs: no rounding is added.  The
 // FP32 form forms phases in FP64, the FP64 form keeps what their rounding leaves
 // out, and both reduce them exactly, where the unfactored FP64 form sums them in
-// radians as the reference does; sums over the nodes are in the form's type and no
-// longer than there.  2 pi is built from a float-rounded pi (MRI.h:13).
+// radians as the reference does; sums over the nodes are in the form's type, cut at
+// kGemmFold.  2 pi is built from a float-rounded pi (MRI.h:13).
 //
 // Block: a tile of rows x (q, v) pairs, 8 x 4 (FP64: 4 x 4) per thread, operands
 // of 16 nodes at a time in shared memory.  Forming a pair of elements costs some
@@ -512,22 +512,21 @@ static void gemm_shape(int64_t P, int64_t C, int64_t V, GemmPlan &g) {
 // add up, at a rate that grows with the warps there (latency: 8 / warps on top);
 // a block costs about 3 stages to set up and write, and a round of blocks 30 more
 // in latency and uneven ends; partial sums are written and read back at some 20 MB
-// a stage.  Splits of at least 64 nodes and 256 MB of partial sums, and at least as many as the unfactored form takes, so
-// that no sum in the form's type is longer than there.
-static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int least) {
+// a stage.  Splits of at least 64 nodes and within 256 MB of partial sums.
+static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes) {
   const int64_t units = (int64_t)g.products * g.nr * g.nc;
   const int64_t per_sm = std::max(1, std::min(65536 / (128 * g.threads), 228 * 1024 / (g.smem + 1024)));
-  int best = least;
+  int best = 1;
   double best_cost = 0.0;
-  int64_t most = out_bytes > 0 ? (256LL << 20) / out_bytes : 1;
+  int64_t most = out_bytes > 0 ? kPartialBytes / out_bytes : 1;
   if (most > 512) most = 512;
-  for (int s = least; s == least || (s <= most && N / s >= 64); ++s) {
+  for (int s = 1; s == 1 || (s <= most && N / s >= 64); ++s) {
     const int64_t on_sm = ceil_div(units * s, (int64_t)kSmCount);
     const double warps = (double)std::min(on_sm, per_sm) * (g.threads / 32);
     const double cost = (double)on_sm * ((double)N / s / kGemmStage) * (1.0 + 8.0 / warps) +
                         3.0 * (double)on_sm + 30.0 * (double)ceil_div(on_sm, per_sm) +
                         (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
-    if (s == least || cost < best_cost) {
+    if (s == 1 || cost < best_cost) {
       best = s;
       best_cost = cost;
     }
@@ -536,7 +535,7 @@ static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int leas
 }
 
 template <typename T>
-void plan_gemm(const fm_signal_args *a, const PrepDev &pr, int least, GemmPlan (&g)[2]) {
+void plan_gemm(const fm_signal_args *a, const PrepDev &pr, GemmPlan (&g)[2]) {
   const int64_t V = a->n_vencs, out_bytes = pr.S * V * 2 * (int64_t)sizeof(T);
   g[0] = g[1] = GemmPlan{};
   if (pr.S == 0 || V == 0 || pr.N == 0) return;
@@ -549,7 +548,7 @@ void plan_gemm(const fm_signal_args *a, const PrepDev &pr, int least, GemmPlan (
     g[1].products = pr.n_ro;
   }
   for (GemmPlan &k : g)
-    if (k.products > 0) k.splits = gemm_splits(k, pr.N, out_bytes, least);
+    if (k.products > 0) k.splits = gemm_splits(k, pr.N, out_bytes);
 }
 
 template <typename T>
@@ -592,8 +591,8 @@ int launch_gemm(const fm_signal_args *a, const PrepDev &pr, const GemmPlan (&g)[
   return FM_OK;
 }
 
-template void plan_gemm<float>(const fm_signal_args *, const PrepDev &, int, GemmPlan (&)[2]);
-template void plan_gemm<double>(const fm_signal_args *, const PrepDev &, int, GemmPlan (&)[2]);
+template void plan_gemm<float>(const fm_signal_args *, const PrepDev &, GemmPlan (&)[2]);
+template void plan_gemm<double>(const fm_signal_args *, const PrepDev &, GemmPlan (&)[2]);
 template int launch_gemm<float>(const fm_signal_args *, const PrepDev &, const GemmPlan (&)[2], float *, float *,
                                 cudaStream_t);
 template int launch_gemm<double>(const fm_signal_args *, const PrepDev &, const GemmPlan (&)[2], double *, double *,

@@ -50,12 +50,14 @@ constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an
 // equal shares, so that 128 of them would put two on some SMs (8 columns, 100,003
 // nodes: 592 us, 877 us with two).  One column fits two blocks either way.
 template <int VMAX, int BLOCKS>
-__global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(PlainDev<double> p, int v0) {
+__global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(PlainDev<double> p, int v0,
+                                                                            bool either) {
   __shared__ double4 s_pos[kPlainNodes];         // moved x, y, z and phi * t
   __shared__ double s_w[kPlainNodes][2 * VMAX];  // decayed M * Mxy columns v0 .. v0 + VMAX
 
   const int n_tiles = *p.n_tiles;
   const int64_t items = (int64_t)n_tiles * p.splits;
+  if (either && (items <= kSmCount) != (BLOCKS == 1)) return;  // the other instance's
   for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
     const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
     __syncthreads();  // the previous tile's readers of s_pos / s_w are done
@@ -273,27 +275,44 @@ static void launch_plain(const PlainDev<T> &p, int64_t tiles, int64_t max_tiles,
   const unsigned grid = (unsigned)(most < kPlainBlocks ? most : kPlainBlocks);
   if constexpr (sizeof(T) == 4) {
     signal_plain32_kernel<VMAX><<<grid, kPlain32Threads, 0, st>>>(p, v0);
-    return;
-  } else if constexpr (VMAX > 1) {
-    if (tiles * p.splits <= kSmCount) {
-      signal_plain_kernel<VMAX, 1><<<grid, kPlainThreads, 0, st>>>(p, v0);
-      return;
+    count_launch();
+  } else {
+    // slabs that are not runs make more tiles than planned, so the device decides
+    const bool either = VMAX > 1 && tiles * p.splits <= kSmCount;
+    if constexpr (VMAX > 1) {
+      if (either) {
+        signal_plain_kernel<VMAX, 1><<<grid, kPlainThreads, 0, st>>>(p, v0, true);
+        count_launch();
+      }
     }
+    signal_plain_kernel<VMAX, 2><<<grid, kPlainThreads, 0, st>>>(p, v0, either);
+    count_launch();
   }
-  if constexpr (sizeof(T) == 8) signal_plain_kernel<VMAX, 2><<<grid, kPlainThreads, 0, st>>>(p, v0);
 }
 
-// Split count for slabs cut to `tiles` tiles: the most tiles that a block takes,
-// over the splits, and 1% a split for its partial sums; at least 1024 nodes a
-// split and 256 MB of partial sums (`out_bytes` a split).  128 tiles go to 592
-// blocks in 9 splits, 2 for each block and 0.22 of a tile's time; in the fewest
-// splits that give every block one (5), it is 0.4.
-constexpr int64_t kPartialBytes = 256LL << 20;
+// Split count for slabs cut to `tiles` tiles, within kPartialBytes (`out_bytes` a
+// split).
+// FP32, an SM holding four blocks: the most tiles that a block takes, over the
+// splits, and 1% a split for its partial sums; at least 1024 nodes a split.  128
+// tiles go to 592 blocks in 9 splits, 2 for each block and 0.22 of a tile's time; in
+// the fewest splits that give every block one (5), it is 0.4.
+// FP64, two blocks: the tiles of the fullest SM, whose blocks share its FP64 pipe
+// (the first alone leaves a third of it idle), and 0.2% a split; at least 512 nodes.
+// 512 tiles of 2,003 nodes are 4 for some SMs in one split, 7 halves in two: 1107 us
+// and 1005 us a call (one column).
+template <typename T>
 static int choose_splits(int64_t tiles, int64_t N, int64_t out_bytes) {
+  constexpr bool f64 = sizeof(T) == 8;
   int best = 1;
   double best_cost = 0.0;
-  for (int s = 1; s <= 64 && (s == 1 || (N / s >= 1024 && s * out_bytes <= kPartialBytes)); ++s) {
-    const double cost = (double)ceil_div(tiles * s, (int64_t)kPlainBlocks) / s * (1.0 + 0.01 * s);
+  for (int s = 1; s <= 64 && (s == 1 || (N / s >= (f64 ? 512 : 1024) && s * out_bytes <= kPartialBytes)); ++s) {
+    double cost;
+    if constexpr (f64) {
+      const int64_t on_sm = ceil_div(tiles * s, (int64_t)kSmCount);
+      cost = (1.5 * (double)(on_sm / 2 * 2) + 2.0 * (double)(on_sm % 2)) / s * (1.0 + 0.002 * s);
+    } else {
+      cost = (double)ceil_div(tiles * s, (int64_t)kPlainBlocks) / s * (1.0 + 0.01 * s);
+    }
     if (s == 1 || cost < best_cost) {
       best = s;
       best_cost = cost;
@@ -322,8 +341,8 @@ static void carve_plain(Carve &c, const fm_signal_args *a, PlainPlan<T> &pl) {
   pl.dev = c.take<PrepDev>(1);
   carve_prep(c, a, pl.tile, false, 0, sizeof(T), ctl, pl.prep);
   pl.tiles = S > 0 ? a->n_ro * ceil_div(a->n_lines * a->n_kz, (int64_t)pl.tile) : 1;
-  pl.splits = choose_splits(pl.tiles, N, S * V * 2 * (int64_t)sizeof(T));
-  plan_gemm<T>(a, pl.prep, pl.splits, pl.gemm);
+  pl.splits = choose_splits<T>(pl.tiles, N, S * V * 2 * (int64_t)sizeof(T));
+  plan_gemm<T>(a, pl.prep, pl.gemm);
   const int most = std::max(pl.splits, std::max(pl.gemm[0].splits, pl.gemm[1].splits));
   pl.partials = most > 1 ? c.take<T>((size_t)most * S * V * 2) : nullptr;
 }
@@ -381,7 +400,6 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
     else if (nv <= 2) launch_plain<T, 2>(p, pl.tiles, max_tiles, v0, st);
     else if (nv <= 4) launch_plain<T, 4>(p, pl.tiles, max_tiles, v0, st);
     else launch_plain<T, 8>(p, pl.tiles, max_tiles, v0, st);
-    count_launch();
     FM_TRY(check_launch("signal_plain_kernel"));
   }
   FM_TRY(launch_gemm<T>(a, pl.prep, pl.gemm, out, pl.partials, st));

@@ -45,3 +45,10 @@ def test_partial_sums_of_small_tensor_core_problems(n, grid, V):
     """Few nodes: no more than 16 splits' sums, as a served request is counted."""
     S = grid[0] * grid[1] * grid[2]
     assert _bytes(n, V, grid, "bf16x3") <= 16 * S * V * 8 + 64 * S + n * (16 * V + 32) + MB
+
+
+def test_unfactored_fp64_tiles_are_split_evenly():
+    """512 tiles are up to 4 for an SM, or 7 halves: two splits' sums are held."""
+    grid, n, V = (16, 8192, 1), 2003, 1
+    S = grid[0] * grid[1]
+    assert _bytes(n, V, grid, "f64") - _bytes(1, V, grid, "f64") >= 2 * S * V * 16
