@@ -32,14 +32,21 @@ namespace fm {
 
 constexpr int kMaxNb = 10;
 
+// Triplets that a warp orders: four to ten times what the nodes of a mesh of
+// good elements have (24 tetrahedra or 8 hexahedra around a node).
+template <int NB>
+constexpr int kWarpTriplets = NB <= 5 ? 256 : 512;
+constexpr int kColWarps = 4;
+
 // Element matrices, Me(i, j) at vals[(e nb + j) nb + i] so that the entries of a
-// column lie together, and each element's place among those of its nodes.
+// column lie together, and each element's place among those of its nodes; `over`
+// is set where a node has more elements than a warp orders.
 template <typename T, int NB>
 __global__ void __launch_bounds__(128) mass_local_kernel(int64_t E, const int *__restrict__ elems, int64_t N,
                                                          const T *__restrict__ nodes, int Q, const T *__restrict__ qw,
                                                          const T *__restrict__ tab, T *__restrict__ vals,
                                                          int *__restrict__ degree, int *__restrict__ place,
-                                                         int *__restrict__ bad) {
+                                                         int *__restrict__ bad, int *__restrict__ over) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
   T X[NB][3];
@@ -50,7 +57,9 @@ __global__ void __launch_bounds__(128) mass_local_kernel(int64_t E, const int *_
       atomicExch(bad, 1);
       v = 0;
     }
-    place[e * NB + i] = atomicAdd(degree + v, 1);
+    const int at = atomicAdd(degree + v, 1);
+    if (at == kWarpTriplets<NB> / NB) *over = 1;
+    place[e * NB + i] = at;
     X[i][0] = nodes[3 * (int64_t)v + 0];
     X[i][1] = nodes[3 * (int64_t)v + 1];
     X[i][2] = nodes[3 * (int64_t)v + 2];
@@ -96,19 +105,13 @@ __global__ void __launch_bounds__(128) mass_local_kernel(int64_t E, const int *_
 template <int NB>
 __global__ void mass_around_kernel(int64_t count, const int *__restrict__ elems, int64_t N,
                                    const int *__restrict__ start, const int *__restrict__ place,
-                                   int *__restrict__ around) {
+                                   int *__restrict__ around, const int *__restrict__ over) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
+  if (k >= count || *over) return;
   int v = elems[k];
   if (v < 0 || v >= N) v = 0;
   around[start[v] + place[k]] = (int)k;
 }
-
-// Triplets that a warp orders: four to ten times what the nodes of a mesh of
-// good elements have (24 tetrahedra or 8 hexahedra around a node).
-template <int NB>
-constexpr int kWarpTriplets = NB <= 5 ? 256 : 512;
-constexpr int kColWarps = 4;
 
 // One warp per column: its distinct rows, ascending, and the sums of their
 // triplets at rows/data[start[c] nb ..], their number in count[c]; or, with
@@ -120,21 +123,14 @@ __global__ void __launch_bounds__(32 * kColWarps) mass_columns_kernel(int64_t N,
                                                                       const int *__restrict__ around,
                                                                       int *__restrict__ rows_out, T *__restrict__ data_out,
                                                                       int *__restrict__ count, T *__restrict__ lump,
-                                                                      int *__restrict__ over) {
+                                                                      const int *__restrict__ over) {
   constexpr int CAP = kWarpTriplets<NB>;
   __shared__ __align__(16) int s_row[kColWarps][CAP], s_sorted[kColWarps][CAP];
   __shared__ __align__(16) T s_val[kColWarps][CAP], s_vsorted[kColWarps][CAP];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t c = (int64_t)blockIdx.x * kColWarps + warp;
-  if (c >= N) return;
+  if (c >= N || *over) return;  // (the matrix is sorted then)
   const int first = start[c], d = start[c + 1] - first, m = d * NB;
-  if (d > CAP / NB) {
-    if (lane == 0) {
-      atomicExch(over, 1);
-      if (count) count[c] = 0;
-    }
-    return;
-  }
   int *row = s_row[warp], *sorted = s_sorted[warp];
   T *val = s_val[warp], *vsorted = s_vsorted[warp];
   // the elements around the node in element order
@@ -344,14 +340,14 @@ static void mass_elements(const fm_mass_args *a, MassPlan &p, cudaStream_t st) {
   mass_local_kernel<T, NB><<<(unsigned)ceil_div(a->n_elems, 128), 128, 0, st>>>(
       a->n_elems, a->elems, a->n_nodes, static_cast<const T *>(a->nodes), a->n_qpoints,
       static_cast<const T *>(a->qweights), static_cast<const T *>(a->tabulated), static_cast<T *>(p.vals), p.degree,
-      p.place, p.status + kMassBad);
+      p.place, p.status + kMassBad, p.status + kMassOver);
   count_launch();
 }
 template <typename T, int NB>
 static void mass_columns(const fm_mass_args *a, MassPlan &p, T *lump, cudaStream_t st) {
   const int64_t count = a->n_elems * NB;
   mass_around_kernel<NB><<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(count, a->elems, a->n_nodes, p.start, p.place,
-                                                                         p.around);
+                                                                         p.around, p.status + kMassOver);
   count_launch();
   mass_columns_kernel<T, NB><<<(unsigned)ceil_div(a->n_nodes, kColWarps), 32 * kColWarps, 0, st>>>(
       a->n_nodes, a->elems, static_cast<const T *>(p.vals), p.start, p.around, p.rows, static_cast<T *>(p.data),
