@@ -43,6 +43,7 @@
 // 2,410 (with runs as columns, kTcRuns).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "signal_common.cuh"
@@ -530,6 +531,58 @@ __device__ inline void tc_request_block(const TcNodeArgs &a, int64_t n0, unsigne
   if (a.mstage) ptx::bulk_copy_g2s((void *)v.modes, a.modes + n0 * a.mstage, tc_mode_bytes(a.mstage), rawfull);
 }
 
+// motion_disp's sum over the modes of a POD term in W modes a load.  A warp's
+// nodes are rows apart, so each load is 32 requests whatever its width, and the two
+// node warps must keep the pace that the whole block once set: 20,011 nodes x 64 x 64
+// samples on a B200, 20 modes 676 us with single reads, 425 us; 64 modes 2029 us,
+// 799 us (with nodes formed by four warps it was 620 us and 1633 us).
+template <int W>
+__device__ __forceinline__ void tc_pod_sum(const float *Phi, const float *wk, int r, float &tx, float &ty, float &tz) {
+  using V = typename std::conditional<W == 4, float4, typename std::conditional<W == 2, float2, float>::type>::type;
+  tx = 0.f; ty = 0.f; tz = 0.f;
+#pragma unroll 3  // (what the kernel's registers take best; 1 leaves reads one after the other)
+  for (int m = 0; m < r; m += W) {
+    const V a = __ldg(reinterpret_cast<const V *>(Phi + m)), b = __ldg(reinterpret_cast<const V *>(Phi + r + m)),
+            c = __ldg(reinterpret_cast<const V *>(Phi + 2 * r + m));
+    const float *pa = reinterpret_cast<const float *>(&a), *pb = reinterpret_cast<const float *>(&b),
+                *pc = reinterpret_cast<const float *>(&c);
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const float wm = wk[m + i];
+      tx = fmaf(pa[i], wm, tx);
+      ty = fmaf(pb[i], wm, ty);
+      tz = fmaf(pc[i], wm, tz);
+    }
+  }
+}
+
+// motion_disp, the modes of each POD term read as wide as its rows are aligned.
+__device__ __forceinline__ void tc_motion_disp(const MotionDev &md, const float *w, int64_t n, float &dx, float &dy,
+                                               float &dz) {
+  float sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < md.n_terms; ++k) {
+    const fm_motion_term &T = md.terms[k];
+    const float *wk = w + md.slot0[k];
+    float tx, ty, tz;
+    if (T.kind == FM_TERM_RESPIRATORY) {
+      tx = __fmul_rn(wk[0], T.direction[0]);
+      ty = __fmul_rn(wk[0], T.direction[1]);
+      tz = __fmul_rn(wk[0], T.direction[2]);
+    } else {
+      const int r = T.n_modes;
+      const float *Phi = T.modes + (size_t)n * 3 * r;
+      const unsigned by = (unsigned)(uintptr_t)T.modes | 4u * r;  // rows start, and components lie, at multiples of it
+      if (by % 16 == 0) tc_pod_sum<4>(Phi, wk, r, tx, ty, tz);
+      else if (by % 8 == 0) tc_pod_sum<2>(Phi, wk, r, tx, ty, tz);
+      else tc_pod_sum<1>(Phi, wk, r, tx, ty, tz);
+    }
+    if (k == 0) { sx = tx; sy = ty; sz = tz; }
+    else { sx = __fadd_rn(sx, tx); sy = __fadd_rn(sy, ty); sz = __fadd_rn(sz, tz); }
+  }
+  dx = sx; dy = sy; dz = sz;
+}
+
 // Node quantities of the block at n0 into a node buffer (one warp, nodes lane,
 // lane + 32 ..): moved position (in FP64 for the phase
 // products) and the decayed, off-resonance rotated weights
@@ -540,26 +593,26 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
                                          const TcRawView &raw, unsigned char *buf, float *wblk, int slot0) {
   constexpr int kPer = kTcBlockNodes / 32, kStep = 32;
   double *pos = reinterpret_cast<double *>(buf);
-  float x[kPer], y[kPer], z[kPer], t2[kPer], phi[kPer];
   bool in[kPer];
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int slot = slot0 + i * kStep;
-    const int64_t n = n0 + slot;
-    in[i] = n < n_end;
+  for (int i = 0; i < kPer; ++i) in[i] = n0 + slot0 + i * kStep < n_end;
+  auto place = [&](int slot, bool inside, float &x, float &y, float &z) {
     if (staged) {
-      x[i] = raw.r0[3 * slot]; y[i] = raw.r0[3 * slot + 1]; z[i] = raw.r0[3 * slot + 2];
-      t2[i] = raw.T2[slot];
-      phi[i] = raw.phi[slot];
-    } else if (in[i]) {
-      x[i] = a.r0[3 * n]; y[i] = a.r0[3 * n + 1]; z[i] = a.r0[3 * n + 2];
-      t2[i] = a.T2[n];
-      phi[i] = a.phi[n];
+      x = raw.r0[3 * slot]; y = raw.r0[3 * slot + 1]; z = raw.r0[3 * slot + 2];
+    } else if (inside) {
+      const float *r = a.r0 + 3 * (n0 + slot);
+      x = r[0]; y = r[1]; z = r[2];
     } else {
-      x[i] = y[i] = z[i] = phi[i] = 0.f;
-      t2[i] = 1.f;
+      x = y = z = 0.f;
     }
-  }
+  };
+  int rmax = 0;
+  auto put_place = [&](int slot, float x, float y, float z) {
+    pos[slot] = (double)x;
+    pos[kTcBlockNodes + slot] = (double)y;
+    pos[2 * kTcBlockNodes + slot] = (double)z;
+    rmax = max(rmax, __float_as_int(fabsf(x) + fabsf(y) + fabsf(z)) & 0x7fffffff);
+  };
   if (staged && a.mstage) {
     // the single POD term's sum (motion_disp's products in its order), the
     // mode rows read from the staged block
@@ -580,35 +633,41 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
     }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      x[i] = x[i] + dx[i]; y[i] = y[i] + dy[i]; z[i] = z[i] + dz[i];
+      float x, y, z;
+      place(slot0 + i * kStep, true, x, y, z);
+      put_place(slot0 + i * kStep, x + dx[i], y + dy[i], z + dz[i]);
     }
   } else if (a.wrun || a.table) {
 #pragma unroll 1
-    for (int i = 0; i < kPer; ++i) {
-      const int64_t n = n0 + slot0 + i * kStep;
-      if (n >= n_end) continue;
-      float dx, dy, dz;
-      if (a.wrun) {
-        motion_disp(p.md, a.wrun, n, p.N, dx, dy, dz);
-      } else {
-        dx = a.table[3 * n]; dy = a.table[3 * n + 1]; dz = a.table[3 * n + 2];
-      }
-      // (compile-time indices keep the arrays in registers)
-#pragma unroll
-      for (int q = 0; q < kPer; ++q)
-        if (q == i) {
-          x[q] = x[q] + dx; y[q] = y[q] + dy; z[q] = z[q] + dz;
+    for (int slot = slot0; slot < kTcBlockNodes; slot += kStep) {
+      const int64_t n = n0 + slot;
+      float x, y, z;
+      place(slot, n < n_end, x, y, z);
+      if (n < n_end) {
+        float dx, dy, dz;
+        if (a.wrun) {
+          tc_motion_disp(p.md, a.wrun, n, dx, dy, dz);
+        } else {
+          dx = a.table[3 * n]; dy = a.table[3 * n + 1]; dz = a.table[3 * n + 2];
         }
+        x = x + dx; y = y + dy; z = z + dz;
+      }
+      put_place(slot, x, y, z);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      float x, y, z;
+      place(slot0 + i * kStep, in[i], x, y, z);
+      put_place(slot0 + i * kStep, x, y, z);
     }
   }
-  int rmax = 0;
+  float t2[kPer], phi[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     const int slot = slot0 + i * kStep;
-    pos[slot] = (double)x[i];
-    pos[kTcBlockNodes + slot] = (double)y[i];
-    pos[2 * kTcBlockNodes + slot] = (double)z[i];
-    rmax = max(rmax, __float_as_int(fabsf(x[i]) + fabsf(y[i]) + fabsf(z[i])) & 0x7fffffff);
+    t2[i] = staged ? raw.T2[slot] : (in[i] ? a.T2[n0 + slot] : 1.f);
+    phi[i] = staged ? raw.phi[slot] : (in[i] ? a.phi[n0 + slot] : 0.f);
   }
   // decay exp(-t / T2) and off-resonance rotation exp(i phi t) of a run: the
   // fast exponential of -t (1 / T2), and the phase phi t reduced in cycles in
