@@ -9,8 +9,8 @@
 //           stretch, which slabs are one run and factor, whether M is diagonal
 //   runs    run starts and times, compacted in order; rows of an M of as many
 //           entries as rows that is not diagonal
-//   items   M Mxy (of such an M or a diagonal one), motion weights, factored runs
-//           and tiles counted
+//   items   M Mxy (of such an M or a diagonal one), motion weights, the largest
+//           |phi| and |t|, factored runs and tiles counted
 //   fill    factored runs and tiles, compacted in order
 // These phases are a few microseconds of work each, so launches bound them:
 // one chain per problem (33 launches and copies, the scans two each) took
@@ -123,19 +123,6 @@ __device__ inline int block_sum(int v) {
   return s;
 }
 
-// Largest of v over the block's threads, in every thread.
-__device__ inline int block_max(int v) {
-  __shared__ int part[kPrepThreads / 32];
-  v = __reduce_max_sync(0xffffffffu, v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int s = part[0];
-#pragma unroll
-  for (int i = 1; i < kPrepThreads / 32; ++i) s = max(s, part[i]);
-  return s;
-}
-
 // Exclusive prefix of v over the block's threads; `total` the block's sum.
 __device__ inline int block_exclusive(int v, int &total) {
   __shared__ int part[kPrepThreads / 32];
@@ -180,12 +167,6 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   const T *t = static_cast<const T *>(p.t);
   const T *kc[3] = {static_cast<const T *>(p.kx), static_cast<const T *>(p.ky), static_cast<const T *>(p.kz)};
   int flags = 0;
-  int phi_max = 0, t_max = 0;  // float bits
-  if (p.turns) {
-    const T *phi = static_cast<const T *>(p.phi);
-    for (int64_t n = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; n < p.N; n += (int64_t)gridDim.x * kPrepThreads)
-      phi_max = max(phi_max, __float_as_int((float)phi[n]) & 0x7fffffff);
-  }
   const int c = blockIdx.x;
   if (c < p.n_chunks) {
     const int64_t s0 = (int64_t)c * p.chunk, s1 = min(p.S, s0 + p.chunk);
@@ -193,7 +174,6 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
     for (int64_t s = s0 + threadIdx.x; s < s1; s += kPrepThreads) {
       const bool first = starts_run(t, s);
       starts += first ? 1 : 0;
-      if (p.turns && t[s] == t[s]) t_max = max(t_max, __float_as_int((float)t[s]) & 0x7fffffff);
       const int i = (int)((unsigned)s / (unsigned)p.Ls), w = (int)s - i * p.Ls;
       if (first != (w == 0)) {
         // slab i is not exactly one run (nor the slab before it, when a run
@@ -253,12 +233,6 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   }
   flags = __reduce_or_sync(0xffffffffu, flags);
   if ((threadIdx.x & 31) == 0 && flags) atomicOr(p.ctl + kCtlFlags, flags);
-  if (p.turns) {
-    phi_max = block_max(phi_max);
-    t_max = block_max(t_max);
-    if (threadIdx.x == 0 && phi_max) atomicMax(p.ctl + kCtlPhi, phi_max);
-    if (threadIdx.x == 0 && t_max) atomicMax(p.ctl + kCtlTime, t_max);
-  }
 }
 
 // ---- runs ----------------------------------------------------------------
@@ -424,6 +398,17 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
   const PrepDev &p = probs[blockIdx.y];
   const int n_runs = p.ctl[kCtlRuns];
   const int64_t tid = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x, stride = (int64_t)gridDim.x * kPrepThreads;
+  int phi_max = 0, t_max = 0;
+  if (p.turns) {
+    // |x| as float bits, which compare as numbers do and NaN above them
+    auto size_bits = [](float x) { return __float_as_int(x) & 0x7fffffff; };
+    for (int64_t i = tid; i < max(p.N, (int64_t)n_runs); i += stride) {
+      const T phi = i < p.N ? static_cast<const T *>(p.phi)[i] : T(0);
+      const double t = i < n_runs ? p.run_t[i] : 0.0;
+      phi_max = max(phi_max, size_bits((float)phi));
+      if (t == t) t_max = max(t_max, size_bits((float)t));
+    }
+  }
   if (p.diag && !(p.ctl[kCtlFlags] & kFlagNotDiagonal)) {
     const T *m = static_cast<const T *>(p.data);
     const C *x = static_cast<const C *>(p.Mxy);
@@ -445,6 +430,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
     for (int64_t idx = tid; idx < total; idx += stride) {
       const int64_t g = idx / p.md.slots;
       p.weights[idx] = motion_weight(p.md, (int)(idx - g * p.md.slots), p.run_t[g]);
+    }
+  }
+  if (p.turns) {
+    phi_max = __reduce_max_sync(0xffffffffu, phi_max);
+    t_max = __reduce_max_sync(0xffffffffu, t_max);
+    if ((threadIdx.x & 31) == 0) {
+      if (phi_max) atomicMax(p.ctl + kCtlPhi, phi_max);
+      if (t_max) atomicMax(p.ctl + kCtlTime, t_max);
     }
   }
   if (tid == 0 && prep_table_mismatch(p)) atomicOr(p.ctl + kCtlError, kErrTableCalls);
