@@ -40,6 +40,7 @@ struct PlainDev {
 };
 
 constexpr int kPlainNodes = 128;            // nodes staged at a time
+constexpr int kPlainFold64 = 1024;          // nodes in one FP64 sum
 constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an SM holds in FP32
 
 // FP64.  Bound by the FP64 pipe's latency in sincos, so by the warps there:
@@ -77,7 +78,21 @@ __global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(Pla
     const int64_t n_begin = (int64_t)split * p.chunk;
     const int64_t n_end = min(p.N, n_begin + p.chunk);
     const float *wrun = p.weights ? p.weights + (int64_t)g * p.md.slots : nullptr;
-    for (int64_t nb = n_begin; nb < n_end; nb += kPlainNodes) {
+    double *dst = p.out + ((int64_t)split * p.S * p.V + (int64_t)s * p.V + v0) * 2;
+    for (int64_t nb = n_begin;; nb += kPlainNodes) {
+      // a sum of kPlainFold64 nodes in registers at a time, then added to the output
+      if (nb >= n_end || (nb > n_begin && (nb - n_begin) % kPlainFold64 == 0)) {
+        const bool first = nb - n_begin <= kPlainFold64;
+#pragma unroll
+        for (int v = 0; v < VMAX; ++v) {
+          if (in && v < nv) {
+            dst[2 * v + 0] = first ? acc_r[v] : dst[2 * v + 0] + acc_r[v];
+            dst[2 * v + 1] = first ? acc_i[v] : dst[2 * v + 1] + acc_i[v];
+          }
+          acc_r[v] = acc_i[v] = 0.0;
+        }
+        if (nb >= n_end) break;
+      }
       const int cnt = (int)min((int64_t)kPlainNodes, n_end - nb);
       __syncthreads();
       for (int j = threadIdx.x; j < cnt; j += kPlainThreads) {
@@ -120,15 +135,6 @@ __global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(Pla
       }
     }
 
-    if (!in) continue;
-    double *dst = p.out + ((int64_t)split * p.S * p.V + (int64_t)s * p.V + v0) * 2;
-#pragma unroll
-    for (int v = 0; v < VMAX; ++v) {
-      if (v < nv) {
-        dst[2 * v + 0] = acc_r[v];
-        dst[2 * v + 1] = acc_i[v];
-      }
-    }
   }  // tiles
 }
 

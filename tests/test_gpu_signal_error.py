@@ -1,6 +1,9 @@
-"""Error of the split-BF16 form where its accumulation, not the split, makes it:
-like nodes, whose terms are equal, so that the sum of 512 nodes is 32 times that of
-16 but for what the accumulators truncate."""
+"""Error where accumulation makes it.  The split-BF16 form on like nodes, whose terms
+are equal, so that the sum of 512 nodes is 32 times that of 16 but for what the
+accumulators truncate; the unfactored FP64 form on a plain sum."""
+import math
+
+import numpy as np
 import pytest
 import torch
 
@@ -35,3 +38,25 @@ def test_wide_tiles_truncate_no_more_than_narrow_ones(cuda):
         return ((many / 32 - few).abs() / few.abs()).mean().item()
     wide, narrow = error(128), error(16)
     assert 0 < wide < 1.15 * narrow
+
+
+def test_fp64_sums_are_cut(cuda):
+    """592 tiles are four for each SM, so the nodes are not split.  Nodes at one place
+    and samples at k = 0 of motion forms (unfactored): the result is the plain sum of
+    M Mxy.  Rounding of a sum of n positive terms is some u sqrt(n) / 3 of it (u =
+    2^-53): 47 u for 20,000 in one sum, 3 u in sums of 1,024."""
+    n, V = 20_000, 8
+    rng = np.random.default_rng(3)
+    traj = W.radial3d(n_ro=592, n_spokes=4)
+    up = lambda a, d=torch.float64: torch.from_numpy(np.ascontiguousarray(a)).to(device=cuda, dtype=d)  # noqa: E731
+    idx = torch.arange(n + 1, dtype=torch.int32, device=cuda)
+    cols = rng.uniform(0.5, 1.5, (n, V)) + 1j * rng.uniform(0.5, 1.5, (n, V))
+    inp = ops.SignalInputs(M=ops.SparseCSC((n, n), idx, idx[:n], up(np.ones(n))), kx=up(0 * traj.kx),
+                           ky=up(0 * traj.ky), kz=up(0 * traj.kz), t=up(traj.t), r0=up(np.zeros((n, 3))),
+                           phi=up(np.zeros(n)), T2=up(np.full(n, np.inf)), Mxy=up(cols, torch.complex128))
+    motion = lower(W.sinusoidal_pod(n, n_modes=1), n, cuda)
+    K = ops.signal(inp, motion, "f64").cpu().numpy().reshape(-1, V)
+    assert (K == K[0]).all()  # every sample sums alike
+    exact = np.array([complex(math.fsum(c.real), math.fsum(c.imag)) for c in cols.T])
+    rel = np.concatenate([(K[0] - exact).real / exact.real, (K[0] - exact).imag / exact.imag])
+    assert np.sqrt((rel ** 2).mean()) < 15 * 2.0 ** -53
