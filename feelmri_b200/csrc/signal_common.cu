@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(kPrepThreads) prep_runs_kernel(const PrepDev *
   if (prep_listed(p)) prep_link_rows(p);
   if (c >= p.n_chunks) return;
   if (!(p.ctl[kCtlFlags] & kFlagRuns)) {  // run g is slab g
-    for (int g = c * kPrepThreads + threadIdx.x; g < p.n_ro; g += p.n_chunks * kPrepThreads) {
-      p.start[g] = g * p.Ls;
-      p.run_t[g] = (double)t[(int64_t)g * p.Ls];
+    for (int64_t g = c * kPrepThreads + threadIdx.x; g < p.n_ro; g += p.n_chunks * kPrepThreads) {
+      p.start[g] = (int)(g * p.Ls);
+      p.run_t[g] = (double)t[g * p.Ls];
     }
     if (c == 0 && threadIdx.x == 0) {
       p.start[p.n_ro] = (int)p.S;
@@ -444,12 +444,12 @@ __global__ void __launch_bounds__(kPrepThreads) prep_items_kernel(const PrepDev 
   const int c = blockIdx.x;
   if (c >= p.n_chunks) return;
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = prep_unlisted(p) ? 0 : min(n_runs, (c + 1) * per);
+  const int64_t g1 = prep_unlisted(p) ? 0 : min((int64_t)n_runs, (int64_t)(c + 1) * per);
   int nf = 0, nt = 0;
-  for (int g = c * per + threadIdx.x; g < g1; g += kPrepThreads) {
+  for (int64_t g = (int64_t)c * per + threadIdx.x; g < g1; g += kPrepThreads) {
     bool fac;
     int tiles;
-    prep_run_items(p, g, fac, tiles);
+    prep_run_items(p, (int)g, fac, tiles);
     nf += fac ? 1 : 0;
     nt += tiles;
   }
@@ -472,16 +472,16 @@ __global__ void __launch_bounds__(kPrepThreads) prep_fill_kernel(const PrepDev *
   int t0 = block_prefix(p.chunk_tiles, c);
   const int n_runs = p.ctl[kCtlRuns];
   const int per = (n_runs + p.n_chunks - 1) / p.n_chunks;
-  const int g1 = prep_unlisted(p) ? 0 : min(n_runs, (c + 1) * per);
-  for (int gb = c * per; gb < g1; gb += kPrepThreads) {
-    const int g = gb + threadIdx.x;
+  const int64_t g1 = prep_unlisted(p) ? 0 : min((int64_t)n_runs, (int64_t)(c + 1) * per);
+  for (int64_t gb = (int64_t)c * per; gb < g1; gb += kPrepThreads) {
+    const int64_t g = gb + threadIdx.x;
     bool fac = false;
     int tiles = 0, nf, nt;
-    if (g < g1) prep_run_items(p, g, fac, tiles);
+    if (g < g1) prep_run_items(p, (int)g, fac, tiles);
     const int f = f0 + block_exclusive(fac ? 1 : 0, nf);
     const int k = t0 + block_exclusive(tiles, nt);
-    if (fac) p.frun[f] = g;
-    for (int i = 0; i < tiles; ++i) p.tiles[k + i] = make_int2(g, i * p.tile);
+    if (fac) p.frun[f] = (int)g;
+    for (int i = 0; i < tiles; ++i) p.tiles[k + i] = make_int2((int)g, i * p.tile);
     f0 += nf;
     t0 += nt;
   }

@@ -40,7 +40,7 @@ struct PlainDev {
 };
 
 constexpr int kPlainNodes = 128;            // nodes staged at a time
-constexpr int kPlainFold64 = 1024;          // nodes in one FP64 sum
+constexpr int kPlainFold64 = 512;           // nodes in one FP64 sum
 constexpr int kPlainBlocks = 4 * kSmCount;  // blocks sharing the tiles: what an SM holds in FP32
 
 // FP64.  Bound by the FP64 pipe's latency in sincos, so by the warps there:
@@ -63,8 +63,8 @@ __global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(Pla
     const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
     __syncthreads();  // the previous tile's readers of s_pos / s_w are done
     const int g = p.tiles[tile].x;
-    const int s = p.run_start[g] + p.tiles[tile].y + threadIdx.x;
-    const bool in = s < p.run_start[g + 1];
+    const int s_begin = p.run_start[g] + p.tiles[tile].y, s = s_begin + threadIdx.x;
+    const bool in = (int)threadIdx.x < p.run_start[g + 1] - s_begin;  // (s itself may pass 2^31)
     const double tg = p.run_t[g];
     const int nv = (int)min((int64_t)VMAX, p.V - v0);
     // kx_ = two_pi * kloc[0](i,j,k)   (MRI.cpp:138-140)
@@ -159,14 +159,15 @@ __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(Plai
     const int split = (int)(item / n_tiles), tile = (int)(item - (int64_t)split * n_tiles);
     __syncthreads();  // the previous tile's readers of s_pos / s_w are done
     const int g = p.tiles[tile].x;
-    const int s0 = p.run_start[g] + p.tiles[tile].y + threadIdx.x, s1 = s0 + kPlain32Threads;
-    const int s_end = p.run_start[g + 1];
+    const int s_begin = p.run_start[g] + p.tiles[tile].y, left = p.run_start[g + 1] - s_begin;
+    const int s0 = s_begin + threadIdx.x, s1 = s0 + kPlain32Threads;
+    const bool in0 = (int)threadIdx.x < left, in1 = (int)threadIdx.x + kPlain32Threads < left;  // (s1 may pass 2^31)
     const float tg = (float)p.run_t[g];
     const int nv = (int)min((int64_t)VMAX, p.V - v0);
     // -k in units of 2 pi with a float-rounded pi
-    auto scaled = [&](const float *k, int s) { return s < s_end ? -(double)k[s] * kPiRatio : 0.0; };
-    const double kx0 = scaled(p.kx, s0), ky0 = scaled(p.ky, s0), kz0 = scaled(p.kz, s0);
-    const double kx1 = scaled(p.kx, s1), ky1 = scaled(p.ky, s1), kz1 = scaled(p.kz, s1);
+    auto scaled = [&](const float *k, int s, bool in) { return in ? -(double)k[s] * kPiRatio : 0.0; };
+    const double kx0 = scaled(p.kx, s0, in0), ky0 = scaled(p.ky, s0, in0), kz0 = scaled(p.kz, s0, in0);
+    const double kx1 = scaled(p.kx, s1, in1), ky1 = scaled(p.ky, s1, in1), kz1 = scaled(p.kz, s1, in1);
     float2 acc0[VMAX], acc1[VMAX];
     // nodes are rows of a sparse matrix of 32-bit indices
     const int n_begin = (int)((int64_t)split * p.chunk);
@@ -233,8 +234,8 @@ __global__ void __launch_bounds__(kPlain32Threads, 4) signal_plain32_kernel(Plai
       };
 #pragma unroll
       for (int v = 0; v < VMAX; ++v) {
-        if (v < nv && s0 < s_end) put(dst[(int64_t)s0 * p.V + v], acc0[v]);
-        if (v < nv && s1 < s_end) put(dst[(int64_t)s1 * p.V + v], acc1[v]);
+        if (v < nv && in0) put(dst[(int64_t)s0 * p.V + v], acc0[v]);
+        if (v < nv && in1) put(dst[(int64_t)s1 * p.V + v], acc1[v]);
       }
       fold = fold_end;
       if (fold >= n_end) break;

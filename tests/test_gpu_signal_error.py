@@ -44,7 +44,7 @@ def test_fp64_sums_are_cut(cuda):
     """592 tiles are four for each SM, so the nodes are not split.  Nodes at one place
     and samples at k = 0 of motion forms (unfactored): the result is the plain sum of
     M Mxy.  Rounding of a sum of n positive terms is some u sqrt(n) / 3 of it (u =
-    2^-53): 47 u for 20,000 in one sum, 3 u in sums of 1,024."""
+    2^-53): 47 u for 20,000 in one sum, 3 u in sums of 512."""
     n, V = 20_000, 8
     rng = np.random.default_rng(3)
     traj = W.radial3d(n_ro=592, n_spokes=4)
