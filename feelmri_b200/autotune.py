@@ -3,9 +3,10 @@
 The persistent launch splits every problem into work units of (run, row tile,
 column tile, node range).  Two knobs shape the units (fm_tc_tuning): the
 nodes per unit along the node range, and the most kz values per tile of a
-factored run.  Fewer, longer units pay less per-unit setup (phase tables,
-the last accumulator fold, the split sums); more, shorter units balance the
-persistent blocks better across the 148 SMs.  The best point depends on the
+factored run (problems whose runs become the columns of a tile have no such
+tiles, and take the same time at every cap).  Fewer, longer units pay less
+per-unit setup (the wave vectors, the last accumulator fold, the split sums);
+more, shorter units balance the persistent blocks better across the 148 SMs.  The best point depends on the
 batch's shape, so the tuner times the candidates on the batch itself (CUDA
 events, after a warm-up call) and caches the winner per shape class, in
 memory and, when FEELMRI_B200_TUNING names a file, on disk.

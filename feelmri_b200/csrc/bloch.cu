@@ -118,7 +118,8 @@ __device__ inline void bloch_prep_range(int64_t n_time, float gamma, int flat_ru
 
 __global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, float gamma, int flat_rule,
                                                                 const float2 *__restrict__ rf,
-                                                                const float *__restrict__ G, const float *__restrict__ dt,
+                                                                const float *__restrict__ G,
+                                                                const float *__restrict__ dt,
                                                                 float4 *__restrict__ sa, float4 *__restrict__ sb,
                                                                 int *__restrict__ seg, double *__restrict__ call_t) {
   bloch_prep_range(n_time, gamma, flat_rule, rf, G, dt, sa, sb, seg, call_t);
@@ -129,9 +130,9 @@ __global__ void __launch_bounds__(kPrepSteps) bloch_prep_kernel(int64_t n_time, 
 // more than steps); its segment list at offset_b + b (n_time_b + 1 ints).
 // Its motion calls are the samples offset_b .. offset_b + n_time_b - 1.
 __global__ void __launch_bounds__(kPrepSteps) bloch_seq_prep_kernel(
-    const fm_bloch_block *__restrict__ blocks, float gamma, int flat_rule, const float2 *__restrict__ rf, const float *__restrict__ G,
-    const float *__restrict__ dt, float4 *__restrict__ sa, float4 *__restrict__ sb, int *__restrict__ seg,
-    double *__restrict__ call_t, int *__restrict__ call_block) {
+    const fm_bloch_block *__restrict__ blocks, float gamma, int flat_rule, const float2 *__restrict__ rf,
+    const float *__restrict__ G, const float *__restrict__ dt, float4 *__restrict__ sa, float4 *__restrict__ sb,
+    int *__restrict__ seg, double *__restrict__ call_t, int *__restrict__ call_block) {
   const int b = blockIdx.x;
   const int64_t o = blocks[b].offset, nt = blocks[b].n_time, step0 = o - b;
   bloch_prep_range(nt, gamma, flat_rule, rf + o, G + 3 * o, dt + o, sa + step0, sb + step0, seg + o + b,
@@ -267,9 +268,9 @@ __device__ __forceinline__ void bloch_position(const BlochDev &p, const BlochNod
 // parameters from sa / sb, first motion call call0.  HIST:
 // history columns written through hist_m / hist_z (the first step's column).
 template <int MODE, int RMAX, bool HIST>
-__device__ __forceinline__ void bloch_segment(const BlochDev &p, BlochNode<RMAX> &s, int flags, bool flat, const float4 *sa,
-                                              const float4 *sb, int count, int64_t call0, float2 *hist_m,
-                                              float *hist_z) {
+__device__ __forceinline__ void bloch_segment(const BlochDev &p, BlochNode<RMAX> &s, int flags, bool flat,
+                                              const float4 *sa, const float4 *sb, int count, int64_t call0,
+                                              float2 *hist_m, float *hist_z) {
   const float *wrow = (MODE == 4) ? p.weights + call0 * p.md.slots + p.md.slot0[p.pod_term] : nullptr;
   const float M0 = p.M0;
   if (flags & kSegDt) {
@@ -745,7 +746,8 @@ int fm_bloch_solve_f32(fm_ctx *ctx, const fm_bloch_args *a, void *workspace, siz
                      ceil_div(a->n_pos, (int64_t)128) <= kSmCount;
   if (!small) {
     bloch_prep_kernel<<<1, kPrepSteps, 0, st>>>(a->n_time, a->gamma, flat_rule(md),
-                                                reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa, sb, seg, md.kind == FM_MOTION_TERMS ? call_t : nullptr);
+                                                reinterpret_cast<const float2 *>(a->rf), a->G, a->dt, sa, sb, seg,
+                                                md.kind == FM_MOTION_TERMS ? call_t : nullptr);
     count_launch();
     FM_TRY(check_launch("bloch_prep_kernel"));
     FM_TRY(launch_motion_weights(md, call_t, a->n_time, weights, st, seg));
@@ -818,7 +820,8 @@ int fm_bloch_sequence_f32(fm_ctx *ctx, const fm_bloch_sequence_args *a, void *wo
   if (terms) {
     const int64_t total = a->n_samples * md.slots;
     motion_weights_seq_kernel<<<(unsigned)ceil_div(total, 128), 128, 0, st>>>(md, w.call_t, a->n_samples,
-                                                                               w.call_block, w.blocks, w.weights, w.seg);
+                                                                              w.call_block, w.blocks, w.weights,
+                                                                              w.seg);
     count_launch();
     FM_TRY(check_launch("motion_weights_seq_kernel"));
   }

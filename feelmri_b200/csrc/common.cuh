@@ -41,7 +41,6 @@ inline void count_launch(int n = 1) { g_launches.fetch_add(n, std::memory_order_
 // Returns FM_ERR_CUDA with a message when the last launch failed.
 int check_launch(const char *what);
 
-
 #define FM_TRY(expr)                 \
   do {                               \
     int _st = (expr);                \

@@ -121,7 +121,8 @@ __global__ void __launch_bounds__(32 * kColWarps) mass_columns_kernel(int64_t N,
                                                                       const T *__restrict__ vals,
                                                                       const int *__restrict__ start,
                                                                       const int *__restrict__ around,
-                                                                      int *__restrict__ rows_out, T *__restrict__ data_out,
+                                                                      int *__restrict__ rows_out,
+                                                                      T *__restrict__ data_out,
                                                                       int *__restrict__ count, T *__restrict__ lump,
                                                                       const int *__restrict__ over) {
   constexpr int CAP = kWarpTriplets<NB>;

@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(kPrepThreads) prep_scan_kernel(const PrepDev *
   }
   if (p.diag) {
     bool diag = true;
-    for (int64_t k = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; k < p.N; k += (int64_t)gridDim.x * kPrepThreads) {
+    const int64_t stride = (int64_t)gridDim.x * kPrepThreads;
+    for (int64_t k = (int64_t)blockIdx.x * kPrepThreads + threadIdx.x; k < p.N; k += stride) {
       diag = diag && p.indices[k] == (int)k && p.indptr[k] == (int)k;
       p.csr.fill[k] = -1;
     }

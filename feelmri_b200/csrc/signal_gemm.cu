@@ -28,7 +28,7 @@
 //
 // Kernel time on a B200, one sin/cos per node-sample (signal_plain_kernel)
 // against this: FP32 50,021 nodes x 48 runs x 48 lines x 16 kz x 4 columns with
-// flow 6152 us -> 2050 us (the multiply-adds alone take 820 us), FP64 20,011
+// flow 6152 us -> 2020 us (the multiply-adds alone take 820 us), FP64 20,011
 // nodes x 64 runs x 64 lines 1403 us -> 68 us (multiply-adds 18 us).
 #include <algorithm>
 

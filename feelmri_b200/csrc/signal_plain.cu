@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(Pla
 // reference rounds the phase in radians to FP32; what comes after is FP32 as
 // there.  Bound by issue: per sample-node some 40 instructions for the phase and
 // its sin/cos and 4 a column, 77% of the issue rate.  20,011 nodes x 128 runs x
-// 255 samples x 8 columns on a B200: 2944 us with sincosf of a rounded phase, one
-// sample per thread and tiles dealt out split by split, 1830 us now.
+// 255 samples x 8 columns, a call on a B200: 3117 us with sincosf of a rounded phase,
+// one sample per thread and tiles dealt out split by split, 1900 us now.
 constexpr int kPlain32Threads = 128;
 constexpr int kPlainFold = 2048;  // nodes in one sum: a longer one is the largest error of the form
 template <int VMAX>
@@ -252,9 +252,9 @@ struct SplitCounts {
 };
 constexpr int kReduceLanes = 8, kReduceElems = 32;
 template <typename T>
-__global__ void __launch_bounds__(kReduceLanes *kReduceElems) split_reduce_kernel(const T *__restrict__ part, SplitCounts c,
-                                                                                  const int *__restrict__ ctl,
-                                                                                  int64_t count, T *__restrict__ out) {
+__global__ void __launch_bounds__(kReduceLanes *kReduceElems)
+    split_reduce_kernel(const T *__restrict__ part, SplitCounts c, const int *__restrict__ ctl, int64_t count,
+                        T *__restrict__ out) {
   __shared__ T sums[kReduceLanes][kReduceElems];
   const int splits = c.splits[prep_form(c.run_cover, c.slab_cover, ctl)];
   if (splits <= 1) return;
@@ -413,8 +413,8 @@ int signal_plain(fm_ctx *ctx, const fm_signal_args *a, void *ws, size_t ws_bytes
   if (pl.partials) {
     const int64_t count = S * V * 2, blocks = ceil_div(count, kReduceElems);
     const SplitCounts c{pl.prep.run_cover, pl.prep.slab_cover, {pl.gemm[0].splits, pl.gemm[1].splits, pl.splits}};
-    split_reduce_kernel<T><<<(unsigned)(blocks < 32 * kSmCount ? blocks : 32 * kSmCount), kReduceLanes * kReduceElems, 0,
-                             st>>>(pl.partials, c, pl.prep.ctl, count, out);
+    const unsigned grid = (unsigned)(blocks < 32 * kSmCount ? blocks : 32 * kSmCount);
+    split_reduce_kernel<T><<<grid, kReduceLanes * kReduceElems, 0, st>>>(pl.partials, c, pl.prep.ctl, count, out);
     count_launch();
     FM_TRY(check_launch("split_reduce_kernel"));
   }

@@ -104,7 +104,7 @@ struct TcItem {
 constexpr int kTcSlab = 0;     // factored runs: rows lines, columns (kz, v)
 constexpr int kTcGeneric = 1;  // other runs: rows samples, columns v
 // Runs as columns, for a problem without motion whose k factors between the
-// run and the place in the slab (kFlagStatic*): rows are the samples of a
+// run and the place in the slab (prep_static): rows are the samples of a
 // slab, columns (run, v); A = exp(-2 pi i k_slab . r), B = exp(-2 pi i k_run . r)
 // exp(-t / T2) exp(i phi t) M Mxy.  Slabs of few kz values then give wide
 // tiles: a 32 x 32 x 8 grid of one coil has 64 units of 8 pairs as lines x kz
@@ -143,7 +143,7 @@ struct TcDev {
 
 // Shared-memory layout of a launch, the same for all its entries (the warps
 // cross from one unit to the next on their own, so a ring slot or node buffer
-// must not move): barriers, `ring` stages, two node buffers (positions,
+// must not move): barriers, `ring` stages, two to four node buffers (positions,
 // weight rows), two staging areas of raw node blocks.
 struct TcGeom {
   uint32_t stage_bytes, ring;
@@ -975,7 +975,10 @@ __device__ __forceinline__ void tc_final(const TcDev &p, const TcWork &W, const 
 template <bool kNarrow>
 __device__ __forceinline__ void tc_issue(uint32_t stage_addr, uint32_t tmem, uint32_t idesc, uint32_t idesc2,
                                          uint32_t d_blo, bool first) {
-  // Descriptors (ptx::smem_desc_sw64): the tiles of a stage differ only in
+  // Shared-memory matrix descriptors: K-major operands in the 64-byte swizzled
+  // layout (rows of 64 bytes, 16-byte chunks XOR-permuted by address bits 7-8,
+  // 8-row groups 512 bytes apart), LBO unused (1), version 1, swizzle mode 64B (4);
+  // the second K step starts 32 bytes on.  The tiles of a stage differ only in
   // the start-address field, address / 16 (below 2^14 in shared memory, and
   // every tile and stage offset a multiple of 16), so the stage's field is
   // formed once and each tile's is one add; the high word is constant.
@@ -1484,7 +1487,7 @@ static void carve_tc(Carve &c, const fm_signal_args *a, int *ctl, TcPlan &pl) {
   pl.partials = c.take<float2>((size_t)pl.max_splits * S * a->n_vencs);
 }
 
-// Entries of a launch: per problem, per column group, both run kinds.
+// Entries of a launch: per problem and column group one of each kind.
 static int tc_n_entries(const fm_signal_args *probs, int n) {
   int e = 0;
   for (int i = 0; i < n; ++i) e += kTcKinds * tc_groups(probs[i].n_vencs);
@@ -1750,7 +1753,8 @@ static int tc_batch(fm_ctx *ctx, const fm_signal_args *probs, int n, const fm_tc
   const int64_t rb = ceil_div(widest, 256);
   for (size_t i0 = 0; i0 < prep.size(); i0 += 65535) {
     const unsigned y = (unsigned)(prep.size() - i0 < 65535 ? prep.size() - i0 : 65535);
-    tc_reduce_kernel<<<dim3((unsigned)(rb < 4 * kSmCount ? rb : 4 * kSmCount), y), 256, 0, st>>>(b.entries, b.first + i0);
+    tc_reduce_kernel<<<dim3((unsigned)(rb < 4 * kSmCount ? rb : 4 * kSmCount), y), 256, 0, st>>>(b.entries,
+                                                                                                 b.first + i0);
     count_launch();
     FM_TRY(check_launch("tc_reduce_kernel"));
   }

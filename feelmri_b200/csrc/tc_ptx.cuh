@@ -115,34 +115,6 @@ __device__ inline void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ inline void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ inline void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor, no swizzle ("interleaved" core matrices of
-// 8 rows x 16 bytes): start address, leading byte offset (between the two
-// 8-element halves of a 16-element K slice), stride byte offset (between
-// 8-row groups), descriptor version 1.
-__device__ inline uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;  // version
-  return d;                // base offset 0, legacy LBO mode, layout SWIZZLE_NONE
-}
-
-// Shared-memory matrix descriptor of a K-major operand in the 64-byte
-// swizzled layout (rows of 64 bytes, 16-byte chunks XOR-permuted by address
-// bits 7-8, 8-row groups 512 bytes apart): start address (a tile start, or
-// plus 32 bytes for the second K step of 16 elements), LBO unused (encoded
-// 1), SBO 512, descriptor version 1, base offset 0, swizzle mode 64B (4).
-__device__ inline uint64_t smem_desc_sw64(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)1 << 16;                  // LBO (ignored within one swizzle row)
-  d |= (uint64_t)(512 >> 4) << 32;         // SBO
-  d |= (uint64_t)1 << 46;                  // version
-  d |= (uint64_t)4 << 61;                  // SWIZZLE_64B
-  return d;
-}
-
 // Instruction descriptor of kind::f16 with BF16 A and B, FP32 accumulate,
 // both operands K-major, shape M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
@@ -198,10 +170,6 @@ __device__ inline void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
 __device__ inline void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ inline void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ inline void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 
 }  // namespace ptx
 }  // namespace fm

@@ -452,7 +452,7 @@ def signal(inp: SignalInputs, motion: LoweredMotion, precision: str = "f32",
 class Tuning:
     """Work-unit shape of the batched tensor-core Signal (fm_tc_tuning):
     nodes per unit (0: spread each problem over the SMs) and the most kz
-    values per tile (0: up to 64)."""
+    values per tile (0: up to 64; tiles whose columns are runs have none)."""
     split_nodes: int = 0
     kz_cap: int = 0
 

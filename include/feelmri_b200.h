@@ -358,7 +358,9 @@ typedef struct fm_tc_tuning {
   int32_t split_nodes;  /* nodes per unit along the node range (0: spread one
                            problem's units evenly over the SMs)             */
   int32_t kz_cap;       /* most kz values per tile of a factored run (0: up
-                           to 64 within 128 (kz, column) pairs)             */
+                           to 64 within 128 (kz, column) pairs); without
+                           effect where runs are the columns of a tile
+                           (nothing moves and k factors that way)           */
   int32_t reserved[2];
 } fm_tc_tuning;
 
