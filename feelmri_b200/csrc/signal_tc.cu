@@ -77,8 +77,8 @@ constexpr int kTcMmaWarp = 15;
 // keep it near 1e-5.  On wide tiles all three products go to one accumulator, on
 // narrow ones two (tensor memory below): where runs are columns, which makes wide
 // tiles of problems that had narrow ones, 21 stages (126 MMAs) keep the error at
-// that of a narrow tile's 32 (128 MMAs).  512 like nodes are off by
-// 4.0e-6 of their sum on a narrow tile, by 5.2e-6 on a wide one with 32, 2.6e-6 with 21.
+// that of a narrow tile's 32 (128 MMAs).  512 like nodes are off by 2.1e-6 of their
+// sum on a narrow tile, by 3.1e-6 on a wide one with 32, 1.6e-6 with 21.
 constexpr int kTcDrain = 32, kTcDrainRuns = 21;
 // Node buffers: one is written while others are still read.  The operand
 // warps are up to a ring apart, so with two buffers of eight stages the next
@@ -106,7 +106,8 @@ constexpr int kTcGeneric = 1;  // other runs: rows samples, columns v
 // Runs as columns, for a problem without motion whose k factors between the
 // run and the place in the slab (prep_static): rows are the samples of a
 // slab, columns (run, v); A = exp(-2 pi i k_slab . r), B = exp(-2 pi i k_run . r)
-// exp(-t / T2) exp(i phi t) M Mxy.  Slabs of few kz values then give wide
+// exp(-t / T2) exp(i phi t) M Mxy, each node rotated by a turn of its own in A and
+// back in B (tc_runs_row).  Slabs of few kz values then give wide
 // tiles: a 32 x 32 x 8 grid of one coil has 64 units of 8 pairs as lines x kz
 // (16 pairs of columns for 128 lines of 4 runs) and 2 units of 32 pairs here.
 constexpr int kTcRuns = 2;
@@ -234,7 +235,7 @@ __device__ inline TcItem tc_item(const TcDev &p, const TcWork &W, int i) {
 // parts, kWStride floats each (padded, so that 16-byte reads of different
 // rows fall in different banks).
 constexpr int kWStride = kTcBlockNodes + 4;
-constexpr uint32_t kTcPosBytes = 3 * kTcBlockNodes * 8;  // x, y, z rows of a node buffer (FP64)
+constexpr uint32_t kTcPosBytes = 4 * kTcBlockNodes * 8;  // x, y, z rows of a node buffer and one more (FP64)
 constexpr int kTcComps = 4;  // x, y, z and (runs as columns) the run's time
 constexpr uint32_t kTcSmemMax = 232448;  // dynamic shared memory a block may opt in to
 
@@ -469,6 +470,29 @@ __device__ inline int tc_abs_sum(double x, double y, double z) {
   return __float_as_int((float)(fabs(x) + fabs(y) + fabs(z))) & 0x7fffffff;
 }
 
+// Rows of a node buffer where runs are columns: the components of k that go with the
+// run come first, for B, which reads rows 0 to 2; A reads rows 1 to 3, the last of
+// which is a turn of each node's own, in cycles, by which A is rotated and the
+// weights back.  A is a function of the place alone there, so nodes in line have the
+// same A, and with it the same error of its split; the errors of a line then add up
+// to that of its whole sum.  With a turn of its own each node's error is another.
+// 196,955 nodes of a grid, 105 x 105 x 16 samples, on a B200: error 1.24e-5 without
+// turns, 8.2e-6 with them or as lines x kz, whose A holds the nodes' decay.
+// Where no component goes with the run, A takes all three and there is no turn.
+__device__ inline int tc_runs_row(int cmask, int c) {
+  const int in = __popc(cmask & ((1 << c) - 1));  // components before c that go with the run
+  if (cmask == 0) return c + 1;
+  return (cmask >> c) & 1 ? in : __popc(cmask) + c - in;
+}
+
+// A turn for node n in [0, 1): the bits of n well mixed.
+__device__ inline double tc_node_turn(int64_t n) {
+  uint32_t h = (uint32_t)n * 0x9e3779b1u;
+  h = (h ^ (h >> 15)) * 0x85ebca77u;
+  h ^= h >> 13;
+  return (double)h * 0x1p-32;
+}
+
 // ---- node blocks ---------------------------------------------------------
 
 // Raw data of one node block in a staging area.
@@ -495,7 +519,8 @@ struct TcNodeArgs {
   const float *r0, *T2, *phi, *modes, *wrun, *table;
   const float2 *MM;
   int VG, mm_ld, mstage, wrows, nrun;
-  bool stacked, runs;
+  bool stacked, runs, turns;
+  int row[3];  // rows of x, y, z in the node buffer
   float t;  // the run's time; stacked: lane k holds run k's
   float w;  // lane k: motion weight k of a staged term
 };
@@ -510,6 +535,9 @@ __device__ inline TcNodeArgs tc_node_args(const TcDev &p, const TcUnit &U, int l
   a.table = p.table ? p.table + (int64_t)U.it.run * p.N * 3 : nullptr;
   a.stacked = p.stacked != 0;
   a.runs = p.kind == kTcRuns;
+  const int cmask = a.runs ? prep_run_comps(p.ctl) : 0;
+  a.turns = cmask != 0;
+  for (int c = 0; c < 3; ++c) a.row[c] = a.runs ? tc_runs_row(cmask, c) : c;
   a.t = (float)p.run_t[U.it.run + (a.stacked && lane < a.nrun ? lane : 0)];
   a.w = p.mstage && 3 * lane < p.mstage ? a.wrun[p.md.slot0[0] + lane] : 0.f;
   return a;
@@ -534,13 +562,13 @@ __device__ inline void tc_request_block(const TcNodeArgs &a, int64_t n0, unsigne
 // motion_disp's sum over the modes of a POD term in W modes a load.  A warp's
 // nodes are rows apart, so each load is 32 requests whatever its width, and the two
 // node warps must keep the pace that the whole block once set: 20,011 nodes x 64 x 64
-// samples on a B200, 20 modes 676 us with single reads, 425 us; 64 modes 2029 us,
-// 799 us (with nodes formed by four warps it was 620 us and 1633 us).
+// samples on a B200, 20 modes 676 us with single reads, 410 us; 64 modes 2029 us,
+// 785 us (with nodes formed by four warps it was 620 us and 1633 us).
 template <int W>
 __device__ __forceinline__ void tc_pod_sum(const float *Phi, const float *wk, int r, float &tx, float &ty, float &tz) {
   using V = typename std::conditional<W == 4, float4, typename std::conditional<W == 2, float2, float>::type>::type;
   tx = 0.f; ty = 0.f; tz = 0.f;
-#pragma unroll 3  // (what the kernel's registers take best; 1 leaves reads one after the other)
+#pragma unroll 2  // (what the kernel's registers take best)
   for (int m = 0; m < r; m += W) {
     const V a = __ldg(reinterpret_cast<const V *>(Phi + m)), b = __ldg(reinterpret_cast<const V *>(Phi + r + m)),
             c = __ldg(reinterpret_cast<const V *>(Phi + 2 * r + m));
@@ -608,9 +636,9 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
   };
   int rmax = 0;
   auto put_place = [&](int slot, float x, float y, float z) {
-    pos[slot] = (double)x;
-    pos[kTcBlockNodes + slot] = (double)y;
-    pos[2 * kTcBlockNodes + slot] = (double)z;
+    pos[a.row[0] * kTcBlockNodes + slot] = (double)x;
+    pos[a.row[1] * kTcBlockNodes + slot] = (double)y;
+    pos[a.row[2] * kTcBlockNodes + slot] = (double)z;
     rmax = max(rmax, __float_as_int(fabsf(x) + fabsf(y) + fabsf(z)) & 0x7fffffff);
   };
   if (staged && a.mstage) {
@@ -674,8 +702,8 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
   // FP64 before the fast sin/cos (cycles_cos_sin), as the A and B tiles do
   // (both within a few 1e-7 of the accurate functions).  Stacked: the weights
   // without decay (B), then one D_r = decay e^{i phi t_r} row per run (A).
-  // Runs as columns: the weights without decay, then 1 / T2 and (FP64) phi in
-  // cycles, from which B forms each run's factor.
+  // Runs as columns: the weights without decay, rotated by the node's turn, then
+  // 1 / T2 and (FP64) phi in cycles, from which B forms each run's factor.
   const int nd = a.runs ? 0 : (a.stacked ? a.nrun : 1);
   float inv_t2[kPer], er[kPer], ei[kPer];
 #pragma unroll
@@ -684,8 +712,12 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
     double *ph = reinterpret_cast<double *>(wblk + 2 * (a.VG + 1) * kWStride);
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      wblk[2 * a.VG * kWStride + slot0 + i * kStep] = in[i] ? inv_t2[i] : 0.f;
-      ph[slot0 + i * kStep] = (double)phi[i] * 0.15915494309189535;
+      const int slot = slot0 + i * kStep;
+      wblk[2 * a.VG * kWStride + slot] = in[i] ? inv_t2[i] : 0.f;
+      ph[slot] = (double)phi[i] * 0.15915494309189535;
+      const double turn = a.turns ? tc_node_turn(n0 + slot) : 0.0;
+      pos[(a.turns ? 3 : 0) * kTcBlockNodes + slot] = turn;
+      cycles_cos_sin(turn, er[i], ei[i]);  // A = exp(-2 pi i (k . r + turn))
     }
   }
 #pragma unroll 1
@@ -704,7 +736,7 @@ __device__ __forceinline__ int tc_derive(const TcDev &p, const TcNodeArgs &a, in
       }
     }
   }
-  const bool plain = a.stacked || a.runs;
+  const bool plain = a.stacked;
   auto put = [&](int v, int slot, float2 m, float dr, float di) {
     wblk[2 * v * kWStride + slot] = plain ? m.x : m.x * dr - m.y * di;
     wblk[(2 * v + 1) * kWStride + slot] = plain ? m.y : m.x * di + m.y * dr;
@@ -1130,6 +1162,7 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
     const int n_blocks = (nst + kTcStagesPerBlock - 1) / kTcStagesPerBlock;
     const bool stacked = p.stacked != 0, generic = p.kind == kTcGeneric, runs = p.kind == kTcRuns;
     const int cmask = runs ? prep_run_comps(p.ctl) : 0;  // components of k that go with the run
+    const float *kc[3] = {p.kx, p.ky, p.kz};
     const bool drains = warp < kTcDrainWarps;
     // turns: three groups of A warps for a generic unit (they write its B too),
     // else two, and the other warps on B: two per stage (a node half each)
@@ -1178,11 +1211,18 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
         tc_row_line(p, U, row, rr, line);
         a_drow = 2 * (VG + rr) * kWStride;
         const int s_p = (rr == 0 ? U.start : p.start[U.it.run + rr]) + (p.kind == kTcSlab ? line * p.n_kz : line);
-        kd[0] = cmask & 1 ? 0.0 : (double)p.kx[s_p];
-        kd[1] = cmask & 2 ? 0.0 : (double)p.ky[s_p];
-        kd[2] = cmask & 4 ? 0.0 : (double)p.kz[s_p];
+        // component c lies in row c, or (runs) in row tc_runs_row - 1 from row 1 on
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double k = (cmask >> c) & 1 ? 0.0 : (double)kc[c][s_p];
+          const int at = runs ? tc_runs_row(cmask, c) - 1 : c;
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            if (i == at) kd[i] = k;
+        }
         kmax = tc_abs_sum(kd[0], kd[1], kd[2]);
       }
+      if (cmask) kd[2] = 1.0;  // the row of turns
       const uint32_t row_off = sw64_offset(row, 0), row_off1 = sw64_offset(row, 16);
       const int d_k2 = ((row >> 1) & 1) != 0 ? -16 : 16;
       const int arrive = rg != 0 ? 1 : kTcStageArrivals - (nrg - 1) - (generic ? 0 : b_per);
@@ -1197,7 +1237,8 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
         if (generic)
           for (int quad = rg; quad < 4; quad += nrg)
             tc_write_b_generic(wp, VG, quad, stg + 2 * kAStageBytes, d_lo, d_im);
-        const double *pos = reinterpret_cast<const double *>(smem + G.pos + nbuf * kTcPosBytes) + j * kTcNodes;
+        const double *pos = reinterpret_cast<const double *>(smem + G.pos + nbuf * kTcPosBytes) + j * kTcNodes +
+                            (runs ? kTcBlockNodes : 0);
 #pragma unroll 1
         for (int n = 0; n < 16; n += 8) {
           const uint32_t addr = stg + (n ? row_off1 : row_off);
@@ -1215,6 +1256,12 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
       // the columns q, 32 at a time, or up to 16 of them and both node halves
       const int grp = (warp - nA) / b_per, half0 = both ? lane >> 4 : (warp - nA) - grp * b_per;
       const int lq = both ? lane & 15 : lane, half_step = both ? 2 : b_per;
+      // components of k that go with the run, in the order of their rows
+      const int n_run = __popc(cmask);
+      const float *kr[3];
+      kr[0] = cmask & 1 ? p.kx : (cmask & 2 ? p.ky : p.kz);
+      kr[1] = (cmask & 3) == 3 ? p.ky : p.kz;
+      kr[2] = p.kz;
       r.seek(stage0 + grp, ring);
       for (int st = grp; st < nst && grp < b_groups; st += b_groups) {
         if (drains) fold_before(st);
@@ -1232,9 +1279,8 @@ __device__ __forceinline__ void tc_role_operands(const TcBatchDev &B, TcBars *ba
           double kd[kTcComps] = {0, 0, 0, 0};
           if (runs) {
             const int s_q = p.start[U.it.q0 + q];
-            kd[0] = cmask & 1 ? (double)p.kx[s_q] : 0.0;
-            kd[1] = cmask & 2 ? (double)p.ky[s_q] : 0.0;
-            kd[2] = cmask & 4 ? (double)p.kz[s_q] : 0.0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) kd[i] = i < n_run ? (double)kr[i][s_q] : 0.0;
             kd[3] = p.run_t[U.it.q0 + q];
           } else {
             const int s_q = U.start + U.it.q0 + q;

@@ -60,3 +60,32 @@ def test_fp64_sums_are_cut(cuda):
     exact = np.array([complex(math.fsum(c.real), math.fsum(c.imag)) for c in cols.T])
     rel = np.concatenate([(K[0] - exact).real / exact.real, (K[0] - exact).imag / exact.imag])
     assert np.sqrt((rel ** 2).mean()) < 15 * 2.0 ** -53
+
+
+def test_split_errors_of_nodes_in_line_are_independent(cuda):
+    """Nodes of a regular grid, all alike, nothing moving: a row factor of place alone
+    is the same for the 24 nodes of a line, and so is the error of its split.  The
+    residual of a split is up to 2^-18 of an element, so with independent errors a
+    sample is off by about 2^-18 of the root of the sum of squares, 3.8e-6 w sqrt(N);
+    with the errors of a line in step, where the lines' own sums are large (the runs
+    at kx about 0), by sqrt(24) times that.  The bound is 2 x 2^-18."""
+    m, w = 24, 1.234567e-3
+    n = m ** 3
+    axis = (np.arange(m) - (m - 1) / 2) * 0.0031
+    r0 = np.stack(np.meshgrid(axis, axis, axis, indexing="ij"), -1).reshape(-1, 3)
+    traj = W.cartesian(res=(40, 40, 8))
+
+    def form(precision):
+        real, cplx = (torch.float64, torch.complex128) if precision == "f64" else (torch.float32, torch.complex64)
+        up = lambda a: torch.from_numpy(np.ascontiguousarray(np.float32(a))).to(device=cuda, dtype=real)  # noqa: E731
+        idx = torch.arange(n + 1, dtype=torch.int32, device=cuda)
+        inp = ops.SignalInputs(M=ops.SparseCSC((n, n), idx, idx[:n], up(np.full(n, w))), kx=up(traj.kx), ky=up(traj.ky),
+                               kz=up(traj.kz), t=up(traj.t), r0=up(r0), phi=up(np.zeros(n)), T2=up(np.full(n, 70.0)),
+                               Mxy=torch.ones((n, 1), dtype=cplx, device=cuda))
+        return ops.signal(inp, lower(None, n, cuda), precision).cpu().numpy()[..., 0].astype(np.complex128)
+    K, ref = form("bf16x3"), form("f64")
+    kx = np.abs(traj.kx)
+    line = kx <= 1.01 * kx.min()             # the runs whose lines sum up
+    weak = np.abs(ref) < 0.02 * n * w        # (at a peak the accumulators' rounding counts)
+    assert (line & weak).sum() > 200
+    assert np.sqrt((np.abs(K - ref)[line & weak] ** 2).mean()) < 2 * 2.0 ** -18 * w * np.sqrt(n)
