@@ -512,21 +512,22 @@ static void gemm_shape(int64_t P, int64_t C, int64_t V, GemmPlan &g) {
 // add up, at a rate that grows with the warps there (latency: 8 / warps on top);
 // a block costs about 3 stages to set up and write, and a round of blocks 30 more
 // in latency and uneven ends; partial sums are written and read back at some 20 MB
-// a stage.  Splits of at least 64 nodes and within 256 MB of partial sums.
-static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes) {
+// a stage.  Splits of at least 64 nodes and within 256 MB of partial sums, and at
+// least `least`.
+static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes, int least) {
   const int64_t units = (int64_t)g.products * g.nr * g.nc;
   const int64_t per_sm = std::max(1, std::min(65536 / (128 * g.threads), 228 * 1024 / (g.smem + 1024)));
-  int best = 1;
+  int best = least;
   double best_cost = 0.0;
   int64_t most = out_bytes > 0 ? kPartialBytes / out_bytes : 1;
   if (most > 512) most = 512;
-  for (int s = 1; s == 1 || (s <= most && N / s >= 64); ++s) {
+  for (int s = least; s == least || (s <= most && N / s >= 64); ++s) {
     const int64_t on_sm = ceil_div(units * s, (int64_t)kSmCount);
     const double warps = (double)std::min(on_sm, per_sm) * (g.threads / 32);
     const double cost = (double)on_sm * ((double)N / s / kGemmStage) * (1.0 + 8.0 / warps) +
                         3.0 * (double)on_sm + 30.0 * (double)ceil_div(on_sm, per_sm) +
                         (s > 1 ? 2.0 * s * (double)out_bytes / 2e7 : 0.0);
-    if (s == 1 || cost < best_cost) {
+    if (s == least || cost < best_cost) {
       best = s;
       best_cost = cost;
     }
@@ -535,7 +536,7 @@ static int gemm_splits(const GemmPlan &g, int64_t N, int64_t out_bytes) {
 }
 
 template <typename T>
-void plan_gemm(const fm_signal_args *a, const PrepDev &pr, GemmPlan (&g)[2]) {
+void plan_gemm(const fm_signal_args *a, const PrepDev &pr, int least, GemmPlan (&g)[2]) {
   const int64_t V = a->n_vencs, out_bytes = pr.S * V * 2 * (int64_t)sizeof(T);
   g[0] = g[1] = GemmPlan{};
   if (pr.S == 0 || V == 0 || pr.N == 0) return;
@@ -548,7 +549,7 @@ void plan_gemm(const fm_signal_args *a, const PrepDev &pr, GemmPlan (&g)[2]) {
     g[1].products = pr.n_ro;
   }
   for (GemmPlan &k : g)
-    if (k.products > 0) k.splits = gemm_splits(k, pr.N, out_bytes);
+    if (k.products > 0) k.splits = gemm_splits(k, pr.N, out_bytes, least);
 }
 
 template <typename T>
@@ -591,8 +592,8 @@ int launch_gemm(const fm_signal_args *a, const PrepDev &pr, const GemmPlan (&g)[
   return FM_OK;
 }
 
-template void plan_gemm<float>(const fm_signal_args *, const PrepDev &, GemmPlan (&)[2]);
-template void plan_gemm<double>(const fm_signal_args *, const PrepDev &, GemmPlan (&)[2]);
+template void plan_gemm<float>(const fm_signal_args *, const PrepDev &, int, GemmPlan (&)[2]);
+template void plan_gemm<double>(const fm_signal_args *, const PrepDev &, int, GemmPlan (&)[2]);
 template int launch_gemm<float>(const fm_signal_args *, const PrepDev &, const GemmPlan (&)[2], float *, float *,
                                 cudaStream_t);
 template int launch_gemm<double>(const fm_signal_args *, const PrepDev &, const GemmPlan (&)[2], double *, double *,

@@ -17,8 +17,9 @@ struct GemmPlan {
 // Most bytes of the partial sums of a call's node splits.
 constexpr int64_t kPartialBytes = 256LL << 20;
 
+// `least`: node splits that fill the GPU by the tiles of an unfactored form.
 template <typename T>
-void plan_gemm(const fm_signal_args *a, const PrepDev &pr, GemmPlan (&g)[2]);
+void plan_gemm(const fm_signal_args *a, const PrepDev &pr, int least, GemmPlan (&g)[2]);
 
 template <typename T>
 int launch_gemm(const fm_signal_args *a, const PrepDev &pr, const GemmPlan (&g)[2], T *out, T *partials,
