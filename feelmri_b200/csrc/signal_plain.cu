@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kPlainThreads, BLOCKS) signal_plain_kernel(Pla
 // which the rest leaves idle, and its reduction exact (cycles.cuh), where the
 // reference rounds the phase in radians to FP32; what comes after is FP32 as
 // there.  Bound by issue: per sample-node some 40 instructions for the phase and
-// its sin/cos and 4 a column, 77% of the issue rate.  20,011 nodes x 128 runs x
+// its sin/cos and 4 a column, 75% of the issue rate.  20,011 nodes x 128 runs x
 // 255 samples x 8 columns, a call on a B200: 3117 us with sincosf of a rounded phase,
 // one sample per thread and tiles dealt out split by split, 1900 us now.
 constexpr int kPlain32Threads = 128;
