@@ -75,11 +75,13 @@ constexpr int kTcMmaWarp = 15;
 // tensor core's FP32 accumulation truncates, so its error grows with the
 // number of MMAs added into one accumulator; 32 stages (512 nodes, 192 MMAs)
 // keep it near 1e-5.  On wide tiles all three products go to one accumulator, on
-// narrow ones two (tensor memory below): where runs are columns, which makes wide
-// tiles of problems that had narrow ones, 21 stages (126 MMAs) keep the error at
-// that of a narrow tile's 32 (128 MMAs).  512 like nodes are off by 2.1e-6 of their
-// sum on a narrow tile, by 3.1e-6 on a wide one with 32, 1.6e-6 with 21.
-constexpr int kTcDrain = 32, kTcDrainRuns = 21;
+// narrow ones two (tensor memory below), and where runs are columns the turns
+// (tc_runs_row) leave no element of the strongest samples 0: there 12 stages (72
+// MMAs) keep the error at what such problems had as narrow or generic tiles.
+// 198,606 nodes, 78 x 22 samples x 2 columns, on a B200: error 3.5e-6 with 32 stages,
+// 2.1e-6 with 21, 1.3e-6 with 12 (1.4e-6 as generic tiles); uneven batch 1% slower
+// than with 21.
+constexpr int kTcDrain = 32, kTcDrainRuns = 12;
 // Node buffers: one is written while others are still read.  The operand
 // warps are up to a ring apart, so with two buffers of eight stages the next
 // block was often late.

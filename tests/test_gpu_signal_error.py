@@ -28,11 +28,11 @@ def _k(n, runs, dev):
 
 def test_wide_tiles_truncate_no_more_than_narrow_ones(cuda):
     """Each MMA on an accumulator truncates it.  A narrow tile of 32 stages adds 4 a
-    stage to its main accumulator, 128; a wide one adds 6 and is folded after 21
-    stages, 126 and then 66.  The truncation of a growing sum adds up to half an ulp
-    an MMA over the mean of the sum, in proportion to the MMAs of a group: 0.82 times
-    the narrow tile's on average, and 1.5 times if a wide tile collected 32 stages.
-    The bound lies between."""
+    stage to its main accumulator, 128; a wide one adds 6 and is folded after 12
+    stages, 72.  The truncation of a growing sum adds up to half an ulp an MMA over
+    the mean of the sum, in proportion to the MMAs of a group: about half the narrow
+    tile's, and 1.5 times if a wide tile collected 32 stages.  The bound lies
+    between."""
     def error(runs):
         few, many = _k(16, runs, cuda), _k(512, runs, cuda)
         return ((many / 32 - few).abs() / few.abs()).mean().item()

@@ -12,7 +12,7 @@ BLOCK, OPERANDS, DRAINS, ARRIVALS = 8, 13, 8, 6
 
 def drain_of(generic, narrow):
     """Stages of an accumulation group."""
-    return 32 if generic or narrow else 21
+    return 32 if generic or narrow else 12
 
 
 class Bar:
