@@ -27,7 +27,7 @@
 // layout; warps 13 and 14 form the node blocks (128 nodes: moved positions,
 // weights) ahead of them; one thread of warp 15 issues the MMAs of each written
 // stage and releases its slot by tcgen05.commit.  The tensor core's FP32
-// accumulation truncates, so the accumulator only collects 32 stages; warps 0-7
+// accumulation truncates, so the accumulator only collects 32 stages or fewer; warps 0-7
 // then fold it into an FP32 (round-to-nearest) running sum kept in the other
 // half of tensor memory.  Blocks loop over work units (row/column tile of a run
 // x node range), each role on its own.  All waits are bounded: on timeout the
@@ -39,8 +39,8 @@
 // ones.  Measured on a B200, with one barrier for the whole block every two or
 // four stages and one warp writing operands and issuing MMAs before:
 // 200,740 nodes x 96 x 96 x 32 x 4 columns 9,274 -> 8,070 us, radial 50,021 x
-// 65,536 x 8 columns with 10 modes 8,687 -> 5,350, 16 uneven phantoms 3,821 ->
-// 2,410 (with runs as columns, kTcRuns).
+// 65,536 x 8 columns with 10 modes 8,687 -> 5,200, 16 uneven phantoms 3,821 ->
+// 2,470 (with runs as columns, kTcRuns).
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -479,7 +479,7 @@ __device__ inline int tc_abs_sum(double x, double y, double z) {
 // same A, and with it the same error of its split; the errors of a line then add up
 // to that of its whole sum.  With a turn of its own each node's error is another.
 // 196,955 nodes of a grid, 105 x 105 x 16 samples, on a B200: error 1.24e-5 without
-// turns, 8.2e-6 with them or as lines x kz, whose A holds the nodes' decay.
+// turns, 7.6e-6 with them (8.3e-6 as lines x kz, whose A holds the nodes' decay).
 // Where no component goes with the run, A takes all three and there is no turn.
 __device__ inline int tc_runs_row(int cmask, int c) {
   const int in = __popc(cmask & ((1 << c) - 1));  // components before c that go with the run
